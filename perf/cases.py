@@ -175,7 +175,7 @@ def _prepare_pool(c, seed):
             torch.cumsum(counts, 0, dtype=torch.int32, out=segs[1:])
         groups.append(ops.make_group(table, ids, values, segs, [dict(udf=_UDF[c["udf"]], out=out, col=i * dim)], _T[c["table"]],
                                      segments_are_offsets=not c["counts"]))
-    return dict(c, plan=ops.PoolPlan(groups), out=out)
+    return dict(c, plan=ops.PoolPlan(groups), groups=groups, out=out)
 
 
 def _run_pool(s):
@@ -218,7 +218,7 @@ def _prepare_gemm(c, seed):
     r = lambda *sh: torch.randn(sh, generator=g, device="cuda")
     A = r(*((M, K) if c["shared"] else (P, M, K))).to(dt)
     W = (r(P, K, N) / K ** 0.5).to(dt)
-    s = dict(c, A=A, bias=r(P, N) * 0.1)
+    s = dict(c, A=A, W_in=W, bias=r(P, N) * 0.1)
     kw = dict(batch=P, M=M, N=N, K=K, lda=K, bias_kind=capi.XB_BIAS_ROW)
     if c["layout"] == "packed":
         # constants are laid out once when a model is loaded
@@ -403,3 +403,141 @@ def tolerance(case):
     if c["kind"] == "serve":
         return {"rel": 1e-6 if c["form"] == "reference_f32" else 2e-3}
     return {"rel": 2e-3 if c["kind"] == "din" else 2.5e-3}
+
+
+# ---- the same results in 64 bits, by plain torch ----------------------------------------------------------------
+_INVERSE = pow(-7046029254386353131, -1, 1 << 64)
+_INVERSE -= (_INVERSE >> 63) << 64                                   # as a signed 64-bit number
+
+
+def _exact_pool(c, seed):
+    s = _prepare_pool(c, seed)
+    out = torch.zeros((c["batch"], c["groups"], c["dim"]), dtype=torch.float64, device="cuda")
+    for i, grp in enumerate(s["groups"]):
+        table, ids, values, segs, _ = grp._keep
+        lens = segs.long() if c["counts"] else segs.long().diff()
+        # a hashed key is (row + 1) * multiplier, undone by the multiplier's inverse; what gives no row is not in the table
+        row = ids * _INVERSE - 1 if c["hashed"] else ids
+        known = (row >= 0) & (row < c["rows"])
+        seg = torch.repeat_interleave(torch.arange(c["batch"], device="cuda"), lens)[known]
+        x = table.buf[row[known], :c["dim"]].double()
+        if values is not None:
+            x *= values[known].double()[:, None]
+        out[:, i].index_add_(0, seg, x)
+        if c["udf"] == "avg":
+            out[:, i] /= lens.clamp(min=1)[:, None]
+    return out.view(c["batch"], -1)
+
+
+def _exact_sharded(c, seed):
+    s = _prepare_sharded(c, seed)
+    B, gpt = c["batch"], c["groups"]
+    off = s["off"].long()
+    out = torch.zeros((B, c["tables"] * gpt, c["dim"]), dtype=torch.float64, device="cuda")
+    for slot in range(c["tables"] * gpt):
+        o = off[slot * B:(slot + 1) * B + 1]
+        x = s["keep"][slot // gpt].buf[s["ids"][o[0]:o[-1]], :c["dim"]].double()
+        out[:, slot].index_add_(0, torch.repeat_interleave(torch.arange(B, device="cuda"), o.diff()), x)
+    return out.view(B, -1)
+
+
+def _exact_gemm(c, seed):
+    s = _prepare_gemm(c, seed)
+    y = torch.matmul(s["A"].double(), s["W_in"].double()) + s["bias"].double()[:, None]
+    if c["act"] == "prelu":
+        y = torch.where(y < 0, y * 0.25, y)
+    elif c["act"] == "dice":
+        y = _dice(y, *[t.double()[:, None] for t in s["kw"]["ep"]])
+    elif c["act"] == "sigmoid":
+        y = y.sigmoid()
+    return y.permute(1, 0, 2).reshape(c["M"], -1) if c["axis"] == 1 else y.reshape(-1, c["N"])
+
+
+def _exact_mlp(c, seed):
+    s = _prepare_mlp(c, seed)
+    x, ys = s["x"].double(), []
+    for i, y in enumerate(s["layers"]):
+        x = x @ y["W"].double().t() + y["bias"].double()
+        x = x.sigmoid() if i == len(s["layers"]) - 1 else torch.where(x < 0, x * 0.25, x)
+        ys.append(x)
+    return ys
+
+
+def _dice(x, gamma, mean, var):
+    p = ((x - mean) / (var + 1e-8).sqrt()).sigmoid()
+    return (1 - p) * gamma * x + p * x
+
+
+def _exact_model(c, seed):
+    """The model op by op: embeddings, (GRU,) attention unit, (AUGRU,) tower, softmax."""
+    dien_ = c["kind"] == "dien"
+    m = _model(c, seed, workloads.dien_model if dien_ else workloads.din_model)
+    req, D = _requests(m, c, seed), m["dims"]
+    D64 = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to("cuda").double()
+    rows = lambda w, ids: D64(w[ids])
+    R, n, T, d = c["requests"], c["n_cand"], c["T"], D["d"]
+    user = torch.cat([rows(m["user"][g], req["user_ids"][:, g]) for g in range(D["user_groups"])], 1)
+    hist = torch.cat([rows(m["item"], req["hist_item"]), rows(m["cate"], req["hist_cate"])], 1)
+    q = torch.cat([rows(m["item"], req["cand_item"]), rows(m["cate"], req["cand_cate"])], 1)
+    k = torch.zeros((R, T, d), dtype=torch.float64, device="cuda")
+    at = 0
+    for r, ln in enumerate(req["seq_len"].tolist()):                # lists end at the last step
+        k[r, T - ln:] = hist[at:at + ln]
+        at += ln
+    W = lambda group: {x: D64(v) for x, v in m[group].items()}
+    a = W("att")
+    tw = {x: [D64(y) for y in v] if isinstance(v, tuple) else D64(v) for x, v in m["dien_tower" if dien_ else "tower"].items()}
+    h = _exact_gru(k, W("gru")) if dien_ else k
+    act = (lambda x, i: x.sigmoid()) if dien_ else (lambda x, i: _dice(x, a["g" + i], a["m" + i], a["v" + i]))
+    scores = torch.empty((R * n, T), dtype=torch.float64, device="cuda")
+    for r in range(R):
+        qr, kr = q[r * n:(r + 1) * n, None].expand(n, T, d), h[r][None].expand(n, T, d)
+        y = act(torch.cat([qr, kr, qr - kr, qr * kr], 2) @ a["W0"] + a["b0"], "0")
+        scores[r * n:(r + 1) * n] = (act(y @ a["W1"] + a["b1"], "1") @ a["W2"] + a["b2"])[..., 0]
+    if dien_:
+        scores = scores.softmax(1)
+        att = _exact_augru(h, scores, n, W("augru"))
+    else:
+        att = torch.bmm(scores.view(R, n, T), k).view(R * n, d)
+    wide = lambda x: x.repeat_interleave(n, 0)
+    his = wide(k.sum(1))
+    x = torch.cat([wide(user), q, his, q * his, att] + ([] if dien_ else [q - his]), 1)
+    for i in "12":
+        x = x @ tw["W" + i] + tw["b" + i]
+        x = torch.where(x < 0, x * tw["slope" + i], x) if dien_ else _dice(x, *tw["dice" + i])
+    prob = (x @ tw["W3"] + tw["b3"]).softmax(1)
+    if c["kind"] == "serve":
+        return prob.cpu().numpy()
+    return (prob, h.reshape(R, T * d), scores, att) if dien_ else prob
+
+
+def _exact_gru(x, g):
+    R, T, H = x.shape
+    h, ys = torch.zeros((R, H), dtype=torch.float64, device="cuda"), []
+    begun = torch.zeros((R, 1), dtype=torch.bool, device="cuda")
+    for t in range(T):
+        i = x[:, t] @ g["i2h"]
+        begun |= (i[:, :H] != 0).any(1, keepdim=True)               # zero steps in front of a list leave the state at zero
+        i, a = i + g["i2h_bias"], h @ g["h2h"] + g["h2h_bias"]
+        r, z = (i + a)[:, :2 * H].sigmoid().split(H, 1)
+        cand = torch.tanh(i[:, 2 * H:] + r * a[:, 2 * H:])
+        h = torch.where(begun, cand + z * (h - cand), 0.0)
+        ys.append(h)
+    return torch.stack(ys, 1)
+
+
+def _exact_augru(x, scores, n, g):
+    R, T, H = x.shape
+    h = torch.zeros((R * n, H), dtype=torch.float64, device="cuda")
+    for t in range(T):
+        xt = x[:, t].repeat_interleave(n, 0)
+        r, u = (torch.cat([xt, h], 1) @ g["Wg"] + g["bg"]).sigmoid().split(H, 1)
+        cand = torch.tanh(torch.cat([xt, r * h], 1) @ g["Wc"] + g["bc"])
+        u = (1 - scores[:, t:t + 1]) * u
+        h = u * h + (1 - u) * cand
+    return h
+
+
+def exact(case, seed):
+    return {"pool": _exact_pool, "sharded": _exact_sharded, "gemm": _exact_gemm, "mlp": _exact_mlp}.get(
+        case["kind"], _exact_model)(case, seed)
