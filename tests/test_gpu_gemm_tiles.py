@@ -1,0 +1,56 @@
+"""Layouts and tiles of the GEMM engines at the sizes where a tile, a k block or a vector load ends.
+
+Tolerances: a product of K terms summed in fp32 is within K * 2^-24 of its exact value relative to the sum of magnitudes
+(twice that is allowed: the tensor cores do not round every partial sum), and rounding to a 16-bit result adds one
+half-ulp of the value: 2^-11 for fp16, 2^-8 for bf16."""
+import numpy as np
+import pytest
+import torch
+
+import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def _ops():
+    pkg.load()
+    from x_deeplearning_b200 import ops, capi
+    return ops, capi
+
+
+def _bound(A, W, want, K, half_ulp):
+    return half_ulp * np.abs(want) + 2 * K * 2.0 ** -24 * (np.abs(A) @ np.abs(W) + 1) + 2.0 ** -24
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("P,M,N,K,ldb,shared", [
+    (1, 128, 64, 64, 64, False), (1, 130, 80, 16, 80, False), (3, 77, 72, 200, 72, True), (2, 300, 8, 24, 16, False),
+    (1, 515, 320, 136, 320, False), (2, 2600, 200, 72, 256, True), (8, 1000, 128, 256, 128, True), (1, 129, 512, 513, 512, False)])
+def test_weights_in_k_n_layout(dtype, P, M, N, K, ldb, shared):
+    """fp16 / bf16 weights as [K, N]: one and several 64-column boxes, part boxes, wide rows, shared and per-branch
+    inputs, weight tiles that stay resident (many m tiles) and that ride in the ring."""
+    ops, capi = _ops()
+    rng = np.random.default_rng(P * 7 + M + N + K)
+    lda = (K + 7) // 8 * 8
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to("cuda", dtype)
+    A = t(rng.normal(0, 1, ((1 if shared else P), M, lda)))
+    W = t(rng.normal(0, 1, (P, K, ldb)) / np.sqrt(K))
+    bias = torch.from_numpy(rng.normal(0, 0.3, (P, N)).astype(np.float32)).cuda()
+    Y = torch.full((P, M, N), 7.0, dtype=dtype, device="cuda")
+    ops.gemm(A, W, Y=Y, bias=bias, batch=P, M=M, N=N, K=K, lda=lda, ldb=ldb, ldy=N,
+             strides=(0 if shared else M * lda, K * ldb, N, M * N), bias_kind=capi.XB_BIAS_ROW)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    got, f = Y.double().cpu().numpy(), lambda x: x.double().cpu().numpy()
+    for p in range(P):
+        a, w = f(A)[0 if shared else p][:, :K], f(W)[p][:, :N]
+        want = a @ w + f(bias)[p]
+        err = np.abs(got[p] - want)
+        assert (err <= _bound(a, w, want, K, 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8)).all(), float(err.max())
+
+
+def test_explicit_tensor_core_engine_still_wants_k_major_weights():
+    ops, capi = _ops()
+    A, W = torch.zeros((128, 64), dtype=torch.float16, device="cuda"), torch.zeros((64, 64), dtype=torch.float16, device="cuda")
+    with pytest.raises(capi.XbError, match="tcgen05 engine needs"):
+        ops.gemm(A, W, engine=capi.XB_GEMM_TCGEN05)

@@ -2,8 +2,9 @@
 // dispatcher.
 //
 //   Y[b] = act(alpha * A[b] * B[b]^T + beta * bias[b])
-//   A [M,K] row-major (K-major), B [N,K] row-major (K-major), fp16 or bf16,
-//   fp32 accumulation in tensor memory.
+//   A [M,K] row-major (K-major), B [N,K] row-major (K-major) or [K,N] row-major
+//   (N-major, the layout Blaze holds weights in), fp16 or bf16, fp32 accumulation
+//   in tensor memory.
 //
 // Persistent kernel, one CTA per SM, 128 x BLOCK_N output tiles. Warp 0 streams
 // 128x64 A tiles (and BLOCK_Nx64 B tiles) through a shared-memory ring with TMA
@@ -35,10 +36,12 @@ constexpr int BLOCK_K = 64;
 constexpr int MAX_STAGES = 8;       // the launch picks as many as fit in shared memory (at least 2)
 constexpr int SMEM_BUDGET = 220 * 1024;
 constexpr int A_STAGE_BYTES = BLOCK_M * BLOCK_K * 2;
+constexpr int MN_BOX_BYTES = 64 * BLOCK_K * 2;      // one N-major box: 64 k rows of 64 columns (128 bytes each)
 
 struct UmmaGemmParams {
   int M, N, K, block_n, tmem_cols, tiles_m, tiles_n, batch, stages;
   int b_resident;        // the B tile (all of K) stays in shared memory while consecutive tiles share it
+  int b_mn;              // B is [K,N] row-major: the MMA reads N-major tiles of 64 columns x 64 k
   uint32_t tiles_per_cta;
   float alpha, beta;
   int a_batched, b_batched;
@@ -236,7 +239,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   using namespace umma;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int b_stage_bytes = p.block_n * BLOCK_K * 2;
+  const int b_stage_bytes = (p.b_mn ? (p.block_n + 63) / 64 * 64 : p.block_n) * BLOCK_K * 2;
   uint8_t* smem_a = smem;
   const int STAGES = p.stages;
   uint8_t* smem_b = smem + STAGES * A_STAGE_BYTES;      // per-stage B tiles, or the resident B tile (all k blocks)
@@ -279,6 +282,14 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
   if (warp == 0) {
     if (lane == 0) {
+      // one k block of B: one box of block_n rows x 64 k, or (N-major) boxes of 64 k rows x 64 columns side by side
+      auto load_b = [&](uint32_t dst, uint32_t bar, int kb, int n0, int b) {
+        if (!p.b_mn) {
+          tma_load_3d(dst, &map_b, bar, kb * BLOCK_K, n0, b);
+        } else {
+          for (int j = 0; j * 64 < p.block_n; ++j) tma_load_3d(dst + j * MN_BOX_BYTES, &map_b, bar, n0 + j * 64, kb * BLOCK_K, b);
+        }
+      };
       int s = 0;
       uint32_t ph = 0;                 // stage and its phase: the stage counter wraps, the phase flips
       uint32_t b_loads = 0;
@@ -295,8 +306,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (!ok) break;
           mbar_arrive_expect_tx(smem_u32(&b_full), (uint32_t)(num_kb * b_stage_bytes));
           for (int kb = 0; kb < num_kb; ++kb)
-            tma_load_3d(smem_u32(smem_b + kb * b_stage_bytes), &map_b, smem_u32(&b_full), kb * BLOCK_K, n0,
-                        p.b_batched ? b : 0);
+            load_b(smem_u32(smem_b + kb * b_stage_bytes), smem_u32(&b_full), kb, n0, p.b_batched ? b : 0);
           ++b_loads;
         }
         for (int kb = 0; kb < num_kb; ++kb, s = (s + 1 == STAGES ? 0 : s + 1), ph ^= (s == 0 ? 1u : 0u)) {
@@ -305,9 +315,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           mbar_arrive_expect_tx(smem_u32(&full_bar[s]), (uint32_t)(A_STAGE_BYTES + b_bytes_per_load));
           tma_load_3d(smem_u32(smem_a + s * A_STAGE_BYTES), &map_a, smem_u32(&full_bar[s]), kb * BLOCK_K, m0,
                       p.a_batched ? b : 0);
-          if (!bres)
-            tma_load_3d(smem_u32(smem_b + s * b_stage_bytes), &map_b, smem_u32(&full_bar[s]), kb * BLOCK_K, n0,
-                        p.b_batched ? b : 0);
+          if (!bres) load_b(smem_u32(smem_b + s * b_stage_bytes), smem_u32(&full_bar[s]), kb, n0, p.b_batched ? b : 0);
         }
       }
     }
@@ -342,7 +350,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
           for (int k = 0; k < BLOCK_K / 16; ++k) {
             const uint64_t da = make_desc_sw128(a_addr + k * 32, 1024);
-            const uint64_t db = make_desc_sw128(b_addr + k * 32, 1024);
+            const uint64_t db = p.b_mn ? make_desc_sw128_mn(b_addr + k * 2048, MN_BOX_BYTES) : make_desc_sw128(b_addr + k * 32, 1024);
             mma_f16_ss_elect(tmem_acc, da, db, p.idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           mma_commit_elect(smem_u32(&empty_bar[s]));     // slot free once these MMAs have read it
@@ -506,7 +514,8 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// [batch, rows, K] tensor of 2-byte elements, box {64, box_rows, 1}, 128-byte swizzle
+// [batch, rows, K] tensor of 2-byte elements, box {64, box_rows, 1}, 128-byte swizzle (an N-major B is the same with
+// its k rows as rows and its columns as the inner extent)
 int make_map(CUtensorMap* map, const void* base, int is_bf16, int64_t K, int64_t rows, int64_t ld, int64_t batch,
              int64_t batch_stride, int box_rows) {
   EncodeTiledFn fn = encode_fn();
@@ -530,11 +539,11 @@ int pick_block_n(int N) {
 
 bool umma_eligible(const xb_gemm_args& a) {
   if (a.ab_dtype != XB_F16 && a.ab_dtype != XB_BF16) return false;
-  if (a.trans_a || !a.trans_b) return false;
+  if (a.trans_a) return false;
   if (a.y_dtype != XB_F16 && a.y_dtype != XB_BF16 && a.y_dtype != XB_F32) return false;
   if (a.lda % 8 || a.ldb % 8 || a.stride_a % 8 || a.stride_b % 8) return false;
   if ((reinterpret_cast<uintptr_t>(a.A) & 15) || (reinterpret_cast<uintptr_t>(a.B) & 15)) return false;
-  if (a.lda < a.K || a.ldb < a.K) return false;
+  if (a.lda < a.K || a.ldb < (a.trans_b ? a.K : a.N)) return false;
   return true;
 }
 
@@ -563,10 +572,13 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   p.epi.kind = a.epilogue; p.epi.a = a.ep_a; p.epi.b = a.ep_b; p.epi.c = a.ep_c;
   p.epi.count = a.ep_count; p.epi.nosqrt = a.dice_nosqrt; p.stride_ep = a.stride_ep;
   const int is_bf16 = a.ab_dtype == XB_BF16;
-  p.idesc = umma::make_idesc(BLOCK_M, p.block_n, is_bf16);
+  p.b_mn = !a.trans_b;
+  p.idesc = umma::make_idesc(BLOCK_M, p.block_n, is_bf16) | (p.b_mn ? umma::IDESC_B_MN : 0u);
   CUtensorMap ma, mb;
   if (int rc = make_map(&ma, a.A, is_bf16, a.K, a.M, a.lda, p.a_batched ? a.batch : 1, a.stride_a, BLOCK_M)) return rc;
-  if (int rc = make_map(&mb, a.B, is_bf16, a.K, a.N, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, p.block_n)) return rc;
+  if (int rc = p.b_mn ? make_map(&mb, a.B, is_bf16, a.N, a.K, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, BLOCK_K)
+                      : make_map(&mb, a.B, is_bf16, a.K, a.N, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, p.block_n))
+    return rc;
   p.tiles_m = (a.M + BLOCK_M - 1) / BLOCK_M;
   p.tiles_n = (a.N + p.block_n - 1) / p.block_n;
   p.batch = a.batch;
@@ -578,7 +590,7 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   // When the whole B tile (all of K) is small and several m tiles share it, it is loaded once and stays in
   // shared memory: re-reading it from L2 for every tile doubles the L2-to-SM traffic of a thin GEMM, which
   // then bounds the kernel below the HBM rate.
-  const int b_stage_bytes = p.block_n * BLOCK_K * 2;
+  const int b_stage_bytes = (p.b_mn ? (p.block_n + 63) / 64 * 64 : p.block_n) * BLOCK_K * 2;
   const int num_kb = (a.K + BLOCK_K - 1) / BLOCK_K;
   const int grid_ctas = (int)std::min<int64_t>(total, sm_count());
   p.tiles_per_cta = (uint32_t)((total + grid_ctas - 1) / grid_ctas);
@@ -732,7 +744,7 @@ static int validate_gemm(const xb_gemm_args* a) {
 }
 
 extern "C" int xb_gemm_uses_tcgen05(const xb_gemm_args* a) {
-  if (!a || a->engine == XB_GEMM_SIMT) return 0;
+  if (!a || a->engine == XB_GEMM_SIMT || (a->engine == XB_GEMM_TCGEN05 && !a->trans_b)) return 0;
   return umma_eligible(*a) ? 1 : 0;
 }
 
@@ -740,7 +752,7 @@ extern "C" int xb_gemm(const xb_gemm_args* a, xb_stream_t stream) {
   if (int rc = validate_gemm(a)) return rc;
   if (a->M == 0 || a->N == 0 || a->batch == 0) return 0;
   if (a->engine == XB_GEMM_TCGEN05) {
-    XB_REQUIRE(umma_eligible(*a), XB_ERR_UNSUPPORTED,
+    XB_REQUIRE(a->trans_b && umma_eligible(*a), XB_ERR_UNSUPPORTED,
                "xb_gemm: tcgen05 engine needs fp16/bf16, A [M,K] and B [N,K] row-major, 16-byte aligned, "
                "leading dimensions and batch strides multiples of 8");
     XB_REQUIRE(a->K > 0, XB_ERR_ARG, "xb_gemm: K = 0");
