@@ -12,6 +12,14 @@
 // fp32 registers; it is rounded to fp16 only as an MMA operand. Only the final state is written (the model reads
 // nothing else), the input sequence is read once per CTA instead of once per candidate.
 //
+// What bounds it is the chain of a step: gate product, gates, candidate product, blend. The tanh units alone need 54
+// paired instructions a row and step at H = 36 (864 cycles of a scheduler's SFU); the rest of a step is tensor-memory
+// round trips and MMA latency. So three warpgroups share a tile, a third of the columns each (a row's columns are
+// independent between the products): every scheduler then has three warps to fill the waits of one another, r*h goes
+// out before the update gate is evaluated, and the update gate's SFU work hides the candidate product. H is a
+// compile-time constant: a run-time H made the update gates a local-memory array. 128 tiles of 100 steps, H = 36: 121 us,
+// 382 with one warpgroup a tile.
+//
 // Cell semantics: VecAttGRUCell.call, xdl-algorithm-solution/DIEN/script/utils.py:178-207 (the reference ships no
 // inference operator for it). Shapes: H padded to Hp = 8*ceil(H/8) must leave 4 or more spare slots (H = 36 does).
 #pragma once
@@ -19,8 +27,10 @@
 namespace xb {
 namespace {
 
-constexpr int AU_THREADS = 160;           // 4 worker warps (one candidate row per thread) + 1 MMA-issuing warp
-constexpr int AU_MMA_WARP = 4;
+constexpr int AU_GROUPS = 3;              // worker warpgroups: one candidate row per thread, a third of the columns
+constexpr int AU_WORKERS = AU_GROUPS * 128;
+constexpr int AU_MMA_WARP = AU_GROUPS * 4;
+constexpr int AU_THREADS = AU_WORKERS + 32;
 
 struct AuGeom {
   int hp, nch, selpos, k, n1, n2, ngrp;   // k: MMA K (h, selector slots, zero chunk); n1 = pad16(2H), n2 = pad16(H)
@@ -29,8 +39,8 @@ struct AuGeom {
   int o_b1, o_b2, o_att, o_x, total;      // shared memory
 };
 
-__host__ __device__ inline AuGeom au_geom(int H, int T) {
-  AuGeom g;
+__host__ __device__ constexpr AuGeom au_geom(int H, int T) {
+  AuGeom g{};
   g.hp = (H + 7) / 8 * 8;
   g.nch = g.hp / 8;
   g.selpos = H & 7;
@@ -69,15 +79,128 @@ __device__ __forceinline__ int au_chunk_off(const AuGeom& g, int blk, int c, int
   return (g.nch - 1 + g.ngrp) * blk;
 }
 
-// HP2: compile-time bound of the fp16 pairs of a state row (the state lives in registers)
-template <int HP2>
-__global__ void __launch_bounds__(AU_THREADS, 2) augru_tc_kernel(const __grid_constant__ AuParams p) {
+// N consecutive tensor-memory columns of this thread's lane
+template <int N>
+__device__ __forceinline__ void au_tmem_st(uint32_t at, const uint32_t* r) {
+  using namespace umma;
+  if constexpr (N >= 8) { tmem_st8(at, r); au_tmem_st<N - 8>(at + 8, r + 8); }
+  else if constexpr (N >= 4) { tmem_st4(at, r[0], r[1], r[2], r[3]); au_tmem_st<N - 4>(at + 4, r + 4); }
+  else if constexpr (N >= 2) { tmem_st2(at, r[0], r[1]); au_tmem_st<N - 2>(at + 2, r + 2); }
+  else if constexpr (N == 1) tmem_st1(at, r[0]);
+}
+
+// The steps of one worker thread: candidate row `row` of the tile, columns [C0, C0 + NC) of the state (NC even).
+// The last group also writes the selector slots, which follow the state in the A operand.
+template <int H, int GRP>
+__device__ __forceinline__ void au_worker(const AuParams& p, const __half* att_row, uint32_t lane_addr, __half* out, bool valid,
+                                          uint64_t* a1_full, uint64_t* acc1_full, uint64_t* a2_full, uint64_t* acc2_full) {
+  using namespace umma;
+  constexpr AuGeom G = au_geom(H, 1);                       // tensor-memory columns do not depend on T
+  constexpr int CPG = (H + 2 * AU_GROUPS - 1) / (2 * AU_GROUPS) * 2;
+  constexpr int C0 = GRP * CPG < H ? GRP * CPG : H;
+  constexpr int NC = GRP == AU_GROUPS - 1 ? H - C0 : (C0 + CPG <= H ? CPG : H - C0);
+  constexpr int NP = NC / 2;
+  constexpr bool LAST = GRP == AU_GROUPS - 1;
+  constexpr int NST = NP + (LAST ? 2 : 0);                  // pairs written per operand: the state's and the selector's
+  const int T = p.T, lane = threadIdx.x & 31;
+  const uint32_t a1t = lane_addr + G.c_a1 + C0 / 2, a2t = lane_addr + G.c_a2 + C0 / 2;
+  float h[NC > 0 ? NC : 1];
+  uint32_t pk[NST > 0 ? NST : 1], upk[NP > 0 ? NP : 1];
+#pragma unroll
+  for (int i = 0; i < NC; ++i) h[i] = 0.f;
+#pragma unroll
+  for (int i = 0; i < NST; ++i) pk[i] = 0u;
+  auto publish = [&](uint32_t at, uint64_t* bar, int t) {
+    if constexpr (LAST) {
+      const uint32_t one = (t & 1) ? 0x3C000000u : 0x3C00u;   // 1.0 in slot t % 4 of the four
+      pk[NP] = (t & 2) ? 0u : one;
+      pk[NP + 1] = (t & 2) ? one : 0u;
+    }
+    au_tmem_st<NST>(at, pk);
+    tmem_wait_st();
+    tc_fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(bar));
+  };
+  if constexpr (LAST) {
+    // what follows the selector slots (up to the operand's end) stays zero
+    constexpr int Z0 = H / 2 + 2, ZN = G.k / 2 - Z0;
+    constexpr int ZA = ZN > 0 ? ZN : 1;
+    uint32_t z[ZA];
+#pragma unroll
+    for (int i = 0; i < ZA; ++i) z[i] = 0u;
+    au_tmem_st<ZN>(lane_addr + G.c_a1 + Z0, z);
+    au_tmem_st<ZN>(lane_addr + G.c_a2 + Z0, z);
+  }
+  publish(a1t, a1_full, 0);                                 // h_0 = 0 with the selector of step 0
+  bool ok = true;
+  for (int t = 0; t < T; ++t) {
+    const uint32_t ph = (uint32_t)t & 1u;
+    // ---- gates: [r|u] = sigmoid(acc1); r*h becomes the A operand of the candidate product
+    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc1_full), ph, 32));
+    if (!ok) break;
+    tc_fence_after_sync();
+    uint32_t vr[32], vu[32];
+    // (a load may reach past the group's columns: still inside the allocation, the extra values are not used)
+    if constexpr (NC > 16) { tmem_ld32_nowait(lane_addr + C0, vr); tmem_ld32_nowait(lane_addr + H + C0, vu); }
+    else if constexpr (NC > 0) { tmem_ld16_lo_nowait(lane_addr + C0, vr); tmem_ld16_lo_nowait(lane_addr + H + C0, vu); }
+    if constexpr (NC > 16) { tmem_wait_ld(vr); tmem_wait_ld(vu); }
+    else if constexpr (NC > 0) {
+      tmem_wait_ld(*reinterpret_cast<uint32_t(*)[16]>(&vr));
+      tmem_wait_ld(*reinterpret_cast<uint32_t(*)[16]>(&vu));
+    }
+    // sigmoid(z) = 1/2 + 1/2 tanh(z/2), two columns per SFU instruction
+    auto sigm2 = [](uint32_t a, uint32_t b) {
+      const __half2 z = __floats2half2_rn(0.5f * __uint_as_float(a), 0.5f * __uint_as_float(b));
+      const __half2 th = bits_h2(tanh_f16x2(h2_bits(z)));
+      return __hfma2(th, __floats2half2_rn(0.5f, 0.5f), __floats2half2_rn(0.5f, 0.5f));
+    };
+#pragma unroll
+    for (int e = 0; e < NP; ++e) {
+      const float2 rf = __half22float2(sigm2(vr[2 * e], vr[2 * e + 1]));
+      pk[e] = h2_bits(__floats2half2_rn(rf.x * h[2 * e], rf.y * h[2 * e + 1]));
+    }
+    publish(a2t, a2_full, t);
+#pragma unroll
+    for (int e = 0; e < NP; ++e) upk[e] = h2_bits(sigm2(vu[2 * e], vu[2 * e + 1]));
+    // ---- candidate and blend
+    const float a = __half2float(att_row[t]);
+    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc2_full), ph, 33));
+    if (!ok) break;
+    tc_fence_after_sync();
+    if constexpr (NC > 16) { tmem_ld32_nowait(lane_addr + G.c_acc2 + C0, vr); tmem_wait_ld(vr); }
+    else if constexpr (NC > 0) {
+      tmem_ld16_lo_nowait(lane_addr + G.c_acc2 + C0, vr);
+      tmem_wait_ld(*reinterpret_cast<uint32_t(*)[16]>(&vr));
+    }
+#pragma unroll
+    for (int e = 0; e < NP; ++e) {
+      const __half2 z = __floats2half2_rn(__uint_as_float(vr[2 * e]), __uint_as_float(vr[2 * e + 1]));
+      const float2 c = __half22float2(bits_h2(tanh_f16x2(h2_bits(z))));
+      const float2 u = __half22float2(bits_h2(upk[e]));
+      const float u0 = (1.f - a) * u.x, u1 = (1.f - a) * u.y;
+      h[2 * e] = u0 * h[2 * e] + (1.f - u0) * c.x;
+      h[2 * e + 1] = u1 * h[2 * e + 1] + (1.f - u1) * c.y;
+      pk[e] = h2_bits(__floats2half2_rn(h[2 * e], h[2 * e + 1]));
+    }
+    if (t + 1 < T) publish(a1t, a1_full, t + 1);
+  }
+  if (ok && valid) {
+#pragma unroll
+    for (int i = 0; i < NP; ++i) *reinterpret_cast<uint32_t*>(out + C0 + 2 * i) = pk[i];      // H is even: 4-byte aligned
+  }
+}
+
+template <int H>
+__global__ void __launch_bounds__(AU_THREADS, H <= 40 ? 2 : 1) augru_tc_kernel(const __grid_constant__ AuParams p) {
   using namespace umma;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t bars[4];
   __shared__ uint32_t tmem_base_s;
-  const AuGeom G = au_geom(p.H, p.T);
-  const int H = p.H, T = p.T, hp = G.hp, nch = G.nch, tpp = (T + 7) / 8 * 8;
+  const AuGeom G = au_geom(H, p.T);
+  constexpr AuGeom G1 = au_geom(H, 1);
+  constexpr int hp = G1.hp, nch = G1.nch;
+  const int T = p.T, tpp = (T + 7) / 8 * 8;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = blockIdx.x / p.tiles_per_req, tile = blockIdx.x % p.tiles_per_req;
   const int rows = min(128, p.n_cand - tile * 128);
@@ -107,55 +230,70 @@ __global__ void __launch_bounds__(AU_THREADS, 2) augru_tc_kernel(const __grid_co
   cp_async_commit();
   // recurrent weights as MMA B operands (row n = output column, k = index into h): chunk-major 8 x 16-byte blocks;
   // the last h chunk shares its block with the selector slots and is replicated into every selector block
-  for (int idx = threadIdx.x; idx < G.n1 * hp; idx += AU_THREADS) {
-    const int n = idx / hp, i = idx - n * hp;
+  for (int idx = threadIdx.x; idx < G1.n1 * hp; idx += AU_THREADS) {
+    const int i = idx / G1.n1, n = idx - i * G1.n1;
     const __half v = (n < 2 * H && i < H) ? p.Wg[(int64_t)(H + i) * 2 * H + n] : zero;
     const int c = i >> 3, e = i & 7;
-    if (c < nch - 1) reinterpret_cast<__half*>(b1s + c * G.blk1)[n * 8 + e] = v;
-    else for (int g = 0; g < G.ngrp; ++g) reinterpret_cast<__half*>(b1s + (nch - 1 + g) * G.blk1)[n * 8 + e] = v;
+    if (c < nch - 1) reinterpret_cast<__half*>(b1s + c * G1.blk1)[n * 8 + e] = v;
+    else for (int g = 0; g < G.ngrp; ++g) reinterpret_cast<__half*>(b1s + (nch - 1 + g) * G1.blk1)[n * 8 + e] = v;
   }
-  for (int idx = threadIdx.x; idx < G.n2 * hp; idx += AU_THREADS) {
-    const int n = idx / hp, i = idx - n * hp;
+  for (int idx = threadIdx.x; idx < G1.n2 * hp; idx += AU_THREADS) {
+    const int i = idx / G1.n2, n = idx - i * G1.n2;
     const __half v = (n < H && i < H) ? p.Wc[(int64_t)(H + i) * H + n] : zero;
     const int c = i >> 3, e = i & 7;
-    if (c < nch - 1) reinterpret_cast<__half*>(b2s + c * G.blk2)[n * 8 + e] = v;
-    else for (int g = 0; g < G.ngrp; ++g) reinterpret_cast<__half*>(b2s + (nch - 1 + g) * G.blk2)[n * 8 + e] = v;
+    if (c < nch - 1) reinterpret_cast<__half*>(b2s + c * G1.blk2)[n * 8 + e] = v;
+    else for (int g = 0; g < G.ngrp; ++g) reinterpret_cast<__half*>(b2s + (nch - 1 + g) * G1.blk2)[n * 8 + e] = v;
   }
-  for (int i = threadIdx.x; i < G.blk1 / 16; i += AU_THREADS)
-    reinterpret_cast<uint4*>(b1s + (nch - 1 + G.ngrp) * G.blk1)[i] = make_uint4(0, 0, 0, 0);
-  for (int i = threadIdx.x; i < G.blk2 / 16; i += AU_THREADS)
-    reinterpret_cast<uint4*>(b2s + (nch - 1 + G.ngrp) * G.blk2)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < G1.blk1 / 16; i += AU_THREADS)
+    reinterpret_cast<uint4*>(b1s + (nch - 1 + G.ngrp) * G1.blk1)[i] = make_uint4(0, 0, 0, 0);
+  for (int i = threadIdx.x; i < G1.blk2 / 16; i += AU_THREADS)
+    reinterpret_cast<uint4*>(b2s + (nch - 1 + G.ngrp) * G1.blk2)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();                       // xs and the weight blocks are in place
   // request-side terms into the selector slots: slot t % 4 of selector block t / 4 holds, for output column n,
   //   B1: x_t Wg_x[:, n] + bg[n]      B2: x_t Wc_x[:, n] + bc[n]     (fp32 sums, rounded once)
-  for (int idx = threadIdx.x; idx < G.ngrp * 4 * (G.n1 + G.n2); idx += AU_THREADS) {
-    const int t = idx / (G.n1 + G.n2), nn = idx - t * (G.n1 + G.n2);
-    const bool first = nn < G.n1;
-    const int n = first ? nn : nn - G.n1;
-    const int width = first ? 2 * H : H;
-    float v = 0.f;
-    if (t < T && n < width) {
+  // A thread keeps one weight column in registers and takes every AU_GROUPS-th step.
+  if (threadIdx.x < AU_WORKERS) {
+    for (int nn = threadIdx.x & 127; nn < G1.n1 + G1.n2; nn += 128) {
+      const bool first = nn < G1.n1;
+      const int n = first ? nn : nn - G1.n1;
+      const int width = first ? 2 * H : H;
+      const bool in = n < width;
       const __half* W = first ? p.Wg : p.Wc;
-      v = __half2float(first ? p.bg[n] : p.bc[n]);
-      for (int i = 0; i < H; ++i) v = fmaf(__half2float(xs[t * hp + i]), __half2float(__ldg(W + (int64_t)i * width + n)), v);
+      uint8_t* blks = first ? b1s + (nch - 1) * G1.blk1 : b2s + (nch - 1) * G1.blk2;
+      const int blk = first ? G1.blk1 : G1.blk2;
+      float w[H];
+#pragma unroll
+      for (int i = 0; i < H; ++i) w[i] = in ? __half2float(__ldg(W + i * width + n)) : 0.f;
+      const float bias = in ? __half2float(first ? p.bg[n] : p.bc[n]) : 0.f;
+      for (int t = threadIdx.x >> 7; t < G.ngrp * 4; t += AU_GROUPS) {
+        float v = 0.f;
+        if (t < T) {
+          v = bias;
+#pragma unroll
+          for (int i = 0; i < H; i += 2) {
+            const float2 xv = __half22float2(*reinterpret_cast<const __half2*>(xs + t * hp + i));
+            v = fmaf(xv.x, w[i], v);
+            v = fmaf(xv.y, w[i + 1], v);
+          }
+        }
+        reinterpret_cast<__half*>(blks + (t >> 2) * blk)[n * 8 + G1.selpos + (t & 3)] = __float2half_rn(v);
+      }
     }
-    uint8_t* blk = first ? b1s + (nch - 1 + t / 4) * G.blk1 : b2s + (nch - 1 + t / 4) * G.blk2;
-    reinterpret_cast<__half*>(blk)[n * 8 + G.selpos + (t & 3)] = __float2half_rn(v);
   }
-  // barriers: a1_full (4 worker warps: h operand of a step written), acc1_full (gate product done),
-  //           a2_full (4 worker warps: r*h written), acc2_full (candidate product done)
+  // barriers: a1_full (every worker warp: h operand of a step written), acc1_full (gate product done),
+  //           a2_full (every worker warp: r*h written), acc2_full (candidate product done)
   uint64_t* a1_full = &bars[0];
   uint64_t* acc1_full = &bars[1];
   uint64_t* a2_full = &bars[2];
   uint64_t* acc2_full = &bars[3];
   if (threadIdx.x == 0) {
-    mbar_init(smem_u32(a1_full), 4);
+    mbar_init(smem_u32(a1_full), AU_WORKERS / 32);
     mbar_init(smem_u32(acc1_full), 1);
-    mbar_init(smem_u32(a2_full), 4);
+    mbar_init(smem_u32(a2_full), AU_WORKERS / 32);
     mbar_init(smem_u32(acc2_full), 1);
     fence_barrier_init();
   }
-  if (warp == AU_MMA_WARP) tmem_alloc(smem_u32(&tmem_base_s), (uint32_t)G.tmem_cols);
+  if (warp == AU_MMA_WARP) tmem_alloc(smem_u32(&tmem_base_s), (uint32_t)G1.tmem_cols);
   cp_async_wait_all();
   fence_proxy_async_smem();
   tc_fence_before_sync();
@@ -166,7 +304,7 @@ __global__ void __launch_bounds__(AU_THREADS, 2) augru_tc_kernel(const __grid_co
   if (warp == AU_MMA_WARP) {
     // whole warp in uniform control flow, one elected lane issues: the descriptors stay in uniform registers
     {
-      const int nks = G.k / 16, sel_ks = (nch - 1) / 2;            // nks <= 4 (H <= 64)
+      constexpr int nks = G1.k / 16, sel_ks = (nch - 1) / 2;            // nks <= 4 (H <= 64)
       const uint32_t b1a = smem_u32(b1s), b2a = smem_u32(b2s);
       // descriptors for selector group 0; only the k step with the selector chunk moves with the group
       uint64_t d1[4], d2[4], delta1 = 0, delta2 = 0;
@@ -174,13 +312,13 @@ __global__ void __launch_bounds__(AU_THREADS, 2) augru_tc_kernel(const __grid_co
       for (int ks = 0; ks < 4; ++ks) {
         d1[ks] = d2[ks] = 0;
         if (ks < nks) {
-          const uint32_t o0 = au_chunk_off(G, G.blk1, 2 * ks, 0), o1 = au_chunk_off(G, G.blk1, 2 * ks + 1, 0);
-          const uint32_t q0 = au_chunk_off(G, G.blk2, 2 * ks, 0), q1 = au_chunk_off(G, G.blk2, 2 * ks + 1, 0);
+          const uint32_t o0 = au_chunk_off(G, G1.blk1, 2 * ks, 0), o1 = au_chunk_off(G, G1.blk1, 2 * ks + 1, 0);
+          const uint32_t q0 = au_chunk_off(G, G1.blk2, 2 * ks, 0), q1 = au_chunk_off(G, G1.blk2, 2 * ks + 1, 0);
           d1[ks] = make_desc_interleaved(b1a + o0, o1 - o0, 128);
           d2[ks] = make_desc_interleaved(b2a + q0, q1 - q0, 128);
           if (ks == sel_ks && G.ngrp > 1) {
-            const uint32_t r0 = au_chunk_off(G, G.blk1, 2 * ks, 1), r1 = au_chunk_off(G, G.blk1, 2 * ks + 1, 1);
-            const uint32_t s0 = au_chunk_off(G, G.blk2, 2 * ks, 1), s1 = au_chunk_off(G, G.blk2, 2 * ks + 1, 1);
+            const uint32_t r0 = au_chunk_off(G, G1.blk1, 2 * ks, 1), r1 = au_chunk_off(G, G1.blk1, 2 * ks + 1, 1);
+            const uint32_t s0 = au_chunk_off(G, G1.blk2, 2 * ks, 1), s1 = au_chunk_off(G, G1.blk2, 2 * ks + 1, 1);
             delta1 = make_desc_interleaved(b1a + r0, r1 - r0, 128) - d1[ks];
             delta2 = make_desc_interleaved(b2a + s0, s1 - s0, 128) - d2[ks];
           }
@@ -194,140 +332,34 @@ __global__ void __launch_bounds__(AU_THREADS, 2) augru_tc_kernel(const __grid_co
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           if (ks < nks)
-            mma_f16_ts_elect(tmem0, tmem0 + G.c_a1 + 8 * ks, d1[ks] + (ks == sel_ks ? grp * delta1 : 0ull), p.idesc1, ks > 0 ? 1u : 0u);
+            mma_f16_ts_elect(tmem0, tmem0 + G1.c_a1 + 8 * ks, d1[ks] + (ks == sel_ks ? grp * delta1 : 0ull), p.idesc1, ks > 0 ? 1u : 0u);
         mma_commit_elect(smem_u32(acc1_full));
         if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(a2_full), ph, 31))) break;
         tc_fence_after_sync();
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           if (ks < nks)
-            mma_f16_ts_elect(tmem0 + G.c_acc2, tmem0 + G.c_a2 + 8 * ks, d2[ks] + (ks == sel_ks ? grp * delta2 : 0ull), p.idesc2,
+            mma_f16_ts_elect(tmem0 + G1.c_acc2, tmem0 + G1.c_a2 + 8 * ks, d2[ks] + (ks == sel_ks ? grp * delta2 : 0ull), p.idesc2,
                              ks > 0 ? 1u : 0u);
         mma_commit_elect(smem_u32(acc2_full));
       }
     }
   } else {
-    const int row = warp * 32 + lane;
-    const bool valid = row < rows;
-    const uint32_t lane_addr = tmem0 + ((uint32_t)(warp * 32) << 16);
-    const uint32_t a1t = lane_addr + G.c_a1, a2t = lane_addr + G.c_a2;
-    float h[2 * HP2];
-#pragma unroll
-    for (int i = 0; i < 2 * HP2; ++i) h[i] = 0.f;
-    // an A operand row: chunks of 8 halves = 4 tensor-memory columns; chunk nch-1 carries the selector slots,
-    // the chunk after it (if k > hp) stays zero
-    auto store_operand = [&](uint32_t at, const uint32_t* pk /* hp/2 packed pairs */, int t) {
-      const int hpos = G.selpos + (t & 3);
-#pragma unroll
-      for (int c = 0; c < HP2 / 4; ++c) {
-        if (c < nch) {
-          uint32_t w0 = pk[4 * c], w1 = pk[4 * c + 1], w2 = pk[4 * c + 2], w3 = pk[4 * c + 3];
-          if (c == nch - 1) {
-            const uint32_t one = 0x3C00u << ((hpos & 1) * 16);
-            const int reg = hpos >> 1;
-            w0 |= reg == 0 ? one : 0u; w1 |= reg == 1 ? one : 0u; w2 |= reg == 2 ? one : 0u; w3 |= reg == 3 ? one : 0u;
-          }
-          tmem_st4(at + 4 * c, w0, w1, w2, w3);
-        }
-      }
-    };
-    uint32_t pk[HP2];
-#pragma unroll
-    for (int i = 0; i < HP2; ++i) pk[i] = 0u;
-    if (G.k > hp) {
-      tmem_st4(a1t + 4 * nch, 0u, 0u, 0u, 0u);
-      tmem_st4(a2t + 4 * nch, 0u, 0u, 0u, 0u);
-    }
-    store_operand(a1t, pk, 0);             // h_0 = 0 with the selector of step 0
-    tmem_wait_st();
-    tc_fence_before_sync();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(a1_full));
-    bool ok = true;
-    const int npair = (H + 1) / 2;
-    for (int t = 0; t < T && ok; ++t) {
-      const uint32_t ph = (uint32_t)t & 1u;
-      // ---- gates: [r|u] = sigmoid(acc1); r*h becomes the A operand of the candidate product
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc1_full), ph, 32));
-      if (!ok) break;
-      tc_fence_after_sync();
-      uint32_t upk[HP2];                   // update gate as fp16 pairs
-#pragma unroll
-      for (int blk = 0; blk < (4 * HP2 + 15) / 16; ++blk) {
-        if (blk * 16 < 2 * H) {
-          uint32_t v[16];
-          tmem_ld16_nowait(lane_addr + 16 * blk, v);
-          tmem_wait_ld(v);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const int col = blk * 16 + 2 * e;            // columns col, col + 1 of [r | u]
-            if (col < 2 * H) {
-              // sigmoid(z) = 1/2 + 1/2 tanh(z/2), two columns per SFU instruction
-              const __half2 z = __floats2half2_rn(0.5f * __uint_as_float(v[2 * e]), 0.5f * __uint_as_float(v[2 * e + 1]));
-              const __half2 th = bits_h2(tanh_f16x2(h2_bits(z)));
-              const __half2 sg = __hfma2(th, __floats2half2_rn(0.5f, 0.5f), __floats2half2_rn(0.5f, 0.5f));
-              if (col < H) {
-                // reset gate: r * h (H is even in every supported shape, so a pair never straddles r | u)
-                const float2 rf = __half22float2(sg);
-                pk[col >> 1] = h2_bits(__floats2half2_rn(rf.x * h[col], col + 1 < H ? rf.y * h[col + 1] : 0.f));
-              } else {
-                upk[(col - H) >> 1] = h2_bits(sg);
-              }
-            }
-          }
-        }
-      }
-      store_operand(a2t, pk, t);
-      tmem_wait_st();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(a2_full));
-      // ---- candidate and blend
-      const float a = __half2float(atts[row * tpp + t]);
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc2_full), ph, 33));
-      if (!ok) break;
-      tc_fence_after_sync();
-#pragma unroll
-      for (int blk = 0; blk < (2 * HP2 + 15) / 16; ++blk) {
-        if (blk * 16 < H) {
-          uint32_t v[16];
-          tmem_ld16_nowait(lane_addr + G.c_acc2 + 16 * blk, v);
-          tmem_wait_ld(v);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const int col = blk * 16 + 2 * e;
-            if (col < H) {
-              const __half2 z = __floats2half2_rn(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
-              const float2 c = __half22float2(bits_h2(tanh_f16x2(h2_bits(z))));
-              const float2 u = __half22float2(bits_h2(upk[col >> 1]));
-              const float u0 = (1.f - a) * u.x, u1 = (1.f - a) * u.y;
-              h[col] = u0 * h[col] + (1.f - u0) * c.x;
-              if (col + 1 < H) h[col + 1] = u1 * h[col + 1] + (1.f - u1) * c.y;
-              pk[col >> 1] = h2_bits(__floats2half2_rn(h[col], col + 1 < H ? h[col + 1] : 0.f));
-            }
-          }
-        }
-      }
-      if (t + 1 < T) {
-        store_operand(a1t, pk, t + 1);
-        tmem_wait_st();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(a1_full));
-      }
-    }
-    if (ok && valid) {
-      __half* o = p.y + ((int64_t)r * p.n_cand + tile * 128 + row) * H;
-#pragma unroll
-      for (int i = 0; i < HP2; ++i)
-        if (i < npair) *reinterpret_cast<uint32_t*>(o + 2 * i) = pk[i];      // H is even: whole pairs, 4-byte aligned
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lane_addr = tmem0 + ((uint32_t)((warp & 3) * 32) << 16);
+    const __half* att_row = atts + row * tpp;
+    __half* out = p.y + ((int64_t)r * p.n_cand + tile * 128 + row) * H;
+    switch (warp >> 2) {
+      case 0: au_worker<H, 0>(p, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full); break;
+      case 1: au_worker<H, 1>(p, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full); break;
+      default: au_worker<H, 2>(p, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full); break;
     }
   }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == AU_MMA_WARP) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem0, (uint32_t)G.tmem_cols);
+    tmem_dealloc(tmem0, (uint32_t)G1.tmem_cols);
   }
 }
 
@@ -339,6 +371,14 @@ bool augru_tc_eligible(int H, int T) {
   return g.total <= 200 * 1024 && T >= 1;
 }
 
+template <int H>
+int launch_augru_tc_h(const AuParams& p, unsigned blocks, int smem, cudaStream_t stream) {
+  static PerDeviceOnce attr;                          // per instantiation
+  XB_SET_MAX_SMEM_ONCE(attr, 200 * 1024, (const void*)augru_tc_kernel<H>);
+  augru_tc_kernel<H><<<blocks, AU_THREADS, smem, stream>>>(p);
+  return check_launch("augru_tc_kernel");
+}
+
 int launch_augru_tc(const AuParams& p0, cudaStream_t stream) {
   AuParams p = p0;
   const AuGeom g = au_geom(p.H, p.T);
@@ -347,11 +387,15 @@ int launch_augru_tc(const AuParams& p0, cudaStream_t stream) {
   p.idesc2 = umma::make_idesc(128, g.n2, 0);
   const int64_t blocks = (int64_t)p.requests * p.tiles_per_req;
   XB_REQUIRE(blocks < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_augru_shared: too many tiles");
-  static PerDeviceOnce attr;
-  XB_SET_MAX_SMEM_ONCE(attr, 200 * 1024, (const void*)augru_tc_kernel<20>, (const void*)augru_tc_kernel<32>);
-  if (g.hp <= 40) augru_tc_kernel<20><<<(unsigned)blocks, AU_THREADS, g.total, stream>>>(p);
-  else augru_tc_kernel<32><<<(unsigned)blocks, AU_THREADS, g.total, stream>>>(p);
-  return check_launch("augru_tc_kernel");
+  // one instantiation per eligible H
+  switch (p.H) {
+#define XB_AU_CASE(h) case h: return launch_augru_tc_h<h>(p, (unsigned)blocks, g.total, stream)
+    XB_AU_CASE(4); XB_AU_CASE(10); XB_AU_CASE(12); XB_AU_CASE(18); XB_AU_CASE(20); XB_AU_CASE(26); XB_AU_CASE(28);
+    XB_AU_CASE(34); XB_AU_CASE(36); XB_AU_CASE(42); XB_AU_CASE(44); XB_AU_CASE(50); XB_AU_CASE(52); XB_AU_CASE(58);
+    XB_AU_CASE(60);
+#undef XB_AU_CASE
+    default: return fail(XB_ERR_UNSUPPORTED, "xb_augru_shared: H = %d", p.H);
+  }
 }
 
 }  // namespace
