@@ -54,3 +54,29 @@ def test_explicit_tensor_core_engine_still_wants_k_major_weights():
     A, W = torch.zeros((128, 64), dtype=torch.float16, device="cuda"), torch.zeros((64, 64), dtype=torch.float16, device="cuda")
     with pytest.raises(capi.XbError, match="tcgen05 engine needs"):
         ops.gemm(A, W, engine=capi.XB_GEMM_TCGEN05)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("P,M,N,K,dtype", [(1, 1, 1, 1, "f32"), (1, 33, 17, 15, "f32"), (2, 200, 80, 144, "f32"),
+                                          (1, 20000, 40, 80, "f32"), (1, 3000, 200, 36, "f32"), (1, 700, 129, 18, "f32"),
+                                          (3, 64, 36, 100, "f32"), (2, 130, 45, 37, "f16"), (1, 100, 24, 52, "bf16")])
+def test_cuda_core_engine_tiles_and_layouts(ta, tb, P, M, N, K, dtype):
+    """Every transpose through both the 16-byte and the element loads (sizes that are and are not multiples of four),
+    tiles from 32 x 16 up to 128 x 128, batches."""
+    ops, capi = _ops()
+    rng = np.random.default_rng(M + N + K + 2 * ta + tb)
+    dt = dict(f32=torch.float32, f16=torch.float16, bf16=torch.bfloat16)[dtype]
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to("cuda", dt)
+    A = t(rng.normal(0, 1, (P, K, M) if ta else (P, M, K)))
+    B = t(rng.normal(0, 1, (P, N, K) if tb else (P, K, N)) / np.sqrt(K))
+    bias = torch.from_numpy(rng.normal(0, 0.3, (P, M, N)).astype(np.float32)).cuda()
+    Y = torch.full((P, M, N), 7.0, dtype=torch.float32, device="cuda")
+    ops.gemm(A, B, Y=Y, bias=bias, trans_a=bool(ta), trans_b=bool(tb), alpha=0.5, beta=2.0, batch=P, M=M, N=N, K=K,
+             lda=A.shape[2], ldb=B.shape[2], ldy=N, ldbias=N, strides=(M * K, K * N, M * N, M * N),
+             bias_kind=capi.XB_BIAS_FULL, engine=capi.XB_GEMM_SIMT)
+    f = lambda x: x.double().cpu().numpy()
+    for p in range(P):
+        a, b = (f(A)[p].T if ta else f(A)[p]), (f(B)[p].T if tb else f(B)[p])
+        want = 0.5 * (a @ b) + 2.0 * f(bias)[p]
+        err = np.abs(f(Y)[p] - want)
+        assert (err <= _bound(a, b, want, K, 2.0 ** -23)).all(), float(err.max())
