@@ -31,6 +31,7 @@ struct AttParams {
   int tiles_per_req, tiles_per_cta;
   uint32_t idesc1, idesc2, idesc3;
   const void* packed;      // weight operands laid out by xb_din_attention_pack, or null
+  int split;               // per-step engine: CTAs (one cluster) that share a tile's steps
 };
 
 __device__ __forceinline__ float att_act(int act, float x, float g, float a, float bneg) {

@@ -22,6 +22,13 @@
 // and, after the last step,
 //   MMA   : out[128 x d] = S[128 x T] * K[T x d]          (the weighted sum is a GEMM too)
 //
+// A step costs about 0.67 us of one SM whatever the number of tiles, so a call with few tiles leaves the chip idle
+// and takes T steps all the same. Then a cluster of `split` CTAs shares a tile: each walks a part of the steps and writes
+// its scores into the S operand of the cluster's first CTA, which runs the closing product over all of them, so a result
+// has the same bits whatever the split. Where neither the scores nor a softmax over them is wanted, steps of zero k rows
+// at either end of a list (the padding of a short one) are not walked: whatever their score, they add s * 0.
+// 8 tiles of 100 steps: 20 us as 8 clusters of 8, 72 whole; 2 tiles of a list of 60: 13 us, 72 before.
+//
 // Biases ride in the MMAs: A1 carries a constant-1 column (a padding column of
 // the q segment when d is not a multiple of 8) whose W0 row is b0, and the last
 // k step of layer 2 reads 16 columns shared by all A2 buffers, the first
@@ -242,12 +249,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ __align__(8) uint64_t bars[21];
   __shared__ uint32_t tmem_base_s;
+  __shared__ int range_s[2];               // first and one past the last step whose k row is not zero
+  __shared__ int t0_s;                     // first step this CTA walks
 
   const int d_ = D0 ? D0 : p.d, h0_ = H0 ? H0 : p.h0, h1_ = H1 ? H1 : p.h1;
+  const int split = p.split;
   const TcGeom G = tc_geom(d_, h0_, h1_, p.T);
   const TcSmemLayout L = tc_layout(G, p.T);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.x / p.tiles_per_req, tile = blockIdx.x % p.tiles_per_req;
+  const int ctile = blockIdx.x / split;                                      // the cluster is `split` CTAs along x
+  const int r = ctile / p.tiles_per_req, tile = ctile % p.tiles_per_req;
   const int d = d_, dp = G.dp, nch = G.nch, k1 = G.k1, h0p = G.h0p, k2 = G.k2, h1p = G.h1p, tp = G.tp, np = G.np;
   int tl = p.seq_len ? p.seq_len[r] : p.T;
   tl = tl < 0 ? 0 : (tl > p.T ? p.T : tl);
@@ -323,15 +334,37 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
   for (int idx = threadIdx.x; idx < 128 * tp / 8; idx += TC_THREADS)
     reinterpret_cast<uint4*>(ss)[idx] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x == 0) ATT_TR(6, 120, 3);
+  if (threadIdx.x == 0) { range_s[0] = p.T; range_s[1] = 0; }
   cp_async_wait_all();
   __syncthreads();
+  // the steps this CTA walks: [t0, t0 + tl) of the list
+  const int t_end = tl;
+  int t0 = 0;
+  if (!p.scores && !p.use_softmax) {
+    for (int t = warp; t < tl; t += TC_THREADS / 32) {
+      bool nz = false;
+      for (int i = lane; i < dp / 2; i += 32) nz |= (reinterpret_cast<const uint32_t*>(khs + t * dp)[i] & 0x7FFF7FFFu) != 0u;
+      if (__any_sync(0xffffffffu, nz) && lane == 0) { atomicMin(&range_s[0], t); atomicMax(&range_s[1], t + 1); }
+    }
+    __syncthreads();
+    t0 = range_s[0];
+    tl = max(0, range_s[1] - t0);
+    if (tl == 0) t0 = 0;
+  }
   if (threadIdx.x == 0) ATT_TR(6, 120, 1);
   // K^T operand of the closing product, from the k rows now in shared memory
   for (int idx = threadIdx.x; idx < np * tp; idx += TC_THREADS) {
     const int t = idx / np, e = idx - t * np;
-    const __half v = (e < d && t < tl) ? khs[t * dp + e] : zero;
+    const __half v = (e < d && t < t_end) ? khs[t * dp + e] : zero;
     kts[(t >> 3) * (np * 8) + e * 8 + (t & 7)] = v;
   }
+  if (split > 1) {
+    const int per = (tl + split - 1) / split, first = min(tl, (int)(blockIdx.x % split) * per);
+    t0 += first;
+    tl = min(per, tl - first);
+  }
+  khs += t0 * dp;
+  if (threadIdx.x == 0) t0_s = t0;
   // barriers (b = step & 1, i = step % na1, a = step % na2):
   //   a1_full[i]   2 builder warps       -> layer-1 MMA warp: A1 of a step is in shared memory
   //   acc1_full[i] tcgen05.commit        -> layer-1 warpgroup i: layer-1 accumulator complete; builder: A1 read
@@ -364,7 +397,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
       mbar_init(smem_u32(&a2_full[i]), 4);
       mbar_init(smem_u32(&a2_free[i]), 1);
     }
-    mbar_init(smem_u32(s_full), 8);
+    mbar_init(smem_u32(s_full), 8 * split);          // the layer-2 warps of every CTA of the cluster
     mbar_init(smem_u32(acc3_full), 1);
     fence_barrier_init();
   }
@@ -372,6 +405,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
   fence_proxy_async_smem();          // operands were written through the generic proxy
   tc_fence_before_sync();
   __syncthreads();
+  if (split > 1) cluster_sync();     // the first CTA's S is cleared and its barrier initialised before anyone writes there
   tc_fence_after_sync();
   const uint32_t tmem0 = tmem_base_s;
   if (threadIdx.x == 0) ATT_TR(6, 120, 2);
@@ -445,7 +479,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
       if (++w1 == G.na1) { w1 = 0; ph1 ^= 1u; }
     }
     // weighted sum over the steps: out = S * K
-    if (ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(s_full), 0, 14))) {
+    if (p.split > 1) {
+      ok = blockIdx.x % p.split == 0 && ok && __all_sync(0xffffffffu, mbar_wait_cluster(smem_u32(s_full), 0, 14));
+      fence_proxy_async_smem();                               // scores of other CTAs came through their generic proxy
+    } else {
+      ok = ok && __all_sync(0xffffffffu, mbar_wait(smem_u32(s_full), 0, 14));
+    }
+    if (ok) {
       tc_fence_after_sync();
       const uint64_t da_step = (uint64_t)((2 * 128 * 16) >> 4);
       uint64_t da = make_desc_interleaved(smem_u32(ss), 128 * 16, 128);
@@ -677,8 +717,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
       const float2 f0 = __half22float2(part[0]), f1 = __half22float2(part[1]);
       const float2 f2 = __half22float2(part[2]), f3 = __half22float2(part[3]);
       const float s = p.b2 + ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
-      if (p.scores && valid && !p.use_softmax) p.scores[((int64_t)r * p.n_cand + n) * p.T + j] = s;
-      ss[(j >> 3) * (128 * 8) + row * 8 + (j & 7)] = __float2half_rn(s);
+      if (p.scores && valid && !p.use_softmax) p.scores[((int64_t)r * p.n_cand + n) * p.T + t0_s + j] = s;
+      const int t = t0_s + j;
+      __half* e = &ss[(t >> 3) * (128 * 8) + row * 8 + (t & 7)];
+      if (p.split > 1) st_cluster_u16(smem_u32(e), 0, __half_as_ushort(__float2half_rn(s)));
+      else *e = __float2half_rn(s);
     }
 
     if (p.use_softmax) asm volatile("bar.sync 1, 256;" ::: "memory");     // both parities' scores are in S
@@ -696,10 +739,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_u32(s_full));
+    if (lane == 0) {
+      if (p.split > 1) mbar_arrive_cluster(smem_u32(s_full), 0);
+      else mbar_arrive(smem_u32(s_full));
+    }
 
     if (lane == 0 && warp == 16) ATT_TR(6, 121, 0);
-    if (wb == 0) ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(acc3_full), 0, 22));
+    if (p.split > 1 && blockIdx.x % p.split != 0) ok = false;             // the cluster's first CTA writes the result
+    if (wb == 0 && ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc3_full), 0, 22));
     tc_fence_after_sync();
     if (lane == 0 && warp == 16) ATT_TR(6, 121, 1);
     if (ok && wb == 0) {
@@ -731,6 +778,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
   tc_fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0) ATT_TR(6, 121, 3);
+  if (p.split > 1) cluster_sync();                            // no CTA leaves while another may still write to it
   if (warp == MMA1_TC_WARP) {
     tc_fence_after_sync();
     tmem_dealloc(tmem0, TMEM_COLS);
@@ -768,26 +816,78 @@ int launch_att_pack(const AttParams& p, int act, void* dst, cudaStream_t stream)
   return check_launch("att_pack_kernel");
 }
 
+// CTAs that can be resident at once as clusters of `split` (one CTA per SM: all of tensor memory): a GPU processing
+// cluster whose SM count is no multiple of `split` leaves some of them out. Asked once per device.
+int cluster_slots(int lg) {
+  static std::atomic<int> cache[64][4];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = cache[dev][lg].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1u << lg; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1u << lg); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = 200 * 1024;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, din_att_tc_kernel<XB_ACT_DICE, 0, 0, 0>, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    n = clusters > 0 ? clusters << lg : -1;
+    cache[dev][lg].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// How many CTAs share a tile: the time is (waves of CTAs) x (steps of one CTA + what a CTA spends around them, about
+// 8 steps' worth), plus about 3 for the cluster's barriers. 592 tiles of 100 steps stay whole (4 x 108 against 8 x 58);
+// 8 tiles take clusters of 8 (13 + 8 + 3 against 108).
+int pick_split(int64_t tiles, int T) {
+  int best = 1;
+  int64_t cost = ((tiles + sm_count() - 1) / sm_count()) * (T + 8);
+  for (int lg = 1; lg <= 3; ++lg) {
+    const int s = 1 << lg, slots = s <= T ? cluster_slots(lg) : 0;
+    if (slots <= 0) continue;
+    const int64_t c = ((tiles * s + slots - 1) / slots) * ((T + s - 1) / s + 8) + 3;
+    if (c < cost) { cost = c; best = s; }
+  }
+  return best;
+}
+
 int launch_att_tc(AttParams& p, const xb_din_att_args& a, cudaStream_t stream) {
   const TcGeom g = tc_geom(a.d, a.h0, a.h1, a.T);
   p.tiles_per_req = (a.n_cand + 127) / 128;
   p.idesc1 = umma::make_idesc(128, g.h0p, 0);
   p.idesc2 = umma::make_idesc(128, g.h1p, 0);
   p.idesc3 = umma::make_idesc(128, g.np, 0);
-  const TcSmemLayout L = tc_layout(g, p.T);
   static PerDeviceOnce attr_set;
   XB_SET_MAX_SMEM_ONCE(attr_set, 220 * 1024, (const void*)din_att_tc_kernel<XB_ACT_NONE, 0, 0, 0>,
                        (const void*)din_att_tc_kernel<XB_ACT_SIGMOID, 0, 0, 0>, (const void*)din_att_tc_kernel<XB_ACT_DICE, 0, 0, 0>,
                        (const void*)din_att_tc_kernel<XB_ACT_SIGMOID, 36, 80, 40>, (const void*)din_att_tc_kernel<XB_ACT_DICE, 36, 80, 40>);
-  const int64_t blocks = (int64_t)a.requests * p.tiles_per_req;
-  XB_REQUIRE(blocks < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_din_attention: too many tiles");
+  const int64_t tiles = (int64_t)a.requests * p.tiles_per_req;
+  XB_REQUIRE(tiles < ((int64_t)1 << 28), XB_ERR_LIMIT, "xb_din_attention: too many tiles");
+  p.split = a.use_softmax ? 1 : pick_split(tiles, p.T);        // the softmax needs all scores of a row in one place
+  const TcSmemLayout L = tc_layout(g, p.T);
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)p.split; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * p.split)); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = (size_t)L.total;
+  cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = p.split > 1 ? 1 : 0;
   // the shape of the DIN / DIEN attention unit (d = 36, MLP 144-80-40-1) has instantiations of its own
   const bool din_shape = a.d == 36 && a.h0 == 80 && a.h1 == 40;
-  if (din_shape && a.act == XB_ACT_DICE) din_att_tc_kernel<XB_ACT_DICE, 36, 80, 40><<<(unsigned)blocks, TC_THREADS, L.total, stream>>>(p);
-  else if (din_shape && a.act == XB_ACT_SIGMOID) din_att_tc_kernel<XB_ACT_SIGMOID, 36, 80, 40><<<(unsigned)blocks, TC_THREADS, L.total, stream>>>(p);
-  else if (a.act == XB_ACT_DICE) din_att_tc_kernel<XB_ACT_DICE, 0, 0, 0><<<(unsigned)blocks, TC_THREADS, L.total, stream>>>(p);
-  else if (a.act == XB_ACT_SIGMOID) din_att_tc_kernel<XB_ACT_SIGMOID, 0, 0, 0><<<(unsigned)blocks, TC_THREADS, L.total, stream>>>(p);
-  else din_att_tc_kernel<XB_ACT_NONE, 0, 0, 0><<<(unsigned)blocks, TC_THREADS, L.total, stream>>>(p);
+  cudaError_t e;
+  if (din_shape && a.act == XB_ACT_DICE) e = cudaLaunchKernelEx(&cfg, din_att_tc_kernel<XB_ACT_DICE, 36, 80, 40>, p);
+  else if (din_shape && a.act == XB_ACT_SIGMOID) e = cudaLaunchKernelEx(&cfg, din_att_tc_kernel<XB_ACT_SIGMOID, 36, 80, 40>, p);
+  else if (a.act == XB_ACT_DICE) e = cudaLaunchKernelEx(&cfg, din_att_tc_kernel<XB_ACT_DICE, 0, 0, 0>, p);
+  else if (a.act == XB_ACT_SIGMOID) e = cudaLaunchKernelEx(&cfg, din_att_tc_kernel<XB_ACT_SIGMOID, 0, 0, 0>, p);
+  else e = cudaLaunchKernelEx(&cfg, din_att_tc_kernel<XB_ACT_NONE, 0, 0, 0>, p);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(XB_ERR_CUDA, "din_att_tc_kernel launch failed: %s", cudaGetErrorString(e));
+  }
   return check_launch("din_att_tc_kernel");
 }
 
