@@ -84,12 +84,60 @@ __global__ void softmax_kernel(const void* x, void* y, int64_t n, int c, int64_t
   }
 }
 
+// Contiguous rows (w == 1) of 16 and more columns: one warp per row, so that a row is read in coalesced pieces, and up to
+// 256 columns stay in registers between the three passes. 16 000 rows of 100 fp32: 7.3 us, 34 before (one thread per row
+// touches 32 rows with every load).
+template <int PER>
+__global__ void __launch_bounds__(256) softmax_rows_kernel(const void* x, void* y, int64_t n, int c, int dt) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * 8;
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < n; r += warps) {
+    const int64_t base = r * c;
+    float v[PER], m = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int j = lane + 32 * i;
+      v[i] = j < c ? load_as_f32(x, base + j, dt) : -INFINITY;
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) m = fmaxf(m, v[i]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      v[i] = lane + 32 * i < c ? __expf(v[i] - m) : 0.f;
+      s += v[i];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int j = lane + 32 * i;
+      if (j < c) store_from_f32(y, base + j, dt, v[i] / s);
+    }
+  }
+}
+
 struct EwParams {
   int op, dt;
   const void *a, *b, *c;
   void* y;
   int64_t as[4], bs[4], cs[4], shape[4];
 };
+
+__device__ __forceinline__ float ew_apply(int op, float av, float bv) {
+  switch (op) {
+    case XB_EW_ADD: return av + bv;
+    case XB_EW_SUB: return av - bv;
+    case XB_EW_MUL: return av * bv;
+    case XB_EW_DIV: return av / bv;
+    case XB_EW_MAX: return fmaxf(av, bv);
+    case XB_EW_MIN: return fminf(av, bv);
+    case XB_EW_EQ: return av == bv ? 1.f : 0.f;
+    default: return av != bv ? 1.f : 0.f;
+  }
+}
 
 __global__ void elementwise_kernel(const __grid_constant__ EwParams p) {
   const int64_t total = p.shape[0] * p.shape[1] * p.shape[2] * p.shape[3];
@@ -109,19 +157,38 @@ __global__ void elementwise_kernel(const __grid_constant__ EwParams p) {
     } else if (p.op == XB_EW_BROADCAST_TO) {
       out = load_as_f32(p.a, ia, p.dt);
     } else {
-      const float av = load_as_f32(p.a, ia, p.dt), bv = load_as_f32(p.b, ib, p.dt);
-      switch (p.op) {
-        case XB_EW_ADD: out = av + bv; break;
-        case XB_EW_SUB: out = av - bv; break;
-        case XB_EW_MUL: out = av * bv; break;
-        case XB_EW_DIV: out = av / bv; break;
-        case XB_EW_MAX: out = fmaxf(av, bv); break;
-        case XB_EW_MIN: out = fminf(av, bv); break;
-        case XB_EW_EQ: out = av == bv ? 1.f : 0.f; break;
-        default: out = av != bv ? 1.f : 0.f; break;
-      }
+      out = ew_apply(p.op, load_as_f32(p.a, ia, p.dt), load_as_f32(p.b, ib, p.dt));
     }
     store_from_f32(p.y, i, p.dt, out);
+  }
+}
+
+// Four fp32 elements of the innermost axis per thread: 16-byte accesses (an operand that repeats along that axis is read
+// once), 32-bit index arithmetic and one decomposition of the index per four elements; the kernel above spends its time
+// on four 64-bit divisions per element. The launcher merges axes that every operand walks contiguously and sees to
+// alignment. [500, 100, 36] - [1, 100, 36]: 3.3 us, 14 before
+__global__ void __launch_bounds__(256) elementwise4_kernel(const __grid_constant__ EwParams p) {
+  const uint32_t s1 = (uint32_t)p.shape[1], s2 = (uint32_t)p.shape[2], s3 = (uint32_t)p.shape[3] / 4;
+  const uint32_t total = (uint32_t)p.shape[0] * s1 * s2 * s3;
+  const bool rep_a = p.as[3] == 0, rep_b = p.bs[3] == 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    uint32_t r = i / s3;
+    const uint32_t i3 = i - r * s3;
+    uint32_t q = r / s2;
+    const uint32_t i2 = r - q * s2;
+    const uint32_t i0 = q / s1, i1 = q - i0 * s1;
+    auto load4 = [&](const void* base, const int64_t* st, bool rep) {
+      const float* f = reinterpret_cast<const float*>(base) + (int64_t)i0 * st[0] + (int64_t)i1 * st[1] + (int64_t)i2 * st[2];
+      if (rep) { const float v = *f; return make_float4(v, v, v, v); }
+      return *reinterpret_cast<const float4*>(f + 4 * i3);
+    };
+    const float4 a = load4(p.a, p.as, rep_a);
+    float4 o = a;
+    if (p.op != XB_EW_BROADCAST_TO) {
+      const float4 b = load4(p.b, p.bs, rep_b);
+      o = make_float4(ew_apply(p.op, a.x, b.x), ew_apply(p.op, a.y, b.y), ew_apply(p.op, a.z, b.z), ew_apply(p.op, a.w, b.w));
+    }
+    reinterpret_cast<float4*>(p.y)[i] = o;
   }
 }
 
@@ -129,7 +196,8 @@ __global__ void copy2d_kernel(const void* src, int64_t src_ld, int sdt, void* ds
                               int64_t rows, int64_t cols) {
   const int64_t total = rows * cols;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / cols, c = i - r * cols;
+    // 32-bit division where it will do: the 64-bit one is most of the instructions of an element
+    const int64_t r = total < ((int64_t)1 << 31) ? (int64_t)((uint32_t)i / (uint32_t)cols) : i / cols, c = i - r * cols;
     if (sdt == XB_I32 && ddt == XB_I32)
       reinterpret_cast<int32_t*>(dst)[r * dst_ld + c] = reinterpret_cast<const int32_t*>(src)[r * src_ld + c];
     else if (sdt == XB_I64 && ddt == XB_I64)
@@ -139,12 +207,32 @@ __global__ void copy2d_kernel(const void* src, int64_t src_ld, int sdt, void* ds
   }
 }
 
+// Same-type copies of rows whose pieces of sizeof(V) bytes are aligned in source and destination: one piece per thread and
+// 32-bit index arithmetic (element by element the kernel above is bound by its 64-bit division). 50 000 rows of 36 fp32
+// into rows of 144: 1.9 us, 5 before
+template <typename V>
+__global__ void __launch_bounds__(256) copy2d_vec_kernel(const V* src, int64_t src_ld, V* dst, int64_t dst_ld, uint32_t total, uint32_t cols) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t r = i / cols, c = i - r * cols;
+    dst[(int64_t)r * dst_ld + c] = src[(int64_t)r * src_ld + c];
+  }
+}
+
 __global__ void reduce_sum_kernel(const void* x, void* y, int64_t outer, int64_t r, int64_t inner, int dt) {
   const int64_t total = outer * inner;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t o = i / inner, in = i - o * inner;
     float s = 0.f;
-    for (int64_t j = 0; j < r; ++j) s += load_as_f32(x, (o * r + j) * inner + in, dt);
+    // eight loads in flight, added in order
+    int64_t j = 0;
+    for (; j + 8 <= r; j += 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = load_as_f32(x, (o * r + j + u) * inner + in, dt);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; j < r; ++j) s += load_as_f32(x, (o * r + j) * inner + in, dt);
     store_from_f32(y, i, dt, s);
   }
 }
@@ -178,7 +266,15 @@ __global__ void __launch_bounds__(256) din_tower_input_kernel(const __half* user
   if ((int)threadIdx.x < G * d) {
     const int gi = threadIdx.x / d, e = threadIdx.x - gi * d;
     float s = 0.f;
-    for (int t = gi; t < T; t += G) s += __half2float(k[((int64_t)r * T + t) * ldk + e]);
+    // eight steps requested together, added in order
+    for (int t = gi; t < T; t += 8 * G) {
+      __half v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = t + u * G < T ? k[((int64_t)r * T + t + u * G) * ldk + e] : __float2half(0.f);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (t + u * G < T) s += __half2float(v[u]);
+    }
     part[gi * d + e] = s;
   }
   for (int e = threadIdx.x; e < du; e += blockDim.x) us[e] = __half2float(user[(int64_t)r * ldu + e]);
@@ -191,6 +287,41 @@ __global__ void __launch_bounds__(256) din_tower_input_kernel(const __half* user
   __syncthreads();
   const int n0 = blockIdx.x * 64;
   const int rows = min(64, n_cand - n0);
+  if (pairs_ok == 2) {
+    // four columns (8 bytes) at a time: 16 000 rows of 328 columns take 17 us, 23 two at a time
+    const int wq = (int)(ldx >> 2);
+    for (int idx = threadIdx.x; idx < rows * wq; idx += blockDim.x) {
+      const int nl = idx / wq, c = (idx - nl * wq) * 4;
+      const int64_t row = (int64_t)r * n_cand + n0 + nl;
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (c < du) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = us[c + u];
+      } else if (c < du + 5 * d) {
+        const int seg = (c - du) / d, e = (c - du) - seg * d;
+        if (seg == 1) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) v[u] = hs[e + u];
+        } else {
+          const uint2 raw = *reinterpret_cast<const uint2*>(seg == 3 ? att + row * ldatt + e : q + row * ldq + e);
+          const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+          v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+          if (seg == 2) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] *= hs[e + u];
+          } else if (seg == 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] -= hs[e + u];
+          }
+        }
+      }
+      const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
+      uint2 w;
+      w.x = *reinterpret_cast<const uint32_t*>(&a); w.y = *reinterpret_cast<const uint32_t*>(&b);
+      *reinterpret_cast<uint2*>(X + row * ldx + c) = w;
+    }
+    return;
+  }
   if (pairs_ok) {
     const int wp = (int)(ldx >> 1);                    // half2 units per row
     for (int idx = threadIdx.x; idx < rows * wp; idx += blockDim.x) {
@@ -246,7 +377,15 @@ __global__ void __launch_bounds__(256) din_tower_split_kernel(const __half* user
   if ((int)threadIdx.x < G * d) {
     const int gi = threadIdx.x / d, e = threadIdx.x - gi * d;
     float s = 0.f;
-    for (int t = gi; t < T; t += G) s += __half2float(k[((int64_t)r * T + t) * ldk + e]);
+    // eight steps requested together, added in order
+    for (int t = gi; t < T; t += 8 * G) {
+      __half v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = t + u * G < T ? k[((int64_t)r * T + t + u * G) * ldk + e] : __float2half(0.f);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (t + u * G < T) s += __half2float(v[u]);
+    }
     part[gi * d + e] = s;
   }
   __syncthreads();
@@ -342,6 +481,13 @@ extern "C" int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t 
   XB_REQUIRE(x && y && n >= 0 && c > 0 && w > 0, XB_ERR_ARG, "xb_softmax: bad arguments");
   XB_REQUIRE(float_dtype(dtype), XB_ERR_UNSUPPORTED, "xb_softmax: dtype %d", dtype);
   if (n == 0) return 0;
+  if (w == 1 && c >= 16 && c <= 256) {
+    const unsigned grid = stream_grid(n, 8);
+    if (c <= 64) softmax_rows_kernel<2><<<grid, 256, 0, (cudaStream_t)s>>>(x, y, n, c, dtype);
+    else if (c <= 128) softmax_rows_kernel<4><<<grid, 256, 0, (cudaStream_t)s>>>(x, y, n, c, dtype);
+    else softmax_rows_kernel<8><<<grid, 256, 0, (cudaStream_t)s>>>(x, y, n, c, dtype);
+    return check_launch("softmax_rows_kernel");
+  }
   softmax_kernel<<<stream_grid(n * w, 128), 128, 0, (cudaStream_t)s>>>(x, y, n, c, w, dtype);
   return check_launch("softmax_kernel");
 }
@@ -375,6 +521,28 @@ extern "C" int xb_elementwise(int32_t op, const void* a, const int64_t* as, cons
     total *= shape[i];
   }
   if (total == 0) return 0;
+  if (dtype == XB_F32 && op != XB_EW_WHERE && total < ((int64_t)1 << 31)) {
+    // merge an axis into the one inside it where both operands step over it as over one axis (the output is dense)
+    EwParams m = p;
+    const bool two = op != XB_EW_BROADCAST_TO;
+    for (int i = 2; i >= 0; --i) {
+      const bool merge = m.shape[i] == 1 || (m.as[i] == m.as[3] * m.shape[3] && (!two || m.bs[i] == m.bs[3] * m.shape[3]));
+      if (!merge) break;
+      m.shape[3] *= m.shape[i];
+      for (int j = i; j > 0; --j) { m.shape[j] = m.shape[j - 1]; m.as[j] = m.as[j - 1]; m.bs[j] = m.bs[j - 1]; }
+      m.shape[0] = 1; m.as[0] = m.bs[0] = 0;
+      ++i;                                            // the next outer axis is at the same place now
+      if (m.shape[0] * m.shape[1] * m.shape[2] == 1) break;
+    }
+    auto fits = [&](const void* base, const int64_t* st) {
+      if (st[3] == 0) return true;
+      return st[3] == 1 && (reinterpret_cast<uintptr_t>(base) & 15) == 0 && st[0] % 4 == 0 && st[1] % 4 == 0 && st[2] % 4 == 0;
+    };
+    if (m.shape[3] % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && fits(a, m.as) && (!two || fits(b, m.bs))) {
+      elementwise4_kernel<<<stream_grid(total / 4, 256), 256, 0, (cudaStream_t)s>>>(m);
+      return check_launch("elementwise4_kernel");
+    }
+  }
   elementwise_kernel<<<stream_grid(total, 256), 256, 0, (cudaStream_t)s>>>(p);
   return check_launch("elementwise_kernel");
 }
@@ -385,6 +553,24 @@ extern "C" int xb_copy2d(const void* src, int64_t src_ld, int32_t sdt, void* dst
   XB_REQUIRE(dtype_size(sdt) && dtype_size(ddt), XB_ERR_UNSUPPORTED, "xb_copy2d: dtype %d -> %d", sdt, ddt);
   XB_REQUIRE((sdt == XB_I64) == (ddt == XB_I64), XB_ERR_UNSUPPORTED, "xb_copy2d: int64 converts to nothing else");
   if (rows * cols == 0) return 0;
+  if (sdt == ddt) {
+    // widest piece that divides the row and both pitches and to which both ends are aligned
+    const int64_t es = (int64_t)dtype_size(sdt);
+    const uintptr_t bits = (uintptr_t)src | (uintptr_t)dst | (uintptr_t)(src_ld * es) | (uintptr_t)(dst_ld * es) | (uintptr_t)(cols * es);
+    const int64_t w = bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : 2;
+    const int64_t pieces = rows * cols * es / w;
+    if (bits % 2 == 0 && pieces < ((int64_t)1 << 30)) {
+      const unsigned grid = stream_grid(pieces, 256);
+      const uint32_t pc = (uint32_t)(cols * es / w);
+      const int64_t sl = src_ld * es / w, dl = dst_ld * es / w;
+      const cudaStream_t st = (cudaStream_t)s;
+      if (w == 16) copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint4*)src, sl, (uint4*)dst, dl, (uint32_t)pieces, pc);
+      else if (w == 8) copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint2*)src, sl, (uint2*)dst, dl, (uint32_t)pieces, pc);
+      else if (w == 4) copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint32_t*)src, sl, (uint32_t*)dst, dl, (uint32_t)pieces, pc);
+      else copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint16_t*)src, sl, (uint16_t*)dst, dl, (uint32_t)pieces, pc);
+      return check_launch("copy2d_vec_kernel");
+    }
+  }
   copy2d_kernel<<<stream_grid(rows * cols, 256), 256, 0, (cudaStream_t)s>>>(src, src_ld, sdt, dst, dst_ld, ddt, rows, cols);
   return check_launch("copy2d_kernel");
 }
@@ -455,9 +641,12 @@ extern "C" int xb_din_tower_input(const void* user, int64_t ldu, const void* q, 
   // 32-bit accesses need even segment widths and leading dimensions and 4-byte aligned bases
   const int pairs_ok = d % 2 == 0 && du % 2 == 0 && ldx % 2 == 0 && ldq % 2 == 0 && ldatt % 2 == 0 &&
                        (((uintptr_t)q | (uintptr_t)att | (uintptr_t)X) & 3) == 0;
+  // 64-bit ones need the same of multiples of four
+  const int quads_ok = d % 4 == 0 && du % 4 == 0 && ldx % 4 == 0 && ldq % 4 == 0 && ldatt % 4 == 0 &&
+                       (((uintptr_t)q | (uintptr_t)att | (uintptr_t)X) & 7) == 0;
   din_tower_input_kernel<<<grid, 256, sizeof(float) * (9 * d + du + 2), (cudaStream_t)s>>>(
       (const __half*)user, ldu, (const __half*)q, ldq, (const __half*)k, ldk, (const __half*)att, ldatt, (__half*)X,
-      ldx, n_cand, T, d, du, pairs_ok);
+      ldx, n_cand, T, d, du, quads_ok ? 2 : pairs_ok);
   return check_launch("din_tower_input_kernel");
 }
 
