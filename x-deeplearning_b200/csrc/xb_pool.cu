@@ -1292,34 +1292,61 @@ __device__ __forceinline__ int64_t route_segment(const int32_t* __restrict__ seg
   return lo;
 }
 
-// pass 1: per-CTA histogram of owners
-// the segment of the first id of every scatter CTA (one search per thread); the entry after the last CTA closes the
-// last window
-__global__ void route_windows_kernel(const int32_t* __restrict__ seg_offsets, int64_t segments, int64_t n, int64_t blocks,
-                                     int32_t* __restrict__ block_first_seg) {
-  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b > blocks) return;
-  const int64_t first = b * ROUTE_CHUNK;
-  const int32_t last_seg = (int32_t)(segments > 0 ? segments - 1 : 0);
-  block_first_seg[b] = (b < blocks && first < n && segments > 0) ? (int32_t)route_segment(seg_offsets, 0, segments, first) : last_seg;
+// the same search by a whole warp, 33 intervals a step: 4 dependent loads for 330 k segments instead of 18
+__device__ __forceinline__ int64_t route_segment_warp(const int32_t* __restrict__ seg_offsets, int64_t segments, int64_t idx) {
+  int64_t lo = 0, hi = segments;
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 32) / 33, at = lo + (int64_t)((threadIdx.x & 31) + 1) * step;
+    const unsigned m = __ballot_sync(0xffffffffu, at < hi && (int64_t)__ldg(seg_offsets + at) <= idx);
+    const int64_t c = m == 0xffffffffu ? 32 : __ffs(~m) - 1;
+    hi = min(hi, lo + (c + 1) * step);
+    lo += c * step;
+  }
+  return lo;
 }
 
+// pass 1: per-CTA histogram of owners, and the segment of the first id of every scatter CTA (the entry after the last
+// CTA closes the last window). Eight id loads a thread are in flight together; with one shard the owner is known and no
+// id is read. 5.1 M ids, one shard, 330 k segments: 6.4 us; two kernels took 23 + 10
 __global__ void __launch_bounds__(256) route_count_kernel(const int64_t* __restrict__ ids, int64_t n, int shards,
-                                                          int32_t* __restrict__ block_hist) {
+                                                          int32_t* __restrict__ block_hist,
+                                                          const int32_t* __restrict__ seg_offsets, int64_t segments,
+                                                          int32_t* __restrict__ block_first_seg) {
   __shared__ int32_t hist[ROUTE_MAX_SHARDS];
   if (threadIdx.x < ROUTE_MAX_SHARDS) hist[threadIdx.x] = 0;
-
   __syncthreads();
   const int64_t base = (int64_t)blockIdx.x * ROUTE_CHUNK;
   const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < ROUTE_CHUNK; i += 256) {
-    const int64_t idx = base + i;
-    const int owner = idx < n ? route_owner((uint64_t)__ldcs(ids + idx), shards) : -1;
-    // one shared-memory atomic per warp and owner instead of one per id (with two owners every id of a CTA would
-    // queue on the same two words)
-    for (int w = 0; w < shards; ++w) {
-      const unsigned m = __ballot_sync(0xffffffffu, owner == w);
-      if (lane == 0 && m) atomicAdd(&hist[w], __popc(m));                                // integer: order-free
+  if (threadIdx.x < 32) {
+    const int32_t last_seg = (int32_t)(segments > 0 ? segments - 1 : 0);
+    const int64_t seg = (base < n && segments > 0) ? route_segment_warp(seg_offsets, segments, base) : last_seg;
+    if (lane == 0) {
+      block_first_seg[blockIdx.x] = (int32_t)seg;
+      if (blockIdx.x == 0) block_first_seg[gridDim.x] = last_seg;
+    }
+  }
+  if (shards == 1) {
+    if (threadIdx.x == 0) block_hist[blockIdx.x] = (int32_t)max((int64_t)0, min((int64_t)ROUTE_CHUNK, n - base));
+    return;
+  }
+  constexpr int U = 8;
+  for (int i0 = 0; i0 < ROUTE_CHUNK; i0 += 256 * U) {
+    uint64_t id[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t idx = base + i0 + u * 256 + threadIdx.x;
+      id[u] = idx < n ? (uint64_t)__ldcs(ids + idx) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t idx = base + i0 + u * 256 + threadIdx.x;
+      const int owner = idx < n ? route_owner(id[u], shards) : -1;
+      // one shared-memory atomic per warp and owner instead of one per id (with two owners every id of a CTA would
+      // queue on the same two words)
+      for (int w = 0; w < shards; ++w) {
+        const unsigned m = __ballot_sync(0xffffffffu, owner == w);
+        if (lane == 0 && m) atomicAdd(&hist[w], __popc(m));                              // integer: order-free
+      }
     }
   }
   __syncthreads();
@@ -1331,43 +1358,47 @@ __global__ void __launch_bounds__(256) route_count_kernel(const int64_t* __restr
 // With bucket_cap > 0 the buckets have a fixed capacity: bucket w starts at w * bucket_cap, its first slot holds
 // the number of records that follow (the receiver reads it from there), and a bucket that would not fit sets
 // *overflow and is cut at the capacity.
-__global__ void __launch_bounds__(256) route_scan_kernel(int32_t* __restrict__ block_hist, int64_t blocks, int shards,
-                                                         int64_t* __restrict__ owner_counts, int64_t bucket_cap,
-                                                         int64_t* __restrict__ headers, int32_t* __restrict__ overflow) {
-  __shared__ int64_t total_s;
-  __shared__ int32_t part[256];
-  if (threadIdx.x == 0) total_s = 0;
-  __syncthreads();
+__global__ void __launch_bounds__(1024) route_scan_kernel(int32_t* __restrict__ block_hist, int64_t blocks, int shards,
+                                                          int64_t* __restrict__ owner_counts, int64_t bucket_cap,
+                                                          int64_t* __restrict__ headers, int32_t* __restrict__ overflow) {
+  __shared__ int32_t part[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t total = 0;                                          // the same in every thread
   for (int w = 0; w < shards; ++w) {
-    const int64_t start = total_s;
-    for (int64_t b0 = 0; b0 < blocks; b0 += 256) {
+    const int64_t start = total;
+    for (int64_t b0 = 0; b0 < blocks; b0 += 1024) {
       const int64_t b = b0 + threadIdx.x;
       const int32_t v = b < blocks ? block_hist[b * shards + w] : 0;
-      part[threadIdx.x] = v;
-      __syncthreads();
-      // Hillis-Steele inclusive scan of the 256 partials
-      for (int off = 1; off < 256; off <<= 1) {
-        int32_t add = threadIdx.x >= off ? part[threadIdx.x - off] : 0;
-        __syncthreads();
-        part[threadIdx.x] += add;
-        __syncthreads();
+      int32_t incl = v;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int32_t o = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += o;
       }
-      if (b < blocks)
-        block_hist[b * shards + w] = bucket_cap > 0 ? (int32_t)(w * bucket_cap + 1 + (total_s - start) + part[threadIdx.x] - v)
-                                                    : (int32_t)(total_s + part[threadIdx.x] - v);
+      if (lane == 31) part[warp] = incl;
       __syncthreads();
-      if (threadIdx.x == 255) total_s += part[255];
-      __syncthreads();
+      int32_t p = part[lane];                                 // every warp scans the 32 warp totals for itself
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int32_t o = __shfl_up_sync(0xffffffffu, p, off);
+        if (lane >= off) p += o;
+      }
+      const int32_t before = warp > 0 ? __shfl_sync(0xffffffffu, p, warp - 1) : 0;
+      if (b < blocks) {
+        const int64_t at = (total - start) + before + incl - v;
+        block_hist[b * shards + w] = bucket_cap > 0 ? (int32_t)(w * bucket_cap + 1 + at) : (int32_t)(start + at);
+      }
+      total += __shfl_sync(0xffffffffu, p, 31);
+      __syncthreads();                                        // `part` is written again
     }
     if (threadIdx.x == 0) {
-      const int64_t cnt = total_s - start;
+      const int64_t cnt = total - start;
       if (owner_counts) owner_counts[w] = cnt;
       if (bucket_cap > 0) {
         headers[w * bucket_cap] = cnt < bucket_cap ? cnt : bucket_cap - 1;
         if (cnt >= bucket_cap) atomicExch(overflow, 1);
       }
     }
-    __syncthreads();
   }
 }
 
@@ -1390,7 +1421,7 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(const int64_t* __res
   const int64_t base = (int64_t)blockIdx.x * ROUTE_CHUNK;
   if (threadIdx.x < shards) running[0][threadIdx.x] = block_base[(int64_t)blockIdx.x * shards + threadIdx.x];
   // the ids of this CTA are consecutive, so their segments lie between the segment of its first id and that of
-  // the next CTA's first id (both found by route_windows_kernel)
+  // the next CTA's first id (both found by route_count_kernel)
   const int64_t win_lo = __ldg(block_first_seg + blockIdx.x), win_hi = (int64_t)__ldg(block_first_seg + blockIdx.x + 1) + 1;
   const bool tabulated = win_hi - win_lo <= WIN;              // otherwise (mostly empty segments) every id searches the offsets
   if (tabulated) {
@@ -1406,6 +1437,7 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(const int64_t* __res
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool one = shards == 1;                               // every id keeps its place: no ranks to work out
   // Rounds of RK x 256 consecutive ids: thread t takes the ids t, t + 256, ... of a round, so every load and (per
   // owner) every store is coalesced and all RK loads are in flight together. The ranking stays stable: an id is
   // preceded by the ids of earlier rounds, of earlier sub-rounds, of lower warps in its sub-round and of lower lanes
@@ -1423,14 +1455,15 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(const int64_t* __res
       const int64_t idx = base + i0 + k * 256 + threadIdx.x;
       owner[k] = idx < n ? route_owner(id[k], shards) : -1;
       rank_in_warp[k] = 0;
+      if (one) continue;
       for (int w = 0; w < shards; ++w) {
         const unsigned m = __ballot_sync(0xffffffffu, owner[k] == w);
         if (owner[k] == w) rank_in_warp[k] = __popc(m & ((1u << lane) - 1));
         if (lane == 0) warp_cnt[rnd][k][warp][w] = __popc(m);
       }
     }
-    __syncthreads();                                          // the counts of this round are written
-    if (threadIdx.x < shards) {
+    if (!one) __syncthreads();                                // the counts of this round are written
+    if (!one && threadIdx.x < shards) {
       // counts -> exclusive prefixes in (sub-round, warp) order, starting from the ids of the rounds before
       int acc = running[rnd][threadIdx.x];
       for (int k = 0; k < RK; ++k)
@@ -1441,13 +1474,14 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(const int64_t* __res
         }
       running[rnd ^ 1][threadIdx.x] = acc;
     }
-    __syncthreads();                                          // the prefixes are written
+    if (!one) __syncthreads();                                // the prefixes are written
 #pragma unroll
     for (int k = 0; k < RK; ++k) {
       const int64_t idx = base + i0 + k * 256 + threadIdx.x;
       if (idx < n) {
         const int ow = owner[k];
-        const int64_t pos = (int64_t)warp_cnt[rnd][k][warp][ow] + rank_in_warp[k];
+        const int64_t pos = one ? (int64_t)running[0][0] + i0 + k * 256 + threadIdx.x
+                                : (int64_t)warp_cnt[rnd][k][warp][ow] + rank_in_warp[k];
         // segment of this id: last offset <= idx
         const int64_t lo = tabulated ? win_lo + seg_rel[i0 + k * 256 + threadIdx.x] : route_segment(seg_offsets, win_lo, win_hi, idx);
         const uint64_t row = route_row(id[k], shards);
@@ -1658,9 +1692,8 @@ extern "C" int xb_route_ids(const int64_t* ids, const float* values, const int32
   const int64_t blocks = std::max<int64_t>((n_ids + ROUTE_CHUNK - 1) / ROUTE_CHUNK, 1);
   int32_t* hist = reinterpret_cast<int32_t*>(scratch);
   int32_t* first_seg = hist + blocks * shards;
-  route_count_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, n_ids, shards, hist);
-  route_windows_kernel<<<(unsigned)((blocks + 256) / 256), 256, 0, stream>>>(seg_offsets, segments, n_ids, blocks, first_seg);
-  route_scan_kernel<<<1, 256, 0, stream>>>(hist, blocks, shards, owner_counts, 0, nullptr, nullptr);
+  route_count_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, n_ids, shards, hist, seg_offsets, segments, first_seg);
+  route_scan_kernel<<<1, 1024, 0, stream>>>(hist, blocks, shards, owner_counts, 0, nullptr, nullptr);
   route_scatter_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, values, seg_offsets, segments, n_ids, shards, hist, out_rows,
                                                              out_values, out_tags, 0, first_seg);
   return check_launch("route kernels");
@@ -1681,9 +1714,8 @@ extern "C" int xb_route_ids_padded(const int64_t* ids, const int32_t* seg_offset
   const int64_t blocks = std::max<int64_t>((n_ids + ROUTE_CHUNK - 1) / ROUTE_CHUNK, 1);
   int32_t* hist = reinterpret_cast<int32_t*>(scratch);
   int32_t* first_seg = hist + blocks * shards;
-  route_count_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, n_ids, shards, hist);
-  route_windows_kernel<<<(unsigned)((blocks + 256) / 256), 256, 0, stream>>>(seg_offsets, segments, n_ids, blocks, first_seg);
-  route_scan_kernel<<<1, 256, 0, stream>>>(hist, blocks, shards, nullptr, bucket_cap, out_records, overflow);
+  route_count_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, n_ids, shards, hist, seg_offsets, segments, first_seg);
+  route_scan_kernel<<<1, 1024, 0, stream>>>(hist, blocks, shards, nullptr, bucket_cap, out_records, overflow);
   route_scatter_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, nullptr, seg_offsets, segments, n_ids, shards, hist, out_records,
                                                              nullptr, nullptr, bucket_cap, first_seg);
   return check_launch("route kernels (fixed-capacity buckets)");
