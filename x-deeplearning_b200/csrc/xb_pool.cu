@@ -38,7 +38,8 @@ struct PoolGroupDev {
   int32_t lpr;                 // lanes per row
   int32_t tl;                  // lanes per segment (team)
   int32_t vhalf;               // per-id weights are fp16
-  int32_t segs;                // specialised kernel: rounds of segments per warp
+  int32_t segs;                // specialised kernels: rounds of segments per warp; queue kernel: segments per warp
+  int32_t counts;              // pool_fast_kernel: `offsets` holds the counts, prefix sums are made by the warps
   PoolItemDev items[XB_MAX_POOL_ITEMS];
 };
 
@@ -57,6 +58,8 @@ struct ScanParams {
   int32_t* chunk_sums[XB_MAX_POOL_GROUPS];
   int32_t chunk_begin[XB_MAX_POOL_GROUPS + 1];
 };
+
+constexpr int POOL_INLINE_COUNTS = 1024;      // longest count array that pool_fast_kernel adds up itself
 
 __device__ __forceinline__ uint64_t mix64(uint64_t x) {
   x ^= x >> 33; x *= 0xff51afd7ed558ccdULL; x ^= x >> 33;
@@ -215,9 +218,11 @@ __device__ __forceinline__ int64_t lookup_row(const PoolGroupDev& g, int64_t key
   uint64_t h = mix64((uint64_t)key) & (uint64_t)g.slot_mask;
   // bounded probe: an index built by xb_table_build_index_host is at most half full
   for (int64_t probes = 0; probes <= g.slot_mask; ++probes) {
-    int32_t r = __ldg(g.slot_rows + h);
+    // both requested at once: the key of an empty slot is read for nothing, that of a full one does not wait for its row
+    const int32_t r = __ldg(g.slot_rows + h);
+    const int64_t k = __ldg(g.slot_keys + h);
     if (r < 0) return -1;
-    if (__ldg(g.slot_keys + h) == key) return r;
+    if (k == key) return r;
     h = (h + 1) & (uint64_t)g.slot_mask;
   }
   return -1;
@@ -503,6 +508,28 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
       nm = __ldg(g.offsets + sg + 1) - st;
     }
   };
+  // Short count arrays (segs is 1): the warp adds up the counts before its first segment itself, which takes less than
+  // the launch of a scan kernel in front of this one. A segment's start: those, and the counts of the teams before its.
+  auto span_from_counts = [&](int& st, int& nm) {
+    const int first = (int)(seg_first - lane / tl);
+    int sum = 0;
+    for (int i0 = 0; i0 < first; i0 += 256) {
+      int c[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) { const int i = i0 + u * 32 + lane; c[u] = i < first ? __ldg(g.offsets + i) : 0; }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) sum += c[u];
+    }
+    nm = seg_first < batch ? __ldg(g.offsets + seg_first) : 0;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(FULL, sum, off);
+    int incl = nm;
+    for (int off = tl; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(FULL, incl, off);
+      if (lane >= off) incl += o;
+    }
+    st = sum + incl - nm;
+  };
   // one id, value and table row number per lane: position base + tlane of the segment
   auto load_ids = [&](int st, int nm, int base, int& row, float& v) {
     const int idx = base + tlane;
@@ -520,8 +547,13 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
 
   int st0, nm0, st1, nm1, st2, nm2, row, row_next;
   float v, v_next;
-  load_span(0, st0, nm0);
-  load_span(1, st1, nm1);
+  if (g.counts) {
+    span_from_counts(st0, nm0);
+    st1 = nm1 = 0;
+  } else {
+    load_span(0, st0, nm0);
+    load_span(1, st1, nm1);
+  }
   load_ids(st0, nm0, 0, row, v);
   for (int i = 0; i < segs; ++i) {
     const int64_t seg = seg_first + (int64_t)i * spw;
@@ -712,7 +744,7 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
 }
 
 // Sum / average pooling with one sub-team (LPR lanes) per segment and a per-warp segment queue: a warp
-// owns 32 consecutive segments, its 32/LPR sub-teams each take the next unclaimed one as soon as they
+// owns up to 32 consecutive segments, its 32/LPR sub-teams each take the next unclaimed one as soon as they
 // finish theirs, so lanes stay busy whatever the spread of segment lengths. A sub-team adds the ids of its
 // segment strictly in order (no cross-lane combine). The ids of the batch after the current one are
 // requested before the rows of the current one, so both latencies overlap.
@@ -741,8 +773,8 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
   const char* wrow = g.weights + tlane * 16;
   const int pitch = (int)g.pitch;
   const uint64_t keep = l2_policy_keep();
-  const int64_t s0 = (warp_id - g.warp_begin) * 32;
-  const int nseg = (int)min((int64_t)32, g.batch - s0);
+  const int64_t s0 = (warp_id - g.warp_begin) * g.segs;
+  const int nseg = (int)min((int64_t)g.segs, g.batch - s0);
 
   // lane l keeps the span of segment s0 + l
   int my_start = 0, my_num = 0;
@@ -1036,6 +1068,12 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
         (groups[i].n_items != 1 || groups[i].items[0].udf == XB_UDF_ASSIGN || (double)groups[i].n_ids >= 3.0 * (double)groups[i].batch))
       all_short = false;
   }
+  // Segments a warp of the queue kernel owns: 32 keep its sub-teams busy whatever the spread of lengths, fewer where the
+  // launch would otherwise not fill the chip with resident warps.
+  // 8 groups of 8192 segments of 15.5 ids (25 M x 32 fp16 table): 43 us at 32 a warp (0.43 of a wave), 33 at 8. 32 such
+  // groups: 89 us at 32 (1.7 waves), 100 at 16, so a launch that fills the chip keeps 32.
+  int queue_segs = 32;
+  while (queue_segs > 8 && call_segments / queue_segs < (int64_t)sm_count() * 32) queue_segs >>= 1;
   all_short = all_short && (call_segments + 31) / 32 >= (int64_t)sm_count() * 8;
   for (int i = 0; i < n_groups; ++i) {
     const xb_pool_group& h = groups[i];
@@ -1108,17 +1146,6 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
       d.items[k].assign_stride = it.udf == XB_UDF_ASSIGN ? it.assign_stride : 0;
       d.items[k].out = it.out; d.items[k].stride = it.stride;
     }
-    if (h.segments_are_offsets) {
-      d.offsets = h.segments;
-    } else {
-      int32_t* off = reinterpret_cast<int32_t*>((char*)scratch + soff);
-      soff += align256(((size_t)h.batch + 1) * 4);
-      sp.chunk_sums[sp.n] = reinterpret_cast<int32_t*>((char*)scratch + soff);
-      soff += align256(scan_chunks(h.batch) * 4);
-      sp.chunk_begin[sp.n + 1] = sp.chunk_begin[sp.n] + (int32_t)scan_chunks(h.batch);
-      sp.counts[sp.n] = h.segments; sp.offsets[sp.n] = off; sp.batch[sp.n] = h.batch; ++sp.n;
-      d.offsets = off;
-    }
     int lg = 0;
     while ((2 << lg) < d.lpr) ++lg;                 // lanes per row 2, 4, 8, 16 -> 0..3
     const int bucket = (d.tdtype == XB_F32 ? 0 : 4) + lg;
@@ -1135,12 +1162,33 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
     d.warp_begin = dst.total_warps;
     const int spw = 32 / d.tl;
     const int64_t rounds = (h.batch + spw - 1) / spw;
+    const bool counts_ok = fast && !short_ok && !queue_ok && !h.segments_are_offsets && h.batch <= POOL_INLINE_COUNTS;
+    if (counts_ok) {
+      d.offsets = h.segments;
+      d.counts = 1;
+    } else if (h.segments_are_offsets) {
+      d.offsets = h.segments;
+    } else {
+      int32_t* off = reinterpret_cast<int32_t*>((char*)scratch + soff);
+      soff += align256(((size_t)h.batch + 1) * 4);
+      sp.chunk_sums[sp.n] = reinterpret_cast<int32_t*>((char*)scratch + soff);
+      soff += align256(scan_chunks(h.batch) * 4);
+      sp.chunk_begin[sp.n + 1] = sp.chunk_begin[sp.n] + (int32_t)scan_chunks(h.batch);
+      sp.counts[sp.n] = h.segments; sp.offsets[sp.n] = off; sp.batch[sp.n] = h.batch; ++sp.n;
+      d.offsets = off;
+    }
     // the specialised kernel gives a warp several rounds, as long as every SM still gets dozens of warps
     d.segs = 1;
     if (fast) d.segs = (int)std::max<int64_t>(1, std::min<int64_t>(8, rounds / ((int64_t)sm_count() * 48)));
     // the short-segment kernel walks 8 rounds per warp (its prefetch needs a few), fewer only for small groups
     if (short_ok) d.segs = (int)std::max<int64_t>(1, std::min<int64_t>(8, rounds / ((int64_t)sm_count() * 16)));
-    dst.total_warps += queue_ok && !short_ok ? (h.batch + 31) / 32 : (rounds + d.segs - 1) / d.segs;
+    if (queue_ok && !short_ok) {
+      d.segs = queue_segs;
+      if (d.segs < spw) d.segs = spw;
+      dst.total_warps += (h.batch + d.segs - 1) / d.segs;
+    } else {
+      dst.total_warps += (rounds + d.segs - 1) / d.segs;
+    }
     dst.g[dst.n_groups++] = d;
   }
   if (sp.n) {
