@@ -80,3 +80,50 @@ def test_cuda_core_engine_tiles_and_layouts(ta, tb, P, M, N, K, dtype):
         want = 0.5 * (a @ b) + 2.0 * f(bias)[p]
         err = np.abs(f(Y)[p] - want)
         assert (err <= _bound(a, b, want, K, 2.0 ** -23)).all(), float(err.max())
+
+
+@pytest.mark.parametrize("P,M,N,K,dtype,out,epi", [
+    (1, 128 * 148, 256, 256, "bf16", "bf16", "prelu"),       # whole 256-row tiles, one column of them
+    (1, 9500, 512, 320, "f16", "f16", "sigmoid"),            # ragged rows: the second CTA of the last pair has 28 of 128
+    (2, 4890, 512, 1000, "f16", "f32", "dice"),              # the last pair's second CTA has no rows; ragged K; batches
+    (1, 2432, 2048, 384, "bf16", "f16", "none")])
+def test_two_cta_tiles(P, M, N, K, dtype, out, epi):
+    ops, capi = _ops()
+    rng = np.random.default_rng(M + N + K)
+    dt = dict(f16=torch.float16, bf16=torch.bfloat16, f32=torch.float32)
+    lda = (K + 7) // 8 * 8
+    t = lambda a, d: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).to("cuda", d)
+    A, W = t(rng.normal(0, 1, (P, M, lda)), dt[dtype]), t(rng.normal(0, 1, (P, N, lda)) / np.sqrt(K), dt[dtype])
+    W[:, :, K:] = 0
+    bias = t(rng.normal(0, 0.3, (P, N)), torch.float32)
+    Y = torch.full((P, M, N), 7.0, dtype=dt[out], device="cuda")
+    kw = {}
+    if epi == "prelu":
+        kw = dict(epilogue=capi.XB_EPI_PRELU, ep=(torch.full((1,), 0.25, device="cuda"), None, None), ep_count=1)
+    elif epi == "sigmoid":
+        kw = dict(epilogue=capi.XB_EPI_SIGMOID)
+    elif epi == "dice":
+        ep = [t(rng.uniform(0.1, 0.5, (P, N)), torch.float32) for _ in range(3)]
+        kw = dict(epilogue=capi.XB_EPI_DICE, ep=ep, stride_ep=N)
+    ops.gemm(A, W, Y=Y, bias=bias, trans_b=True, batch=P, M=M, N=N, K=K, lda=lda, ldb=lda, ldy=N,
+             strides=(M * lda, N * lda, N, M * N), bias_kind=capi.XB_BIAS_ROW, **kw)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    half_ulp = dict(f16=2.0 ** -11, bf16=2.0 ** -8, f32=2.0 ** -23)[out]
+    for p in range(P):
+        a, w = A[p, :, :K].double(), W[p, :, :K].double()
+        pre = a @ w.t() + bias[p].double()
+        want = pre
+        if epi == "prelu":
+            want = torch.where(pre < 0, pre * 0.25, pre)
+        elif epi == "sigmoid":
+            want = pre.sigmoid()
+        elif epi == "dice":
+            g, m, v = [e[p].double() for e in ep]
+            s = ((pre - m) / (v + 1e-8).sqrt()).sigmoid()
+            want = (1 - s) * g * pre + s * pre
+        # the activations' slopes are at most about 1 (sigmoid, PReLU) and 4 (Dice with var >= 0.1); __expf and the fast
+        # division add 2^-20 of the value
+        scale = a.abs() @ w.abs().t() + 1
+        tol = (half_ulp + 2.0 ** -20) * want.abs() + (4 if epi == "dice" else 1) * 2 * K * 2.0 ** -24 * scale
+        assert ((Y[p].double() - want).abs() <= tol).all(), float((Y[p].double() - want).abs().max())

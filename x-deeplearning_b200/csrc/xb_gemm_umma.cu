@@ -42,6 +42,7 @@ struct UmmaGemmParams {
   int M, N, K, block_n, tmem_cols, tiles_m, tiles_n, batch, stages;
   int b_resident;        // the B tile (all of K) stays in shared memory while consecutive tiles share it
   int b_mn;              // B is [K,N] row-major: the MMA reads N-major tiles of 64 columns x 64 k
+  int n_fast;            // consecutive tiles walk n first
   uint32_t tiles_per_cta;
   float alpha, beta;
   int a_batched, b_batched;
@@ -68,7 +69,9 @@ __device__ __forceinline__ void store_row16(TOut* dst, const float (&v)[16], int
 #pragma unroll
     for (int i = 0; i < 4; ++i) d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
   } else {
-    for (int i = 0; i < valid; ++i) dst[i] = from_f32<TOut>(v[i]);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (i < valid) dst[i] = from_f32<TOut>(v[i]);
   }
 }
 
@@ -232,6 +235,73 @@ __device__ __forceinline__ void epi_tile_fast(uint32_t tmem_row, int c_begin, in
   }
 }
 
+// bias and activation parameters of output column gn into entry e of the staged columns
+__device__ __forceinline__ void stage_columns(const UmmaGemmParams& p, int b, int gn, int e, float* s_bias, float* s_a, float* s_b,
+                                              float* s_c) {
+  const bool in = gn < p.N;
+  float bv = 0.f, pa = 0.f, pb = 0.f, pc = 0.f;
+  if (in && p.bias_kind == XB_BIAS_ROW) bv = p.beta * load_as_f32(p.bias, (int64_t)b * p.stride_bias + gn, p.bias_dtype);
+  if (in && p.epi.kind == XB_EPI_PRELU) pa = p.epi.a[(int64_t)b * p.stride_ep + (p.epi.count == 1 ? 0 : gn)];
+  if (in && p.epi.kind == XB_EPI_DICE) {
+    const float var = p.epi.c[(int64_t)b * p.stride_ep + gn];
+    pa = p.epi.a[(int64_t)b * p.stride_ep + gn];                            // gamma
+    pc = p.epi.nosqrt ? 1.f / var : rsqrtf(var + 1e-8f);                    // 1/std
+    pb = -p.epi.b[(int64_t)b * p.stride_ep + gn] * pc;                      // -mean/std
+  }
+  s_bias[e] = bv; s_a[e] = pa; s_b[e] = pb; s_c[e] = pc;
+}
+
+// Epilogue of any tile: checks rows and columns against the output, adds a full bias matrix where there is one.
+template <typename TOut>
+__device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t tmem_row, int c_begin, int c_end, const float* s_bias,
+                                              const float* s_a, const float* s_b, const float* s_c, TOut* yrow, int b, int gm,
+                                              int brow, int n0, bool vec_base) {
+  using namespace umma;
+  for (int cg = c_begin; cg < c_end; ++cg) {
+    uint32_t raw[16];
+    tmem_ld16_nowait(tmem_row + (uint32_t)(cg * 16), raw);
+    tmem_wait_ld(raw);
+    const int c = cg * 16, gn0 = n0 + c, valid = min(p.N - gn0, 16);
+    if (valid <= 0) continue;                                        // uniform across the warp
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = fmaf(p.alpha, __uint_as_float(raw[i]), s_bias[c + i]);
+    if (p.bias_kind == XB_BIAS_FULL && gm < p.M) {
+      const int64_t base = (int64_t)b * p.stride_bias + (int64_t)brow * p.ldbias + gn0;
+      const float* bf = reinterpret_cast<const float*>(p.bias) + base;
+      if (p.bias_dtype == XB_F32 && valid == 16 && (reinterpret_cast<uintptr_t>(bf) & 15) == 0) {
+        // fp32 rows (the per-group partial product of a pruned GEMM): four 16-byte loads, mostly one
+        // address per warp since consecutive output rows share the bias row
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 t = __ldg(reinterpret_cast<const float4*>(bf) + i);
+          v[4 * i] += p.beta * t.x; v[4 * i + 1] += p.beta * t.y;
+          v[4 * i + 2] += p.beta * t.z; v[4 * i + 3] += p.beta * t.w;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (i < valid) v[i] += p.beta * load_as_f32(p.bias, base + i, p.bias_dtype);
+      }
+    }
+    if (p.epi.kind == XB_EPI_PRELU) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = act_prelu(v[i], s_a[c + i]);
+    } else if (p.epi.kind == XB_EPI_DICE) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float g = s_a[c + i];
+        const float pr = __fdividef(1.f, 1.f + __expf(-fmaf(v[i], s_c[c + i], s_b[c + i])));
+        v[i] = v[i] * fmaf(pr, 1.f - g, g);
+      }
+    } else if (p.epi.kind == XB_EPI_SIGMOID) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[i] = act_sigmoid(v[i]);
+    }
+    if (gm < p.M) store_row16<TOut>(yrow + gn0, v, valid, vec_base && ((gn0 * sizeof(TOut)) % 16 == 0));
+  }
+}
+
 template <typename TOut>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -256,6 +326,14 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const uint32_t tiles_mn = (uint32_t)p.tiles_m * (uint32_t)p.tiles_n;
   const uint32_t total_tiles = tiles_mn * (uint32_t)p.batch;
   const uint32_t acc_stride = (uint32_t)p.tmem_cols / 2;
+  // A tile's place: m fastest, or (n_fast, rings only) n fastest, so that the n tiles of one row of tiles run at the same
+  // time and its A rows come from HBM once.
+  auto place = [&](uint32_t tile, int& b, int& m0, int& n0) {
+    b = (int)(tile / tiles_mn);
+    const uint32_t rem = tile - (uint32_t)b * tiles_mn, inner = (uint32_t)(p.n_fast ? p.tiles_n : p.tiles_m), o = rem / inner, i = rem - o * inner;
+    m0 = (int)(p.n_fast ? o : i) * BLOCK_M;
+    n0 = (int)(p.n_fast ? i : o) * p.block_n;
+  };
   // Tile sequence of this CTA, the same for every role. With a resident B tile each CTA takes a contiguous
   // run (m fastest), so that B changes once or twice per CTA; otherwise CTAs interleave, so that the CTAs
   // running at the same time read the same B tile from L2.
@@ -296,9 +374,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       int cur_n0 = -1, cur_b = -1;
       bool ok = true;
       for (uint32_t tile = tile_first; tile < tile_end && ok; tile += tile_step) {
-        const int b = (int)(tile / tiles_mn);
-        const uint32_t rem = tile - (uint32_t)b * tiles_mn, nt = rem / (uint32_t)p.tiles_m;
-        const int m0 = (int)(rem - nt * (uint32_t)p.tiles_m) * BLOCK_M, n0 = (int)nt * p.block_n;
+        int b, m0, n0;
+        place(tile, b, m0, n0);
         if (bres && (n0 != cur_n0 || b != cur_b)) {
           cur_n0 = n0; cur_b = b;
           // the MMAs that read the previous B tile have completed (signalled after the last tile that used it)
@@ -386,9 +463,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // global memory or the acc_empty barrier: the other epilogue warps may have passed the same wait (each
     // lane keeps its own clock), and they still need this warp at the two named barriers below.
     for (uint32_t tile = tile_first; tile < tile_end; tile += tile_step, ++it) {
-      const int b = (int)(tile / tiles_mn);
-      const uint32_t rem = tile - (uint32_t)b * tiles_mn, nt = rem / (uint32_t)p.tiles_m;
-      const int m0 = (int)(rem - nt * (uint32_t)p.tiles_m) * BLOCK_M, n0 = (int)nt * p.block_n;
+      int b, m0, n0;
+      place(tile, b, m0, n0);
       const int as = it & 1;
       const int gm = m0 + row;
       const int brow = p.bias_group > 1 ? (int)((uint32_t)gm / (uint32_t)p.bias_group) : gm;   // bias row of this output row
@@ -396,19 +472,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         cur_n0 = n0; cur_b = b;
         asm volatile("bar.sync 2, 512;" ::: "memory");                  // everyone is done with the old columns
         const int e = ew * 32 + lane, gn = n0 + e;
-        if (e < p.block_n) {
-          const bool in = gn < p.N;
-          float bv = 0.f, pa = 0.f, pb = 0.f, pc = 0.f;
-          if (in && p.bias_kind == XB_BIAS_ROW) bv = p.beta * load_as_f32(p.bias, (int64_t)b * p.stride_bias + gn, p.bias_dtype);
-          if (in && p.epi.kind == XB_EPI_PRELU) pa = p.epi.a[(int64_t)b * p.stride_ep + (p.epi.count == 1 ? 0 : gn)];
-          if (in && p.epi.kind == XB_EPI_DICE) {
-            const float var = p.epi.c[(int64_t)b * p.stride_ep + gn];
-            pa = p.epi.a[(int64_t)b * p.stride_ep + gn];                            // gamma
-            pc = p.epi.nosqrt ? 1.f / var : rsqrtf(var + 1e-8f);                    // 1/std
-            pb = -p.epi.b[(int64_t)b * p.stride_ep + gn] * pc;                      // -mean/std
-          }
-          s_bias[e] = bv; s_a[e] = pa; s_b[e] = pb; s_c[e] = pc;
-        }
+        if (e < p.block_n) stage_columns(p, b, gn, e, s_bias, s_a, s_b, s_c);
         asm volatile("bar.sync 2, 512;" ::: "memory");
       }
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&acc_full[as]), (uint32_t)(it >> 1) & 1u, 3));
@@ -434,54 +498,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         if (lane == 0) mbar_arrive(smem_u32(&acc_empty[as]));
         continue;
       }
-      for (int cg = c_begin; cg < c_end; ++cg) {
-        uint32_t raw[1][16];
-        tmem_ld16_nowait(tmem_acc + (uint32_t)(cg * 16), raw[0]);
-        tmem_wait_ld(raw[0]);
-        for (int u = 0; u < 1; ++u) {
-          const int c = (cg + u) * 16;
-          const int gn0 = n0 + c;
-          int valid = p.N - gn0;
-          valid = valid > 16 ? 16 : valid;
-          if (cg + u >= c_end || valid <= 0) continue;                   // uniform across the warp
-          float v[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = fmaf(p.alpha, __uint_as_float(raw[u][i]), s_bias[c + i]);
-          if (p.bias_kind == XB_BIAS_FULL && gm < p.M) {
-            const int64_t base = (int64_t)b * p.stride_bias + (int64_t)brow * p.ldbias + gn0;
-            const float* bf = reinterpret_cast<const float*>(p.bias) + base;
-            if (p.bias_dtype == XB_F32 && valid == 16 && (reinterpret_cast<uintptr_t>(bf) & 15) == 0) {
-              // fp32 rows (the per-group partial product of a pruned GEMM): four 16-byte loads, mostly one
-              // address per warp since consecutive output rows share the bias row
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float4 t = __ldg(reinterpret_cast<const float4*>(bf) + i);
-                v[4 * i] += p.beta * t.x; v[4 * i + 1] += p.beta * t.y;
-                v[4 * i + 2] += p.beta * t.z; v[4 * i + 3] += p.beta * t.w;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 16; ++i)
-                if (i < valid) v[i] += p.beta * load_as_f32(p.bias, base + i, p.bias_dtype);
-            }
-          }
-          if (p.epi.kind == XB_EPI_PRELU) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = act_prelu(v[i], s_a[c + i]);
-          } else if (p.epi.kind == XB_EPI_DICE) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float g = s_a[c + i];
-              const float pr = __fdividef(1.f, 1.f + __expf(-fmaf(v[i], s_c[c + i], s_b[c + i])));
-              v[i] = v[i] * fmaf(pr, 1.f - g, g);
-            }
-          } else if (p.epi.kind == XB_EPI_SIGMOID) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = act_sigmoid(v[i]);
-          }
-          if (gm < p.M) store_row16<TOut>(yrow + gn0, v, valid, vec_base && ((gn0 * sizeof(TOut)) % 16 == 0));
-        }
-      }
+      epi_tile_edge<TOut>(p, tmem_acc, c_begin, c_end, s_bias, s_a, s_b, s_c, yrow, b, gm, brow, n0, vec_base);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&acc_empty[as]));              // one arrival per epilogue warp
@@ -556,8 +573,7 @@ int launch_umma(const CUtensorMap& ma, const CUtensorMap& mb, const UmmaGemmPara
   return check_launch("gemm_umma_kernel");
 }
 
-int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
-  UmmaGemmParams p;
+void fill_umma_params(UmmaGemmParams& p, const xb_gemm_args& a) {
   memset(&p, 0, sizeof(p));
   p.M = a.M; p.N = a.N; p.K = a.K;
   p.block_n = pick_block_n(a.N);
@@ -571,17 +587,66 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   p.Y = a.Y; p.ldy = a.ldy; p.stride_y = a.stride_y; p.y_dtype = a.y_dtype;
   p.epi.kind = a.epilogue; p.epi.a = a.ep_a; p.epi.b = a.ep_b; p.epi.c = a.ep_c;
   p.epi.count = a.ep_count; p.epi.nosqrt = a.dice_nosqrt; p.stride_ep = a.stride_ep;
-  const int is_bf16 = a.ab_dtype == XB_BF16;
+  p.batch = a.batch;
   p.b_mn = !a.trans_b;
-  p.idesc = umma::make_idesc(BLOCK_M, p.block_n, is_bf16) | (p.b_mn ? umma::IDESC_B_MN : 0u);
+  p.idesc = umma::make_idesc(BLOCK_M, p.block_n, a.ab_dtype == XB_BF16) | (p.b_mn ? umma::IDESC_B_MN : 0u);
+}
+
+// Two-CTA tiles where they fill the chip (a 256 x 256 tile for every pair of SMs) and the epilogue is the plain one: whole
+// 256-column tiles, aligned output rows, no bias matrix. Below that the one-CTA kernel spreads the work over more SMs.
+// [65536, 1280] x [1280, 1024] and the two layers after it (bf16): 207 us as pairs, 290 one CTA at a time.
+bool pair_wanted(const xb_gemm_args& a) {
+  const int64_t es = a.y_dtype == XB_F32 ? 4 : 2;
+  return a.trans_b && a.N % 256 == 0 && a.K >= 256 && !(a.bias && a.bias_kind == XB_BIAS_FULL) &&
+         (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0 && (a.ldy * es) % 16 == 0 && (a.stride_y * es) % 16 == 0 &&
+         ((int64_t)a.M + 255) / 256 * (a.N / 256) * a.batch >= sm_count() / 2;
+}
+
+}  // namespace
+}  // namespace xb
+
+#include "xb_gemm_umma_pair.cuh"
+
+namespace xb {
+namespace {
+
+template <typename TOut>
+int launch_umma_pair(const CUtensorMap& ma, const CUtensorMap& mb, const UmmaGemmParams& p, dim3 grid, size_t smem, cudaStream_t s) {
+  static PerDeviceOnce attr_set;   // per instantiation
+  XB_SET_MAX_SMEM_ONCE(attr_set, 226 * 1024, (const void*)gemm_umma_pair_kernel<TOut>);
+  gemm_umma_pair_kernel<TOut><<<grid, GEMM_THREADS, smem, s>>>(ma, mb, p);
+  return check_launch("gemm_umma_pair_kernel");
+}
+
+int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
+  UmmaGemmParams p;
+  fill_umma_params(p, a);
+  const int is_bf16 = a.ab_dtype == XB_BF16;
   CUtensorMap ma, mb;
   if (int rc = make_map(&ma, a.A, is_bf16, a.K, a.M, a.lda, p.a_batched ? a.batch : 1, a.stride_a, BLOCK_M)) return rc;
+  // after the ring: per-column epilogue parameters [4][256] fp32, then the epilogue warps' staging areas
+  const int tail = 4 * 256 * (int)sizeof(float) + (a.y_dtype == XB_F32 ? 0 : EPI_WARPS * EPI_STAGE_BYTES);
+  if (pair_wanted(a)) {
+    if (int rc = make_map(&mb, a.B, is_bf16, a.K, a.N, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, PAIR_N / 2)) return rc;
+    p.tiles_m = (a.M + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
+    p.tiles_n = a.N / PAIR_N;
+    p.idesc = umma::make_idesc(2 * BLOCK_M, PAIR_N, is_bf16);
+    p.stages = std::min(PAIR_MAX_STAGES, (225 * 1024 - tail) / PAIR_STAGE_BYTES);
+    const size_t smem = (size_t)p.stages * PAIR_STAGE_BYTES + tail + 1024;
+    const int64_t total = (int64_t)p.tiles_m * p.tiles_n * p.batch;
+    XB_REQUIRE(total < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)total);
+    const dim3 grid(2 * (unsigned)std::min<int64_t>(total, sm_count() / 2));
+    switch (a.y_dtype) {
+      case XB_F16: return launch_umma_pair<__half>(ma, mb, p, grid, smem, stream);
+      case XB_BF16: return launch_umma_pair<__nv_bfloat16>(ma, mb, p, grid, smem, stream);
+      default: return launch_umma_pair<float>(ma, mb, p, grid, smem, stream);
+    }
+  }
   if (int rc = p.b_mn ? make_map(&mb, a.B, is_bf16, a.N, a.K, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, BLOCK_K)
                       : make_map(&mb, a.B, is_bf16, a.K, a.N, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, p.block_n))
     return rc;
   p.tiles_m = (a.M + BLOCK_M - 1) / BLOCK_M;
   p.tiles_n = (a.N + p.block_n - 1) / p.block_n;
-  p.batch = a.batch;
   const int64_t total = (int64_t)p.tiles_m * p.tiles_n * p.batch;
   XB_REQUIRE(total < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)total);
   // persistent: one CTA per SM walks the tiles; the accumulator is double-buffered in TMEM so the
@@ -595,8 +660,11 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   const int grid_ctas = (int)std::min<int64_t>(total, sm_count());
   p.tiles_per_cta = (uint32_t)((total + grid_ctas - 1) / grid_ctas);
   p.b_resident = (int64_t)num_kb * b_stage_bytes <= 96 * 1024 && p.tiles_m >= 4 && p.tiles_per_cta >= 2;
-  // after the ring: per-column epilogue parameters [4][256] fp32, then the epilogue warps' staging areas
-  const int tail = 4 * 256 * (int)sizeof(float) + (a.y_dtype == XB_F32 ? 0 : EPI_WARPS * EPI_STAGE_BYTES);
+  // n first where the CTAs that run together then share A rows instead of fetching them again for every n tile (the whole
+  // weight matrix stays in L2 either way at the sizes of a dense tower); m first where A fits L2 itself, since a CTA then
+  // keeps its columns and stages their parameters once. (A of the 65536-row tower's first
+  // layer is 168 MB and was read four times.)
+  p.n_fast = !p.b_resident && p.tiles_n > 1 && (int64_t)a.M * a.K * 2 > (32 << 20) && (int64_t)a.N * a.K * 2 <= (32 << 20);
   size_t smem;
   if (p.b_resident) {
     const int b_bytes = num_kb * b_stage_bytes;
