@@ -22,6 +22,74 @@ const std::vector<size_t> kEmptyShape;
 }  // namespace
 
 // ---- impl classes ---------------------------------------------------------------------------------
+// Small feeds on their way to the device. A request is some dozens of arrays of a few KB; a cudaMemcpyAsync for each costs
+// the host more than the bytes do. So Feed copies a small array into pinned memory that the device can read (the caller's
+// buffer is free as soon as Feed returns) and one kernel brings all of them over, enqueued before anything that could see
+// the inputs. 36 arrays of a request: 7 us on the device instead of 63, and the call 110 us shorter.
+class FeedStage {
+ public:
+  static constexpr size_t kMaxFeed = 32 << 10;       // longer arrays: the copy engine is as cheap as the host's memcpy
+  FeedStage() = default;
+  FeedStage(const FeedStage&) = delete;
+  ~FeedStage() {
+    if (in_flight_) cudaDeviceSynchronize();          // (as blobs do before they give their memory back)
+    if (host_) cudaFreeHost(host_);
+  }
+
+  bool pending(const Blob* b) const {
+    for (const Item& i : items_)
+      if (i.blob == b) return true;
+    return false;
+  }
+  // a later feed of the same blob replaces the one that waits
+  void Drop(const Blob* b) {
+    for (size_t i = 0; i < items_.size(); ++i)
+      if (items_[i].blob == b) { items_.erase(items_.begin() + (long)i); return; }
+  }
+  void Add(Blob* b, const void* data, size_t len, cudaStream_t stream) {
+    if (!host_) {
+      CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&host_), kBytes, cudaHostAllocMapped | cudaHostAllocPortable));
+      CUDA_CHECK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&dev_), host_, 0));
+    }
+    Drop(b);
+    if (items_.size() == kMaxItems || used_ + len > kBytes) Flush(stream);
+    if (in_flight_) {                                 // what the last kernel read may still be on its way
+      CUDA_CHECK(cudaStreamSynchronize(stream));
+      Done();
+    }
+    memcpy(host_ + used_, data, len);
+    items_.push_back(Item{b, used_, len});
+    used_ = (used_ + len + 15) / 16 * 16;
+  }
+  // enqueues the copies that wait
+  void Flush(cudaStream_t stream) {
+    if (items_.empty()) return;
+    xb_copy_item* d = reinterpret_cast<xb_copy_item*>(host_);
+    size_t longest = 0;
+    for (size_t i = 0; i < items_.size(); ++i) {
+      d[i].src = dev_ + items_[i].at; d[i].dst = items_[i].blob->as<void>(); d[i].bytes = (int64_t)items_[i].len;
+      longest = std::max(longest, items_[i].len);
+    }
+    const int n = (int)items_.size();
+    items_.clear();
+    in_flight_ = true;
+    XB_CHECK(xb_copy_segments(reinterpret_cast<const xb_copy_item*>(dev_), n, (int64_t)longest, stream));
+  }
+  // the stream has been synchronised since the last Flush
+  void Done() {
+    if (items_.empty()) used_ = kMaxItems * sizeof(xb_copy_item);
+    in_flight_ = false;
+  }
+
+ private:
+  struct Item { Blob* blob; size_t at, len; };
+  static constexpr size_t kMaxItems = 128, kBytes = 512 << 10;
+  char *host_ = nullptr, *dev_ = nullptr;            // [descriptors][arrays]
+  size_t used_ = kMaxItems * sizeof(xb_copy_item);
+  std::vector<Item> items_;
+  bool in_flight_ = false;
+};
+
 class PredictorImpl {
  public:
   PredictorImpl(const NetDef& def, std::shared_ptr<store::SparsePuller> puller, std::shared_ptr<ConstantStore> constants) {
@@ -45,6 +113,7 @@ class PredictorImpl {
   std::unordered_map<std::string, int> in_types_;
   std::unordered_map<std::string, ValueInfo> feed_cfg_;
   std::vector<char> staging_;
+  FeedStage feeds_;
   std::vector<size_t> scratch_shape_;
   bool profile_ = false;
   // request batching (InitScheduler(enable_batching = true)): the queue of this model and device, and
@@ -178,6 +247,10 @@ FeedNameConfig Predictor::GetFeedNameConfig(const std::string& feed_name) {
 bool Predictor::ReshapeInput(const char* name, const std::vector<size_t>& shape) {
   try {
     Blob* b = impl_->InputBlob(name);
+    if (impl_->feeds_.pending(b)) {                  // fed at its old shape
+      CUDA_CHECK(cudaSetDevice(impl_->net_->device_id()));
+      impl_->feeds_.Flush(impl_->net_->stream());
+    }
     b->set_data_type(impl_->in_types_[name]);
     b->Reshape(shape);
     return true;
@@ -194,6 +267,11 @@ bool Predictor::Feed(const char* name, const void* data, size_t len) {
     BLAZE_CONDITION_THROW(len == b->bytes(), "feed of ", name, ": len=", len, " blob bytes=", b->bytes());
     if (len == 0) return true;
     CUDA_CHECK(cudaSetDevice(impl_->net_->device_id()));
+    if (len <= FeedStage::kMaxFeed) {
+      impl_->feeds_.Add(b, data, len, impl_->net_->stream());
+      return true;
+    }
+    impl_->feeds_.Drop(b);
     CUDA_CHECK(cudaMemcpyAsync(b->as<void>(), data, len, cudaMemcpyHostToDevice, impl_->net_->stream()));
     return true;
   } catch (const std::exception& e) { SetError(e.what()); return false; }
@@ -217,6 +295,7 @@ bool Predictor::Forward(const PredictorCallback&& cb) {
   try {
     CUDA_CHECK(cudaSetDevice(impl_->net_->device_id()));
     impl_->async_error_.clear();
+    impl_->feeds_.Flush(impl_->net_->stream());
     if (cb && impl_->queue_) {
       // asynchronous: the batch thread stacks this request with others of the same model, runs them
       // as one net and calls cb once this predictor's outputs are in place
@@ -243,6 +322,7 @@ bool Predictor::Forward(const PredictorCallback&& cb) {
     impl_->net_->profile = impl_->profile_;
     if (!impl_->net_->Run()) return false;
     CUDA_CHECK(cudaStreamSynchronize(impl_->net_->stream()));
+    impl_->feeds_.Done();
     impl_->net_->CheckDeviceStatus();
     if (cb) cb();
     return true;
@@ -257,6 +337,10 @@ bool Predictor::Output(const char* name, void** data, size_t* len) {
     BLAZE_CONDITION_THROW(impl_->async_error_.empty(), impl_->async_error_);
     Blob* b = impl_->ws_.GetBlob(name);
     BLAZE_CONDITION_THROW(b != nullptr, "output ", name, " does not exist");
+    if (impl_->feeds_.pending(b)) {
+      CUDA_CHECK(cudaSetDevice(impl_->net_->device_id()));
+      impl_->feeds_.Flush(impl_->net_->stream());
+    }
     impl_->staging_.resize(std::max<size_t>(b->bytes(), 1));
     if (b->bytes()) {
       CUDA_CHECK(cudaMemcpyAsync(impl_->staging_.data(), b->as<void>(), b->bytes(), cudaMemcpyDeviceToHost, impl_->net_->stream()));
@@ -542,6 +626,7 @@ int Blaze_B200_PredictorFeedDevice(PredictorHandle h, const char* name, const vo
   PredictorImpl* impl = PredictorManagerImpl::ImplOf(static_cast<CPredictor*>(h)->p);
   Blob* b = impl->InputBlob(name);
   BLAZE_CONDITION_THROW(len == b->bytes(), "feed of ", name, ": len=", len, " blob bytes=", b->bytes());
+  impl->feeds_.Drop(b);
   if (len) CUDA_CHECK(cudaMemcpyAsync(b->as<void>(), device_data, len, cudaMemcpyDeviceToDevice, impl->net_->stream()));
   API_END();
 }
@@ -550,6 +635,10 @@ int Blaze_B200_PredictorOutputDevice(PredictorHandle h, const char* name, void**
   PredictorImpl* impl = PredictorManagerImpl::ImplOf(static_cast<CPredictor*>(h)->p);
   Blob* b = impl->ws_.GetBlob(name);
   BLAZE_CONDITION_THROW(b != nullptr, "output ", name, " does not exist");
+  if (impl->feeds_.pending(b)) {
+    CUDA_CHECK(cudaSetDevice(impl->net_->device_id()));
+    impl->feeds_.Flush(impl->net_->stream());
+  }
   *device_data = b->as<void>();
   *len = b->bytes();
   API_END();
