@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(AU_THREADS, H <= 40 ? 2 : 1) augru_tc_kernel(c
   __half* atts = reinterpret_cast<__half*>(smem + G.o_att);
   __half* xs = reinterpret_cast<__half*>(smem + G.o_x);
   const __half zero = __float2half(0.f);
+  pdl_begin();
 
   // ---- prologue -------------------------------------------------------------------------------------------
   // attention scores of the tile and the request's input sequence: asynchronous copies where alignment allows
@@ -375,7 +376,7 @@ template <int H>
 int launch_augru_tc_h(const AuParams& p, unsigned blocks, int smem, cudaStream_t stream) {
   static PerDeviceOnce attr;                          // per instantiation
   XB_SET_MAX_SMEM_ONCE(attr, 200 * 1024, (const void*)augru_tc_kernel<H>);
-  augru_tc_kernel<H><<<blocks, AU_THREADS, smem, stream>>>(p);
+  launch_dependent(augru_tc_kernel<H>, blocks, AU_THREADS, smem, stream, p);
   return check_launch("augru_tc_kernel");
 }
 

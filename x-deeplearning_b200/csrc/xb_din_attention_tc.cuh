@@ -260,6 +260,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
   const int ctile = blockIdx.x / split;                                      // the cluster is `split` CTAs along x
   const int r = ctile / p.tiles_per_req, tile = ctile % p.tiles_per_req;
   const int d = d_, dp = G.dp, nch = G.nch, k1 = G.k1, h0p = G.h0p, k2 = G.k2, h1p = G.h1p, tp = G.tp, np = G.np;
+  pdl_begin();
   int tl = p.seq_len ? p.seq_len[r] : p.T;
   tl = tl < 0 ? 0 : (tl > p.T ? p.T : tl);
 
@@ -870,12 +871,14 @@ int launch_att_tc(AttParams& p, const xb_din_att_args& a, cudaStream_t stream) {
   XB_REQUIRE(tiles < ((int64_t)1 << 28), XB_ERR_LIMIT, "xb_din_attention: too many tiles");
   p.split = a.use_softmax ? 1 : pick_split(tiles, p.T);        // the softmax needs all scores of a row in one place
   const TcSmemLayout L = tc_layout(g, p.T);
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)p.split; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;         // as launch_dependent
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)p.split; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(tiles * p.split)); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = (size_t)L.total;
-  cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = p.split > 1 ? 1 : 0;
+  cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = p.split > 1 ? 2 : 1;
   // the shape of the DIN / DIEN attention unit (d = 36, MLP 144-80-40-1) has instantiations of its own
   const bool din_shape = a.d == 36 && a.h0 == 80 && a.h1 == 40;
   cudaError_t e;

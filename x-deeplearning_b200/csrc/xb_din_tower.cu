@@ -160,6 +160,7 @@ __global__ void tower_pack_kernel(const __grid_constant__ TowerParams p, uint8_t
 // at once and only then waits for any (at du + d = 180 and T = 100 that is everything). One request: 5.8 us, 8.2 before
 constexpr int PT_COLS = 64, PT_SLICES = 8, PT_W = 24, PT_T = 16;
 __global__ void __launch_bounds__(PT_COLS * PT_SLICES) din_tower_partial_kernel(const __grid_constant__ TowerParams p) {
+  pdl_begin();
   extern __shared__ float sm[];            // [d] his_sum, [du] user row, [G][d] step sums, [PT_SLICES][PT_COLS]
   const int r = blockIdx.x, d = p.d, du = p.du;
   float* hs = sm;
@@ -234,7 +235,8 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
   const int d = p.d, dp = G.dp, nch = G.nch, n1p = G.n1p, n2p = G.n2p, n3 = p.n3;
   const int64_t total_tiles = (int64_t)p.requests * p.tiles_per_req;
 
-  // weight image: asynchronous 16-byte copies, all in flight at once
+  // weight image: asynchronous 16-byte copies, all in flight at once. Requested before pdl_begin: the kernel before is
+  // din_tower_partial_kernel, which has passed its own pdl_begin, so whatever wrote the image has completed.
   {
     for (int i = threadIdx.x; i < G.image_bytes / 16; i += TW_THREADS) cp_async16(smem + 16 * i, p.packed + 16 * i);
     cp_async_commit();
@@ -259,6 +261,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem0 = tmem_base_s;
+  pdl_begin();
 
   if (warp == TW_MMA_WARP) {
     // the whole warp runs the issue loop in uniform control flow and one elected lane issues: the descriptors
@@ -591,13 +594,18 @@ extern "C" int xb_din_tower(const xb_din_tower_args* a, void* workspace, size_t 
   p.idesc1 = umma::make_idesc(128, g.n1p, 0);
   p.idesc2 = umma::make_idesc(128, g.n2p, 0);
   XB_REQUIRE(a->requests <= 65535 * 32, XB_ERR_LIMIT, "xb_din_tower: too many requests per call");
-  din_tower_partial_kernel<<<dim3(a->requests, (a->n1 + PT_COLS - 1) / PT_COLS), PT_COLS * PT_SLICES,
-                             sizeof(float) * (9 * a->d + a->du + PT_COLS * PT_SLICES + 2), stream>>>(p);
+  const int64_t tiles = (int64_t)a->requests * p.tiles_per_req;
+  const dim3 pgrid(a->requests, (a->n1 + PT_COLS - 1) / PT_COLS);
+  const size_t psmem = sizeof(float) * (9 * a->d + a->du + PT_COLS * PT_SLICES + 2);
+  // A large call's kernels start on a chip that the one before has left: with every link of pooling -> attention -> partial ->
+  // tower -> next pooling made early, the attention's tiles spread unevenly over the SMs and some walk a fifth one of four
+  // (74 requests of 1000: 393 us a pass, 348 with this link plain, 357 with none early).
+  if (tiles <= sm_count()) launch_dependent(din_tower_partial_kernel, pgrid, PT_COLS * PT_SLICES, psmem, stream, p);
+  else din_tower_partial_kernel<<<pgrid, PT_COLS * PT_SLICES, psmem, stream>>>(p);
   if (int rc = check_launch("din_tower_partial_kernel")) return rc;
   static PerDeviceOnce attr_set;
   XB_SET_MAX_SMEM_ONCE(attr_set, 220 * 1024, (const void*)din_tower_tc_kernel);
-  const int64_t tiles = (int64_t)a->requests * p.tiles_per_req;
   const int grid = (int)std::min<int64_t>(tiles, sm_count());
-  din_tower_tc_kernel<<<grid, TW_THREADS, g.total, stream>>>(p);
+  launch_dependent(din_tower_tc_kernel, grid, TW_THREADS, g.total, stream, p);
   return check_launch("din_tower_tc_kernel");
 }

@@ -96,6 +96,7 @@ struct SimtSlice {
 
 template <int TM, int TN>
 __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(const __grid_constant__ SimtGemmParams p) {
+  pdl_begin();
   constexpr int BM = 16 * TM, BN = 16 * TN;
   using SliceA = SimtSlice<BM>;
   using SliceB = SimtSlice<BN>;
@@ -187,13 +188,13 @@ __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(c
 template <int TM>
 static void launch_simt_tm(const SimtGemmParams& p, int tn, dim3 grid, cudaStream_t s) {
   switch (tn) {
-    case 1: gemm_simt_kernel<TM, 1><<<grid, 256, 0, s>>>(p); break;
-    case 2: gemm_simt_kernel<TM, 2><<<grid, 256, 0, s>>>(p); break;
-    case 3: gemm_simt_kernel<TM, 3><<<grid, 256, 0, s>>>(p); break;
-    case 4: gemm_simt_kernel<TM, 4><<<grid, 256, 0, s>>>(p); break;
-    case 5: gemm_simt_kernel<TM, 5><<<grid, 256, 0, s>>>(p); break;
-    case 6: gemm_simt_kernel<TM, 6><<<grid, 256, 0, s>>>(p); break;
-    default: gemm_simt_kernel<TM, 8><<<grid, 256, 0, s>>>(p); break;
+    case 1: launch_dependent(gemm_simt_kernel<TM, 1>, grid, 256, 0, s, p); break;
+    case 2: launch_dependent(gemm_simt_kernel<TM, 2>, grid, 256, 0, s, p); break;
+    case 3: launch_dependent(gemm_simt_kernel<TM, 3>, grid, 256, 0, s, p); break;
+    case 4: launch_dependent(gemm_simt_kernel<TM, 4>, grid, 256, 0, s, p); break;
+    case 5: launch_dependent(gemm_simt_kernel<TM, 5>, grid, 256, 0, s, p); break;
+    case 6: launch_dependent(gemm_simt_kernel<TM, 6>, grid, 256, 0, s, p); break;
+    default: launch_dependent(gemm_simt_kernel<TM, 8>, grid, 256, 0, s, p); break;
   }
 }
 

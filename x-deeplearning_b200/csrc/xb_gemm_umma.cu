@@ -357,6 +357,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
+  pdl_begin();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -577,7 +578,7 @@ int launch_umma(const CUtensorMap& ma, const CUtensorMap& mb, const UmmaGemmPara
                 cudaStream_t s) {
   static PerDeviceOnce attr_set;   // per instantiation
   XB_SET_MAX_SMEM_ONCE(attr_set, SMEM_BUDGET + 6 * 1024, (const void*)gemm_umma_kernel<TOut>);
-  gemm_umma_kernel<TOut><<<grid, GEMM_THREADS, smem, s>>>(ma, mb, p);
+  launch_dependent(gemm_umma_kernel<TOut>, grid, GEMM_THREADS, smem, s, ma, mb, p);
   return check_launch("gemm_umma_kernel");
 }
 
@@ -622,7 +623,7 @@ template <typename TOut>
 int launch_umma_pair(const CUtensorMap& ma, const CUtensorMap& mb, const UmmaGemmParams& p, dim3 grid, size_t smem, cudaStream_t s) {
   static PerDeviceOnce attr_set;   // per instantiation
   XB_SET_MAX_SMEM_ONCE(attr_set, 226 * 1024, (const void*)gemm_umma_pair_kernel<TOut>);
-  gemm_umma_pair_kernel<TOut><<<grid, GEMM_THREADS, smem, s>>>(ma, mb, p);
+  launch_dependent(gemm_umma_pair_kernel<TOut>, grid, GEMM_THREADS, smem, s, ma, mb, p);
   return check_launch("gemm_umma_pair_kernel");
 }
 

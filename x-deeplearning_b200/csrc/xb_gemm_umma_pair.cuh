@@ -86,6 +86,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   cluster_sync();                                                  // the other CTA's barriers are initialised too
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
+  pdl_begin();
 
   if (warp == 0) {
     if (lane == 0) {

@@ -41,6 +41,7 @@ static inline unsigned stream_grid(int64_t work_items, int per_block) {
 
 __global__ void dice_kernel(const void* x, void* y, int64_t size, int c, const void* gamma,
                             const void* mean, const void* var, int nosqrt, int dt) {
+  pdl_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (int64_t)gridDim.x * blockDim.x) {
     int col = (int)(i % c);
     float v = load_as_f32(x, i, dt);
@@ -51,17 +52,20 @@ __global__ void dice_kernel(const void* x, void* y, int64_t size, int c, const v
 }
 
 __global__ void prelu_kernel(const void* x, void* y, int64_t size, const void* w, int64_t inner, int dt, int wdt) {
+  pdl_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (int64_t)gridDim.x * blockDim.x)
     store_from_f32(y, i, dt, act_prelu(load_as_f32(x, i, dt), load_as_f32(w, i % inner, wdt)));
 }
 
 __global__ void sigmoid_kernel(const void* x, void* y, int64_t size, int dt) {
+  pdl_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (int64_t)gridDim.x * blockDim.x)
     store_from_f32(y, i, dt, act_sigmoid(load_as_f32(x, i, dt)));
 }
 
 __global__ void batchnorm_kernel(const void* x, void* y, int64_t size, int c, const void* gamma, const void* beta,
                                  const void* mean, const void* var, float eps, int nosqrt, int dt) {
+  pdl_begin();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (int64_t)gridDim.x * blockDim.x) {
     int col = (int)(i % c);
     float vr = load_as_f32(var, col, dt);
@@ -72,6 +76,7 @@ __global__ void batchnorm_kernel(const void* x, void* y, int64_t size, int c, co
 
 // one thread per (outer, inner) pair walks the c axis three times (max, sum, divide)
 __global__ void softmax_kernel(const void* x, void* y, int64_t n, int c, int64_t w, int dt) {
+  pdl_begin();
   const int64_t total = n * w;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t base = (i / w) * c * w + (i % w);
@@ -89,6 +94,7 @@ __global__ void softmax_kernel(const void* x, void* y, int64_t n, int c, int64_t
 // touches 32 rows with every load).
 template <int PER>
 __global__ void __launch_bounds__(256) softmax_rows_kernel(const void* x, void* y, int64_t n, int c, int dt) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * 8;
   for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < n; r += warps) {
@@ -140,6 +146,7 @@ __device__ __forceinline__ float ew_apply(int op, float av, float bv) {
 }
 
 __global__ void elementwise_kernel(const __grid_constant__ EwParams p) {
+  pdl_begin();
   const int64_t total = p.shape[0] * p.shape[1] * p.shape[2] * p.shape[3];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int64_t r = i;
@@ -168,6 +175,7 @@ __global__ void elementwise_kernel(const __grid_constant__ EwParams p) {
 // on four 64-bit divisions per element. The launcher merges axes that every operand walks contiguously and sees to
 // alignment. [500, 100, 36] - [1, 100, 36]: 3.3 us, 14 before
 __global__ void __launch_bounds__(256) elementwise4_kernel(const __grid_constant__ EwParams p) {
+  pdl_begin();
   const uint32_t s1 = (uint32_t)p.shape[1], s2 = (uint32_t)p.shape[2], s3 = (uint32_t)p.shape[3] / 4;
   const uint32_t total = (uint32_t)p.shape[0] * s1 * s2 * s3;
   const bool rep_a = p.as[3] == 0, rep_b = p.bs[3] == 0;
@@ -194,6 +202,7 @@ __global__ void __launch_bounds__(256) elementwise4_kernel(const __grid_constant
 
 __global__ void copy2d_kernel(const void* src, int64_t src_ld, int sdt, void* dst, int64_t dst_ld, int ddt,
                               int64_t rows, int64_t cols) {
+  pdl_begin();
   const int64_t total = rows * cols;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     // 32-bit division where it will do: the 64-bit one is most of the instructions of an element
@@ -212,6 +221,7 @@ __global__ void copy2d_kernel(const void* src, int64_t src_ld, int sdt, void* ds
 // into rows of 144: 1.9 us, 5 before
 template <typename V>
 __global__ void __launch_bounds__(256) copy2d_vec_kernel(const V* src, int64_t src_ld, V* dst, int64_t dst_ld, uint32_t total, uint32_t cols) {
+  pdl_begin();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const uint32_t r = i / cols, c = i - r * cols;
     dst[(int64_t)r * dst_ld + c] = src[(int64_t)r * src_ld + c];
@@ -219,6 +229,7 @@ __global__ void __launch_bounds__(256) copy2d_vec_kernel(const V* src, int64_t s
 }
 
 __global__ void reduce_sum_kernel(const void* x, void* y, int64_t outer, int64_t r, int64_t inner, int dt) {
+  pdl_begin();
   const int64_t total = outer * inner;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t o = i / inner, in = i - o * inner;
@@ -256,6 +267,7 @@ __global__ void __launch_bounds__(256) din_tower_input_kernel(const __half* user
                                                               int64_t ldq, const __half* k, int64_t ldk,
                                                               const __half* att, int64_t ldatt, __half* X, int64_t ldx,
                                                               int n_cand, int T, int d, int du, int pairs_ok) {
+  pdl_begin();
   extern __shared__ float hs[];      // [d] his_sum, then [du] user row
   float* us = hs + d;
   const int r = blockIdx.y;
@@ -370,6 +382,7 @@ __global__ void __launch_bounds__(256) din_tower_split_kernel(const __half* user
                                                               const __half* att, int64_t ldatt, __half* Xu, int64_t ldxu,
                                                               __half* Xc, int64_t ldxc, int n_cand, int T, int d, int du,
                                                               int pairs_ok) {
+  pdl_begin();
   extern __shared__ float hs[];      // [d] his_sum, then [G][d] partial sums
   float* part = hs + d;
   const int r = blockIdx.y;
@@ -456,7 +469,7 @@ extern "C" int xb_dice(const void* x, void* y, int64_t rows, int32_t c, const vo
   XB_REQUIRE(x && y && gamma && mean && var && c > 0 && rows >= 0, XB_ERR_ARG, "xb_dice: bad arguments");
   XB_REQUIRE(float_dtype(dtype), XB_ERR_UNSUPPORTED, "xb_dice: dtype %d", dtype);
   if (rows == 0) return 0;
-  dice_kernel<<<stream_grid(rows * c, 256), 256, 0, (cudaStream_t)s>>>(x, y, rows * c, c, gamma, mean, var, nosqrt, dtype);
+  launch_dependent(dice_kernel, stream_grid(rows * c, 256), 256, 0, (cudaStream_t)s, x, y, rows * c, c, gamma, mean, var, nosqrt, dtype);
   return check_launch("dice_kernel");
 }
 
@@ -465,7 +478,7 @@ extern "C" int xb_prelu(const void* x, void* y, int64_t size, const void* w, int
   XB_REQUIRE(x && y && w && inner > 0 && size >= 0, XB_ERR_ARG, "xb_prelu: bad arguments");
   XB_REQUIRE(float_dtype(dtype) && float_dtype(w_dtype), XB_ERR_UNSUPPORTED, "xb_prelu: dtype %d/%d", dtype, w_dtype);
   if (size == 0) return 0;
-  prelu_kernel<<<stream_grid(size, 256), 256, 0, (cudaStream_t)s>>>(x, y, size, w, inner, dtype, w_dtype);
+  launch_dependent(prelu_kernel, stream_grid(size, 256), 256, 0, (cudaStream_t)s, x, y, size, w, inner, dtype, w_dtype);
   return check_launch("prelu_kernel");
 }
 
@@ -473,7 +486,7 @@ extern "C" int xb_sigmoid(const void* x, void* y, int64_t size, int32_t dtype, x
   XB_REQUIRE(x && y && size >= 0, XB_ERR_ARG, "xb_sigmoid: bad arguments");
   XB_REQUIRE(float_dtype(dtype), XB_ERR_UNSUPPORTED, "xb_sigmoid: dtype %d", dtype);
   if (size == 0) return 0;
-  sigmoid_kernel<<<stream_grid(size, 256), 256, 0, (cudaStream_t)s>>>(x, y, size, dtype);
+  launch_dependent(sigmoid_kernel, stream_grid(size, 256), 256, 0, (cudaStream_t)s, x, y, size, dtype);
   return check_launch("sigmoid_kernel");
 }
 
@@ -483,12 +496,12 @@ extern "C" int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t 
   if (n == 0) return 0;
   if (w == 1 && c >= 16 && c <= 256) {
     const unsigned grid = stream_grid(n, 8);
-    if (c <= 64) softmax_rows_kernel<2><<<grid, 256, 0, (cudaStream_t)s>>>(x, y, n, c, dtype);
-    else if (c <= 128) softmax_rows_kernel<4><<<grid, 256, 0, (cudaStream_t)s>>>(x, y, n, c, dtype);
-    else softmax_rows_kernel<8><<<grid, 256, 0, (cudaStream_t)s>>>(x, y, n, c, dtype);
+    if (c <= 64) launch_dependent(softmax_rows_kernel<2>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
+    else if (c <= 128) launch_dependent(softmax_rows_kernel<4>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
+    else launch_dependent(softmax_rows_kernel<8>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
     return check_launch("softmax_rows_kernel");
   }
-  softmax_kernel<<<stream_grid(n * w, 128), 128, 0, (cudaStream_t)s>>>(x, y, n, c, w, dtype);
+  launch_dependent(softmax_kernel, stream_grid(n * w, 128), 128, 0, (cudaStream_t)s, x, y, n, c, w, dtype);
   return check_launch("softmax_kernel");
 }
 
@@ -498,7 +511,7 @@ extern "C" int xb_batchnorm(const void* x, void* y, int64_t size, int32_t c, con
   XB_REQUIRE(x && y && gamma && beta && mean && var && c > 0 && size >= 0, XB_ERR_ARG, "xb_batchnorm: bad arguments");
   XB_REQUIRE(float_dtype(dtype), XB_ERR_UNSUPPORTED, "xb_batchnorm: dtype %d", dtype);
   if (size == 0) return 0;
-  batchnorm_kernel<<<stream_grid(size, 256), 256, 0, (cudaStream_t)s>>>(x, y, size, c, gamma, beta, mean, var, eps, nosqrt, dtype);
+  launch_dependent(batchnorm_kernel, stream_grid(size, 256), 256, 0, (cudaStream_t)s, x, y, size, c, gamma, beta, mean, var, eps, nosqrt, dtype);
   return check_launch("batchnorm_kernel");
 }
 
@@ -539,11 +552,11 @@ extern "C" int xb_elementwise(int32_t op, const void* a, const int64_t* as, cons
       return st[3] == 1 && (reinterpret_cast<uintptr_t>(base) & 15) == 0 && st[0] % 4 == 0 && st[1] % 4 == 0 && st[2] % 4 == 0;
     };
     if (m.shape[3] % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && fits(a, m.as) && (!two || fits(b, m.bs))) {
-      elementwise4_kernel<<<stream_grid(total / 4, 256), 256, 0, (cudaStream_t)s>>>(m);
+      launch_dependent(elementwise4_kernel, stream_grid(total / 4, 256), 256, 0, (cudaStream_t)s, m);
       return check_launch("elementwise4_kernel");
     }
   }
-  elementwise_kernel<<<stream_grid(total, 256), 256, 0, (cudaStream_t)s>>>(p);
+  launch_dependent(elementwise_kernel, stream_grid(total, 256), 256, 0, (cudaStream_t)s, p);
   return check_launch("elementwise_kernel");
 }
 
@@ -564,14 +577,14 @@ extern "C" int xb_copy2d(const void* src, int64_t src_ld, int32_t sdt, void* dst
       const uint32_t pc = (uint32_t)(cols * es / w);
       const int64_t sl = src_ld * es / w, dl = dst_ld * es / w;
       const cudaStream_t st = (cudaStream_t)s;
-      if (w == 16) copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint4*)src, sl, (uint4*)dst, dl, (uint32_t)pieces, pc);
-      else if (w == 8) copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint2*)src, sl, (uint2*)dst, dl, (uint32_t)pieces, pc);
-      else if (w == 4) copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint32_t*)src, sl, (uint32_t*)dst, dl, (uint32_t)pieces, pc);
-      else copy2d_vec_kernel<<<grid, 256, 0, st>>>((const uint16_t*)src, sl, (uint16_t*)dst, dl, (uint32_t)pieces, pc);
+      if (w == 16) launch_dependent(copy2d_vec_kernel<uint4>, grid, 256, 0, st, (const uint4*)src, sl, (uint4*)dst, dl, (uint32_t)pieces, pc);
+      else if (w == 8) launch_dependent(copy2d_vec_kernel<uint2>, grid, 256, 0, st, (const uint2*)src, sl, (uint2*)dst, dl, (uint32_t)pieces, pc);
+      else if (w == 4) launch_dependent(copy2d_vec_kernel<uint32_t>, grid, 256, 0, st, (const uint32_t*)src, sl, (uint32_t*)dst, dl, (uint32_t)pieces, pc);
+      else launch_dependent(copy2d_vec_kernel<uint16_t>, grid, 256, 0, st, (const uint16_t*)src, sl, (uint16_t*)dst, dl, (uint32_t)pieces, pc);
       return check_launch("copy2d_vec_kernel");
     }
   }
-  copy2d_kernel<<<stream_grid(rows * cols, 256), 256, 0, (cudaStream_t)s>>>(src, src_ld, sdt, dst, dst_ld, ddt, rows, cols);
+  launch_dependent(copy2d_kernel, stream_grid(rows * cols, 256), 256, 0, (cudaStream_t)s, src, src_ld, sdt, dst, dst_ld, ddt, rows, cols);
   return check_launch("copy2d_kernel");
 }
 
@@ -579,6 +592,7 @@ extern "C" int xb_copy2d(const void* src, int64_t src_ld, int32_t sdt, void* dst
 // and the length allow it, single bytes otherwise (id lists and segment counts of odd lengths).
 constexpr int64_t COPY_PIECE = 32 * 1024;
 __global__ void copy_segments_kernel(const xb_copy_item* __restrict__ items) {
+  pdl_begin();
   const xb_copy_item it = items[blockIdx.x];
   const int64_t begin = (int64_t)blockIdx.y * COPY_PIECE;
   if (begin >= it.bytes) return;
@@ -601,7 +615,7 @@ extern "C" int xb_copy_segments(const xb_copy_item* items, int32_t n_items, int6
   const int64_t pieces = (max_bytes + COPY_PIECE - 1) / COPY_PIECE;
   XB_REQUIRE(pieces <= 65535, XB_ERR_LIMIT, "xb_copy_segments: a copy of %lld bytes is too long for one call", (long long)max_bytes);
   dim3 grid((unsigned)n_items, (unsigned)pieces);
-  copy_segments_kernel<<<grid, 256, 0, (cudaStream_t)s>>>(items);
+  launch_dependent(copy_segments_kernel, grid, 256, 0, (cudaStream_t)s, items);
   return check_launch("copy_segments_kernel");
 }
 
@@ -610,7 +624,7 @@ extern "C" int xb_reduce_sum(const void* x, void* y, int64_t outer, int64_t r, i
   XB_REQUIRE(x && y && outer >= 0 && r >= 0 && inner >= 0, XB_ERR_ARG, "xb_reduce_sum: bad arguments");
   XB_REQUIRE(float_dtype(dtype), XB_ERR_UNSUPPORTED, "xb_reduce_sum: dtype %d", dtype);
   if (outer * inner == 0) return 0;
-  reduce_sum_kernel<<<stream_grid(outer * inner, 128), 128, 0, (cudaStream_t)s>>>(x, y, outer, r, inner, dtype);
+  launch_dependent(reduce_sum_kernel, stream_grid(outer * inner, 128), 128, 0, (cudaStream_t)s, x, y, outer, r, inner, dtype);
   return check_launch("reduce_sum_kernel");
 }
 
@@ -644,7 +658,7 @@ extern "C" int xb_din_tower_input(const void* user, int64_t ldu, const void* q, 
   // 64-bit ones need the same of multiples of four
   const int quads_ok = d % 4 == 0 && du % 4 == 0 && ldx % 4 == 0 && ldq % 4 == 0 && ldatt % 4 == 0 &&
                        (((uintptr_t)q | (uintptr_t)att | (uintptr_t)X) & 7) == 0;
-  din_tower_input_kernel<<<grid, 256, sizeof(float) * (9 * d + du + 2), (cudaStream_t)s>>>(
+  launch_dependent(din_tower_input_kernel, grid, 256, sizeof(float) * (9 * d + du + 2), (cudaStream_t)s, 
       (const __half*)user, ldu, (const __half*)q, ldq, (const __half*)k, ldk, (const __half*)att, ldatt, (__half*)X,
       ldx, n_cand, T, d, du, quads_ok ? 2 : pairs_ok);
   return check_launch("din_tower_input_kernel");
@@ -665,7 +679,7 @@ extern "C" int xb_din_tower_input_split(const void* user, int64_t ldu, const voi
   dim3 grid(n_cand > 0 ? (n_cand + 63) / 64 : 1, requests);
   const int pairs_ok = d % 2 == 0 && ldxc % 2 == 0 && ldq % 2 == 0 && ldatt % 2 == 0 &&
                        (((uintptr_t)q | (uintptr_t)att | (uintptr_t)Xc) & 3) == 0;
-  din_tower_split_kernel<<<grid, 256, sizeof(float) * (9 * d + 2), (cudaStream_t)s>>>(
+  launch_dependent(din_tower_split_kernel, grid, 256, sizeof(float) * (9 * d + 2), (cudaStream_t)s, 
       (const __half*)user, ldu, (const __half*)q, ldq, (const __half*)k, ldk, (const __half*)att, ldatt, (__half*)Xu,
       ldxu, (__half*)Xc, ldxc, n_cand, T, d, du, pairs_ok);
   return check_launch("din_tower_split_kernel");

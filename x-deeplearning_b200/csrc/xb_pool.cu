@@ -69,6 +69,7 @@ __device__ __forceinline__ uint64_t mix64(uint64_t x) {
 // counts -> exclusive offsets, one CTA per group: 1024 threads x 8 counts per pass (8192 per pass).
 constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 8;
 __global__ void __launch_bounds__(SCAN_THREADS) scan_counts_kernel(const __grid_constant__ ScanParams p) {
+  pdl_begin();
   const int g = blockIdx.x;
   const int32_t* __restrict__ counts = p.counts[g];
   int32_t* __restrict__ offsets = p.offsets[g];
@@ -135,6 +136,7 @@ __device__ __forceinline__ int scan_find_group(const ScanParams& p, int chunk) {
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) scan_sums_kernel(const __grid_constant__ ScanParams p) {
+  pdl_begin();
   const int g = scan_find_group(p, blockIdx.x), lc = blockIdx.x - p.chunk_begin[g];
   const int32_t* __restrict__ counts = p.counts[g];
   const int64_t batch = p.batch[g], i0 = (int64_t)lc * SCAN_THREADS * SCAN_ITEMS + (int64_t)threadIdx.x * SCAN_ITEMS;
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_sums_kernel(const __grid_co
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const __grid_constant__ ScanParams p) {
+  pdl_begin();
   const int g = scan_find_group(p, blockIdx.x), lc = blockIdx.x - p.chunk_begin[g];
   const int32_t* __restrict__ counts = p.counts[g];
   int32_t* __restrict__ offsets = p.offsets[g];
@@ -270,6 +273,7 @@ __device__ __forceinline__ void store_out(void* out, int64_t idx, int out_dtype,
 }
 
 __global__ void __launch_bounds__(256) pool_kernel(const __grid_constant__ PoolParams p) {
+  pdl_begin();
   const int64_t warp_id = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (warp_id >= p.total_warps) return;      // whole warp leaves together
   const int lane = threadIdx.x & 31;
@@ -469,6 +473,7 @@ __device__ __forceinline__ void store_vec(void* out, int64_t o, bool out16, cons
 // in flight.
 template <int TD, int LPR>
 __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant__ PoolParams p) {
+  pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;          // elements per 16-byte chunk
   constexpr int RB = LPR < 4 ? LPR : 4;              // row loads in flight per lane
   constexpr unsigned FULL = 0xffffffffu;
@@ -649,6 +654,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
 // pools 2.6 M segments of 1.9 ids). A segment's rows are added in id order, as everywhere.
 template <int TD, int LPR, bool REC>
 __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__ PoolParams p) {
+  pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;          // elements per 16-byte chunk
   constexpr int SPW = 32 / LPR;                      // segments per warp and round
   constexpr int U = 4;                               // ids of a segment fetched together
@@ -752,6 +758,7 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
 // nothing for it (a run-time test here cost 15 % on tables that do not fit L2)
 template <int TD, int LPR, bool REC>
 __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constant__ PoolParams p) {
+  pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int NT = 32 / LPR;                       // sub-teams per warp
@@ -871,10 +878,10 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
 template <int TD, bool REC>
 static int launch_pool_queue(const PoolParams& p, int lpr, unsigned blocks, cudaStream_t stream) {
   switch (lpr) {
-    case 1: case 2: pool_queue_kernel<TD, 2, REC><<<blocks, 256, 0, stream>>>(p); break;
-    case 4: pool_queue_kernel<TD, 4, REC><<<blocks, 256, 0, stream>>>(p); break;
-    case 8: pool_queue_kernel<TD, 8, REC><<<blocks, 256, 0, stream>>>(p); break;
-    default: pool_queue_kernel<TD, 16, REC><<<blocks, 256, 0, stream>>>(p); break;
+    case 1: case 2: launch_dependent(pool_queue_kernel<TD, 2, REC>, blocks, 256, 0, stream, p); break;
+    case 4: launch_dependent(pool_queue_kernel<TD, 4, REC>, blocks, 256, 0, stream, p); break;
+    case 8: launch_dependent(pool_queue_kernel<TD, 8, REC>, blocks, 256, 0, stream, p); break;
+    default: launch_dependent(pool_queue_kernel<TD, 16, REC>, blocks, 256, 0, stream, p); break;
   }
   return check_launch("pool_queue_kernel");
 }
@@ -882,10 +889,10 @@ static int launch_pool_queue(const PoolParams& p, int lpr, unsigned blocks, cuda
 template <int TD>
 static int launch_pool_fast(const PoolParams& p, int lpr, unsigned blocks, cudaStream_t stream) {
   switch (lpr) {
-    case 1: case 2: pool_fast_kernel<TD, 2><<<blocks, 256, 0, stream>>>(p); break;
-    case 4: pool_fast_kernel<TD, 4><<<blocks, 256, 0, stream>>>(p); break;
-    case 8: pool_fast_kernel<TD, 8><<<blocks, 256, 0, stream>>>(p); break;
-    default: pool_fast_kernel<TD, 16><<<blocks, 256, 0, stream>>>(p); break;
+    case 1: case 2: launch_dependent(pool_fast_kernel<TD, 2>, blocks, 256, 0, stream, p); break;
+    case 4: launch_dependent(pool_fast_kernel<TD, 4>, blocks, 256, 0, stream, p); break;
+    case 8: launch_dependent(pool_fast_kernel<TD, 8>, blocks, 256, 0, stream, p); break;
+    default: launch_dependent(pool_fast_kernel<TD, 16>, blocks, 256, 0, stream, p); break;
   }
   return check_launch("pool_fast_kernel");
 }
@@ -893,10 +900,10 @@ static int launch_pool_fast(const PoolParams& p, int lpr, unsigned blocks, cudaS
 template <int TD, bool REC>
 static int launch_pool_short(const PoolParams& p, int lpr, unsigned blocks, cudaStream_t stream) {
   switch (lpr) {
-    case 1: case 2: pool_short_kernel<TD, 2, REC><<<blocks, 256, 0, stream>>>(p); break;
-    case 4: pool_short_kernel<TD, 4, REC><<<blocks, 256, 0, stream>>>(p); break;
-    case 8: pool_short_kernel<TD, 8, REC><<<blocks, 256, 0, stream>>>(p); break;
-    default: pool_short_kernel<TD, 16, REC><<<blocks, 256, 0, stream>>>(p); break;
+    case 1: case 2: launch_dependent(pool_short_kernel<TD, 2, REC>, blocks, 256, 0, stream, p); break;
+    case 4: launch_dependent(pool_short_kernel<TD, 4, REC>, blocks, 256, 0, stream, p); break;
+    case 8: launch_dependent(pool_short_kernel<TD, 8, REC>, blocks, 256, 0, stream, p); break;
+    default: launch_dependent(pool_short_kernel<TD, 16, REC>, blocks, 256, 0, stream, p); break;
   }
   return check_launch("pool_short_kernel");
 }
@@ -1194,12 +1201,12 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
   if (sp.n) {
     if (sp.chunk_begin[sp.n] > sp.n) {
       // some count array is longer than one chunk: all chunks in parallel, two launches
-      scan_sums_kernel<<<sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream>>>(sp);
+      launch_dependent(scan_sums_kernel, sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream, sp);
       if (int rc = check_launch("scan_sums_kernel")) return rc;
-      scan_apply_kernel<<<sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream>>>(sp);
+      launch_dependent(scan_apply_kernel, sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream, sp);
       if (int rc = check_launch("scan_apply_kernel")) return rc;
     } else {
-      scan_counts_kernel<<<sp.n, SCAN_THREADS, 0, stream>>>(sp);
+      launch_dependent(scan_counts_kernel, sp.n, SCAN_THREADS, 0, stream, sp);
       if (int rc = check_launch("scan_counts_kernel")) return rc;
     }
   }
@@ -1239,7 +1246,7 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
   if (p.n_groups == 0) return 0;
   const int64_t blocks = (p.total_warps + 7) / 8;
   XB_REQUIRE(blocks < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_embedding_pool: too many segments");
-  pool_kernel<<<(unsigned)blocks, 256, 0, stream>>>(p);
+  launch_dependent(pool_kernel, (unsigned)blocks, 256, 0, stream, p);
   return check_launch("pool_kernel");
 }
 
@@ -1360,6 +1367,7 @@ __global__ void __launch_bounds__(256) route_count_kernel(const int64_t* __restr
                                                           int32_t* __restrict__ block_hist,
                                                           const int32_t* __restrict__ seg_offsets, int64_t segments,
                                                           int32_t* __restrict__ block_first_seg) {
+  pdl_begin();
   __shared__ int32_t hist[ROUTE_MAX_SHARDS];
   if (threadIdx.x < ROUTE_MAX_SHARDS) hist[threadIdx.x] = 0;
   __syncthreads();
@@ -1409,6 +1417,7 @@ __global__ void __launch_bounds__(256) route_count_kernel(const int64_t* __restr
 __global__ void __launch_bounds__(1024) route_scan_kernel(int32_t* __restrict__ block_hist, int64_t blocks, int shards,
                                                           int64_t* __restrict__ owner_counts, int64_t bucket_cap,
                                                           int64_t* __restrict__ headers, int32_t* __restrict__ overflow) {
+  pdl_begin();
   __shared__ int32_t part[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int64_t total = 0;                                          // the same in every thread
@@ -1458,6 +1467,7 @@ __global__ void __launch_bounds__(256) route_scatter_kernel(const int64_t* __res
                                                             int64_t* __restrict__ out_rows, float* __restrict__ out_values,
                                                             int32_t* __restrict__ out_tags, int64_t bucket_cap,
                                                             const int32_t* __restrict__ block_first_seg) {
+  pdl_begin();
   // The kernel is bound by instructions per id, not by memory, so the per-id work is kept to a handful: the segment
   // of every id of the CTA is tabulated once in shared memory (each segment of the CTA's window writes its number
   // over its own positions), and the ranks come from prefix sums that `shards` threads make once per round.
@@ -1589,6 +1599,7 @@ __global__ void tag_count_kernel(const int32_t* __restrict__ tags, int64_t n, in
 __global__ void shard_combine_kernel(const float* __restrict__ partial, int shards, int64_t segments, int dim,
                                      const int32_t* __restrict__ seg_len, int avg, void* out, int64_t out_stride,
                                      int64_t seg_per_row, int out_dtype) {
+  pdl_begin();
   const int64_t total = segments * dim;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t s = i / dim;
@@ -1609,6 +1620,7 @@ template <int SHARDS>
 __global__ void __launch_bounds__(256) shard_combine4_kernel(const float4* __restrict__ partial, int shards, int64_t segments,
                                                              int dim4, const int32_t* __restrict__ seg_len, int avg,
                                                              void* out, int64_t out_stride, int64_t rows, int out_dtype) {
+  pdl_begin();
   const int64_t total = segments * dim4;
   const int n_sh = SHARDS ? SHARDS : shards;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1653,6 +1665,7 @@ template <int SHARDS>
 __global__ void __launch_bounds__(256) shard_combine_h8_kernel(const uint4* __restrict__ partial, int shards, int64_t segments,
                                                                int dim8, const int32_t* __restrict__ seg_len, int avg,
                                                                void* out, int64_t out_stride, int64_t rows, int out_dtype) {
+  pdl_begin();
   const int64_t total = segments * dim8;
   const int n_sh = SHARDS ? SHARDS : shards;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1740,9 +1753,9 @@ extern "C" int xb_route_ids(const int64_t* ids, const float* values, const int32
   const int64_t blocks = std::max<int64_t>((n_ids + ROUTE_CHUNK - 1) / ROUTE_CHUNK, 1);
   int32_t* hist = reinterpret_cast<int32_t*>(scratch);
   int32_t* first_seg = hist + blocks * shards;
-  route_count_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, n_ids, shards, hist, seg_offsets, segments, first_seg);
-  route_scan_kernel<<<1, 1024, 0, stream>>>(hist, blocks, shards, owner_counts, 0, nullptr, nullptr);
-  route_scatter_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, values, seg_offsets, segments, n_ids, shards, hist, out_rows,
+  launch_dependent(route_count_kernel, (unsigned)blocks, 256, 0, stream, ids, n_ids, shards, hist, seg_offsets, segments, first_seg);
+  launch_dependent(route_scan_kernel, 1, 1024, 0, stream, hist, blocks, shards, owner_counts, 0, nullptr, nullptr);
+  launch_dependent(route_scatter_kernel, (unsigned)blocks, 256, 0, stream, ids, values, seg_offsets, segments, n_ids, shards, hist, out_rows,
                                                              out_values, out_tags, 0, first_seg);
   return check_launch("route kernels");
 }
@@ -1762,9 +1775,9 @@ extern "C" int xb_route_ids_padded(const int64_t* ids, const int32_t* seg_offset
   const int64_t blocks = std::max<int64_t>((n_ids + ROUTE_CHUNK - 1) / ROUTE_CHUNK, 1);
   int32_t* hist = reinterpret_cast<int32_t*>(scratch);
   int32_t* first_seg = hist + blocks * shards;
-  route_count_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, n_ids, shards, hist, seg_offsets, segments, first_seg);
-  route_scan_kernel<<<1, 1024, 0, stream>>>(hist, blocks, shards, nullptr, bucket_cap, out_records, overflow);
-  route_scatter_kernel<<<(unsigned)blocks, 256, 0, stream>>>(ids, nullptr, seg_offsets, segments, n_ids, shards, hist, out_records,
+  launch_dependent(route_count_kernel, (unsigned)blocks, 256, 0, stream, ids, n_ids, shards, hist, seg_offsets, segments, first_seg);
+  launch_dependent(route_scan_kernel, 1, 1024, 0, stream, hist, blocks, shards, nullptr, bucket_cap, out_records, overflow);
+  launch_dependent(route_scatter_kernel, (unsigned)blocks, 256, 0, stream, ids, nullptr, seg_offsets, segments, n_ids, shards, hist, out_records,
                                                              nullptr, nullptr, bucket_cap, first_seg);
   return check_launch("route kernels (fixed-capacity buckets)");
 }
@@ -1817,12 +1830,12 @@ extern "C" int xb_scan_counts(const int32_t* counts, int64_t counts_stride, int3
   }
   if (batch == 0) return 0;
   if (sp.chunk_begin[sp.n] > sp.n) {
-    scan_sums_kernel<<<sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream>>>(sp);
+    launch_dependent(scan_sums_kernel, sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream, sp);
     if (int rc = check_launch("scan_sums_kernel")) return rc;
-    scan_apply_kernel<<<sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream>>>(sp);
+    launch_dependent(scan_apply_kernel, sp.chunk_begin[sp.n], SCAN_THREADS, 0, stream, sp);
     return check_launch("scan_apply_kernel");
   }
-  scan_counts_kernel<<<sp.n, SCAN_THREADS, 0, stream>>>(sp);
+  launch_dependent(scan_counts_kernel, sp.n, SCAN_THREADS, 0, stream, sp);
   return check_launch("scan_counts_kernel");
 }
 
@@ -1957,6 +1970,7 @@ extern "C" int xb_shard_pool_padded(const xb_table_desc* const* tables, const in
 // same segment number add once. counts[src * segments + tag]; a tag outside [0, segments) is dropped.
 __global__ void record_count_kernel(const int64_t* __restrict__ packed, int sources, int64_t cap, int64_t segments,
                                     int32_t* __restrict__ counts) {
+  pdl_begin();
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (int64_t)gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   for (int src = 0; src < sources; ++src) {
@@ -1980,7 +1994,7 @@ extern "C" int xb_record_counts_padded(const int64_t* packed, int32_t sources, i
   XB_REQUIRE(packed && counts && sources >= 1 && sources <= ROUTE_MAX_SHARDS && bucket_cap >= 2 && segments >= 0, XB_ERR_ARG,
              "xb_record_counts_padded: bad arguments");
   XB_CUDA(cudaMemsetAsync(counts, 0, (size_t)sources * (size_t)segments * sizeof(int32_t), stream));
-  record_count_kernel<<<sm_count() * 8, 256, 0, stream>>>(packed, sources, bucket_cap, segments, counts);
+  launch_dependent(record_count_kernel, sm_count() * 8, 256, 0, stream, packed, sources, bucket_cap, segments, counts);
   return check_launch("record_count_kernel");
 }
 
@@ -2046,10 +2060,10 @@ extern "C" int xb_shard_combine(const void* partial_, int32_t partial_dtype, int
       const int64_t blocks8 = std::min<int64_t>((segments * dim8 + 255) / 256, (int64_t)sm_count() * 16);
       const uint4* p8 = reinterpret_cast<const uint4*>(partial_);
       switch (shards) {
-        case 2: shard_combine_h8_kernel<2><<<(unsigned)blocks8, 256, 0, stream>>>(p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
-        case 4: shard_combine_h8_kernel<4><<<(unsigned)blocks8, 256, 0, stream>>>(p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
-        case 8: shard_combine_h8_kernel<8><<<(unsigned)blocks8, 256, 0, stream>>>(p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
-        default: shard_combine_h8_kernel<0><<<(unsigned)blocks8, 256, 0, stream>>>(p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
+        case 2: launch_dependent(shard_combine_h8_kernel<2>, (unsigned)blocks8, 256, 0, stream, p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
+        case 4: launch_dependent(shard_combine_h8_kernel<4>, (unsigned)blocks8, 256, 0, stream, p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
+        case 8: launch_dependent(shard_combine_h8_kernel<8>, (unsigned)blocks8, 256, 0, stream, p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
+        default: launch_dependent(shard_combine_h8_kernel<0>, (unsigned)blocks8, 256, 0, stream, p8, shards, segments, dim8, seg_len, avg, out, out_stride, rows, out_dtype); break;
       }
       return check_launch("shard_combine_h8_kernel");
     }
@@ -2071,15 +2085,15 @@ extern "C" int xb_shard_combine(const void* partial_, int32_t partial_dtype, int
     const int64_t blocks4 = std::min<int64_t>((segments * dim4 + 255) / 256, (int64_t)sm_count() * 16);
     const float4* p4 = reinterpret_cast<const float4*>(partial);
     switch (shards) {
-      case 2: shard_combine4_kernel<2><<<(unsigned)blocks4, 256, 0, stream>>>(p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
-      case 4: shard_combine4_kernel<4><<<(unsigned)blocks4, 256, 0, stream>>>(p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
-      case 8: shard_combine4_kernel<8><<<(unsigned)blocks4, 256, 0, stream>>>(p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
-      default: shard_combine4_kernel<0><<<(unsigned)blocks4, 256, 0, stream>>>(p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
+      case 2: launch_dependent(shard_combine4_kernel<2>, (unsigned)blocks4, 256, 0, stream, p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
+      case 4: launch_dependent(shard_combine4_kernel<4>, (unsigned)blocks4, 256, 0, stream, p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
+      case 8: launch_dependent(shard_combine4_kernel<8>, (unsigned)blocks4, 256, 0, stream, p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
+      default: launch_dependent(shard_combine4_kernel<0>, (unsigned)blocks4, 256, 0, stream, p4, shards, segments, dim4, seg_len, avg, out, out_stride, rows, out_dtype); break;
     }
     return check_launch("shard_combine4_kernel");
   }
   const int64_t blocks = std::min<int64_t>((segments * dim + 255) / 256, (int64_t)sm_count() * 8);
-  shard_combine_kernel<<<(unsigned)blocks, 256, 0, stream>>>(partial, shards, segments, dim, seg_len, avg, out, out_stride, groups,
+  launch_dependent(shard_combine_kernel, (unsigned)blocks, 256, 0, stream, partial, shards, segments, dim, seg_len, avg, out, out_stride, groups,
                                                              out_dtype);
   return check_launch("shard_combine_kernel");
 }

@@ -34,6 +34,7 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int steps, int H,
                                                       const T* __restrict__ i2h, const T* __restrict__ h2h,
                                                       const T* __restrict__ bi, const T* __restrict__ bh) {
+  pdl_begin();
   constexpr int HP = gru_hp(NV);
   extern __shared__ __align__(16) float gru_sm[];
   float* xs = gru_sm;                              // [GRU_CHUNK][HP]
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
 // the candidates of one request), and only the final state is written (y is [B, H]).
 __global__ void augru_kernel(const void* x, const void* att, void* y, int T, int H, const void* Wg_, const void* bg_,
                              const void* Wc_, const void* bc_, int dt, int share) {
+  pdl_begin();
   extern __shared__ float sm[];
   float* Wg = sm;                     // [2H][2H]
   float* Wc = Wg + 4 * H * H;         // [2H][H]
@@ -188,7 +190,7 @@ int launch_gru_nv(const T* x, T* y, int64_t batch, int steps, int H, const T* i2
   const size_t smem = sizeof(float) * GRU_CHUNK * (size_t)(gru_hp(NV) + 3 * H);
   static PerDeviceOnce attr;                       // per instantiation
   XB_SET_MAX_SMEM_ONCE(attr, sizeof(float) * GRU_CHUNK * 4 * gru_hp(NV), (const void*)gru_kernel<T, NV>);
-  gru_kernel<T, NV><<<(unsigned)batch, (4 * H + 31) / 32 * 32, smem, s>>>(x, y, steps, H, i2h, h2h, bi, bh);
+  launch_dependent(gru_kernel<T, NV>, (unsigned)batch, (4 * H + 31) / 32 * 32, smem, s, x, y, steps, H, i2h, h2h, bi, bh);
   return check_launch("gru_kernel");
 }
 template <typename T>
@@ -243,7 +245,7 @@ extern "C" int xb_augru(const void* x, const void* att, void* y, int64_t batch, 
   static PerDeviceOnce attr;
   XB_SET_MAX_SMEM_ONCE(attr, 110 * 1024, (const void*)augru_kernel);
   const int threads = (2 * H + 31) / 32 * 32;
-  augru_kernel<<<(unsigned)batch, threads, smem, (cudaStream_t)s>>>(x, att, y, T, H, Wg, bg, Wc, bc, dtype, 0);
+  launch_dependent(augru_kernel, (unsigned)batch, threads, smem, (cudaStream_t)s, x, att, y, T, H, Wg, bg, Wc, bc, dtype, 0);
   return check_launch("augru_kernel");
 }
 
@@ -272,6 +274,6 @@ extern "C" int xb_augru_shared(const void* x, const void* att, void* y_final, in
   static PerDeviceOnce attr;
   XB_SET_MAX_SMEM_ONCE(attr, 110 * 1024, (const void*)augru_kernel);
   const int threads = (2 * H + 31) / 32 * 32;
-  augru_kernel<<<(unsigned)batch, threads, smem, (cudaStream_t)s>>>(x, att, y_final, T, H, Wg, bg, Wc, bc, XB_F16, n_cand);
+  launch_dependent(augru_kernel, (unsigned)batch, threads, smem, (cudaStream_t)s, x, att, y_final, T, H, Wg, bg, Wc, bc, XB_F16, n_cand);
   return check_launch("augru_kernel");
 }

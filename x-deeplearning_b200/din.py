@@ -173,8 +173,9 @@ class DinModel:
         check(lib().xb_softmax(ops.ptr(p["logit"]), ops.ptr(p["prob"]), R * n_cand, D["tower"][2], 1, capi.XB_F32, s))
         return p["prob"]
 
-    # kernels launched by one forward_device call (pool scan + pool + attention + the two tower kernels)
-    LAUNCHES_PER_FORWARD = 5
+    # kernels launched by one forward_device call (pool + attention + the two tower kernels; the pooling call scans its
+    # counts in a launch of their own from 1025 requests on)
+    LAUNCHES_PER_FORWARD = 4
 
     def forward(self, staged):
         """End to end: host ids -> device -> probabilities back on the host."""
