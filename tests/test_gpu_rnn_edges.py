@@ -53,3 +53,23 @@ def test_augru_column_groups(H, R, n_cand, T):
     f = lambda t: t.float().cpu().numpy()
     want = orc.augru(np.repeat(f(dx), n_cand, axis=0), f(da), f(dWg), f(dbg), f(dWc), f(dbc))[:, T - 1, :]
     np.testing.assert_allclose(f(y), want, rtol=0, atol=8e-3)
+
+
+@pytest.mark.parametrize("H", [1, 5, 16, 32, 33, 64])
+@pytest.mark.parametrize("R,n_cand,T", [(2, 7, 33), (1, 4, 64), (3, 1, 1)])
+def test_augru_shared_in_fp32(H, R, n_cand, T):
+    """Widths without selector slots take the fp32 kernel: chunks of 32 steps, four candidates a block."""
+    ops, capi, L = _ops()
+    rng = np.random.default_rng(H + T)
+    h16 = lambda a: torch.from_numpy(a.astype(np.float32)).to("cuda", torch.float16)
+    x, att = rng.normal(0, 0.7, (R, T, H)), rng.dirichlet(np.ones(T) * 0.3, R * n_cand)
+    Wg, bg = rng.normal(0, 1 / np.sqrt(2 * H), (2 * H, 2 * H)), rng.normal(0.5, 0.2, 2 * H)
+    Wc, bc = rng.normal(0, 1 / np.sqrt(2 * H), (2 * H, H)), rng.normal(0, 0.1, H)
+    dx, da, dWg, dbg, dWc, dbc = h16(x), h16(att), h16(Wg), h16(bg), h16(Wc), h16(bc)
+    y = torch.full((R * n_cand, H), 9.0, dtype=torch.float16, device="cuda")
+    capi.check(L.xb_augru_shared(ops.ptr(dx), ops.ptr(da), ops.ptr(y), R, n_cand, T, H, ops.ptr(dWg), ops.ptr(dbg),
+                                 ops.ptr(dWc), ops.ptr(dbc), capi.XB_GEMM_SIMT, ops.stream()))
+    f = lambda t: t.float().cpu().numpy()
+    want = orc.augru(np.repeat(f(dx), n_cand, axis=0), f(da), f(dWg), f(dbg), f(dWc), f(dbc))[:, T - 1, :]
+    # fp32 throughout (2e-5 over the recurrence, as for the GRU), then one fp16 rounding: half an ulp of values below 1
+    np.testing.assert_allclose(f(y), want, rtol=0, atol=2.0 ** -12 + 2e-5)

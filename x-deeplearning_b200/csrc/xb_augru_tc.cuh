@@ -17,8 +17,8 @@
 // round trips and MMA latency. So three warpgroups share a tile, a third of the columns each (a row's columns are
 // independent between the products): every scheduler then has three warps to fill the waits of one another, r*h goes
 // out before the update gate is evaluated, and the update gate's SFU work hides the candidate product. H is a
-// compile-time constant: a run-time H made the update gates a local-memory array. 128 tiles of 100 steps, H = 36: 121 us,
-// 382 with one warpgroup a tile.
+// compile-time constant: a run-time H made the update gates a local-memory array. 128 tiles of 100 steps, H = 36: 115 us,
+// 121 with a copy of the code per group, 382 with one warpgroup a tile.
 //
 // Cell semantics: VecAttGRUCell.call, xdl-algorithm-solution/DIEN/script/utils.py:178-207 (the reference ships no
 // inference operator for it). Shapes: H padded to Hp = 8*ceil(H/8) must leave 4 or more spare slots (H = 36 does).
@@ -89,105 +89,111 @@ __device__ __forceinline__ void au_tmem_st(uint32_t at, const uint32_t* r) {
   else if constexpr (N == 1) tmem_st1(at, r[0]);
 }
 
-// The steps of one worker thread: candidate row `row` of the tile, columns [C0, C0 + NC) of the state (NC even).
-// The last group also writes the selector slots, which follow the state in the A operand.
-template <int H, int GRP>
-__device__ __forceinline__ void au_worker(const AuParams& p, const __half* att_row, uint32_t lane_addr, __half* out, bool valid,
+// The steps of one worker thread: candidate row `row` of the tile, columns [C0, C0 + 2 np) of the state. The groups run the
+// same code with their own offsets (a copy each would not stay in the instruction cache that they share); the last group
+// also writes the selector slots, which follow the state in the A operand.
+template <int H>
+__device__ __forceinline__ void au_worker(const AuParams& p, int grp, const __half* att_row, uint32_t lane_addr, __half* out, bool valid,
                                           uint64_t* a1_full, uint64_t* acc1_full, uint64_t* a2_full, uint64_t* acc2_full) {
   using namespace umma;
   constexpr AuGeom G = au_geom(H, 1);                       // tensor-memory columns do not depend on T
-  constexpr int CPG = (H + 2 * AU_GROUPS - 1) / (2 * AU_GROUPS) * 2;
-  constexpr int C0 = GRP * CPG < H ? GRP * CPG : H;
-  constexpr int NC = GRP == AU_GROUPS - 1 ? H - C0 : (C0 + CPG <= H ? CPG : H - C0);
-  constexpr int NP = NC / 2;
-  constexpr bool LAST = GRP == AU_GROUPS - 1;
-  constexpr int NST = NP + (LAST ? 2 : 0);                  // pairs written per operand: the state's and the selector's
+  constexpr int CPG = (H + 2 * AU_GROUPS - 1) / (2 * AU_GROUPS) * 2, NP = CPG / 2;
+  constexpr bool EVEN = CPG * AU_GROUPS == H;               // every group has CPG columns
+  const int C0 = min(grp * CPG, H), np = EVEN ? NP : min(CPG, H - C0) / 2;
+  const bool last = grp == AU_GROUPS - 1;
   const int T = p.T, lane = threadIdx.x & 31;
   const uint32_t a1t = lane_addr + G.c_a1 + C0 / 2, a2t = lane_addr + G.c_a2 + C0 / 2;
-  float h[NC > 0 ? NC : 1];
-  uint32_t pk[NST > 0 ? NST : 1], upk[NP > 0 ? NP : 1];
+  float h[CPG];
+  uint32_t pk[NP], upk[NP];
 #pragma unroll
-  for (int i = 0; i < NC; ++i) h[i] = 0.f;
+  for (int i = 0; i < CPG; ++i) h[i] = 0.f;
 #pragma unroll
-  for (int i = 0; i < NST; ++i) pk[i] = 0u;
-  auto publish = [&](uint32_t at, uint64_t* bar, int t) {
-    if constexpr (LAST) {
-      const uint32_t one = (t & 1) ? 0x3C000000u : 0x3C00u;   // 1.0 in slot t % 4 of the four
-      pk[NP] = (t & 2) ? 0u : one;
-      pk[NP + 1] = (t & 2) ? one : 0u;
+  for (int i = 0; i < NP; ++i) pk[i] = upk[i] = 0u;
+  auto publish = [&](uint32_t at, uint32_t operand, uint64_t* bar, int t) {
+    if constexpr (EVEN) {
+      au_tmem_st<NP>(at, pk);
+    } else {
+#pragma unroll
+      for (int e = 0; e < NP; ++e)
+        if (e < np) tmem_st1(at + e, pk[e]);
     }
-    au_tmem_st<NST>(at, pk);
+    if (last) {
+      const uint32_t one = (t & 1) ? 0x3C000000u : 0x3C00u;   // 1.0 in slot t % 4 of the four
+      tmem_st2(operand + H / 2, (t & 2) ? 0u : one, (t & 2) ? one : 0u);
+    }
     tmem_wait_st();
     tc_fence_before_sync();
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(bar));
   };
-  if constexpr (LAST) {
+  if (last) {
     // what follows the selector slots (up to the operand's end) stays zero
-    constexpr int Z0 = H / 2 + 2, ZN = G.k / 2 - Z0;
-    constexpr int ZA = ZN > 0 ? ZN : 1;
-    uint32_t z[ZA];
-#pragma unroll
-    for (int i = 0; i < ZA; ++i) z[i] = 0u;
-    au_tmem_st<ZN>(lane_addr + G.c_a1 + Z0, z);
-    au_tmem_st<ZN>(lane_addr + G.c_a2 + Z0, z);
+    for (int c = H / 2 + 2; c < G.k / 2; ++c) { tmem_st1(lane_addr + G.c_a1 + c, 0u); tmem_st1(lane_addr + G.c_a2 + c, 0u); }
   }
-  publish(a1t, a1_full, 0);                                 // h_0 = 0 with the selector of step 0
+  publish(a1t, lane_addr + G.c_a1, a1_full, 0);             // h_0 = 0 with the selector of step 0
   bool ok = true;
+  // 16 or 32 columns in one load: more than the group's, still inside the allocation, the extra values are not used
+  uint32_t vr[32], vu[32];
+  auto load = [&](uint32_t at, uint32_t (&v)[32]) {
+    if constexpr (CPG > 16) tmem_ld32_nowait(at, v);
+    else tmem_ld16_lo_nowait(at, v);
+  };
+  auto loaded = [&](uint32_t (&v)[32]) {
+    if constexpr (CPG > 16) tmem_wait_ld(v);
+    else tmem_wait_ld(*reinterpret_cast<uint32_t(*)[16]>(&v));
+  };
+  // sigmoid(z) = 1/2 + 1/2 tanh(z/2), two columns per SFU instruction
+  auto sigm2 = [](uint32_t a, uint32_t b) {
+    const __half2 z = __floats2half2_rn(0.5f * __uint_as_float(a), 0.5f * __uint_as_float(b));
+    const __half2 th = bits_h2(tanh_f16x2(h2_bits(z)));
+    return __hfma2(th, __floats2half2_rn(0.5f, 0.5f), __floats2half2_rn(0.5f, 0.5f));
+  };
   for (int t = 0; t < T; ++t) {
     const uint32_t ph = (uint32_t)t & 1u;
     // ---- gates: [r|u] = sigmoid(acc1); r*h becomes the A operand of the candidate product
     ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc1_full), ph, 32));
     if (!ok) break;
     tc_fence_after_sync();
-    uint32_t vr[32], vu[32];
-    // (a load may reach past the group's columns: still inside the allocation, the extra values are not used)
-    if constexpr (NC > 16) { tmem_ld32_nowait(lane_addr + C0, vr); tmem_ld32_nowait(lane_addr + H + C0, vu); }
-    else if constexpr (NC > 0) { tmem_ld16_lo_nowait(lane_addr + C0, vr); tmem_ld16_lo_nowait(lane_addr + H + C0, vu); }
-    if constexpr (NC > 16) { tmem_wait_ld(vr); tmem_wait_ld(vu); }
-    else if constexpr (NC > 0) {
-      tmem_wait_ld(*reinterpret_cast<uint32_t(*)[16]>(&vr));
-      tmem_wait_ld(*reinterpret_cast<uint32_t(*)[16]>(&vu));
-    }
-    // sigmoid(z) = 1/2 + 1/2 tanh(z/2), two columns per SFU instruction
-    auto sigm2 = [](uint32_t a, uint32_t b) {
-      const __half2 z = __floats2half2_rn(0.5f * __uint_as_float(a), 0.5f * __uint_as_float(b));
-      const __half2 th = bits_h2(tanh_f16x2(h2_bits(z)));
-      return __hfma2(th, __floats2half2_rn(0.5f, 0.5f), __floats2half2_rn(0.5f, 0.5f));
-    };
+    load(lane_addr + C0, vr);
+    load(lane_addr + H + C0, vu);
+    loaded(vr);
+    loaded(vu);
 #pragma unroll
     for (int e = 0; e < NP; ++e) {
-      const float2 rf = __half22float2(sigm2(vr[2 * e], vr[2 * e + 1]));
-      pk[e] = h2_bits(__floats2half2_rn(rf.x * h[2 * e], rf.y * h[2 * e + 1]));
+      if (e < np) {
+        const float2 rf = __half22float2(sigm2(vr[2 * e], vr[2 * e + 1]));
+        pk[e] = h2_bits(__floats2half2_rn(rf.x * h[2 * e], rf.y * h[2 * e + 1]));
+      }
     }
-    publish(a2t, a2_full, t);
+    publish(a2t, lane_addr + G.c_a2, a2_full, t);
 #pragma unroll
-    for (int e = 0; e < NP; ++e) upk[e] = h2_bits(sigm2(vu[2 * e], vu[2 * e + 1]));
+    for (int e = 0; e < NP; ++e)
+      if (e < np) upk[e] = h2_bits(sigm2(vu[2 * e], vu[2 * e + 1]));
     // ---- candidate and blend
     const float a = __half2float(att_row[t]);
     ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(acc2_full), ph, 33));
     if (!ok) break;
     tc_fence_after_sync();
-    if constexpr (NC > 16) { tmem_ld32_nowait(lane_addr + G.c_acc2 + C0, vr); tmem_wait_ld(vr); }
-    else if constexpr (NC > 0) {
-      tmem_ld16_lo_nowait(lane_addr + G.c_acc2 + C0, vr);
-      tmem_wait_ld(*reinterpret_cast<uint32_t(*)[16]>(&vr));
-    }
+    load(lane_addr + G.c_acc2 + C0, vr);
+    loaded(vr);
 #pragma unroll
     for (int e = 0; e < NP; ++e) {
-      const __half2 z = __floats2half2_rn(__uint_as_float(vr[2 * e]), __uint_as_float(vr[2 * e + 1]));
-      const float2 c = __half22float2(bits_h2(tanh_f16x2(h2_bits(z))));
-      const float2 u = __half22float2(bits_h2(upk[e]));
-      const float u0 = (1.f - a) * u.x, u1 = (1.f - a) * u.y;
-      h[2 * e] = u0 * h[2 * e] + (1.f - u0) * c.x;
-      h[2 * e + 1] = u1 * h[2 * e + 1] + (1.f - u1) * c.y;
-      pk[e] = h2_bits(__floats2half2_rn(h[2 * e], h[2 * e + 1]));
+      if (e < np) {
+        const __half2 z = __floats2half2_rn(__uint_as_float(vr[2 * e]), __uint_as_float(vr[2 * e + 1]));
+        const float2 c = __half22float2(bits_h2(tanh_f16x2(h2_bits(z))));
+        const float2 u = __half22float2(bits_h2(upk[e]));
+        const float u0 = (1.f - a) * u.x, u1 = (1.f - a) * u.y;
+        h[2 * e] = u0 * h[2 * e] + (1.f - u0) * c.x;
+        h[2 * e + 1] = u1 * h[2 * e + 1] + (1.f - u1) * c.y;
+        pk[e] = h2_bits(__floats2half2_rn(h[2 * e], h[2 * e + 1]));
+      }
     }
-    if (t + 1 < T) publish(a1t, a1_full, t + 1);
+    if (t + 1 < T) publish(a1t, lane_addr + G.c_a1, a1_full, t + 1);
   }
   if (ok && valid) {
 #pragma unroll
-    for (int i = 0; i < NP; ++i) *reinterpret_cast<uint32_t*>(out + C0 + 2 * i) = pk[i];      // H is even: 4-byte aligned
+    for (int i = 0; i < NP; ++i)
+      if (i < np) *reinterpret_cast<uint32_t*>(out + C0 + 2 * i) = pk[i];      // H is even: 4-byte aligned
   }
 }
 
@@ -350,11 +356,7 @@ __global__ void __launch_bounds__(AU_THREADS, H <= 40 ? 2 : 1) augru_tc_kernel(c
     const uint32_t lane_addr = tmem0 + ((uint32_t)((warp & 3) * 32) << 16);
     const __half* att_row = atts + row * tpp;
     __half* out = p.y + ((int64_t)r * p.n_cand + tile * 128 + row) * H;
-    switch (warp >> 2) {
-      case 0: au_worker<H, 0>(p, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full); break;
-      case 1: au_worker<H, 1>(p, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full); break;
-      default: au_worker<H, 2>(p, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full); break;
-    }
+    au_worker<H>(p, warp >> 2, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full);
   }
   tc_fence_before_sync();
   __syncthreads();

@@ -5,6 +5,7 @@
 // global atomics between blocks, blaze/blaze/operator/op/gru_op.cu:73-85; nothing
 // here waits on another CTA). Latency-bound by design: throughput comes from
 // batch-many independent CTAs.
+#include <algorithm>
 #include <cstring>
 
 #include "xb_common.cuh"
@@ -18,16 +19,26 @@ __device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cas
 
 __device__ __forceinline__ float sigm(float v) { return 1.f / (1.f + expf(-v)); }
 
+}  // namespace
+}  // namespace xb
+
+#include "xb_augru_tc.cuh"
+
+namespace xb {
+namespace {
+
 // x [B,T,H], y [B,T,H]; i2h, h2h [H,3H] (gate order r, z, candidate); biases [3H].
 // Follows GRUKernel, blaze/blaze/operator/op/gru_op.cc:33-93: leading steps whose first H
 // input pre-activations (before the bias) are all zero emit zeros and leave h at zero.
 //
-// What bounds it is the chain h(t) -> h(t+1); everything else is kept off that chain. The input products of up to
-// GRU_CHUNK steps are made first, one gate column per thread with its weights in registers (they do not depend on h).
-// Then a step is: four lanes per unit, each with a quarter of the unit's three recurrent columns in registers, read
-// their part of h as 16-byte vectors, add up over the lanes with two shuffles, and all four evaluate the gates; the
-// new h goes to the other of two buffers, so a step needs one barrier. 16 sequences of 100 steps, H = 36: 77 us,
-// 156 before (weights in shared memory, three barriers a step).
+// What bounds it is the chain h(t) -> h(t+1), some 250 instructions of which each waits for the one before; everything else
+// is kept off that chain. The input products of up to GRU_CHUNK steps are made first, one gate column per thread with its
+// weights in registers (they do not depend on h). Then a step is: four lanes per unit, each with a quarter of the unit's
+// three recurrent columns in registers, read their part of h as 16-byte vectors and add up over the lanes with three
+// shuffles that leave the reset gate's sum in lane 0, the update gate's in lane 1 and the candidate's in lane 2; lanes 0
+// and 1 evaluate their sigmoids in the same instructions, lane 2 the candidate and the new h, which goes to the other of two
+// buffers, so a step needs one barrier. 16 sequences of 100 steps, H = 36: 62 us; 77 with
+// six shuffles and every lane evaluating both sigmoids, 156 with the weights in shared memory and three barriers.
 constexpr int GRU_CHUNK = 64;
 __host__ __device__ constexpr int gru_hp(int nv) { return 16 * nv; }          // h and x rows padded with zeros
 template <typename T, int NV>
@@ -57,9 +68,7 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
       wh[g][i] = (unit && k < H) ? to_f32<T>(h2h[k * G + g * H + u]) : 0.f;
     }
   const float bij = tid < G ? to_f32<T>(bi[tid]) : 0.f;
-  float bhu[3];
-#pragma unroll
-  for (int g = 0; g < 3; ++g) bhu[g] = unit ? to_f32<T>(bh[g * H + u]) : 0.f;
+  const float bh_l = (unit && l < 3) ? to_f32<T>(bh[l * H + u]) : 0.f;
   for (int i = tid; i < 2 * HP; i += blockDim.x) (&hbuf[0][0])[i] = 0.f;
   bool started = false;
   float h = 0.f;
@@ -67,23 +76,39 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
     const int n = min(GRU_CHUNK, steps - t0);
     __syncthreads();                               // the last chunk's rows have been used
     const T* xb = x + (b * steps + t0) * H;
-    for (int i = tid; i < n * HP; i += blockDim.x) {
-      const int t = i / HP, k = i - t * HP;
-      xs[i] = k < H ? to_f32<T>(xb[t * H + k]) : 0.f;
+    for (int i0 = tid; i0 < n * HP; i0 += 8 * blockDim.x) {       // eight loads in flight
+      float v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = i0 + e * (int)blockDim.x, t = i / HP, k = i - t * HP;
+        v[e] = i < n * HP && k < H ? to_f32<T>(xb[t * H + k]) : 0.f;
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = i0 + e * (int)blockDim.x;
+        if (i < n * HP) xs[i] = v[e];
+      }
     }
     for (int i = tid; i < n; i += blockDim.x) nonzero[i] = 0;
     __syncthreads();
     if (tid < G) {
-#pragma unroll 4
-      for (int t = 0; t < n; ++t) {
-        float p = 0.f;
+      for (int t = 0; t < n; t += 4) {                            // four independent chains (rows past n are not kept)
+        float q[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int k = 0; k < HP; k += 4) {
-          const float4 v = *reinterpret_cast<const float4*>(xs + t * HP + k);
-          p = fmaf(v.x, wi[k], p); p = fmaf(v.y, wi[k + 1], p); p = fmaf(v.z, wi[k + 2], p); p = fmaf(v.w, wi[k + 3], p);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float4 v = *reinterpret_cast<const float4*>(xs + (t + e) * HP + k);
+            q[e] = fmaf(v.x, wi[k], q[e]); q[e] = fmaf(v.y, wi[k + 1], q[e]); q[e] = fmaf(v.z, wi[k + 2], q[e]); q[e] = fmaf(v.w, wi[k + 3], q[e]);
+          }
         }
-        if (tid < H && p != 0.f) nonzero[t] = 1;
-        pre[t * G + tid] = p + bij;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (t + e < n) {
+            if (tid < H && q[e] != 0.f) nonzero[t + e] = 1;
+            pre[(t + e) * G + tid] = q[e] + bij;
+          }
+        }
       }
     }
     __syncthreads();
@@ -94,8 +119,7 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
         if (unit && l == 0) y[at] = from_f32<T>(0.f);
         continue;
       }
-      float pr = 0.f, pz = 0.f, pc = 0.f;
-      if (unit) { pr = pre[t * G + u]; pz = pre[t * G + H + u]; pc = pre[t * G + 2 * H + u]; }
+      const float pre_l = (unit && l < 3) ? pre[t * G + l * H + u] : 0.f;      // lane 0: r, lane 1: z, lane 2: candidate
       const float4* hv = reinterpret_cast<const float4*>(hbuf[t & 1]);
       float a[3][2] = {};
 #pragma unroll
@@ -109,19 +133,18 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
           a[g][1] = fmaf(v.w, wh[g][4 * i + 3], a[g][1]);
         }
       }
-      float s[3];
-#pragma unroll
-      for (int g = 0; g < 3; ++g) {
-        s[g] = a[g][0] + a[g][1];
-        s[g] += __shfl_xor_sync(0xffffffffu, s[g], 1);
-        s[g] += __shfl_xor_sync(0xffffffffu, s[g], 2);
-        s[g] += bhu[g];
-      }
-      const float r = sigm(pr + s[0]);
-      const float z = sigm(pz + s[1]);
-      const float c = tanhf(pc + r * s[2]);
+      const float sr = a[0][0] + a[0][1], sz = a[1][0] + a[1][1], sc = a[2][0] + a[2][1];
+      // even lanes collect r and the candidate, odd lanes z; then lane 0 r, lane 2 the candidate
+      float keep = (l & 1) ? sz : sr;
+      keep += __shfl_xor_sync(0xffffffffu, (l & 1) ? sr : sz, 1);
+      float cand = sc + __shfl_xor_sync(0xffffffffu, sc, 1);
+      const float other = __shfl_xor_sync(0xffffffffu, l == 0 ? cand : keep, 2);
+      const float sum = (l == 2 ? cand : keep) + other + bh_l;
+      const float gate = sigm(pre_l + sum);                                    // lanes 0 and 1
+      const float r = __shfl_sync(0xffffffffu, gate, (threadIdx.x & 28)), z = __shfl_sync(0xffffffffu, gate, (threadIdx.x & 28) + 1);
+      const float c = tanhf(pre_l + r * sum);                                  // lane 2
       h = c + z * (h - c);
-      if (unit && l == 0) {
+      if (unit && l == 2) {
         hbuf[(t + 1) & 1][u] = h;
         y[at] = from_f32<T>(h);
       }
@@ -135,10 +158,8 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
 // AUGRU after VecAttGRUCell.call (xdl-algorithm-solution/DIEN/script/utils.py:139-207):
 // [r|u] = sigmoid([x,h] Wg + bg); c = tanh([x, r*h] Wc + bc); u' = (1 - a_t) u; h' = u' h + (1 - u') c.
 // Wg [2H, 2H] (rows x then h; columns r then u), Wc [2H, H]; att [B, T].
-// `share` > 0: the input sequence is shared by groups of `share` consecutive batch entries (x is [B / share, T, H],
-// the candidates of one request), and only the final state is written (y is [B, H]).
 __global__ void augru_kernel(const void* x, const void* att, void* y, int T, int H, const void* Wg_, const void* bg_,
-                             const void* Wc_, const void* bc_, int dt, int share) {
+                             const void* Wc_, const void* bc_, int dt) {
   pdl_begin();
   extern __shared__ float sm[];
   float* Wg = sm;                     // [2H][2H]
@@ -156,8 +177,7 @@ __global__ void augru_kernel(const void* x, const void* att, void* y, int T, int
   __syncthreads();
   for (int t = 0; t < T; ++t) {
     const int64_t base = (b * T + t) * H;
-    const int64_t xbase = share > 0 ? ((b / share) * T + t) * H : base;
-    if (j < H) xs[j] = load_as_f32(x, xbase + j, dt);
+    if (j < H) xs[j] = load_as_f32(x, base + j, dt);
     __syncthreads();
     if (j < G) {
       float s = bgj;
@@ -176,12 +196,112 @@ __global__ void augru_kernel(const void* x, const void* att, void* y, int T, int
       const float a = load_as_f32(att, b * T + t, dt);
       const float u = (1.f - a) * g[H + j];
       out = u * h[j] + (1.f - u) * tanhf(s);
-      if (share <= 0) store_from_f32(y, base + j, dt, out);
-      else if (t == T - 1) store_from_f32(y, b * H + j, dt, out);
+      store_from_f32(y, base + j, dt, out);
     }
     __syncthreads();
     if (j < H) h[j] = out;
   }
+}
+
+// AUGRU over a request's shared sequence in fp32, for widths the tensor-core engine does not take (and on request): x is
+// [requests, T, H], att [requests * n_cand, T], only the final states y [requests * n_cand, H] are written.
+// A CTA owns AS_CAND candidates of one request. The terms of x_t are the same for all of them: each chunk of steps they
+// are made once, a gate column per thread. A candidate is four lanes per unit with their quarter of the unit's three
+// recurrent columns in registers (as gru_kernel), and two barriers of its own threads a step: r*h, then h.
+// 4 requests of 1000 candidates, 100 steps, H = 32: 418 us,
+// 973 with a block per candidate and the weights in shared memory
+constexpr int AS_CAND = 4, AS_CHUNK = 32;
+template <int NV>
+__global__ void __launch_bounds__(AS_CAND * 64 * NV > 1024 ? 1024 : AS_CAND * 64 * NV)
+augru_shared_kernel(const __half* __restrict__ x, const __half* __restrict__ att, __half* __restrict__ y, int n_cand, int steps, int H,
+                    const __half* __restrict__ Wg, const __half* __restrict__ bg, const __half* __restrict__ Wc,
+                    const __half* __restrict__ bc, int cands, int group_threads, int blocks_per_req) {
+  constexpr int HP = gru_hp(NV);
+  extern __shared__ __align__(16) float as_sm[];
+  float* xs = as_sm;                                           // [AS_CHUNK][HP]
+  float* px = xs + AS_CHUNK * HP;                              // [AS_CHUNK][3H]: x_t Wg_x + bg (r, u), x_t Wc_x + bc
+  __shared__ __align__(16) float hbuf[AS_CAND][2][HP];
+  __shared__ __align__(16) float rhbuf[AS_CAND][HP];
+  pdl_begin();
+  const int tid = threadIdx.x, G = 3 * H;
+  const int r = blockIdx.x / blocks_per_req, cand = tid / group_threads, gt = tid - cand * group_threads;
+  const int n = (blockIdx.x - r * blocks_per_req) * cands + cand;
+  const int u = gt >> 2, l = gt & 3;
+  const bool unit = u < H && n < n_cand;
+  float wr[4 * NV], wu[4 * NV], wc[4 * NV];
+#pragma unroll
+  for (int i = 0; i < 4 * NV; ++i) {
+    const int k = 4 * (4 * (i >> 2) + l) + (i & 3);
+    const bool in = u < H && k < H;
+    wr[i] = in ? __half2float(Wg[(H + k) * 2 * H + u]) : 0.f;
+    wu[i] = in ? __half2float(Wg[(H + k) * 2 * H + H + u]) : 0.f;
+    wc[i] = in ? __half2float(Wc[(H + k) * H + u]) : 0.f;
+  }
+  for (int i = gt; i < 2 * HP; i += group_threads) (&hbuf[cand][0][0])[i] = 0.f;
+  for (int i = gt; i < HP; i += group_threads) rhbuf[cand][i] = 0.f;
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(cand + 1), "r"(group_threads) : "memory"); };
+  const __half* arow = att + ((int64_t)r * n_cand + min(n, n_cand - 1)) * steps;
+  float h = 0.f;
+  for (int t0 = 0; t0 < steps; t0 += AS_CHUNK) {
+    const int m = min(AS_CHUNK, steps - t0);
+    __syncthreads();
+    for (int i = tid; i < m * HP; i += blockDim.x) {
+      const int t = i / HP, k = i - t * HP;
+      xs[i] = k < H ? __half2float(x[((int64_t)r * steps + t0 + t) * H + k]) : 0.f;
+    }
+    __syncthreads();
+    for (int idx = tid; idx < m * G; idx += blockDim.x) {
+      const int t = idx / G, j = idx - t * G;
+      const bool gate = j < 2 * H;
+      const __half* W = gate ? Wg + j : Wc + j - 2 * H;
+      const int ld = gate ? 2 * H : H;
+      float s = __half2float(gate ? bg[j] : bc[j - 2 * H]);
+#pragma unroll 8
+      for (int k = 0; k < H; ++k) s = fmaf(xs[t * HP + k], __half2float(__ldg(W + k * ld)), s);
+      px[idx] = s;
+    }
+    __syncthreads();
+    for (int t = 0; t < m; ++t) {
+      const float a = __half2float(__ldg(arow + t0 + t));
+      float pr = 0.f, pu = 0.f, pc = 0.f;
+      if (unit) { pr = px[t * G + u]; pu = px[t * G + H + u]; pc = px[t * G + 2 * H + u]; }
+      const float4* hv = reinterpret_cast<const float4*>(hbuf[cand][t & 1]);
+      float ar = 0.f, au = 0.f, ac = 0.f;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const float4 v = hv[4 * i + l];
+        ar = fmaf(v.x, wr[4 * i], ar); ar = fmaf(v.y, wr[4 * i + 1], ar); ar = fmaf(v.z, wr[4 * i + 2], ar); ar = fmaf(v.w, wr[4 * i + 3], ar);
+        au = fmaf(v.x, wu[4 * i], au); au = fmaf(v.y, wu[4 * i + 1], au); au = fmaf(v.z, wu[4 * i + 2], au); au = fmaf(v.w, wu[4 * i + 3], au);
+      }
+      ar += __shfl_xor_sync(0xffffffffu, ar, 1); ar += __shfl_xor_sync(0xffffffffu, ar, 2);
+      au += __shfl_xor_sync(0xffffffffu, au, 1); au += __shfl_xor_sync(0xffffffffu, au, 2);
+      const float rg = sigm(pr + ar);
+      if (unit && l == 0) rhbuf[cand][u] = rg * h;
+      group_sync();
+      const float ug = (1.f - a) * sigm(pu + au);
+      const float4* rv = reinterpret_cast<const float4*>(rhbuf[cand]);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const float4 v = rv[4 * i + l];
+        ac = fmaf(v.x, wc[4 * i], ac); ac = fmaf(v.y, wc[4 * i + 1], ac); ac = fmaf(v.z, wc[4 * i + 2], ac); ac = fmaf(v.w, wc[4 * i + 3], ac);
+      }
+      ac += __shfl_xor_sync(0xffffffffu, ac, 1); ac += __shfl_xor_sync(0xffffffffu, ac, 2);
+      h = ug * h + (1.f - ug) * tanhf(pc + ac);
+      if (unit && l == 0) hbuf[cand][(t + 1) & 1][u] = h;
+      group_sync();
+    }
+  }
+  if (unit && l == 0) y[((int64_t)r * n_cand + n) * H + u] = __float2half_rn(h);
+}
+
+template <int NV>
+int launch_augru_shared(const AuParams& p, cudaStream_t s) {
+  const int gt = (4 * p.H + 31) / 32 * 32, cands = std::min(AS_CAND, 1024 / gt), bpr = (p.n_cand + cands - 1) / cands;
+  XB_REQUIRE((int64_t)p.requests * bpr < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_augru_shared: batch too large");
+  const size_t smem = sizeof(float) * AS_CHUNK * (size_t)(gru_hp(NV) + 3 * p.H);
+  launch_dependent(augru_shared_kernel<NV>, (unsigned)(p.requests * bpr), cands * gt, smem, s, p.x, p.att, p.y, p.n_cand, p.T, p.H, p.Wg,
+                   p.bg, p.Wc, p.bc, cands, gt, bpr);
+  return check_launch("augru_shared_kernel");
 }
 
 template <typename T, int NV>
@@ -206,8 +326,6 @@ int launch_gru(const T* x, T* y, int64_t batch, int steps, int H, const T* i2h, 
 
 }  // namespace
 }  // namespace xb
-
-#include "xb_augru_tc.cuh"
 
 namespace xb {
 int rnn_status(int* out) { return umma::read_status_word(out); }
@@ -245,7 +363,7 @@ extern "C" int xb_augru(const void* x, const void* att, void* y, int64_t batch, 
   static PerDeviceOnce attr;
   XB_SET_MAX_SMEM_ONCE(attr, 110 * 1024, (const void*)augru_kernel);
   const int threads = (2 * H + 31) / 32 * 32;
-  launch_dependent(augru_kernel, (unsigned)batch, threads, smem, (cudaStream_t)s, x, att, y, T, H, Wg, bg, Wc, bc, dtype, 0);
+  launch_dependent(augru_kernel, (unsigned)batch, threads, smem, (cudaStream_t)s, x, att, y, T, H, Wg, bg, Wc, bc, dtype);
   return check_launch("augru_kernel");
 }
 
@@ -260,20 +378,17 @@ extern "C" int xb_augru_shared(const void* x, const void* att, void* y_final, in
   const bool tc = engine != XB_GEMM_SIMT && augru_tc_eligible(H, T);
   XB_REQUIRE(tc || engine != XB_GEMM_TCGEN05, XB_ERR_UNSUPPORTED,
              "xb_augru_shared: the tcgen05 engine takes an even H <= 64 whose padding to a multiple of 8 leaves 4 slots");
-  if (tc) {
-    AuParams p;
-    memset(&p, 0, sizeof(p));
-    p.x = (const __half*)x; p.att = (const __half*)att; p.y = (__half*)y_final;
-    p.Wg = (const __half*)Wg; p.bg = (const __half*)bg; p.Wc = (const __half*)Wc; p.bc = (const __half*)bc;
-    p.requests = requests; p.n_cand = n_cand; p.T = T; p.H = H;
-    return launch_augru_tc(p, (cudaStream_t)s);
+  AuParams p;
+  memset(&p, 0, sizeof(p));
+  p.x = (const __half*)x; p.att = (const __half*)att; p.y = (__half*)y_final;
+  p.Wg = (const __half*)Wg; p.bg = (const __half*)bg; p.Wc = (const __half*)Wc; p.bc = (const __half*)bc;
+  p.requests = requests; p.n_cand = n_cand; p.T = T; p.H = H;
+  if (tc) return launch_augru_tc(p, (cudaStream_t)s);
+  XB_REQUIRE((int64_t)requests * n_cand < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_augru_shared: batch too large");
+  switch ((H + 15) / 16) {
+    case 1: return launch_augru_shared<1>(p, (cudaStream_t)s);
+    case 2: return launch_augru_shared<2>(p, (cudaStream_t)s);
+    case 3: return launch_augru_shared<3>(p, (cudaStream_t)s);
+    default: return launch_augru_shared<4>(p, (cudaStream_t)s);
   }
-  const int64_t batch = (int64_t)requests * n_cand;
-  XB_REQUIRE(batch < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_augru_shared: batch too large");
-  const size_t smem = sizeof(float) * ((size_t)6 * H * H + 5 * H);
-  static PerDeviceOnce attr;
-  XB_SET_MAX_SMEM_ONCE(attr, 110 * 1024, (const void*)augru_kernel);
-  const int threads = (2 * H + 31) / 32 * 32;
-  launch_dependent(augru_kernel, (unsigned)batch, threads, smem, (cudaStream_t)s, x, att, y_final, T, H, Wg, bg, Wc, bc, XB_F16, n_cand);
-  return check_launch("augru_kernel");
 }
