@@ -33,7 +33,6 @@ struct PoolGroupDev {
   const void* values;
   const int32_t* offsets;      // exclusive offsets [batch+1]
   int64_t rows, pitch, slot_mask, batch;
-  int64_t warp_begin;          // first warp of this group in the launch
   int32_t dim, tdtype, id_dtype, out_dtype, n_items, has_table;
   int32_t lpr;                 // lanes per row
   int32_t tl;                  // lanes per segment (team)
@@ -46,8 +45,20 @@ struct PoolGroupDev {
 struct PoolParams {
   int32_t n_groups;
   int64_t total_warps;
+  int64_t warp_begin[XB_MAX_POOL_GROUPS];      // first warp of each group in the launch
   PoolGroupDev g[XB_MAX_POOL_GROUPS];
 };
+
+// The group a warp works for. Kernel parameters come through the constant cache, cold at every launch: walking the groups
+// themselves would wait for one line after another (a group is several), so the first warps lie side by side and the lanes
+// look at one each. Twelve groups of 64 lists:
+// 5.9 -> 5.5 us; twenty of 512: 11.2 -> 10.7.
+__device__ __forceinline__ int pool_find_group(const PoolParams& p, int64_t warp_id) {
+  const int lane = threadIdx.x & 31;
+  static_assert(XB_MAX_POOL_GROUPS <= 32, "one lane per group");
+  const unsigned m = __ballot_sync(0xffffffffu, lane < p.n_groups && p.warp_begin[lane < XB_MAX_POOL_GROUPS ? lane : 0] <= warp_id);
+  return 31 - __clz(m);                        // group 0 begins with warp 0
+}
 
 struct ScanParams {
   int32_t n;
@@ -277,8 +288,7 @@ __global__ void __launch_bounds__(256) pool_kernel(const __grid_constant__ PoolP
   const int64_t warp_id = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (warp_id >= p.total_warps) return;      // whole warp leaves together
   const int lane = threadIdx.x & 31;
-  int gi = 0;
-  while (gi + 1 < p.n_groups && p.g[gi + 1].warp_begin <= warp_id) ++gi;
+  const int gi = pool_find_group(p, warp_id);
   const PoolGroupDev& g = p.g[gi];
 
   const int tl = g.tl, lpr = g.lpr;
@@ -287,7 +297,7 @@ __global__ void __launch_bounds__(256) pool_kernel(const __grid_constant__ PoolP
   const int ns = tl / lpr;
   const int epc = (g.tdtype == XB_F32) ? 4 : 8;          // elements per 16-byte chunk
   const int col0 = chunk * epc;
-  const int64_t seg = (warp_id - g.warp_begin) * (32 / tl) + team;
+  const int64_t seg = (warp_id - p.warp_begin[gi]) * (32 / tl) + team;
   const bool active = seg < g.batch;
   const bool loads = active && g.has_table && col0 < g.dim;
 
@@ -480,8 +490,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
   const int64_t warp_id = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (warp_id >= p.total_warps) return;              // whole warp leaves together
   const int lane = threadIdx.x & 31;
-  int gi = 0;
-  while (gi + 1 < p.n_groups && p.g[gi + 1].warp_begin <= warp_id) ++gi;
+  const int gi = pool_find_group(p, warp_id);
   const PoolGroupDev& g = p.g[gi];
   const PoolItemDev& it = g.items[0];
 
@@ -503,7 +512,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
   const int64_t batch = g.batch;
   // this warp walks `segs` consecutive rounds of `spw` segments; the offsets of round i+2 and the ids of
   // round i+1 are fetched while the rows of round i are in flight
-  const int64_t seg_first = (warp_id - g.warp_begin) * segs * spw + lane / tl;
+  const int64_t seg_first = (warp_id - p.warp_begin[gi]) * segs * spw + lane / tl;
 
   auto load_span = [&](int i, int& st, int& nm) {
     const int64_t sg = seg_first + (int64_t)i * spw;
@@ -661,13 +670,12 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
   const int64_t warp_id = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (warp_id >= p.total_warps) return;
   const int lane = threadIdx.x & 31;
-  int gi = 0;
-  while (gi + 1 < p.n_groups && p.g[gi + 1].warp_begin <= warp_id) ++gi;
+  const int gi = pool_find_group(p, warp_id);
   const PoolGroupDev& g = p.g[gi];
   const PoolItemDev& it = g.items[0];
   const int chunk = lane & (LPR - 1);
   const int rounds = g.segs;                         // consecutive rounds of SPW segments this warp walks
-  const int64_t seg0 = (warp_id - g.warp_begin) * rounds * SPW + lane / LPR;
+  const int64_t seg0 = (warp_id - p.warp_begin[gi]) * rounds * SPW + lane / LPR;
   const int64_t batch = g.batch;
   const int dim = g.dim, col0 = chunk * EPC;
   const bool cvalid = col0 < dim;
@@ -765,8 +773,7 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
   const int64_t warp_id = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (warp_id >= p.total_warps) return;
   const int lane = threadIdx.x & 31;
-  int gi = 0;
-  while (gi + 1 < p.n_groups && p.g[gi + 1].warp_begin <= warp_id) ++gi;
+  const int gi = pool_find_group(p, warp_id);
   const PoolGroupDev& g = p.g[gi];
   const PoolItemDev& it = g.items[0];
 
@@ -780,7 +787,7 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
   const char* wrow = g.weights + tlane * 16;
   const int pitch = (int)g.pitch;
   const uint64_t keep = l2_policy_keep();
-  const int64_t s0 = (warp_id - g.warp_begin) * g.segs;
+  const int64_t s0 = (warp_id - p.warp_begin[gi]) * g.segs;
   const int nseg = (int)min((int64_t)g.segs, g.batch - s0);
 
   // lane l keeps the span of segment s0 + l
@@ -1166,7 +1173,7 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
     const bool short_ok = all_short && fast && d.tl == d.lpr &&
                           (hp[bucket].n_groups == 0 || (hp[bucket].g[0].id_dtype == XB_REC64) == (h.id_dtype == XB_REC64));
     PoolParams& dst = short_ok ? hp[bucket] : queue_ok ? qp[bucket] : fast ? fp[bucket] : p;
-    d.warp_begin = dst.total_warps;
+    dst.warp_begin[dst.n_groups] = dst.total_warps;
     const int spw = 32 / d.tl;
     const int64_t rounds = (h.batch + spw - 1) / spw;
     const bool counts_ok = fast && !short_ok && !queue_ok && !h.segments_are_offsets && h.batch <= POOL_INLINE_COUNTS;
@@ -1186,7 +1193,9 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
     }
     // the specialised kernel gives a warp several rounds, as long as every SM still gets dozens of warps
     d.segs = 1;
-    if (fast) d.segs = (int)std::max<int64_t>(1, std::min<int64_t>(8, rounds / ((int64_t)sm_count() * 48)));
+    // (dozens less with a list of one or two ids, whose warp is a chain of latencies: its rounds overlap, while a second
+    // wave of warps would begin the chain again: 2 x 74 000 single ids and their requests' lists 17.7 -> 13.1 us.)
+    if (fast) d.segs = (int)std::max<int64_t>(1, std::min<int64_t>(8, rounds / ((int64_t)sm_count() * (avg < 3.0 ? 12 : 48))));
     // the short-segment kernel walks 8 rounds per warp (its prefetch needs a few), fewer only for small groups
     if (short_ok) d.segs = (int)std::max<int64_t>(1, std::min<int64_t>(8, rounds / ((int64_t)sm_count() * 16)));
     if (queue_ok && !short_ok) {
