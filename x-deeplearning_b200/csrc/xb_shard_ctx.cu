@@ -22,6 +22,10 @@
 #include "xb_common.cuh"
 
 namespace xb {
+
+// xb_pool.cu
+int record_offsets_padded(const int64_t* packed, int sources, int64_t bucket_cap, int32_t* offsets, int64_t segments, cudaStream_t stream);
+
 namespace {
 
 // ---- NCCL, bound at run time -----------------------------------------------------------------------------
@@ -94,14 +98,13 @@ struct xb_shard_ctx {
   cudaEvent_t slot_ready[2] = {nullptr, nullptr};   // recorded when a slot's id exchange has been enqueued
   cudaEvent_t slot_free[2] = {nullptr, nullptr};    // recorded when the pooling that reads a slot has been enqueued
   int begun = 0, finished = 0;                      // steps begun / finished so far (begun - finished <= 2)
-  int32_t *counts = nullptr, *offsets = nullptr;    // [world * S], [world * (S + 1)]
+  int32_t* offsets = nullptr;                       // [world * (S + 1)]
   char *partial = nullptr, *back = nullptr;         // [world * S * dim] partial sums (partial_dtype): the slot in use
   char *partial2[2] = {nullptr, nullptr}, *back2[2] = {nullptr, nullptr};   // two slots: a pooled step and the one before it
   cudaEvent_t back_ready[2] = {nullptr, nullptr};   // recorded when a slot's partial-sum exchange has been enqueued
   cudaEvent_t back_free[2] = {nullptr, nullptr};    // recorded when the combine that reads a slot has been enqueued
   int pooled = 0;                                   // steps whose middle part has been enqueued (finished counts combines)
   void* route_scratch = nullptr; size_t route_scratch_bytes = 0;
-  void* scan_scratch = nullptr; size_t scan_scratch_bytes = 0;
   int32_t* overflow_dev = nullptr;                  // device view of the mapped flag
   volatile int32_t* overflow_host = nullptr;
   // optional phase timing: events recorded at the phase boundaries of the last xb_sharded_pool call
@@ -176,8 +179,6 @@ extern "C" int xb_shard_ctx_create(xb_shard_ctx** out, const void* unique_id128,
   const int W = c->world;
   const size_t esz = c->partial_dtype == XB_F32 ? 4 : 2;
   c->route_scratch_bytes = xb_route_scratch_bytes(c->max_ids, W);
-  const int groups_per_scan = std::min(W, XB_MAX_POOL_GROUPS);
-  c->scan_scratch_bytes = xb_scan_counts_scratch_bytes(groups_per_scan, c->S);
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t at = off; off += align256(bytes); return at; };
   // One rank: what it sends is what it receives, so both exchanges read their source in place (the slots' events order
@@ -186,11 +187,11 @@ extern "C" int xb_shard_ctx_create(xb_shard_ctx** out, const void* unique_id128,
   auto take_recv = [&](size_t bytes, size_t sent) { return W == 1 ? sent : take(bytes); };
   const size_t o_send = take((size_t)W * c->cap * 8), o_recv = take_recv((size_t)W * c->cap * 8, o_send);
   const size_t o_send1 = take((size_t)W * c->cap * 8), o_recv1 = take_recv((size_t)W * c->cap * 8, o_send1);
-  const size_t o_counts = take((size_t)W * c->S * 4), o_offsets = take((size_t)W * (c->S + 1) * 4);
+  const size_t o_offsets = take((size_t)W * (c->S + 1) * 4);
   const size_t partial_bytes = (size_t)W * c->S * c->dim * esz;
   const size_t o_partial = take(partial_bytes), o_back = take_recv(partial_bytes, o_partial);
   const size_t o_partial1 = take(partial_bytes), o_back1 = take_recv(partial_bytes, o_partial1);
-  const size_t o_route = take(c->route_scratch_bytes), o_scan = take(c->scan_scratch_bytes);
+  const size_t o_route = take(c->route_scratch_bytes);
   c->arena_bytes = off;
   XB_CUDA(cudaMalloc(reinterpret_cast<void**>(&c->arena), c->arena_bytes));
   c->send2[0] = reinterpret_cast<int64_t*>(c->arena + o_send); c->recv2[0] = reinterpret_cast<int64_t*>(c->arena + o_recv);
@@ -198,13 +199,13 @@ extern "C" int xb_shard_ctx_create(xb_shard_ctx** out, const void* unique_id128,
   c->send = c->send2[0]; c->recv = c->recv2[0];
   for (cudaEvent_t& e : c->slot_ready) XB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (cudaEvent_t& e : c->slot_free) XB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  c->counts = reinterpret_cast<int32_t*>(c->arena + o_counts); c->offsets = reinterpret_cast<int32_t*>(c->arena + o_offsets);
+  c->offsets = reinterpret_cast<int32_t*>(c->arena + o_offsets);
   c->partial2[0] = c->arena + o_partial; c->back2[0] = c->arena + o_back;
   c->partial2[1] = c->arena + o_partial1; c->back2[1] = c->arena + o_back1;
   c->partial = c->partial2[0]; c->back = c->back2[0];
   for (cudaEvent_t& e : c->back_ready) XB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (cudaEvent_t& e : c->back_free) XB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  c->route_scratch = c->arena + o_route; c->scan_scratch = c->arena + o_scan;
+  c->route_scratch = c->arena + o_route;
   int32_t* flag = nullptr;
   XB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&flag), 64, cudaHostAllocMapped | cudaHostAllocPortable));
   *flag = 0;
@@ -295,13 +296,8 @@ extern "C" int xb_sharded_pool_pool(xb_shard_ctx* c, xb_stream_t stream_) {
   // the combine that read this slot's partial sums two steps ago may still be running on another stream
   if (c->pooled >= 2) XB_CUDA(cudaStreamWaitEvent(stream, c->back_free[slot], 0));
   mark(c, 2, stream);
-  // 2. at the owner: segment lengths per source from the received records, offsets per source
-  if (int rc = xb_record_counts_padded(recv, W, c->cap, c->counts, c->S, stream)) return rc;
-  for (int s0 = 0; s0 < W; s0 += XB_MAX_POOL_GROUPS) {
-    const int n = std::min(W - s0, (int)XB_MAX_POOL_GROUPS);
-    if (int rc = xb_scan_counts(c->counts + (int64_t)s0 * c->S, c->S, c->offsets + (int64_t)s0 * (c->S + 1), c->S + 1, n, c->S,
-                                c->scan_scratch, c->scan_scratch_bytes, stream)) return rc;
-  }
+  // 2. at the owner: the segments' offsets per source from the received records
+  if (int rc = record_offsets_padded(recv, W, c->cap, c->offsets, c->S, stream)) return rc;
   mark(c, 3, stream);
   // 3. pool every (source, table) segment range against that table's shard
   if (int rc = xb_shard_pool_records(c->tables.data(), c->table_segments.data(), c->n_tables, recv, c->cap, c->offsets, W,
