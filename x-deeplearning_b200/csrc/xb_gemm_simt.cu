@@ -4,22 +4,26 @@
 // 1e-6 operator fixtures need true fp32 products, not tf32), transposed A,
 // leading dimensions that break TMA's 16-byte rule, and tiny shapes.
 //
-// 256 threads as 16 x 16, TM x TN outputs each (tile 16*TM x 16*TN), 16-deep k
-// slices double-buffered in shared memory, the next slice on its way to
-// registers while the current one is multiplied; fp32 accumulation with k
-// ascending, whatever the tile.
-// What bounds it is the FMA rate where the launch fills the chip: a thread reads
-// TM values of A as 16-byte vectors (two addresses a warp: a broadcast) and TN
-// scalars of B for TM*TN FMAs, so the shared-memory pipe stays below the FMA
-// pipe from 8 x 4 up. [50000, 144] x [144, 80] fp32
-// with Dice: 114 us, 230 with the 64 x 64 tile of 4 x 4 outputs this replaces (a second column of tiles three
-// quarters empty, four scalar reads of each operand for 16 FMAs).
+// 256 threads, tile 16*TM x 16*TN, 16-deep k slices; fp32 accumulation with k
+// ascending, whatever the tile, so every form gives the same bits.
+// gemm_f32_kernel (fp32, neither operand transposed: Blaze's own layout) keeps
+// a ring of slices in flight with cp.async, which hides the latency that bounds
+// a small launch. What bounds a large one is instructions: with one FMA an
+// instruction the schedulers issued in a third of the cycles (43 % of the stalls
+// were instruction fetches), so two columns' FMAs go into one fma.rn.f32x2
+// (each rounded as an FMA of its own) and a thread owns pairs of adjacent
+// columns. [50000, 144] x [144, 80]: 75 us (scalar FMAs 85, the general
+// kernel 114); [8192, 512] x [512, 512]: 150 us, 29 TFLOP/s.
+// gemm_simt_kernel is the general form: any type, layout and alignment, the next
+// slice on its way to registers while the current one is multiplied.
+#include <algorithm>
+
 #include "xb_common.cuh"
 
 namespace xb {
 
 struct SimtGemmParams {
-  int tiles_n;
+  int tiles_n, y_pairs;
   int M, N, K, trans_a, trans_b, in_dtype, y_dtype, a_vec, b_vec;
   float alpha, beta;
   const void* A; int64_t lda, stride_a;
@@ -94,6 +98,28 @@ struct SimtSlice {
   }
 };
 
+// What an output column needs beside its sum, read once per thread and column; then bias and activation of one output.
+struct Column { float bias, a, b, c; };
+__device__ __forceinline__ Column column_of(const SimtGemmParams& p, int b, int gn) {
+  Column o = {0.f, 0.f, 0.f, 0.f};
+  const int64_t eo = (int64_t)b * p.stride_ep + gn;
+  if (p.bias_kind == XB_BIAS_ROW) o.bias = load_as_f32(p.bias, (int64_t)b * p.stride_bias + gn, p.bias_dtype);
+  if (p.epi.kind == XB_EPI_PRELU) o.a = p.epi.a[p.epi.count == 1 ? (int64_t)b * p.stride_ep : eo];
+  if (p.epi.kind == XB_EPI_DICE) { o.a = p.epi.a[eo]; o.b = p.epi.b[eo]; o.c = dice_rstd(p.epi.c[eo], p.epi.nosqrt); }
+  return o;
+}
+__device__ __forceinline__ float finish(const SimtGemmParams& p, const Column& c, int b, int gm, int gn, float acc) {
+  float v = p.alpha * acc;
+  if (p.bias_kind == XB_BIAS_ROW)
+    v += p.beta * c.bias;
+  else if (p.bias_kind == XB_BIAS_FULL)
+    v += p.beta * load_as_f32(p.bias, (int64_t)b * p.stride_bias + (int64_t)(gm / p.bias_group) * p.ldbias + gn, p.bias_dtype);
+  if (p.epi.kind == XB_EPI_PRELU) return act_prelu(v, c.a);
+  if (p.epi.kind == XB_EPI_DICE) return act_dice(v, c.a, c.b, c.c);
+  if (p.epi.kind == XB_EPI_SIGMOID) return act_sigmoid(v);
+  return v;
+}
+
 template <int TM, int TN>
 __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(const __grid_constant__ SimtGemmParams p) {
   pdl_begin();
@@ -161,49 +187,191 @@ __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(c
     }
   }
 
-  EpiParams epi = p.epi;
-  if (epi.a) epi.a += (int64_t)b * p.stride_ep;
-  if (epi.b) epi.b += (int64_t)b * p.stride_ep;
-  if (epi.c) epi.c += (int64_t)b * p.stride_ep;
 #pragma unroll
   for (int j = 0; j < TN; ++j) {
     const int gn = n0 + tx + 16 * j;
     if (gn >= p.N) continue;
-    const float rb = p.bias_kind == XB_BIAS_ROW ? load_as_f32(p.bias, (int64_t)b * p.stride_bias + gn, p.bias_dtype) : 0.f;
+    const Column c = column_of(p, b, gn);
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       const int gm = m0 + ty * TM + i;
-      if (gm >= p.M) continue;
-      float v = p.alpha * acc[i][j];
-      if (p.bias_kind == XB_BIAS_ROW)
-        v += p.beta * rb;
-      else if (p.bias_kind == XB_BIAS_FULL)
-        v += p.beta * load_as_f32(p.bias, (int64_t)b * p.stride_bias + (int64_t)(gm / p.bias_group) * p.ldbias + gn, p.bias_dtype);
-      v = apply_epilogue(epi, v, gn);
-      store_from_f32(p.Y, (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + gn, p.y_dtype, v);
+      if (gm < p.M) store_from_f32(p.Y, (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + gn, p.y_dtype, finish(p, c, b, gm, gn, acc[i][j]));
     }
   }
 }
 
-template <int TM>
-static void launch_simt_tm(const SimtGemmParams& p, int tn, dim3 grid, cudaStream_t s) {
-  switch (tn) {
-    case 1: launch_dependent(gemm_simt_kernel<TM, 1>, grid, 256, 0, s, p); break;
-    case 2: launch_dependent(gemm_simt_kernel<TM, 2>, grid, 256, 0, s, p); break;
-    case 3: launch_dependent(gemm_simt_kernel<TM, 3>, grid, 256, 0, s, p); break;
-    case 4: launch_dependent(gemm_simt_kernel<TM, 4>, grid, 256, 0, s, p); break;
-    case 5: launch_dependent(gemm_simt_kernel<TM, 5>, grid, 256, 0, s, p); break;
-    case 6: launch_dependent(gemm_simt_kernel<TM, 6>, grid, 256, 0, s, p); break;
-    default: launch_dependent(gemm_simt_kernel<TM, 8>, grid, 256, 0, s, p); break;
+// fp32, A [M, K] and B [K, N] as they lie. A ring of F32_STAGES slices: A as [row][k] (pitch 20: a warp's two rows on other
+// banks), B as [k][column]; 16-byte copies where the operand's rows allow, 4-byte ones otherwise, zeros past the edges.
+constexpr int F32_STAGES = 4, F32_APITCH = SIMT_BK + 4;
+template <int TM, int TN>
+struct F32Tile {
+  static constexpr int BM = 16 * TM, BN = 16 * TN, A_FLOATS = BM * F32_APITCH, B_FLOATS = SIMT_BK * BN;
+  static constexpr int SMEM = F32_STAGES * (A_FLOATS + B_FLOATS) * 4;
+};
+__device__ __forceinline__ void cp_async_zfill16(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_zfill4(uint32_t dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+
+template <int TM, int TN>
+__global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_f32_kernel(const __grid_constant__ SimtGemmParams p) {
+  using Tl = F32Tile<TM, TN>;
+  extern __shared__ __align__(16) float ring[];
+  pdl_begin();
+  const int b = blockIdx.y;
+  const float* A = reinterpret_cast<const float*>(p.A) + (int64_t)b * p.stride_a;
+  const float* B = reinterpret_cast<const float*>(p.B) + (int64_t)b * p.stride_b;
+  const int mt = blockIdx.x / p.tiles_n, m0 = mt * Tl::BM, n0 = (int)(blockIdx.x - (unsigned)mt * p.tiles_n) * Tl::BN;
+  const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;          // rows ty + 32 i, columns 2 tx + 16 j and the next
+  const int nk = (p.K + SIMT_BK - 1) / SIMT_BK;
+  const uint32_t ring_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
+
+  auto request = [&](int kb) {
+    if (kb < nk) {
+      const int k0 = kb * SIMT_BK;
+      const uint32_t as = ring_u32 + (kb % F32_STAGES) * (Tl::A_FLOATS + Tl::B_FLOATS) * 4, bs = as + Tl::A_FLOATS * 4;
+      if (p.a_vec) {
+#pragma unroll
+        for (int q0 = 0; q0 < Tl::BM * 4; q0 += 256) {
+          const int q = q0 + threadIdx.x;
+          if (Tl::BM * 4 % 256 == 0 || q < Tl::BM * 4) {
+            const int r = q / 4, k = q % 4 * 4;
+            const bool in = m0 + r < p.M && k0 + k < p.K;
+            cp_async_zfill16(as + (r * F32_APITCH + k) * 4, in ? A + (int64_t)(m0 + r) * p.lda + k0 + k : A, in);
+          }
+        }
+      } else {
+        for (int q = threadIdx.x; q < Tl::BM * SIMT_BK; q += 256) {
+          const int r = q / SIMT_BK, k = q % SIMT_BK;
+          const bool in = m0 + r < p.M && k0 + k < p.K;
+          cp_async_zfill4(as + (r * F32_APITCH + k) * 4, in ? A + (int64_t)(m0 + r) * p.lda + k0 + k : A, in);
+        }
+      }
+      if (p.b_vec) {
+#pragma unroll
+        for (int q0 = 0; q0 < Tl::BN * 4; q0 += 256) {
+          const int q = q0 + threadIdx.x;
+          if (Tl::BN * 4 % 256 == 0 || q < Tl::BN * 4) {
+            const int k = q / (Tl::BN / 4), n = q % (Tl::BN / 4) * 4;
+            const bool in = n0 + n < p.N && k0 + k < p.K;
+            cp_async_zfill16(bs + (k * Tl::BN + n) * 4, in ? B + (int64_t)(k0 + k) * p.ldb + n0 + n : B, in);
+          }
+        }
+      } else {
+        for (int q = threadIdx.x; q < Tl::BN * SIMT_BK; q += 256) {
+          const int k = q / Tl::BN, n = q % Tl::BN;
+          const bool in = n0 + n < p.N && k0 + k < p.K;
+          cp_async_zfill4(bs + (k * Tl::BN + n) * 4, in ? B + (int64_t)(k0 + k) * p.ldb + n0 + n : B, in);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");        // an empty group keeps the count
+  };
+
+  constexpr int R = TM / 2;                                     // rows of a thread
+  uint64_t acc[R][TN];                                          // pairs of fp32
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+  // one copy of `request`: this loop asks for the first slices too
+#pragma unroll 1
+  for (int kb = 1 - F32_STAGES; kb < nk; ++kb) {
+    if (kb < 0) {
+      request(kb + F32_STAGES - 1);
+      continue;
+    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(F32_STAGES - 2) : "memory");
+    __syncthreads();                                            // slice kb has landed; slice kb - 1 has been read
+    request(kb + F32_STAGES - 1);
+    const float* as = ring + (kb % F32_STAGES) * (Tl::A_FLOATS + Tl::B_FLOATS) + ty * F32_APITCH;
+    const float* bs = ring + (kb % F32_STAGES) * (Tl::A_FLOATS + Tl::B_FLOATS) + Tl::A_FLOATS + 2 * tx;
+#pragma unroll
+    for (int k4 = 0; k4 < SIMT_BK; k4 += 4) {
+      float a[R][4];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(as + 32 * i * F32_APITCH + k4);
+        a[i][0] = x.x; a[i][1] = x.y; a[i][2] = x.z; a[i][3] = x.w;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint64_t bb[TN];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) bb[j] = *reinterpret_cast<const uint64_t*>(bs + (k4 + k) * Tl::BN + 16 * j);
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          uint64_t aa;
+          asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a[i][k]));
+#pragma unroll
+          for (int j = 0; j < TN; ++j) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[i][j]) : "l"(aa), "l"(bb[j]));
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < TN; ++j) {
+    float lo[R], hi[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(lo[i]), "=f"(hi[i]) : "l"(acc[i][j]));
+    const int gn = n0 + 2 * tx + 16 * j;
+    if (gn >= p.N) continue;
+    const Column c0 = column_of(p, b, gn), c1 = column_of(p, b, min(gn + 1, p.N - 1));
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int gm = m0 + ty + 32 * i;
+      if (gm >= p.M) continue;
+      const float v0 = finish(p, c0, b, gm, gn, lo[i]), v1 = gn + 1 < p.N ? finish(p, c1, b, gm, gn + 1, hi[i]) : 0.f;
+      const int64_t at = (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + gn;
+      if (p.y_pairs && gn + 1 < p.N) {
+        *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.Y) + at) = make_float2(v0, v1);
+      } else {
+        store_from_f32(p.Y, at, p.y_dtype, v0);
+        if (gn + 1 < p.N) store_from_f32(p.Y, at + 1, p.y_dtype, v1);
+      }
+    }
   }
 }
 
+template <int TM, int TN>
+static int launch_f32(const SimtGemmParams& p, dim3 grid, cudaStream_t s) {
+  static PerDeviceOnce attr;                                    // per instantiation
+  if (F32Tile<TM, TN>::SMEM > 48 * 1024) XB_SET_MAX_SMEM_ONCE(attr, (F32Tile<TM, TN>::SMEM), (const void*)gemm_f32_kernel<TM, TN>);
+  launch_dependent(gemm_f32_kernel<TM, TN>, grid, 256, F32Tile<TM, TN>::SMEM, s, p);
+  return check_launch("gemm_f32_kernel");
+}
+template <int TM>
+static int launch_f32_tm(const SimtGemmParams& p, int tn, dim3 grid, cudaStream_t s) {
+  switch (tn) {
+    case 1: return launch_f32<TM, 1>(p, grid, s);
+    case 2: return launch_f32<TM, 2>(p, grid, s);
+    case 3: return launch_f32<TM, 3>(p, grid, s);
+    case 4: return launch_f32<TM, 4>(p, grid, s);
+    case 5: return launch_f32<TM, 5>(p, grid, s);
+    case 6: return launch_f32<TM, 6>(p, grid, s);
+    default: return launch_f32<TM, 8>(p, grid, s);
+  }
+}
+template <int TM>
+static int launch_simt_tm(const SimtGemmParams& p, int tn, dim3 grid, cudaStream_t s) {
+  switch (tn) {
+    case 2: launch_dependent(gemm_simt_kernel<TM, 2>, grid, 256, 0, s, p); break;
+    case 4: launch_dependent(gemm_simt_kernel<TM, 4>, grid, 256, 0, s, p); break;
+    default: launch_dependent(gemm_simt_kernel<TM, 8>, grid, 256, 0, s, p); break;
+  }
+  return check_launch("gemm_simt_kernel");
+}
+
 // Tile of a product: a wave of CTAs costs what its busiest SM computes, TM*TN a k slice and output pair, plus what
-// the operand reads and the slice's overhead cost beside it; the tile with the cheapest sum of waves is taken.
-static void pick_simt_tile(int64_t M, int64_t N, int64_t batch, int* tm, int* tn) {
+// the operand reads and the slice's overhead cost beside it; the tile with the cheapest sum of waves is taken. The general
+// kernel has fewer widths.
+static void pick_simt_tile(int64_t M, int64_t N, int64_t batch, bool f32, int* tm, int* tn) {
   double best = 0;
   for (int m : {8, 4, 2}) {
     for (int n : {8, 6, 5, 4, 3, 2, 1}) {
+      if (!f32 && n != 8 && n != 4 && n != 2) continue;
       const int64_t tiles = ((M + 16 * m - 1) / (16 * m)) * ((N + 16 * n - 1) / (16 * n)) * batch;
       const double waves = (double)((tiles + sm_count() - 1) / sm_count());
       const double cost = waves * (m * n + 1.5 * n + 0.75 * m + 4);
@@ -231,17 +399,17 @@ int gemm_simt(const xb_gemm_args& a, cudaStream_t stream) {
   };
   p.a_vec = vec(a.A, a.lda, a.stride_a, a.trans_a ? a.M : a.K);
   p.b_vec = vec(a.B, a.ldb, a.stride_b, a.trans_b ? a.K : a.N);
+  p.y_pairs = a.y_dtype == XB_F32 && (reinterpret_cast<uintptr_t>(a.Y) & 7) == 0 && a.ldy % 2 == 0 && a.stride_y % 2 == 0;
   int tm = 8, tn = 8;
-  pick_simt_tile(a.M, a.N, a.batch, &tm, &tn);
+  const bool f32 = a.ab_dtype == XB_F32 && !a.trans_a && !a.trans_b;
+  pick_simt_tile(a.M, a.N, a.batch, f32, &tm, &tn);
   XB_REQUIRE((a.M + 63) / 64 <= 65535 && a.batch <= 65535, XB_ERR_LIMIT, "xb_gemm: M or batch too large for the SIMT engine");
   p.tiles_n = (a.N + 16 * tn - 1) / (16 * tn);
   const int64_t tiles = (((int64_t)a.M + 16 * tm - 1) / (16 * tm)) * p.tiles_n;
   XB_REQUIRE(tiles < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)tiles);
   dim3 grid((unsigned)tiles, (unsigned)a.batch);
-  if (tm == 8) launch_simt_tm<8>(p, tn, grid, stream);
-  else if (tm == 4) launch_simt_tm<4>(p, tn, grid, stream);
-  else launch_simt_tm<2>(p, tn, grid, stream);
-  return check_launch("gemm_simt_kernel");
+  if (f32) return tm == 8 ? launch_f32_tm<8>(p, tn, grid, stream) : tm == 4 ? launch_f32_tm<4>(p, tn, grid, stream) : launch_f32_tm<2>(p, tn, grid, stream);
+  return tm == 8 ? launch_simt_tm<8>(p, tn, grid, stream) : tm == 4 ? launch_simt_tm<4>(p, tn, grid, stream) : launch_simt_tm<2>(p, tn, grid, stream);
 }
 
 }  // namespace xb
