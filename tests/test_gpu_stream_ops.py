@@ -60,7 +60,7 @@ def test_elementwise_layouts(op, ref, a, b, off):
 
 
 @pytest.mark.parametrize("rows,cols,src_ld,dst_ld,so,do", [
-    (50, 36, 36, 144, 0, 36), (3, 8, 8, 8, 0, 0), (5, 7, 9, 11, 1, 2), (64, 18, 18, 36, 0, 18), (17, 10, 0, 10, 0, 0), (1, 1, 1, 1, 3, 5)])
+    (50, 36, 36, 144, 0, 36), (3, 8, 8, 8, 0, 0), (5, 7, 9, 11, 1, 2), (64, 18, 18, 36, 0, 18), (17, 10, 0, 10, 0, 0), (1, 1, 1, 1, 3, 5), (9, 100, 100, 100, 0, 0), (9, 12, 16, 20, 4, 8)])
 @pytest.mark.parametrize("dtype,to", [("f32", "f32"), ("f16", "f16"), ("f32", "f16"), ("f16", "f32"), ("i32", "i32"), ("i64", "i64")])
 def test_copy2d_pieces(rows, cols, src_ld, dst_ld, so, do, dtype, to):
     capi, ops, L = _L()

@@ -228,6 +228,25 @@ __global__ void __launch_bounds__(256) copy2d_vec_kernel(const V* src, int64_t s
   }
 }
 
+// fp32 <-> fp16 copies, four elements per thread (16 bytes on one side, 8 on the other)
+template <bool TO_HALF>
+__global__ void __launch_bounds__(256) copy2d_convert_kernel(const void* src, int64_t src_ld, void* dst, int64_t dst_ld, uint32_t total, uint32_t cols) {
+  pdl_begin();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const uint32_t r = i / cols, c = i - r * cols;
+    if (TO_HALF) {
+      const float4 v = reinterpret_cast<const float4*>(src)[(int64_t)r * src_ld + c];
+      const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
+      reinterpret_cast<uint2*>(dst)[(int64_t)r * dst_ld + c] =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    } else {
+      const uint2 v = reinterpret_cast<const uint2*>(src)[(int64_t)r * src_ld + c];
+      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+      reinterpret_cast<float4*>(dst)[(int64_t)r * dst_ld + c] = make_float4(a.x, a.y, b.x, b.y);
+    }
+  }
+}
+
 __global__ void reduce_sum_kernel(const void* x, void* y, int64_t outer, int64_t r, int64_t inner, int dt) {
   pdl_begin();
   const int64_t total = outer * inner;
@@ -300,37 +319,52 @@ __global__ void __launch_bounds__(256) din_tower_input_kernel(const __half* user
   const int n0 = blockIdx.x * 64;
   const int rows = min(64, n_cand - n0);
   if (pairs_ok == 2) {
-    // four columns (8 bytes) at a time: 16 000 rows of 328 columns take 17 us, 23 two at a time
-    const int wq = (int)(ldx >> 2);
-    for (int idx = threadIdx.x; idx < rows * wq; idx += blockDim.x) {
-      const int nl = idx / wq, c = (idx - nl * wq) * 4;
-      const int64_t row = (int64_t)r * n_cand + n0 + nl;
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
+    // Four columns (8 bytes) at a time. A thread keeps its columns and takes every few rows, so the columns' place and
+    // what is the same for all rows are worked out once. 16 000 rows of 328 columns: 16 us
+    // behind the AUGRU, 19 without asking for rows ahead
+    const int wq = (int)(ldx >> 2), step = max(1, (int)blockDim.x / wq);
+    for (int q0 = threadIdx.x; q0 < step * wq; q0 += blockDim.x) {
+      const int r0 = q0 / wq, c = (q0 - r0 * wq) * 4;
+      float f[4] = {0.f, 0.f, 0.f, 0.f};
+      int seg = -1, e = 0;                             // -1: the same four values in every row
       if (c < du) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = us[c + u];
+        for (int u = 0; u < 4; ++u) f[u] = us[c + u];
       } else if (c < du + 5 * d) {
-        const int seg = (c - du) / d, e = (c - du) - seg * d;
-        if (seg == 1) {
+        seg = (c - du) / d;
+        e = (c - du) - seg * d;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) v[u] = hs[e + u];
-        } else {
-          const uint2 raw = *reinterpret_cast<const uint2*>(seg == 3 ? att + row * ldatt + e : q + row * ldq + e);
-          const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-          v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
-          if (seg == 2) {
+        for (int u = 0; u < 4; ++u) f[u] = hs[e + u];
+        if (seg == 1) seg = -1;
+      }
+      const __half* src = seg == 3 ? att + e : q + e;
+      const int64_t ld = seg == 3 ? ldatt : ldq, row0 = (int64_t)r * n_cand + n0;
+      constexpr int U = 8;                             // rows requested together (a store would hold back the loads behind it)
+      for (int nl0 = r0; nl0 < rows; nl0 += U * step) {
+        uint2 raw[U];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] *= hs[e + u];
-          } else if (seg == 4) {
+        for (int k = 0; k < U; ++k) {
+          const int nl = nl0 + k * step;
+          raw[k] = make_uint2(0u, 0u);
+          if (seg >= 0 && nl < rows) raw[k] = *reinterpret_cast<const uint2*>(src + (row0 + nl) * ld);
+        }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] -= hs[e + u];
+        for (int k = 0; k < U; ++k) {
+          const int nl = nl0 + k * step;
+          if (nl >= rows) continue;
+          float v[4] = {f[0], f[1], f[2], f[3]};
+          if (seg >= 0) {
+            const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&raw[k].x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&raw[k].y));
+            const float x[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = seg == 2 ? x[u] * f[u] : seg == 4 ? x[u] - f[u] : x[u];
           }
+          const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
+          uint2 w;
+          w.x = *reinterpret_cast<const uint32_t*>(&a); w.y = *reinterpret_cast<const uint32_t*>(&b);
+          *reinterpret_cast<uint2*>(X + (row0 + nl) * ldx + c) = w;
         }
       }
-      const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
-      uint2 w;
-      w.x = *reinterpret_cast<const uint32_t*>(&a); w.y = *reinterpret_cast<const uint32_t*>(&b);
-      *reinterpret_cast<uint2*>(X + row * ldx + c) = w;
     }
     return;
   }
@@ -583,6 +617,14 @@ extern "C" int xb_copy2d(const void* src, int64_t src_ld, int32_t sdt, void* dst
       else launch_dependent(copy2d_vec_kernel<uint16_t>, grid, 256, 0, st, (const uint16_t*)src, sl, (uint16_t*)dst, dl, (uint32_t)pieces, pc);
       return check_launch("copy2d_vec_kernel");
     }
+  }
+  const bool to_half = sdt == XB_F32 && ddt == XB_F16;
+  if ((to_half || (sdt == XB_F16 && ddt == XB_F32)) && src_ld % 4 == 0 && dst_ld % 4 == 0 && cols % 4 == 0 &&
+      ((uintptr_t)src & (to_half ? 15 : 7)) == 0 && ((uintptr_t)dst & (to_half ? 7 : 15)) == 0 && rows * cols < ((int64_t)1 << 31)) {
+    const uint32_t n = (uint32_t)(rows * cols / 4);
+    launch_dependent(to_half ? copy2d_convert_kernel<true> : copy2d_convert_kernel<false>, stream_grid(n, 256), 256, 0, (cudaStream_t)s,
+                     src, src_ld / 4, dst, dst_ld / 4, n, (uint32_t)(cols / 4));
+    return check_launch("copy2d_convert_kernel");
   }
   launch_dependent(copy2d_kernel, stream_grid(rows * cols, 256), 256, 0, (cudaStream_t)s, src, src_ld, sdt, dst, dst_ld, ddt, rows, cols);
   return check_launch("copy2d_kernel");
