@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(PT_COLS * PT_SLICES) din_tower_partial_kernel(
   float* hs = sm;
   float* us = hs + d;
   float* part = us + du;
-  const int G = max(1, min((int)blockDim.x / d, 8));
+  const int G = max(1, min(256 / d, 8));
   float* colsum = part + 8 * d;
   // weight rows 0..du-1 meet the user row, rows du+d..du+2d-1 meet his_sum; x(c) is the matching input
   const int col = threadIdx.x % PT_COLS, slice = threadIdx.x / PT_COLS;
