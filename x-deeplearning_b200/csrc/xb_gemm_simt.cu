@@ -8,12 +8,13 @@
 // ascending, whatever the tile, so every form gives the same bits.
 // gemm_f32_kernel (fp32, neither operand transposed: Blaze's own layout) keeps
 // a ring of slices in flight with cp.async, which hides the latency that bounds
-// a small launch. What bounds a large one is instructions: with one FMA an
-// instruction the schedulers issued in a third of the cycles (43 % of the stalls
-// were instruction fetches), so two columns' FMAs go into one fma.rn.f32x2
-// (each rounded as an FMA of its own) and a thread owns pairs of adjacent
-// columns. [50000, 144] x [144, 80]: 75 us (scalar FMAs 85, the general
-// kernel 114); [8192, 512] x [512, 512]: 150 us, 29 TFLOP/s.
+// a small launch, and puts two columns' FMAs into one fma.rn.f32x2 (each
+// rounded as an FMA of its own), so that a thread owns pairs of adjacent
+// columns. Its outputs leave through shared memory in a rolled loop: what
+// bounded it was the fetching of code that was unrolled over them.
+// [50000, 144] x [144, 80]: 42 us (75 with unrolled outputs, 114 with the
+// general kernel's register prefetch); [8192, 512] x [512, 512]: 117 us,
+// 37 TFLOP/s (150); 45 TFLOP/s of 72 at K = 4096.
 // gemm_simt_kernel is the general form: any type, layout and alignment, the next
 // slice on its way to registers while the current one is multiplied.
 #include <algorithm>
@@ -120,6 +121,11 @@ __device__ __forceinline__ float finish(const SimtGemmParams& p, const Column& c
   return v;
 }
 
+// (one copy of the code: see the outputs of gemm_f32_kernel)
+__device__ __noinline__ void finish_and_store(const SimtGemmParams& p, Column c, int b, int gm, int gn, float acc) {
+  store_from_f32(p.Y, (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + gn, p.y_dtype, finish(p, c, b, gm, gn, acc));
+}
+
 template <int TM, int TN>
 __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(const __grid_constant__ SimtGemmParams p) {
   pdl_begin();
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(c
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
       const int gm = m0 + ty * TM + i;
-      if (gm < p.M) store_from_f32(p.Y, (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + gn, p.y_dtype, finish(p, c, b, gm, gn, acc[i][j]));
+      if (gm < p.M) finish_and_store(p, c, b, gm, gn, acc[i][j]);
     }
   }
 }
@@ -207,6 +213,7 @@ template <int TM, int TN>
 struct F32Tile {
   static constexpr int BM = 16 * TM, BN = 16 * TN, A_FLOATS = BM * F32_APITCH, B_FLOATS = SIMT_BK * BN;
   static constexpr int SMEM = F32_STAGES * (A_FLOATS + B_FLOATS) * 4;
+  static_assert(BM * BN * 4 <= SMEM, "the ring also holds the tile's outputs");
 };
 __device__ __forceinline__ void cp_async_zfill16(uint32_t dst, const void* src, bool in) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
@@ -311,26 +318,30 @@ __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_f32_kernel(co
       }
     }
   }
+  // Outputs go through shared memory (the ring is done with), so that bias, activation and store are one rolled loop: unrolled
+  // over a thread's outputs they are some 100 KB of code that every SM fetches to run once, 40 us whatever K.
+  __syncthreads();
 #pragma unroll
-  for (int j = 0; j < TN; ++j) {
-    float lo[R], hi[R];
+  for (int i = 0; i < R; ++i)
 #pragma unroll
-    for (int i = 0; i < R; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(lo[i]), "=f"(hi[i]) : "l"(acc[i][j]));
-    const int gn = n0 + 2 * tx + 16 * j;
-    if (gn >= p.N) continue;
-    const Column c0 = column_of(p, b, gn), c1 = column_of(p, b, min(gn + 1, p.N - 1));
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int gm = m0 + ty + 32 * i;
-      if (gm >= p.M) continue;
-      const float v0 = finish(p, c0, b, gm, gn, lo[i]), v1 = gn + 1 < p.N ? finish(p, c1, b, gm, gn + 1, hi[i]) : 0.f;
-      const int64_t at = (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + gn;
-      if (p.y_pairs && gn + 1 < p.N) {
-        *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.Y) + at) = make_float2(v0, v1);
-      } else {
-        store_from_f32(p.Y, at, p.y_dtype, v0);
-        if (gn + 1 < p.N) store_from_f32(p.Y, at + 1, p.y_dtype, v1);
-      }
+    for (int j = 0; j < TN; ++j) *reinterpret_cast<uint64_t*>(ring + (ty + 32 * i) * Tl::BN + 2 * tx + 16 * j) = acc[i][j];
+  __syncthreads();
+  constexpr int PAIRS = Tl::BN / 2, STEP = 256 / PAIRS;         // a thread keeps its two columns and takes every STEP-th row
+  const int cp = threadIdx.x % PAIRS, r0 = threadIdx.x / PAIRS, gn = n0 + 2 * cp;
+  if (r0 >= STEP || gn >= p.N) return;
+  const bool two = gn + 1 < p.N;
+  const Column c0 = column_of(p, b, gn), c1 = column_of(p, b, two ? gn + 1 : gn);
+#pragma unroll 1
+  for (int r = r0; r < Tl::BM && m0 + r < p.M; r += STEP) {
+    const int gm = m0 + r;
+    const float2 x = *reinterpret_cast<const float2*>(ring + r * Tl::BN + 2 * cp);
+    const float v0 = finish(p, c0, b, gm, gn, x.x), v1 = two ? finish(p, c1, b, gm, gn + 1, x.y) : 0.f;
+    const int64_t at = (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + gn;
+    if (p.y_pairs && two) {
+      *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.Y) + at) = make_float2(v0, v1);
+    } else {
+      store_from_f32(p.Y, at, p.y_dtype, v0);
+      if (two) store_from_f32(p.Y, at + 1, p.y_dtype, v1);
     }
   }
 }
