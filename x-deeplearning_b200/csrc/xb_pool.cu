@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "xb_common.cuh"
+#include "xb_pool_plan.h"
 
 namespace xb {
 
@@ -522,7 +523,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
       nm = __ldg(g.offsets + sg + 1) - st;
     }
   };
-  // Short count arrays (segs is 1): the warp adds up the counts before its first segment itself, which takes less than
+  // Short count arrays (pool_split gives their warps one round): the warp adds up the counts before its first segment itself, which takes less than
   // the launch of a scan kernel in front of this one. A segment's start: those, and the counts of the teams before its.
   auto span_from_counts = [&](int& st, int& nm) {
     const int first = (int)(seg_first - lane / tl);
@@ -1174,8 +1175,6 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
                           (hp[bucket].n_groups == 0 || (hp[bucket].g[0].id_dtype == XB_REC64) == (h.id_dtype == XB_REC64));
     PoolParams& dst = short_ok ? hp[bucket] : queue_ok ? qp[bucket] : fast ? fp[bucket] : p;
     dst.warp_begin[dst.n_groups] = dst.total_warps;
-    const int spw = 32 / d.tl;
-    const int64_t rounds = (h.batch + spw - 1) / spw;
     const bool counts_ok = fast && !short_ok && !queue_ok && !h.segments_are_offsets && h.batch <= POOL_INLINE_COUNTS;
     if (counts_ok) {
       d.offsets = h.segments;
@@ -1191,20 +1190,10 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
       sp.counts[sp.n] = h.segments; sp.offsets[sp.n] = off; sp.batch[sp.n] = h.batch; ++sp.n;
       d.offsets = off;
     }
-    // the specialised kernel gives a warp several rounds, as long as every SM still gets dozens of warps
-    d.segs = 1;
-    // (dozens less with a list of one or two ids, whose warp is a chain of latencies: its rounds overlap, while a second
-    // wave of warps would begin the chain again: 2 x 74 000 single ids and their requests' lists 17.7 -> 13.1 us.)
-    if (fast) d.segs = (int)std::max<int64_t>(1, std::min<int64_t>(8, rounds / ((int64_t)sm_count() * (avg < 3.0 ? 12 : 48))));
-    // the short-segment kernel walks 8 rounds per warp (its prefetch needs a few), fewer only for small groups
-    if (short_ok) d.segs = (int)std::max<int64_t>(1, std::min<int64_t>(8, rounds / ((int64_t)sm_count() * 16)));
-    if (queue_ok && !short_ok) {
-      d.segs = queue_segs;
-      if (d.segs < spw) d.segs = spw;
-      dst.total_warps += (h.batch + d.segs - 1) / d.segs;
-    } else {
-      dst.total_warps += (rounds + d.segs - 1) / d.segs;
-    }
+    const PoolPath path = short_ok ? PoolPath::SHORT : queue_ok ? PoolPath::QUEUE : fast ? PoolPath::FAST : PoolPath::GENERAL;
+    const PoolSplit split = pool_split(path, h.batch, d.tl, avg, counts_ok, queue_segs, sm_count());
+    d.segs = split.segs;
+    dst.total_warps += split.warps;
     dst.g[dst.n_groups++] = d;
   }
   if (sp.n) {
