@@ -75,3 +75,43 @@ def test_a_request_gets_the_same_bits_alone_and_in_a_batch():
         one = att(q[r * n_cand:(r + 1) * n_cand], k[r * T:(r + 1) * T], 1, n_cand, T, engine=capi.XB_GEMM_TCGEN05)
         assert torch.equal(one, all_[r * n_cand:(r + 1) * n_cand])
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("R,n_cand,T", [(1, 140, 100), (5, 130, 17), (160, 128, 20)])      # split, split, one wave and more
+@pytest.mark.parametrize("lens", [False, True])
+def test_scores_that_are_no_finite_numbers_show_through_zero_rows(R, n_cand, T, lens):
+    """s * 0 is NaN for such a score: a call that walks every step (because it wants the scores) and one that leaves out
+    zero rows agree, whether the odd rows of q meet lists of zeros, short lists or full ones."""
+    pkg.load()
+    from x_deeplearning_b200 import capi, ops
+    rng = np.random.default_rng(R)
+    d = 36
+    w = _weights(rng, d, 80, 40)
+    t = torch.from_numpy
+    att = ops.DinAttention(t(w["W0"]), t(w["b0"]), t(w["W1"]), t(w["b1"]), t(w["W2"]), float(w["b2"][0]),
+                           dice0=[t(w["g0"]), t(w["m0"]), t(w["v0"])], dice1=[t(w["g1"]), t(w["m1"]), t(w["v1"])], act=2)
+    q = rng.normal(0, 0.5, (R, n_cand, d)).astype(np.float16)
+    q[:, 3, 5], q[:, 17, 0], q[:, 40, 35] = np.inf, -np.inf, np.nan
+    q[:, 60], q[:, 61] = 6e4, -6e4                                     # finite, their scores are not
+    k = rng.normal(0, 0.5, (R, T, d)).astype(np.float16)
+    for r in range(R):
+        kind = r % 5
+        if kind == 0:
+            k[r] = 0
+        elif kind == 1:
+            k[r, : T // 2] = 0
+        elif kind == 2:
+            k[r, T // 3:] = -0.0
+        elif kind == 3:
+            k[r, : T // 3] = 0
+            k[r, T - 2:] = 0
+    sl = torch.from_numpy(rng.integers(0, T + 1, R).astype(np.int32)).cuda() if lens else None
+    qd, kd = t(q.reshape(R * n_cand, d)).cuda(), t(k.reshape(R * T, d)).cuda()
+    call = lambda sc: att(qd, kd, R, n_cand, T, seq_len=sl, scores=sc, engine=capi.XB_GEMM_TCGEN05)
+    got, want = call(None).clone(), call(torch.zeros((R * n_cand, T), device="cuda")).clone()
+    assert ops.device_status() == 0
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.nan_to_num(nan=9.0), want.nan_to_num(nan=9.0))
+    rows = got.view(R, n_cand, d)[:, [3, 17, 40]].isfinite().logical_not().all(-1)
+    live = sl.cpu() > 0 if lens else torch.ones(R, dtype=torch.bool)
+    assert rows[live.cuda()].all() and not rows[~live.cuda()].any()            # an odd q row shows unless its list is empty

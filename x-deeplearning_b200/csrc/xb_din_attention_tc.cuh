@@ -25,8 +25,8 @@
 // A step costs about 0.67 us of one SM whatever the number of tiles, so a call with few tiles leaves the chip idle
 // and takes T steps all the same. Then a cluster of `split` CTAs shares a tile: each walks a part of the steps and writes
 // its scores into the S operand of the cluster's first CTA, which runs the closing product over all of them, so a result
-// has the same bits whatever the split. Where neither the scores nor a softmax over them is wanted, steps of zero k rows
-// at either end of a list (the padding of a short one) are not walked: whatever their score, they add s * 0.
+// has the same bits whatever the split. Where neither the scores nor a softmax over them is wanted, of the steps of zero k
+// rows at either end of a list (the padding of a short one) only one is walked: each adds the same s * 0.
 // 8 tiles of 100 steps: 20 us as 8 clusters of 8, 72 whole; 2 tiles of a list of 60: 13 us, 72 before.
 //
 // Biases ride in the MMAs: A1 carries a constant-1 column (a padding column of
@@ -348,9 +348,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
       if (__any_sync(0xffffffffu, nz) && lane == 0) { atomicMin(&range_s[0], t); atomicMax(&range_s[1], t + 1); }
     }
     __syncthreads();
+    // one of the zero rows stays in: all of them have the same score, and one that is no finite fp16 number makes the
+    // result NaN through s * 0 however often it is added
+    int end = range_s[1];
     t0 = range_s[0];
-    tl = max(0, range_s[1] - t0);
-    if (tl == 0) t0 = 0;
+    if (end == 0) { t0 = 0; end = min(tl, 1); }
+    else if (t0 > 0) --t0;
+    else if (end < tl) ++end;
+    tl = end - t0;
   }
   if (threadIdx.x == 0) ATT_TR(6, 120, 1);
   // K^T operand of the closing product, from the k rows now in shared memory
