@@ -49,6 +49,24 @@ def test_weights_in_k_n_layout(dtype, P, M, N, K, ldb, shared):
         assert (err <= _bound(a, w, want, K, 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8)).all(), float(err.max())
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("epi", ["none", "dice"])
+def test_weights_in_k_n_layout_with_fp32_results_keep_the_precision_of_the_cuda_cores(dtype, epi):
+    """K fp32 FMAs in order: within K * 2^-24 of the sum of magnitudes in the worst case; the bits of the explicit engine."""
+    ops, capi = _ops()
+    rng = np.random.default_rng(3)
+    M, N, K = 300, 128, 512
+    t = lambda a, d: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).to("cuda", d)
+    A, W = t(rng.normal(0, 1, (M, K)), dtype), t(rng.normal(0, 1, (K, N)) / np.sqrt(K), dtype)
+    bias = t(rng.normal(0, 0.3, N), torch.float32)
+    kw = {} if epi == "none" else dict(epilogue=capi.XB_EPI_DICE, ep=[t(rng.uniform(0.1, 0.5, N), torch.float32) for _ in range(3)])
+    got, simt = [ops.gemm(A, W, bias=bias, out_dtype=torch.float32, engine=e, **kw) for e in (capi.XB_GEMM_AUTO, capi.XB_GEMM_SIMT)]
+    assert torch.equal(got, simt)
+    if epi == "none":
+        f = lambda x: x.double().cpu().numpy()
+        assert (np.abs(f(got) - (f(A) @ f(W) + f(bias))) <= (K + 2) * 2.0 ** -24 * (np.abs(f(A)) @ np.abs(f(W)) + np.abs(f(bias)))).all()
+
+
 def test_explicit_tensor_core_engine_still_wants_k_major_weights():
     ops, capi = _ops()
     A, W = torch.zeros((128, 64), dtype=torch.float16, device="cuda"), torch.zeros((64, 64), dtype=torch.float16, device="cuda")
