@@ -69,3 +69,39 @@ def test_routing_to_one_shard(segments, mean):
             assert torch.equal(g.cpu(), c)
         g, c = gops.route_packed(t(ids).cuda(), gv, t(off).cuda(), 1), cops.route_packed(t(ids), cv, t(off), 1)
         assert torch.equal(g[0].cpu(), c[0]) and torch.equal(g[2].cpu(), c[2])
+
+
+@pytest.mark.parametrize("sources,cap,S", [(1, 2, 1), (1, 5000, 700), (3, 4099, 6000), (16, 300, 40), (2, 100_000, 3)])
+def test_offsets_and_counts_of_received_records(sources, cap, S):
+    """The two ways to a source's segments agree: offsets straight from the sorted records (what the sharded step uses) and the
+    counts of xb_record_counts_padded added up. Headers that say more than the bucket holds, or less than nothing, and records
+    of segments that do not exist (they belong to none)."""
+    import ctypes
+    pkg.load()
+    from x_deeplearning_b200 import capi, ops
+    rng = np.random.default_rng(S)
+    packed = np.zeros((sources, cap), np.int64)
+    want = np.zeros((sources, S), np.int32)
+    for s in range(sources):
+        cnt = [cap - 1, (cap - 1) // 2, cap + 7, -3, 0][s % 5] if sources > 1 else cap - 1
+        real = max(0, min(cnt, cap - 1))
+        tags = np.sort(rng.integers(0, S, real)) if s % 2 == 0 else np.sort(rng.integers(S // 3, 1 + S // 2, real) // 5 * 5 % S)
+        beyond = min(real, 5) if sources > 1 or cap == 5000 else 0
+        if beyond:
+            tags[real - beyond:] = S + np.arange(beyond)
+            if beyond == 5:
+                tags[real - 1] = (1 << 32) - 9                       # the sign bit of the record
+        for i, t in enumerate(tags):
+            packed[s, 1 + i] = np.uint64((int(t) << 32) | int(rng.integers(0, 1 << 31))).astype(np.int64)
+        packed[s, 0] = cnt
+        want[s] = np.bincount(tags[tags < S], minlength=S)[:S]
+    dp = torch.from_numpy(packed).cuda()
+    counts = torch.full((sources, S), -1, dtype=torch.int32, device="cuda")
+    offsets = torch.full((sources, S + 1), -1, dtype=torch.int32, device="cuda")
+    lib = capi.lib()
+    capi.check(lib.xb_record_counts_padded(ops.ptr(dp), sources, cap, ops.ptr(counts), S, ops.stream()))
+    fn = lib["_ZN2xb21record_offsets_paddedEPKlilPilP11CUstream_st"]         # xb::record_offsets_padded
+    fn.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]
+    assert fn(dp.data_ptr(), sources, cap, offsets.data_ptr(), S, ops.stream()) == 0
+    assert np.array_equal(counts.cpu().numpy(), want)
+    assert np.array_equal(offsets.cpu().numpy(), np.concatenate([np.zeros((sources, 1), np.int64), np.cumsum(want, 1)], 1))

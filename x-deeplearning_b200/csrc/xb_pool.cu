@@ -2083,8 +2083,9 @@ extern "C" int xb_record_counts_padded(const int64_t* packed, int32_t sources, i
 // Exclusive offsets of every segment of a source straight from its received bucket. Records arrive sorted by segment, so a
 // record that begins a new segment is the offset of that segment and of the empty ones before it, and what follows the
 // last record's segment is the count: one pass over the records, no counts, no atomics, no scan. (5.1 M records, 330 k
-// segments: 10 us; counting, clearing and scanning took 24.) offsets [sources, segments + 1]. Segment numbers and counts come from peers: every index is
-// bounded here, and offsets of records that are not sorted are wrong but lie inside the bucket.
+// segments: 10 us; counting, clearing and scanning took 24.) offsets [sources, segments + 1]. Segment numbers and counts come
+// from peers: every index is bounded here, records of a segment that does not exist come last and belong to none (the closing
+// entry is the first of them), and offsets of records that are not sorted are wrong but lie inside the bucket.
 __global__ void __launch_bounds__(256) record_offsets_kernel(const int64_t* __restrict__ packed, int64_t cap, int64_t segments,
                                                              int32_t* __restrict__ offsets) {
   pdl_begin();
@@ -2094,7 +2095,7 @@ __global__ void __launch_bounds__(256) record_offsets_kernel(const int64_t* __re
   int64_t cnt = __ldg(rec);
   cnt = cnt < 0 || segments == 0 ? 0 : (cnt > cap - 1 ? cap - 1 : cnt);
   ++rec;
-  auto segment = [&](int64_t v) { return (int64_t)min((uint64_t)v >> 32, (uint64_t)(segments - 1)); };
+  auto segment = [&](int64_t v) { return (int64_t)min((uint64_t)v >> 32, (uint64_t)segments); };
   // offsets[lo .. hi] = value for every lane; runs of empty segments longer than a few are written by the whole warp
   auto fill = [&](int64_t lo, int64_t hi, int32_t value) {
     if (hi - lo < 8)
