@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(AU_THREADS, H <= 40 ? 2 : 1) augru_tc_kernel(c
   __half* atts = reinterpret_cast<__half*>(smem + G.o_att);
   __half* xs = reinterpret_cast<__half*>(smem + G.o_x);
   const __half zero = __float2half(0.f);
-  pdl_begin();
+  pdl_wait();
 
   // ---- prologue -------------------------------------------------------------------------------------------
   // attention scores of the tile and the request's input sequence: asynchronous copies where alignment allows
@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(AU_THREADS, H <= 40 ? 2 : 1) augru_tc_kernel(c
     __half* out = p.y + ((int64_t)r * p.n_cand + tile * 128 + row) * H;
     au_worker<H>(p, warp >> 2, att_row, lane_addr, out, row < rows, a1_full, acc1_full, a2_full, acc2_full);
   }
+  pdl_release();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == AU_MMA_WARP) {

@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
   const int ctile = blockIdx.x / split;                                      // the cluster is `split` CTAs along x
   const int r = ctile / p.tiles_per_req, tile = ctile % p.tiles_per_req;
   const int d = d_, dp = G.dp, nch = G.nch, k1 = G.k1, h0p = G.h0p, k2 = G.k2, h1p = G.h1p, tp = G.tp, np = G.np;
-  pdl_begin();
+  pdl_wait();
   int tl = p.seq_len ? p.seq_len[r] : p.T;
   tl = tl < 0 ? 0 : (tl > p.T ? p.T : tl);
 
@@ -730,6 +730,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
       else *e = __float2half_rn(s);
     }
 
+    pdl_release();
     if (p.use_softmax) asm volatile("bar.sync 1, 256;" ::: "memory");     // both parities' scores are in S
     if (p.use_softmax && wb == 0) {
       // masked softmax over the steps, in place on this thread's row of S (steps >= tl are masked out)
@@ -781,6 +782,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) din_att_tc_kernel(const __grid_
   }
 
   if (lane == 0 && warp == 16) ATT_TR(6, 121, 2);
+  pdl_release();
   tc_fence_before_sync();
   __syncthreads();
   if (threadIdx.x == 0) ATT_TR(6, 121, 3);

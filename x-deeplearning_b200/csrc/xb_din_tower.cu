@@ -235,8 +235,8 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
   const int d = p.d, dp = G.dp, nch = G.nch, n1p = G.n1p, n2p = G.n2p, n3 = p.n3;
   const int64_t total_tiles = (int64_t)p.requests * p.tiles_per_req;
 
-  // weight image: asynchronous 16-byte copies, all in flight at once. Requested before pdl_begin: the kernel before is
-  // din_tower_partial_kernel, which has passed its own pdl_begin, so whatever wrote the image has completed.
+  // weight image: asynchronous 16-byte copies, all in flight at once. Requested before pdl_wait: the kernel before is
+  // din_tower_partial_kernel, which has passed its own wait, so whatever wrote the image has completed.
   {
     for (int i = threadIdx.x; i < G.image_bytes / 16; i += TW_THREADS) cp_async16(smem + 16 * i, p.packed + 16 * i);
     cp_async_commit();
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem0 = tmem_base_s;
-  pdl_begin();
+  pdl_wait();
 
   if (warp == TW_MMA_WARP) {
     // the whole warp runs the issue loop in uniform control flow and one elected lane issues: the descriptors

@@ -128,7 +128,7 @@ __device__ __noinline__ void finish_and_store(const SimtGemmParams& p, Column c,
 
 template <int TM, int TN>
 __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(const __grid_constant__ SimtGemmParams p) {
-  pdl_begin();
+  pdl_wait();
   constexpr int BM = 16 * TM, BN = 16 * TN;
   using SliceA = SimtSlice<BM>;
   using SliceB = SimtSlice<BN>;
@@ -193,6 +193,7 @@ __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_simt_kernel(c
     }
   }
 
+  pdl_release();
 #pragma unroll
   for (int j = 0; j < TN; ++j) {
     const int gn = n0 + tx + 16 * j;
@@ -226,7 +227,7 @@ template <int TM, int TN>
 __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_f32_kernel(const __grid_constant__ SimtGemmParams p) {
   using Tl = F32Tile<TM, TN>;
   extern __shared__ __align__(16) float ring[];
-  pdl_begin();
+  pdl_wait();
   const int b = blockIdx.y;
   const float* A = reinterpret_cast<const float*>(p.A) + (int64_t)b * p.stride_a;
   const float* B = reinterpret_cast<const float*>(p.B) + (int64_t)b * p.stride_b;
@@ -320,6 +321,7 @@ __global__ void __launch_bounds__(256, TM * TN >= 40 ? 2 : 3) gemm_f32_kernel(co
   }
   // Outputs go through shared memory (the ring is done with), so that bias, activation and store are one rolled loop: unrolled
   // over a thread's outputs they are some 100 KB of code that every SM fetches to run once, 40 us whatever K.
+  pdl_release();
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < R; ++i)

@@ -357,7 +357,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
-  pdl_begin();
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -506,6 +506,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   }
 
+  pdl_release();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {

@@ -86,7 +86,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   cluster_sync();                                                  // the other CTA's barriers are initialised too
   tc_fence_after_sync();
   const uint32_t tmem_base = tmem_base_s;
-  pdl_begin();
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -178,6 +178,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
   }
 
+  pdl_release();
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync();                  // no CTA leaves while the other's MMAs, copies or arrivals may still touch it

@@ -45,7 +45,7 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int steps, int H,
                                                       const T* __restrict__ i2h, const T* __restrict__ h2h,
                                                       const T* __restrict__ bi, const T* __restrict__ bh) {
-  pdl_begin();
+  pdl_wait();
   constexpr int HP = gru_hp(NV);
   extern __shared__ __align__(16) float gru_sm[];
   float* xs = gru_sm;                              // [GRU_CHUNK][HP]
@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
       }
     }
     __syncthreads();
+    if (t0 + n >= steps) pdl_release();            // (not in the steps: they are the chain)
     for (int t = 0; t < n; ++t) {
       const int64_t at = (b * steps + t0 + t) * H + u;
       if (!started) started = nonzero[t] != 0;     // the same for every thread
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
 // Wg [2H, 2H] (rows x then h; columns r then u), Wc [2H, H]; att [B, T].
 __global__ void augru_kernel(const void* x, const void* att, void* y, int T, int H, const void* Wg_, const void* bg_,
                              const void* Wc_, const void* bc_, int dt) {
-  pdl_begin();
+  pdl_wait();
   extern __shared__ float sm[];
   float* Wg = sm;                     // [2H][2H]
   float* Wc = Wg + 4 * H * H;         // [2H][H]
@@ -222,7 +223,7 @@ augru_shared_kernel(const __half* __restrict__ x, const __half* __restrict__ att
   float* px = xs + AS_CHUNK * HP;                              // [AS_CHUNK][3H]: x_t Wg_x + bg (r, u), x_t Wc_x + bc
   __shared__ __align__(16) float hbuf[AS_CAND][2][HP];
   __shared__ __align__(16) float rhbuf[AS_CAND][HP];
-  pdl_begin();
+  pdl_wait();
   const int tid = threadIdx.x, G = 3 * H;
   const int r = blockIdx.x / blocks_per_req, cand = tid / group_threads, gt = tid - cand * group_threads;
   const int n = (blockIdx.x - r * blocks_per_req) * cands + cand;
@@ -261,6 +262,7 @@ augru_shared_kernel(const __half* __restrict__ x, const __half* __restrict__ att
       px[idx] = s;
     }
     __syncthreads();
+    if (t0 + m >= steps) pdl_release();
     for (int t = 0; t < m; ++t) {
       const float a = __half2float(__ldg(arow + t0 + t));
       float pr = 0.f, pu = 0.f, pc = 0.f;
