@@ -86,3 +86,9 @@ def test_tensor_memory_is_allocated_before_the_next_kernel_is_released():
             checked += 1
     assert checked >= 4
 
+
+def test_a_cluster_that_shares_an_attention_tile_has_its_sm_to_itself():
+    text = _sources()["xb_din_attention_tc.cuh"]
+    kb = int(re.search(r"TC_CLUSTER_SMEM = (\d+) \* 1024", text).group(1))
+    assert 2 * kb > 228 and kb <= 220
+    assert re.search(r"p\.split > 1 \? std::max<size_t>\(\(size_t\)L\.total, TC_CLUSTER_SMEM\)", text)

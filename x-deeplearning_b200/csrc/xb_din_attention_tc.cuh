@@ -849,6 +849,8 @@ int cluster_slots(int lg) {
   return n;
 }
 
+constexpr size_t TC_CLUSTER_SMEM = 116 * 1024;       // an SM has 228 KB
+
 // How many CTAs share a tile: the time is (waves of CTAs) x (steps of one CTA + what a CTA spends around them, about
 // 8 steps' worth), plus about 3 for the cluster's barriers. 592 tiles of 100 steps stay whole (4 x 108 against 8 x 58);
 // 8 tiles take clusters of 8 (13 + 8 + 3 against 108).
@@ -884,7 +886,10 @@ int launch_att_tc(AttParams& p, const xb_din_att_args& a, cudaStream_t stream) {
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim.x = (unsigned)p.split; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(tiles * p.split)); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = (size_t)L.total;
+  // The CTAs of a cluster wait for one another with all of tensor memory in hand, so two clusters must never hold an SM each and
+  // wait for the other's: more than half of the shared memory keeps a second CTA off the SM, whatever the register count.
+  const size_t smem = p.split > 1 ? std::max<size_t>((size_t)L.total, TC_CLUSTER_SMEM) : (size_t)L.total;
+  cfg.gridDim = dim3((unsigned)(tiles * p.split)); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = smem;
   cfg.stream = stream; cfg.attrs = at; cfg.numAttrs = p.split > 1 ? 2 : 1;
   // the shape of the DIN / DIEN attention unit (d = 36, MLP 144-80-40-1) has instantiations of its own
   const bool din_shape = a.d == 36 && a.h0 == 80 && a.h1 == 40;
