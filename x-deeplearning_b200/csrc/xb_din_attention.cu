@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cstring>
 
+#include "xb_att_plan.h"
 #include "xb_common.cuh"
 #include "xb_umma.cuh"
 

@@ -851,21 +851,6 @@ int cluster_slots(int lg) {
 
 constexpr size_t TC_CLUSTER_SMEM = 116 * 1024;       // an SM has 228 KB
 
-// How many CTAs share a tile: the time is (waves of CTAs) x (steps of one CTA + what a CTA spends around them, about
-// 8 steps' worth), plus about 3 for the cluster's barriers. 592 tiles of 100 steps stay whole (4 x 108 against 8 x 58);
-// 8 tiles take clusters of 8 (13 + 8 + 3 against 108).
-int pick_split(int64_t tiles, int T) {
-  int best = 1;
-  int64_t cost = ((tiles + sm_count() - 1) / sm_count()) * (T + 8);
-  for (int lg = 1; lg <= 3; ++lg) {
-    const int s = 1 << lg, slots = s <= T ? cluster_slots(lg) : 0;
-    if (slots <= 0) continue;
-    const int64_t c = ((tiles * s + slots - 1) / slots) * ((T + s - 1) / s + 8) + 3;
-    if (c < cost) { cost = c; best = s; }
-  }
-  return best;
-}
-
 int launch_att_tc(AttParams& p, const xb_din_att_args& a, cudaStream_t stream) {
   const TcGeom g = tc_geom(a.d, a.h0, a.h1, a.T);
   p.tiles_per_req = (a.n_cand + 127) / 128;
@@ -877,8 +862,8 @@ int launch_att_tc(AttParams& p, const xb_din_att_args& a, cudaStream_t stream) {
                        (const void*)din_att_tc_kernel<XB_ACT_SIGMOID, 0, 0, 0>, (const void*)din_att_tc_kernel<XB_ACT_DICE, 0, 0, 0>,
                        (const void*)din_att_tc_kernel<XB_ACT_SIGMOID, 36, 80, 40>, (const void*)din_att_tc_kernel<XB_ACT_DICE, 36, 80, 40>);
   const int64_t tiles = (int64_t)a.requests * p.tiles_per_req;
-  XB_REQUIRE(tiles < ((int64_t)1 << 28), XB_ERR_LIMIT, "xb_din_attention: too many tiles");
-  p.split = a.use_softmax ? 1 : pick_split(tiles, p.T);        // the softmax needs all scores of a row in one place
+  XB_REQUIRE(tiles < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_din_attention: too many tiles");
+  p.split = a.use_softmax ? 1 : att_split(tiles, p.T, cluster_slots);        // the softmax needs all scores of a row in one place
   const TcSmemLayout L = tc_layout(g, p.T);
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;         // as launch_dependent
