@@ -302,14 +302,16 @@ __device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t 
   }
 }
 
-template <typename TOut>
+// B_MN is a template parameter because the K-major kernel must not pay for the other layout: with a run-time test of it in the
+// MMA and load loops 8 products of [65536, 256] x [256, 128] took 78 us, 74 without.
+template <typename TOut, bool B_MN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ UmmaGemmParams p) {
   using namespace umma;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int b_stage_bytes = (p.b_mn ? (p.block_n + 63) / 64 * 64 : p.block_n) * BLOCK_K * 2;
+  const int b_stage_bytes = (B_MN ? (p.block_n + 63) / 64 * 64 : p.block_n) * BLOCK_K * 2;
   uint8_t* smem_a = smem;
   const int STAGES = p.stages;
   uint8_t* smem_b = smem + STAGES * A_STAGE_BYTES;      // per-stage B tiles, or the resident B tile (all k blocks)
@@ -363,7 +365,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (lane == 0) {
       // one k block of B: one box of block_n rows x 64 k, or (N-major) boxes of 64 k rows x 64 columns side by side
       auto load_b = [&](uint32_t dst, uint32_t bar, int kb, int n0, int b) {
-        if (!p.b_mn) {
+        if (!B_MN) {
           tma_load_3d(dst, &map_b, bar, kb * BLOCK_K, n0, b);
         } else {
           for (int j = 0; j * 64 < p.block_n; ++j) tma_load_3d(dst + j * MN_BOX_BYTES, &map_b, bar, n0 + j * 64, kb * BLOCK_K, b);
@@ -428,7 +430,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 #pragma unroll
           for (int k = 0; k < BLOCK_K / 16; ++k) {
             const uint64_t da = make_desc_sw128(a_addr + k * 32, 1024);
-            const uint64_t db = p.b_mn ? make_desc_sw128_mn(b_addr + k * 2048, MN_BOX_BYTES) : make_desc_sw128(b_addr + k * 32, 1024);
+            const uint64_t db = B_MN ? make_desc_sw128_mn(b_addr + k * 2048, MN_BOX_BYTES) : make_desc_sw128(b_addr + k * 32, 1024);
             mma_f16_ss_elect(tmem_acc, da, db, p.idesc, (kb > 0 || k > 0) ? 1u : 0u);
           }
           mma_commit_elect(smem_u32(&empty_bar[s]));     // slot free once these MMAs have read it
@@ -578,12 +580,12 @@ bool umma_eligible(const xb_gemm_args& a) {
   return true;
 }
 
-template <typename TOut>
+template <typename TOut, bool B_MN>
 int launch_umma(const CUtensorMap& ma, const CUtensorMap& mb, const UmmaGemmParams& p, dim3 grid, size_t smem,
                 cudaStream_t s) {
   static PerDeviceOnce attr_set;   // per instantiation
-  XB_SET_MAX_SMEM_ONCE(attr_set, SMEM_BUDGET + 6 * 1024, (const void*)gemm_umma_kernel<TOut>);
-  launch_dependent(gemm_umma_kernel<TOut>, grid, GEMM_THREADS, smem, s, ma, mb, p);
+  XB_SET_MAX_SMEM_ONCE(attr_set, SMEM_BUDGET + 6 * 1024, (const void*)gemm_umma_kernel<TOut, B_MN>);
+  launch_dependent(gemm_umma_kernel<TOut, B_MN>, grid, GEMM_THREADS, smem, s, ma, mb, p);
   return check_launch("gemm_umma_kernel");
 }
 
@@ -691,9 +693,10 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
     smem = (size_t)p.stages * stage_bytes + tail + 1024;
   }
   switch (a.y_dtype) {
-    case XB_F16: return launch_umma<__half>(ma, mb, p, grid, smem, stream);
-    case XB_BF16: return launch_umma<__nv_bfloat16>(ma, mb, p, grid, smem, stream);
-    default: return launch_umma<float>(ma, mb, p, grid, smem, stream);
+    case XB_F16: return p.b_mn ? launch_umma<__half, true>(ma, mb, p, grid, smem, stream) : launch_umma<__half, false>(ma, mb, p, grid, smem, stream);
+    case XB_BF16:
+      return p.b_mn ? launch_umma<__nv_bfloat16, true>(ma, mb, p, grid, smem, stream) : launch_umma<__nv_bfloat16, false>(ma, mb, p, grid, smem, stream);
+    default: return launch_umma<float, false>(ma, mb, p, grid, smem, stream);      // (never b_mn: umma_eligible)
   }
 }
 
