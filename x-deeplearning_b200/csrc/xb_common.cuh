@@ -152,13 +152,4 @@ __device__ __forceinline__ float act_prelu(float x, float w) {
 }
 __device__ __forceinline__ float act_sigmoid(float x) { return 1.f / (1.f + __expf(-x)); }
 
-__device__ __forceinline__ float apply_epilogue(const EpiParams& e, float v, int col) {
-  switch (e.kind) {
-    case XB_EPI_PRELU: return act_prelu(v, e.a[e.count == 1 ? 0 : col]);
-    case XB_EPI_DICE: return act_dice(v, e.a[col], e.b[col], dice_rstd(e.c[col], e.nosqrt));
-    case XB_EPI_SIGMOID: return act_sigmoid(v);
-    default: return v;
-  }
-}
-
 }  // namespace xb

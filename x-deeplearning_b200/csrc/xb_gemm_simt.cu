@@ -378,7 +378,8 @@ static int launch_simt_tm(const SimtGemmParams& p, int tn, dim3 grid, cudaStream
 }
 
 // Tile of a product: a wave of CTAs costs what its busiest SM computes, TM*TN a k slice and output pair, plus what
-// the operand reads and the slice's overhead cost beside it; the tile with the cheapest sum of waves is taken. The general
+// the operand reads (1.5 TN + 0.75 TM) and the slice's barrier and index work (4) cost beside it; the tile with the cheapest sum
+// of waves is taken. The three weights are estimates in units of FMAs, not fitted to measurements of each tile. The general
 // kernel has fewer widths.
 static void pick_simt_tile(int64_t M, int64_t N, int64_t batch, bool f32, int* tm, int* tn) {
   double best = 0;
@@ -416,6 +417,7 @@ int gemm_simt(const xb_gemm_args& a, cudaStream_t stream) {
   int tm = 8, tn = 8;
   const bool f32 = a.ab_dtype == XB_F32 && !a.trans_a && !a.trans_b;
   pick_simt_tile(a.M, a.N, a.batch, f32, &tm, &tn);
+  // (the entry point's limits, whatever the tile; a grid of any of them would take more rows)
   XB_REQUIRE((a.M + 63) / 64 <= 65535 && a.batch <= 65535, XB_ERR_LIMIT, "xb_gemm: M or batch too large for the SIMT engine");
   p.tiles_n = (a.N + 16 * tn - 1) / (16 * tn);
   const int64_t tiles = (((int64_t)a.M + 16 * tm - 1) / (16 * tm)) * p.tiles_n;

@@ -341,7 +341,7 @@ extern "C" int xb_gru(const void* x, void* y, int64_t batch, int32_t T, int32_t 
                       const void* i2h_bias, const void* h2h_bias, int32_t dtype, xb_stream_t s) {
   XB_REQUIRE(x && y && i2h && h2h && i2h_bias && h2h_bias, XB_ERR_ARG, "xb_gru: null tensor");
   XB_REQUIRE(batch >= 0 && T >= 0 && H >= 1, XB_ERR_ARG, "xb_gru: bad sizes");
-  XB_REQUIRE(H <= 64, XB_ERR_LIMIT, "xb_gru: hidden size %d, at most 64 (weights are kept in shared memory)", H);
+  XB_REQUIRE(H <= 64, XB_ERR_LIMIT, "xb_gru: hidden size %d, at most 64 (weights are kept in registers)", H);
   XB_REQUIRE(dtype == XB_F32 || dtype == XB_F16, XB_ERR_UNSUPPORTED, "xb_gru: dtype %d", dtype);
   XB_REQUIRE(batch < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gru: batch too large");
   if (batch == 0 || T == 0) return 0;

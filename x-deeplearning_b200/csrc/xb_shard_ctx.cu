@@ -223,10 +223,7 @@ extern "C" int xb_shard_ctx_create(xb_shard_ctx** out, const void* unique_id128,
 
 // slice w of `send` goes to rank w, slice w of `recv` comes from rank w; `bytes` per slice
 static int all_to_all_equal(xb_shard_ctx* c, const void* send, void* recv, size_t bytes, cudaStream_t stream) {
-  if (c->world == 1) {
-    if (recv != send) XB_CUDA(cudaMemcpyAsync(recv, send, bytes, cudaMemcpyDeviceToDevice, stream));
-    return 0;
-  }
+  if (c->world == 1) return 0;                // both sides are one buffer (xb_shard_ctx_create)
   XB_NCCL(nccl().GroupStart());
   for (int w = 0; w < c->world; ++w) {
     XB_NCCL(nccl().Send(static_cast<const char*>(send) + (size_t)w * bytes, bytes, kNcclInt8, w, c->comm, stream));
