@@ -1,0 +1,34 @@
+"""The two tensor-core engines behind xb_augru_shared (few tiles: warp-level MMAs, many: tcgen05) over lists longer than a chunk
+of 128 steps, ragged tiles of four and of eight warps, and a candidate whose scores are no numbers, which no other candidate
+may see. Tolerance as in test_gpu_rnn.py."""
+import numpy as np
+import pytest
+import torch
+
+import orc
+import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,T", [(36, 127), (36, 128), (36, 129), (36, 200), (4, 257), (60, 130), (18, 5)])
+@pytest.mark.parametrize("R,n_cand", [(1, 17), (2, 65), (16, 1000), (80, 130)])
+def test_augru_over_chunks_of_steps(H, T, R, n_cand):
+    pkg.load()
+    from x_deeplearning_b200 import ops, capi
+    rng = np.random.default_rng(H + T)
+    h16 = lambda a: torch.from_numpy(a.astype(np.float32)).to("cuda", torch.float16)
+    x, att = rng.normal(0, 0.7, (R, T, H)), rng.dirichlet(np.ones(T) * 0.3, R * n_cand)
+    Wg, bg = rng.normal(0, 1 / np.sqrt(2 * H), (2 * H, 2 * H)), rng.normal(0.5, 0.2, 2 * H)
+    Wc, bc = rng.normal(0, 1 / np.sqrt(2 * H), (2 * H, H)), rng.normal(0, 0.1, H)
+    dx, da, dWg, dbg, dWc, dbc = h16(x), h16(att), h16(Wg), h16(bg), h16(Wc), h16(bc)
+    bad = n_cand // 2
+    da[bad] = torch.nan
+    y = torch.full((R * n_cand + 1, H), 9.0, dtype=torch.float16, device="cuda")
+    capi.check(capi.lib().xb_augru_shared(ops.ptr(dx), ops.ptr(da), ops.ptr(y), R, n_cand, T, H, ops.ptr(dWg), ops.ptr(dbg),
+                                          ops.ptr(dWc), ops.ptr(dbc), capi.XB_GEMM_TCGEN05, ops.stream()))
+    assert (y[-1] == 9.0).all() and y[bad].isnan().all()
+    few = [i for r in {0, R - 1} for i in range(r * n_cand, (r + 1) * n_cand) if i != bad][:200] + [R * n_cand - 1]
+    f = lambda t: t.float().cpu().numpy()
+    want = orc.augru(f(dx)[np.array(few) // n_cand], f(da)[few], f(dWg), f(dbg), f(dWc), f(dbc))[:, T - 1, :]
+    np.testing.assert_allclose(f(y)[few], want, rtol=0, atol=8e-3)
