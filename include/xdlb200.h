@@ -390,7 +390,7 @@ int xb_pack_weight_kmajor(const void* W, int32_t w_dtype, int32_t K, int32_t N, 
  *   x = [q, k, q-k, q*k] (4d), s = W2'act(W1'act(W0'x+b0)+b1)+b2,
  *   out[n] = sum_t s[n,t] * k[t]     (optionally masked softmax over t first).
  * The 4d-wide concat is built in shared memory and never written to HBM. */
-enum { XB_ACT_NONE = 0, XB_ACT_SIGMOID = 1, XB_ACT_DICE = 2 };
+enum { XB_ACT_NONE = 0, XB_ACT_SIGMOID = 1, XB_ACT_DICE = 2, XB_ACT_PRELU = 3 };   /* PReLU: the tower alone */
 /* `engine` of xb_din_att_args takes XB_GEMM_AUTO / XB_GEMM_SIMT / XB_GEMM_TCGEN05 or this value: the tcgen05
  * engine that regroups layer 1 as q x (Wq + Wd + diag(k_t) Wp) and runs two steps per MMA (needs `packed`). */
 enum { XB_ATT_ENGINE_PAIR = 3,
@@ -470,6 +470,10 @@ typedef struct xb_din_tower_args {
   const void* W3; const float* b3;                                                              /* [n2, n3] */
   int32_t softmax;
   const void* packed;                   /* image written by xb_din_tower_pack */
+  int32_t act;                          /* 0 or XB_ACT_DICE; XB_ACT_PRELU: gamma1 [n1] and gamma2 [n2] are the slopes, mean and
+                                         * var unused; activations and the bias of layer 2 in fp32, logits not rounded to fp16
+                                         * (what xb_gemm with XB_EPI_PRELU and fp16 outputs computes). The same for
+                                         * xb_din_tower_pack and xb_din_tower */
 } xb_din_tower_args;
 
 /* 0 for shapes the kernel does not take (d <= 64, n1 <= 256, n2 <= 128, n3 <= 8). */
@@ -516,6 +520,8 @@ int xb_prelu(const void* x, void* y, int64_t size, const void* w, int64_t inner,
 /* SigmoidOp, blaze/blaze/operator/op/sigmoid_op.cu:11-17 */
 int xb_sigmoid(const void* x, void* y, int64_t size, int32_t dtype, xb_stream_t stream);
 /* SoftmaxOp, blaze/blaze/operator/op/softmax_op.cu:25-67: softmax over c with outer n, inner w */
+/* xb_softmax of n rows of c fp32 scores, written as fp32 and, rounded from it, as fp16 (the gates of xb_augru_shared) */
+int xb_softmax_scores(const float* x, float* y, void* y16, int64_t n, int32_t c, xb_stream_t stream);
 int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t w, int32_t dtype, xb_stream_t stream);
 /* BatchNormalizationOp (inference), blaze/blaze/operator/op/batch_normalization_op.cu:12 */
 int xb_batchnorm(const void* x, void* y, int64_t size, int32_t c, const void* gamma, const void* beta,

@@ -1,0 +1,65 @@
+"""What the DIEN-style model runs around its AUGRU: softmax with an fp16 copy and the fused tower with PReLU, against plain
+torch in 64 bits."""
+import pytest
+import torch
+
+import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def _ops():
+    pkg.load()
+    from x_deeplearning_b200 import ops, capi
+    return ops, capi, capi.lib()
+
+
+@pytest.mark.parametrize("n,c", [(1, 16), (33, 20), (500, 64), (131, 65), (77, 100), (40, 101), (9, 128), (35, 129), (64, 256),
+                                 (5, 257), (7, 3), (50000, 36)])
+def test_softmax_scores(n, c):
+    ops, capi, L = _ops()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    for shift in (0, 1):                                            # rows of whole 16-byte pieces, then misaligned ones
+        x = torch.randn(n * c + 1, generator=g, device="cuda")[shift:shift + n * c] * 6
+        x[0] = -torch.inf
+        y, y16 = torch.full((n, c), 9.0, device="cuda"), torch.full((n, c), 9.0, device="cuda", dtype=torch.float16)
+        capi.check(L.xb_softmax_scores(ops.ptr(x), ops.ptr(y), ops.ptr(y16), n, c, ops.stream()))
+        want = x.double().view(n, c).softmax(1)
+        # __expf: 2 + |x| units in the last place at the most, the sum of them and the division beside it
+        assert ((y.double() - want).abs() <= 64 * 2.0 ** -24 * want + 1e-38).all()
+        assert torch.equal(y16, y.half())
+        z = torch.full_like(y, 9.0)
+        capi.check(L.xb_softmax(ops.ptr(x), ops.ptr(z), n, c, 1, capi.XB_F32, ops.stream()))
+        assert torch.equal(y, z)
+        capi.check(L.xb_softmax(ops.ptr(x), ops.ptr(x), n, c, 1, capi.XB_F32, ops.stream()))       # in place
+        assert torch.equal(y.view(-1), x)
+
+
+@pytest.mark.parametrize("R,n_cand,T,d,du,dims", [(1, 5, 3, 36, 144, (200, 80, 2)), (3, 130, 20, 36, 144, (200, 80, 2)),
+                                                  (2, 300, 7, 32, 40, (64, 32, 1)), (150, 129, 2, 16, 8, (48, 24, 8)),
+                                                  (160, 200, 2, 36, 30, (77, 33, 3))])
+@pytest.mark.parametrize("softmax", [True, False])
+def test_tower_with_prelu(R, n_cand, T, d, du, dims, softmax):
+    ops, capi, _ = _ops()
+    g = torch.Generator().manual_seed(R + d)
+    r = lambda *s: torch.randn(s, generator=g)
+    n1, n2, n3 = dims
+    h = lambda x: x.half().float()
+    W1, W2, W3 = h(r(du + 5 * d, n1) / (du + 5 * d) ** 0.5), h(r(n1, n2) / n1 ** 0.5), h(r(n2, n3) / n2 ** 0.5)
+    b1, b2, b3 = r(n1) * 0.1, r(n2) * 0.1, r(n3) * 0.1
+    s1, s2 = torch.rand(n1, generator=g) * 0.5, torch.rand(n2, generator=g) * 0.5
+    user, q, k, att = [h(r(*s)).half().cuda() for s in ((R, du), (R * n_cand, d), (R * T, d), (R * n_cand, d))]
+    tower = ops.DinTower(d, du, W1, b1, [s1], W2, b2, [s2], W3, b3, softmax=softmax, act=capi.XB_ACT_PRELU)
+    got = tower(user, q, k, att, R, n_cand, T).double().cpu()
+    D = lambda x: x.double().cpu()
+    his = D(k).view(R, T, d).sum(1).half().double().repeat_interleave(n_cand, 0)
+    x = torch.cat([D(user).repeat_interleave(n_cand, 0), D(q), his, (D(q) * his).half().double(), D(att), (D(q) - his).half().double()], 1)
+    for W, b, s in ((W1, b1, s1), (W2, b2, s2)):
+        x = x @ W.double() + b.double()
+        x = torch.where(x < 0, x * s.double(), x).half().double()
+    want = x @ W3.double() + b3.double()
+    # two roundings to fp16 (2^-11 of the value) carried through the layers after them; his_sum may round to its neighbour
+    tol = 2.0 ** -9 * (1 + want.abs().max()) * 1.5
+    if softmax:
+        want = want.softmax(1)
+    assert (got - want).abs().max() <= tol, (float((got - want).abs().max()), float(tol))

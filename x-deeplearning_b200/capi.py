@@ -14,7 +14,7 @@ XB_EPI_NONE, XB_EPI_PRELU, XB_EPI_DICE, XB_EPI_SIGMOID = 0, 1, 2, 3
 XB_BIAS_NONE, XB_BIAS_ROW, XB_BIAS_FULL = 0, 1, 2
 XB_ATT_ENGINE_PAIR, XB_ATT_ENGINE_SPLIT = 3, 4
 XB_GEMM_AUTO, XB_GEMM_SIMT, XB_GEMM_TCGEN05 = 0, 1, 2
-XB_ACT_NONE, XB_ACT_SIGMOID, XB_ACT_DICE = 0, 1, 2
+XB_ACT_NONE, XB_ACT_SIGMOID, XB_ACT_DICE, XB_ACT_PRELU = 0, 1, 2, 3
 XB_MAX_POOL_ITEMS, XB_MAX_POOL_GROUPS = 4, 32
 (XB_EW_ADD, XB_EW_SUB, XB_EW_MUL, XB_EW_DIV, XB_EW_MAX, XB_EW_MIN, XB_EW_EQ, XB_EW_NE,
  XB_EW_BROADCAST_TO, XB_EW_WHERE) = range(10)
@@ -69,7 +69,7 @@ class DinTowerArgs(C.Structure):
                 ("prob", vp), ("requests", i32), ("n_cand", i32), ("T", i32), ("d", i32), ("du", i32), ("n1", i32),
                 ("n2", i32), ("n3", i32), ("W1", vp), ("b1", vp), ("gamma1", vp), ("mean1", vp), ("var1", vp),
                 ("W2", vp), ("b2", vp), ("gamma2", vp), ("mean2", vp), ("var2", vp), ("W3", vp), ("b3", vp),
-                ("softmax", i32), ("packed", vp)]
+                ("softmax", i32), ("packed", vp), ("act", i32)]
 
 
 # every symbol include/xdlb200.h declares: (restype, argtypes)
@@ -140,6 +140,7 @@ SYMBOLS = {
     "xb_prelu": (i32, [vp, vp, i64, vp, i64, i32, i32, vp]),
     "xb_sigmoid": (i32, [vp, vp, i64, i32, vp]),
     "xb_softmax": (i32, [vp, vp, i64, i32, i64, i32, vp]),
+    "xb_softmax_scores": (i32, [vp, vp, vp, i64, i32, vp]),
     "xb_batchnorm": (i32, [vp, vp, i64, i32, vp, vp, vp, vp, f32, i32, i32, vp]),
     "xb_elementwise": (i32, [i32, vp, vp, vp, vp, vp, vp, vp, vp, i32, vp]),
     "xb_copy2d": (i32, [vp, i64, i32, vp, i64, i32, i64, i64, vp]),

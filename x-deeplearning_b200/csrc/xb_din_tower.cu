@@ -18,6 +18,9 @@
 // Eight worker warps in two warpgroups split the columns of every phase; a ninth warp issues the MMAs.
 // Dice runs on packed fp16 pairs with one SFU instruction per pair, as in the attention unit:
 //   Dice(x) = x * (C + D*tanh(A*x + B)), A = rstd/2, B = -mean*rstd/2, C = (1+gamma)/2, D = (1-gamma)/2.
+// PReLU towers (the DIEN-style model: no q-his_sum columns, so their rows of W1 are zero) round where a chain of GEMMs with
+// fp16 outputs and an fp32 one at the end rounds: activations and the bias of layer 2 in fp32, logits unrounded. 16 x 1000
+// candidates: 17 us after what is before them, 45 as feature assembly, three GEMMs and a softmax.
 #include <algorithm>
 #include <cstring>
 
@@ -79,7 +82,7 @@ struct TowerParams {
   float* prob;
   float* hs;            // [requests, d]
   float* partial;       // [requests, n1]
-  int requests, n_cand, T, d, du, n1, n2, n3, softmax, tiles_per_req;
+  int requests, n_cand, T, d, du, n1, n2, n3, softmax, tiles_per_req, act;
   const __half* W1; const float* b1; const float *g1, *m1, *v1;
   const __half* W2; const float* b2; const float *g2, *m2, *v2;
   const __half* W3; const float* b3;
@@ -119,7 +122,7 @@ __global__ void tower_pack_kernel(const __grid_constant__ TowerParams p, uint8_t
     __half v = zero;
     if (n < p.n2) {
       if (kk < p.n1) v = p.W2[(int64_t)kk * p.n2 + n];
-      else if (kk == G.n1p) v = __float2half_rn(p.b2 ? p.b2[n] : 0.f);
+      else if (kk == G.n1p && p.act == XB_ACT_DICE) v = __float2half_rn(p.b2 ? p.b2[n] : 0.f);
     }
     w2[(kk >> 3) * (G.n2p * 8) + n * 8 + (kk & 7)] = v;
   }
@@ -131,6 +134,17 @@ __global__ void tower_pack_kernel(const __grid_constant__ TowerParams p, uint8_t
       const float *gm = layer ? p.g2 : p.g1, *mu = layer ? p.m2 : p.m1, *var = layer ? p.v2 : p.v1;
       uint4* c = layer ? c2 : c1;
       for (int j = threadIdx.x; j < np / 2; j += blockDim.x) {
+        if (p.act == XB_ACT_PRELU) {                // slopes and (layer 2) biases of the two columns, fp32
+          float v[4] = {0, 0, 0, 0};
+          for (int u = 0; u < 2; ++u) {
+            const int col = 2 * j + u;
+            if (col >= n) continue;
+            v[u] = gm[col];
+            v[2 + u] = layer && p.b2 ? p.b2[col] : 0.f;
+          }
+          c[j] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+          continue;
+        }
         float A[2] = {0, 0}, B[2] = {0, 0}, C[2] = {0, 0}, D[2] = {0, 0};
         for (int u = 0; u < 2; ++u) {
           const int col = 2 * j + u;
@@ -225,6 +239,7 @@ __global__ void __launch_bounds__(PT_COLS * PT_SLICES) din_tower_partial_kernel(
 }
 
 // ---- the tower kernel --------------------------------------------------------------------------------
+template <int ACT>
 __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __grid_constant__ TowerParams p) {
   using namespace umma;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -398,16 +413,28 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
           const float4* pp = reinterpret_cast<const float4*>(ps + 16 * b);
           const uint4* cc = c1 + 8 * b;
           uint32_t y[8], th[8];
+          if constexpr (ACT == XB_ACT_PRELU) {
 #pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {
-            const float4 pv = pp[e4];
-            y[2 * e4] = h2u(__floats2half2_rn(__uint_as_float(cur[4 * e4]) + pv.x, __uint_as_float(cur[4 * e4 + 1]) + pv.y));
-            y[2 * e4 + 1] = h2u(__floats2half2_rn(__uint_as_float(cur[4 * e4 + 2]) + pv.z, __uint_as_float(cur[4 * e4 + 3]) + pv.w));
+            for (int e4 = 0; e4 < 4; ++e4) {
+              const float4 pv = pp[e4];
+              const uint4 s0 = cc[2 * e4], s1 = cc[2 * e4 + 1];
+              y[2 * e4] = h2u(__floats2half2_rn(act_prelu(__uint_as_float(cur[4 * e4]) + pv.x, __uint_as_float(s0.x)),
+                                                act_prelu(__uint_as_float(cur[4 * e4 + 1]) + pv.y, __uint_as_float(s0.y))));
+              y[2 * e4 + 1] = h2u(__floats2half2_rn(act_prelu(__uint_as_float(cur[4 * e4 + 2]) + pv.z, __uint_as_float(s1.x)),
+                                                    act_prelu(__uint_as_float(cur[4 * e4 + 3]) + pv.w, __uint_as_float(s1.y))));
+            }
+          } else {
+#pragma unroll
+            for (int e4 = 0; e4 < 4; ++e4) {
+              const float4 pv = pp[e4];
+              y[2 * e4] = h2u(__floats2half2_rn(__uint_as_float(cur[4 * e4]) + pv.x, __uint_as_float(cur[4 * e4 + 1]) + pv.y));
+              y[2 * e4 + 1] = h2u(__floats2half2_rn(__uint_as_float(cur[4 * e4 + 2]) + pv.z, __uint_as_float(cur[4 * e4 + 3]) + pv.w));
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) th[e] = tanh_f16x2(h2u(__hfma2(u2h(y[e]), u2h(cc[e].x), u2h(cc[e].y))));
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = h2u(__hmul2(u2h(y[e]), __hfma2(u2h(th[e]), u2h(cc[e].w), u2h(cc[e].z))));
           }
-#pragma unroll
-          for (int e = 0; e < 8; ++e) th[e] = tanh_f16x2(h2u(__hfma2(u2h(y[e]), u2h(cc[e].x), u2h(cc[e].y))));
-#pragma unroll
-          for (int e = 0; e < 8; ++e) y[e] = h2u(__hmul2(u2h(y[e]), __hfma2(u2h(th[e]), u2h(cc[e].w), u2h(cc[e].z))));
           tmem_st8(a2t + 8 * b, y);
         };
         if (b_begin < b_end) tmem_ld16_nowait(lane_addr + 16 * b_begin, va);
@@ -436,14 +463,24 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
           const uint4* cc = c2 + 8 * b;
           uint32_t y[8], th[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            y[e] = h2u(__floats2half2_rn(__uint_as_float(cur[2 * e]), __uint_as_float(cur[2 * e + 1])));
+          for (int e = 0; e < 8; ++e) {
+            if constexpr (ACT == XB_ACT_PRELU) {
+              const uint4 sb = cc[e];
+              y[e] = h2u(__floats2half2_rn(act_prelu(__uint_as_float(cur[2 * e]) + __uint_as_float(sb.z), __uint_as_float(sb.x)),
+                                           act_prelu(__uint_as_float(cur[2 * e + 1]) + __uint_as_float(sb.w), __uint_as_float(sb.y))));
+            } else {
+              y[e] = h2u(__floats2half2_rn(__uint_as_float(cur[2 * e]), __uint_as_float(cur[2 * e + 1])));
+            }
+          }
+          if constexpr (ACT == XB_ACT_DICE) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) th[e] = tanh_f16x2(h2u(__hfma2(u2h(y[e]), u2h(cc[e].x), u2h(cc[e].y))));
+            for (int e = 0; e < 8; ++e) th[e] = tanh_f16x2(h2u(__hfma2(u2h(y[e]), u2h(cc[e].x), u2h(cc[e].y))));
+          }
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
             // the layer output is an fp16 tensor in the model's graph: round, then feed layer 3 in fp32
-            const float2 f = __half22float2(__hmul2(u2h(y[e]), __hfma2(u2h(th[e]), u2h(cc[e].w), u2h(cc[e].z))));
+            const float2 f = __half22float2(ACT == XB_ACT_DICE ? __hmul2(u2h(y[e]), __hfma2(u2h(th[e]), u2h(cc[e].w), u2h(cc[e].z)))
+                                                               : u2h(y[e]));
             const float* wr = w3 + (16 * b + 2 * e) * TW_MAX_N3;
 #pragma unroll
             for (int j = 0; j < TW_MAX_N3; ++j)
@@ -470,7 +507,8 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
         for (int j = 0; j < TW_MAX_N3; ++j) {
           if (j < n3) {
             // layer-3 output rounded to the model's fp16, as the un-fused graph stores it
-            logit[j] = __half2float(__float2half_rn(logit[j] + lg[row * TW_MAX_N3 + j] + b3[j]));
+            logit[j] = logit[j] + lg[row * TW_MAX_N3 + j] + b3[j];
+            if (ACT == XB_ACT_DICE) logit[j] = __half2float(__float2half_rn(logit[j]));
             mx = fmaxf(mx, logit[j]);
           }
         }
@@ -481,7 +519,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
             if (j < n3) { logit[j] = __expf(logit[j] - mx); sum += logit[j]; }
           const float inv = 1.f / sum;
 #pragma unroll
-          for (int j = 0; j < TW_MAX_N3; ++j) logit[j] *= inv;
+          for (int j = 0; j < TW_MAX_N3; ++j) logit[j] = ACT == XB_ACT_DICE ? logit[j] * inv : logit[j] / sum;
         }
         if (n < p.n_cand) {
           float* o = p.prob + ((int64_t)r * p.n_cand + n) * n3;
@@ -497,6 +535,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
     cp_async_wait_all();
   }
 
+  pdl_release();
   tc_fence_before_sync();
   __syncthreads();
   if (warp == TW_MMA_WARP) {
@@ -525,6 +564,7 @@ void fill_params(TowerParams& p, const xb_din_tower_args& a) {
   p.W2 = (const __half*)a.W2; p.b2 = a.b2; p.g2 = a.gamma2; p.m2 = a.mean2; p.v2 = a.var2;
   p.W3 = (const __half*)a.W3; p.b3 = a.b3;
   p.packed = (const uint8_t*)a.packed;
+  p.act = a.act == XB_ACT_PRELU ? XB_ACT_PRELU : XB_ACT_DICE;
 }
 
 }  // namespace
@@ -540,8 +580,10 @@ using namespace xb;
 static int validate_tower(const xb_din_tower_args* a, const char* who) {
   XB_REQUIRE(a, XB_ERR_ARG, "%s: null arguments", who);
   XB_REQUIRE(a->d > 0 && a->du >= 0 && a->n1 > 0 && a->n2 > 0 && a->n3 > 0, XB_ERR_ARG, "%s: bad sizes", who);
-  XB_REQUIRE(a->W1 && a->W2 && a->W3 && a->gamma1 && a->mean1 && a->var1 && a->gamma2 && a->mean2 && a->var2, XB_ERR_ARG,
-             "%s: missing weights or Dice parameters", who);
+  XB_REQUIRE(a->act == 0 || a->act == XB_ACT_DICE || a->act == XB_ACT_PRELU, XB_ERR_UNSUPPORTED, "%s: activation %d", who, a->act);
+  XB_REQUIRE(a->W1 && a->W2 && a->W3 && a->gamma1 && a->gamma2 &&
+                 (a->act == XB_ACT_PRELU || (a->mean1 && a->var1 && a->mean2 && a->var2)),
+             XB_ERR_ARG, "%s: missing weights or Dice parameters", who);
   int why = 0;
   XB_REQUIRE(tower_eligible(*a, &why), XB_ERR_UNSUPPORTED, "%s: shape outside the fused tower kernel (reason %d)", who, why);
   return 0;
@@ -604,8 +646,9 @@ extern "C" int xb_din_tower(const xb_din_tower_args* a, void* workspace, size_t 
   else din_tower_partial_kernel<<<pgrid, PT_COLS * PT_SLICES, psmem, stream>>>(p);
   if (int rc = check_launch("din_tower_partial_kernel")) return rc;
   static PerDeviceOnce attr_set;
-  XB_SET_MAX_SMEM_ONCE(attr_set, 220 * 1024, (const void*)din_tower_tc_kernel);
+  XB_SET_MAX_SMEM_ONCE(attr_set, 220 * 1024, (const void*)din_tower_tc_kernel<XB_ACT_DICE>, (const void*)din_tower_tc_kernel<XB_ACT_PRELU>);
   const int grid = (int)std::min<int64_t>(tiles, sm_count());
-  launch_dependent(din_tower_tc_kernel, grid, TW_THREADS, g.total, stream, p);
+  if (p.act == XB_ACT_PRELU) launch_dependent(din_tower_tc_kernel<XB_ACT_PRELU>, grid, TW_THREADS, g.total, stream, p);
+  else launch_dependent(din_tower_tc_kernel<XB_ACT_DICE>, grid, TW_THREADS, g.total, stream, p);
   return check_launch("din_tower_tc_kernel");
 }

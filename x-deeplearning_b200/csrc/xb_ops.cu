@@ -125,6 +125,80 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(const void* x, void* 
   }
 }
 
+// The same for fp32 rows, eight lanes a row and four columns a lane at a time: a quarter of the shuffles, loads of 16 bytes
+// where the rows allow them. y16, where given, receives the fp16 rounding of y, which saves the pass that would convert it.
+// 16 000 rows of 100 with the fp16 copy: 5.6 us after the kernel before, 9.5 as two launches.
+template <int PER4>
+__global__ void __launch_bounds__(256) softmax_f32_kernel(const float* x, float* y, __half* y16, int64_t n, int c, int vec) {
+  pdl_begin();
+  const int l = threadIdx.x & 7, sub = threadIdx.x >> 3 & 3;
+  const int64_t rows = (int64_t)gridDim.x * 32;
+  for (int64_t at = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 5) * 4; at < n; at += rows) {       // the same for a warp: its shuffles stay whole
+    const int64_t r = at + sub;
+    const bool in = r < n;
+    const float* xr = x + r * c;
+    float v[PER4][4], m = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < PER4; ++i) {
+      const int j = 4 * (l + 8 * i);
+      if (vec) {
+        const float4 q = in && j < c ? *reinterpret_cast<const float4*>(xr + j) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        v[i][0] = q.x; v[i][1] = q.y; v[i][2] = q.z; v[i][3] = q.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[i][e] = in && j + e < c ? xr[j + e] : -INFINITY;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < PER4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) m = fmaxf(m, v[i][e]);
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < PER4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        v[i][e] = 4 * (l + 8 * i) + e < c ? __expf(v[i][e] - m) : 0.f;
+        s += v[i][e];
+      }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (!in) continue;
+#pragma unroll
+    for (int i = 0; i < PER4; ++i) {
+      const int j = 4 * (l + 8 * i);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[i][e] /= s;
+      if (vec && j < c) {
+        *reinterpret_cast<float4*>(y + r * c + j) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+        if (y16) {
+          const __half2 lo = __floats2half2_rn(v[i][0], v[i][1]), hi = __floats2half2_rn(v[i][2], v[i][3]);
+          *reinterpret_cast<uint2*>(y16 + r * c + j) =
+              make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (j + e < c) {
+            y[r * c + j + e] = v[i][e];
+            if (y16) y16[r * c + j + e] = __float2half_rn(v[i][e]);
+          }
+      }
+    }
+  }
+}
+static int launch_softmax_f32(const float* x, float* y, __half* y16, int64_t n, int c, cudaStream_t s) {
+  const int vec = c % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
+                  (reinterpret_cast<uintptr_t>(y16) & 7) == 0;
+  const unsigned grid = stream_grid(n, 32);
+  if (c <= 64) launch_dependent(softmax_f32_kernel<2>, grid, 256, 0, s, x, y, y16, n, c, vec);
+  else if (c <= 128) launch_dependent(softmax_f32_kernel<4>, grid, 256, 0, s, x, y, y16, n, c, vec);
+  else launch_dependent(softmax_f32_kernel<8>, grid, 256, 0, s, x, y, y16, n, c, vec);
+  return check_launch("softmax_f32_kernel");
+}
+
 struct EwParams {
   int op, dt;
   const void *a, *b, *c;
@@ -529,6 +603,7 @@ extern "C" int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t 
   XB_REQUIRE(float_dtype(dtype), XB_ERR_UNSUPPORTED, "xb_softmax: dtype %d", dtype);
   if (n == 0) return 0;
   if (w == 1 && c >= 16 && c <= 256) {
+    if (dtype == XB_F32) return launch_softmax_f32((const float*)x, (float*)y, nullptr, n, c, (cudaStream_t)s);
     const unsigned grid = stream_grid(n, 8);
     if (c <= 64) launch_dependent(softmax_rows_kernel<2>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
     else if (c <= 128) launch_dependent(softmax_rows_kernel<4>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
@@ -537,6 +612,14 @@ extern "C" int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t 
   }
   launch_dependent(softmax_kernel, stream_grid(n * w, 128), 128, 0, (cudaStream_t)s, x, y, n, c, w, dtype);
   return check_launch("softmax_kernel");
+}
+
+extern "C" int xb_softmax_scores(const float* x, float* y, void* y16, int64_t n, int32_t c, xb_stream_t s) {
+  XB_REQUIRE(x && y && y16 && n >= 0 && c > 0, XB_ERR_ARG, "xb_softmax_scores: bad arguments");
+  if (n == 0) return 0;
+  if (c >= 16 && c <= 256) return launch_softmax_f32(x, y, (__half*)y16, n, c, (cudaStream_t)s);
+  if (int rc = xb_softmax(x, y, n, c, 1, XB_F32, s)) return rc;
+  return xb_copy2d(y, c, XB_F32, y16, c, XB_F16, n, c, s);
 }
 
 extern "C" int xb_batchnorm(const void* x, void* y, int64_t size, int32_t c, const void* gamma, const void* beta,

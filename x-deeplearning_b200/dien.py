@@ -6,8 +6,8 @@ xdl-algorithm-solution/DIEN/script/utils.py:139-207, attention MLP and tower as 
     s[n, t]   = MLP_sigmoid([q_n, h_t, q_n - h_t, q_n * h_t])       raw scores, then softmax over t
     f[n]      = last state of AUGRU(h[r], s[n])                      [H]
     prob[n]   = softmax(PReLU-MLP([user | q_n | his_sum | q_n*his_sum | f_n]))
-Pooling, GRU, the fused attention unit (scores only), AUGRU and the tcgen05 GEMMs with PReLU epilogues run as
-kernels of the library; the feature assembly uses the strided-copy and elementwise kernels.
+Pooling, GRU, the fused attention unit (scores only), softmax, AUGRU and the fused tower with PReLU run as kernels of the
+library; with an engine of the caller's choice the tower is its assembly kernel and GEMMs of that engine.
 """
 import ctypes as C
 
@@ -43,6 +43,12 @@ class DienModel(DinModel):
         self.dW3 = ops.pack_weight_kmajor(t(tw["W3"]).to(device), torch.float16)
         self.db = [f32(tw["b1"]), f32(tw["b2"]), f32(tw["b3"])]
         self.dslope = [f32(tw["slope1"]), f32(tw["slope2"])]
+        # the same tower in one kernel: the layer input's columns up to the fourth candidate-side segment, which is where that
+        # kernel has the attention output, and zero rows for the fifth
+        W1 = np.zeros((self.dtin + D["d"], tw["W1"].shape[1]), np.float32)
+        W1[:self.dtin] = tw["W1"]
+        self.dtower = ops.DinTower(D["d"], D["user_groups"] * D["emb"], t(W1), t(tw["b1"]), [t(tw["slope1"])], t(tw["W2"]),
+                                   t(tw["b2"]), [t(tw["slope2"])], t(tw["W3"]), t(tw["b3"]), device=device, act=capi.XB_ACT_PRELU)
 
     def forward_dien(self, p):
         """Inputs already uploaded by DinModel.upload(). Returns probabilities [R*n_cand, 2] fp32."""
@@ -62,15 +68,19 @@ class DienModel(DinModel):
         raw = torch.empty((N, T), dtype=torch.float32, device=dev)
         self.att_sig(q, hseq.view(R * T, H), R, n_cand, T, out=p["att"], scores=raw)
         sm = torch.empty_like(raw)
-        check(L.xb_softmax(ops.ptr(raw), ops.ptr(sm), N, T, 1, F32, s))
         score16 = e16(N, T)
-        check(L.xb_copy2d(ops.ptr(sm), T, F32, ops.ptr(score16), T, F16, N, T, s))
+        check(L.xb_softmax_scores(ops.ptr(raw), ops.ptr(sm), ops.ptr(score16), N, T, s))
         # interest evolution: every candidate runs the AUGRU over its request's GRU states, which are read once
         # per 128-candidate tile; only the final state is kept
         final = e16(N, H)
         a = self.augru
         check(L.xb_augru_shared(ops.ptr(hseq), ops.ptr(score16), ops.ptr(final), R, n_cand, T, H, ops.ptr(a["Wg"]),
                                 ops.ptr(a["bg"]), ops.ptr(a["Wc"]), ops.ptr(a["bc"]), self.augru_engine, s))
+        if self.engine == capi.XB_GEMM_AUTO:
+            ws = self.dtower.workspace(R, dev)
+            prob = self.dtower(p["user_emb"], q, k.view(R * T, H), final, R, n_cand, T, ws=ws)
+            p["dien_keep"] = (hseq, raw, sm, score16, final, ws)                      # alive until the stream drains
+            return prob, dict(hseq=hseq, scores=sm, final=final)
         # tower input [user | q | his_sum | q*his_sum | final state | (q - his_sum: zero weights)]
         X = e16(N, self.dldx)
         check(L.xb_din_tower_input(ops.ptr(p["user_emb"]), du, ops.ptr(q), H, ops.ptr(k), H, ops.ptr(final), H, ops.ptr(X),

@@ -197,15 +197,19 @@ def device_status():
 
 
 class DinTower:
-    """Weights of the DIN tower (du+5d -> n1 -> n2 -> n3, Dice after the first two layers) packed for
-    xb_din_tower. W1 [du+5d, n1], W2 [n1, n2], W3 [n2, n3] are float32 CPU tensors in Blaze's [K, N] layout."""
+    """Weights of the DIN tower (du+5d -> n1 -> n2 -> n3, Dice after the first two layers, or PReLU) packed for
+    xb_din_tower. W1 [du+5d, n1], W2 [n1, n2], W3 [n2, n3] are float32 CPU tensors in Blaze's [K, N] layout; dice1, dice2:
+    (gamma, mean, var), or with act XB_ACT_PRELU (slopes,)."""
 
-    def __init__(self, d, du, W1, b1, dice1, W2, b2, dice2, W3, b3, softmax=True, device="cuda"):
+    def __init__(self, d, du, W1, b1, dice1, W2, b2, dice2, W3, b3, softmax=True, device="cuda", act=capi.XB_ACT_DICE):
         h = lambda x: x.to(device=device, dtype=torch.float16).contiguous()
         f = lambda x: x.to(device=device, dtype=torch.float32).contiguous()
         self.d, self.du = d, du
         self.n1, self.n2, self.n3 = W1.shape[1], W2.shape[1], W3.shape[1]
         assert W1.shape[0] == du + 5 * d and W2.shape[0] == self.n1 and W3.shape[0] == self.n2
+        self.act = act
+        if act == capi.XB_ACT_PRELU:
+            dice1, dice2 = [dice1[0]] * 3, [dice2[0]] * 3           # only the first of each is read
         self.keep = [h(W1), f(b1), f(dice1[0]), f(dice1[1]), f(dice1[2]), h(W2), f(b2), f(dice2[0]), f(dice2[1]),
                      f(dice2[2]), h(W3), f(b3)]
         self.softmax = softmax
@@ -223,7 +227,7 @@ class DinTower:
         k = self.keep
         a.W1, a.b1, a.gamma1, a.mean1, a.var1 = k[0].data_ptr(), k[1].data_ptr(), k[2].data_ptr(), k[3].data_ptr(), k[4].data_ptr()
         a.W2, a.b2, a.gamma2, a.mean2, a.var2 = k[5].data_ptr(), k[6].data_ptr(), k[7].data_ptr(), k[8].data_ptr(), k[9].data_ptr()
-        a.W3, a.b3 = k[10].data_ptr(), k[11].data_ptr()
+        a.W3, a.b3, a.act = k[10].data_ptr(), k[11].data_ptr(), self.act
         a.packed = self.packed.data_ptr()
         return a
 
