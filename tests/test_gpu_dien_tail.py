@@ -63,3 +63,30 @@ def test_tower_with_prelu(R, n_cand, T, d, du, dims, softmax):
     if softmax:
         want = want.softmax(1)
     assert (got - want).abs().max() <= tol, (float((got - want).abs().max()), float(tol))
+
+
+@pytest.mark.parametrize("R,n_cand,T,d,du,dims", [(150, 129, 3, 36, 144, (200, 80, 2)), (310, 100, 2, 20, 8, (48, 24, 5))])
+def test_dice_tower_over_several_tiles_a_block(R, n_cand, T, d, du, dims):
+    """More tiles than SMs: a block begins its next tile between the two epilogues of the one before."""
+    ops, capi, _ = _ops()
+    g = torch.Generator().manual_seed(R)
+    r = lambda *s: torch.randn(s, generator=g)
+    u = lambda n, lo, hi: torch.rand(n, generator=g) * (hi - lo) + lo
+    n1, n2, n3 = dims
+    h = lambda x: x.half().float()
+    W1, W2, W3 = h(r(du + 5 * d, n1) / (du + 5 * d) ** 0.5), h(r(n1, n2) / n1 ** 0.5), h(r(n2, n3) / n2 ** 0.5)
+    b1, b2, b3 = r(n1) * 0.1, r(n2) * 0.1, r(n3) * 0.1
+    dice = [[u(n, 0, 0.5), u(n, -0.1, 0.1), u(n, 0.5, 1.5)] for n in (n1, n2)]
+    user, q, k, att = [h(r(*s)).half().cuda() for s in ((R, du), (R * n_cand, d), (R * T, d), (R * n_cand, d))]
+    got = ops.DinTower(d, du, W1, b1, dice[0], W2, b2, dice[1], W3, b3, softmax=False)(user, q, k, att, R, n_cand, T).double().cpu()
+    D = lambda x: x.double().cpu()
+    his = D(k).view(R, T, d).sum(1).half().double().repeat_interleave(n_cand, 0)
+    x = torch.cat([D(user).repeat_interleave(n_cand, 0), D(q), his, (D(q) * his).half().double(), D(att), (D(q) - his).half().double()], 1)
+    for W, b, (ga, mu, va) in ((W1, b1, dice[0]), (W2, b2, dice[1])):
+        x = x @ W.double() + b.double()
+        p = ((x - mu.double()) / (va.double() + 1e-8).sqrt()).sigmoid()
+        x = (1 - p) * ga.double() * x + p * x
+    want = x @ W3.double() + b3.double()
+    # Dice on fp16 pairs: half-precision tanh (5e-4) and three roundings (2^-11) of a value, twice, and the logits' rounding
+    tol = 4e-3 * (1 + float((x.abs() @ W3.double().abs()).max()))
+    assert (got - want).abs().max() <= tol, (float((got - want).abs().max()), tol)
