@@ -171,12 +171,13 @@ __global__ void tower_pack_kernel(const __grid_constant__ TowerParams p, uint8_t
 
 // ---- once per launch: his_sum and the per-request product of layer 1 -------------------------------
 // partial[r][n] = b1[n] + sum_c user[r][c] * W1[c][n] + sum_e fp16(his_sum[r][e]) * W1[du+d+e][n]
-// One CTA per (request, 64 output columns): 8 groups of 64 threads split the du + d weight rows; the group sums are added
-// in group order. his_sum: the T steps are split over groups of d threads and added in group order.
-// A chain of memory latencies is all this kernel is, so each thread requests its first 24 weights and its first 16 steps
-// at once and only then waits for any (at du + d = 180 and T = 100 that is everything). One request: 5.8 us, 8.2 before
-constexpr int PT_COLS = 64, PT_SLICES = 8, PT_W = 24, PT_T = 16;
-__global__ void __launch_bounds__(PT_COLS * PT_SLICES) din_tower_partial_kernel(const __grid_constant__ TowerParams p) {
+// One CTA per (request, 64 output columns): 16 warps split the du + d weight rows, a lane has two columns; the warps' sums are
+// added in order. his_sum: the T steps are split over groups of d threads and added in group order.
+// A chain of memory latencies is all this kernel is, so each thread requests its first 12 pairs of weights and its first 16
+// steps at once and only then waits for any (at du + d = 180 and T = 100 that is everything), and two CTAs fit an SM: 74
+// requests are one wave. 74 requests: 6.9 us, 11.3 with 8 groups of 64 threads, 88 registers each; one request: 5.0, 5.8.
+constexpr int PT_COLS = 64, PT_SLICES = 16, PT_W = 12, PT_T = 16, PT_THREADS = PT_COLS / 2 * PT_SLICES;
+__global__ void __launch_bounds__(PT_THREADS, 2) din_tower_partial_kernel(const __grid_constant__ TowerParams p) {
   pdl_begin();
   extern __shared__ float sm[];            // [d] his_sum, [du] user row, [G][d] step sums, [PT_SLICES][PT_COLS]
   const int r = blockIdx.x, d = p.d, du = p.du;
@@ -186,16 +187,21 @@ __global__ void __launch_bounds__(PT_COLS * PT_SLICES) din_tower_partial_kernel(
   const int G = max(1, min(256 / d, 8));
   float* colsum = part + 8 * d;
   // weight rows 0..du-1 meet the user row, rows du+d..du+2d-1 meet his_sum; x(c) is the matching input
-  const int col = threadIdx.x % PT_COLS, slice = threadIdx.x / PT_COLS;
+  const int col = threadIdx.x % 32 * 2, slice = threadIdx.x / 32;
   const int n = blockIdx.y * PT_COLS + col;
   const int rows = du + d, per = (rows + PT_SLICES - 1) / PT_SLICES;
   const int c_begin = slice * per, c_end = n < p.n1 ? min(rows, c_begin + per) : 0;
-  __half w[PT_W];
+  const bool pairs = p.n1 % 2 == 0 && (reinterpret_cast<uintptr_t>(p.W1) & 3) == 0;
+  __half2 w[PT_W];
   auto load_w = [&](int c0) {
 #pragma unroll
     for (int u = 0; u < PT_W; ++u) {
       const int c = c0 + u;
-      w[u] = c < c_end ? p.W1[(int64_t)(c < du ? c : c + d) * p.n1 + n] : __float2half(0.f);      // skips the q rows of W1
+      w[u] = __floats2half2_rn(0.f, 0.f);
+      if (c < c_end) {
+        const __half* at = p.W1 + (int64_t)(c < du ? c : c + d) * p.n1 + n;                        // skips the q rows of W1
+        w[u] = pairs ? *reinterpret_cast<const __half2*>(at) : __halves2half2(at[0], n + 1 < p.n1 ? at[1] : __float2half(0.f));
+      }
     }
   };
   load_w(c_begin);
@@ -223,21 +229,28 @@ __global__ void __launch_bounds__(PT_COLS * PT_SLICES) din_tower_partial_kernel(
     if (blockIdx.y == 0) p.hs[(int64_t)r * d + e] = s;
   }
   __syncthreads();
-  float acc = 0.f;
+  float2 acc = make_float2(0.f, 0.f);
   for (int c0 = c_begin; c0 < c_end; c0 += PT_W) {
     if (c0 > c_begin) load_w(c0);
 #pragma unroll
     for (int u = 0; u < PT_W; ++u) {
       const int c = c0 + u;
-      if (c < c_end) acc = fmaf(c < du ? us[c] : hs[c - du], __half2float(w[u]), acc);
+      if (c < c_end) {
+        const float x = c < du ? us[c] : hs[c - du];
+        const float2 f = __half22float2(w[u]);
+        acc.x = fmaf(x, f.x, acc.x); acc.y = fmaf(x, f.y, acc.y);
+      }
     }
   }
-  colsum[slice * PT_COLS + col] = acc;
+  colsum[slice * PT_COLS + col] = acc.x;
+  colsum[slice * PT_COLS + col + 1] = acc.y;
   __syncthreads();
-  if (slice == 0 && n < p.n1) {
-    float s = p.b1 ? p.b1[n] : 0.f;
-    for (int g = 0; g < PT_SLICES; ++g) s += colsum[g * PT_COLS + col];
-    p.partial[(int64_t)r * p.n1 + n] = s;
+  const int out = blockIdx.y * PT_COLS + threadIdx.x;
+  if (threadIdx.x < PT_COLS && out < p.n1) {
+    float s = p.b1 ? p.b1[out] : 0.f;
+#pragma unroll
+    for (int g = 0; g < PT_SLICES; ++g) s += colsum[g * PT_COLS + threadIdx.x];
+    p.partial[(int64_t)r * p.n1 + out] = s;
   }
 }
 
@@ -669,8 +682,8 @@ extern "C" int xb_din_tower(const xb_din_tower_args* a, void* workspace, size_t 
   // A large call's kernels start on a chip that the one before has left: with every link of pooling -> attention -> partial ->
   // tower -> next pooling made early, the attention's tiles spread unevenly over the SMs and some walk a fifth one of four
   // (74 requests of 1000: 393 us a pass, 348 with this link plain, 357 with none early).
-  if (tiles <= sm_count()) launch_dependent(din_tower_partial_kernel, pgrid, PT_COLS * PT_SLICES, psmem, stream, p);
-  else din_tower_partial_kernel<<<pgrid, PT_COLS * PT_SLICES, psmem, stream>>>(p);
+  if (tiles <= sm_count()) launch_dependent(din_tower_partial_kernel, pgrid, PT_THREADS, psmem, stream, p);
+  else din_tower_partial_kernel<<<pgrid, PT_THREADS, psmem, stream>>>(p);
   if (int rc = check_launch("din_tower_partial_kernel")) return rc;
   static PerDeviceOnce attr_set;
   XB_SET_MAX_SMEM_ONCE(attr_set, 220 * 1024, (const void*)din_tower_tc_kernel<XB_ACT_DICE, 2>, (const void*)din_tower_tc_kernel<XB_ACT_PRELU, 2>,
