@@ -32,46 +32,67 @@ namespace {
 // Follows GRUKernel, blaze/blaze/operator/op/gru_op.cc:33-93: leading steps whose first H
 // input pre-activations (before the bias) are all zero emit zeros and leave h at zero.
 //
-// What bounds it is the chain h(t) -> h(t+1), some 250 instructions of which each waits for the one before; everything else
-// is kept off that chain. The input products of up to GRU_CHUNK steps are made first, one gate column per thread with its
-// weights in registers (they do not depend on h). Then a step is: four lanes per unit, each with a quarter of the unit's
-// three recurrent columns in registers, read their part of h as 16-byte vectors and add up over the lanes with three
-// shuffles that leave the reset gate's sum in lane 0, the update gate's in lane 1 and the candidate's in lane 2; lanes 0
-// and 1 evaluate their sigmoids in the same instructions, lane 2 the candidate and the new h, which goes to the other of two
-// buffers, so a step needs one barrier. 16 sequences of 100 steps, H = 36: 62 us; 77 with
-// six shuffles and every lane evaluating both sigmoids, 156 with the weights in shared memory and three barriers.
+// What bounds it is the chain h(t) -> h(t+1), in which every instruction waits for the one before; everything else is kept off
+// it. The input products of up to GRU_CHUNK steps are made first (they do not depend on h). Then a thread owns one of the 3H
+// gate columns, its recurrent weights in registers, and a step is: read h as broadcast 16-byte vectors, four chains of FMAs,
+// the reset and update threads evaluate their gates and leave them in shared memory, the candidate threads the candidate and the
+// new h. Two barriers a step, but no shuffles, and each scheduler has one warp (H = 36).
+// fp16 sequences evaluate the gates with the hardware's exponential and reciprocal (gate_tanh below; the state stays fp32, and
+// what their few units in the last place of fp32 leave of a result that is rounded to fp16 is nothing: the same error against
+// 64 bits, 2.0e-4); fp32 sequences keep expf, tanhf and the division.
+// 16 sequences of 100 steps, H = 36: 36 us fp16, 39 fp32; 62 and 58 with four lanes a unit, three shuffles and one barrier a step.
+// 1000 sequences 180 and 275, 16 of H = 64 52 and 70. (The register bound lets the compiler have every h vector of a step on its
+// way at once: at 128 registers, which it picks otherwise, 56 us.)
 constexpr int GRU_CHUNK = 64;
 __host__ __device__ constexpr int gru_hp(int nv) { return 16 * nv; }          // h and x rows padded with zeros
+
+__device__ __forceinline__ float ex2_approx(float v) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v)); return y; }
+__device__ __forceinline__ float rcp_approx(float v) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v)); return y; }
+template <typename T> __device__ __forceinline__ float gate_sigmoid(float v) {
+  if constexpr (sizeof(T) == 4) return sigm(v);
+  else return rcp_approx(1.f + ex2_approx(-1.4426950408889634f * v));
+}
+// tanh from one exponential, 1 - 2 / (1 + e^2x); below 1/2, where that would cancel, x + x^3 P(x^2) with P of degree 3 fitted to
+// (tanh x - x) / x^3 by iteratively reweighted least squares (Lawson's method), 1.5e-8 relative. Both are evaluated: a branch
+// would take longer.
+template <typename T> __device__ __forceinline__ float gate_tanh(float x) {
+  if constexpr (sizeof(T) == 4) {
+    return tanhf(x);
+  } else {
+    const float s = x * x;
+    float p = fmaf(s, 0.01724149f, -0.05304549f);
+    p = fmaf(p, s, 0.13325879f);
+    p = fmaf(p, s, -0.33333144f);
+    const float small = fmaf(x * s, p, x), large = fmaf(-2.f, rcp_approx(1.f + ex2_approx(2.8853900817779268f * x)), 1.f);
+    return fabsf(x) < 0.5f ? small : large;
+  }
+}
+
 template <typename T, int NV>
-__global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int steps, int H,
-                                                      const T* __restrict__ i2h, const T* __restrict__ h2h,
-                                                      const T* __restrict__ bi, const T* __restrict__ bh) {
+__global__ void __launch_bounds__((48 * NV + 31) / 32 * 32, 1) gru_kernel(const T* x, T* y, int steps, int H,
+                                                                       const T* __restrict__ i2h, const T* __restrict__ h2h,
+                                                                       const T* __restrict__ bi, const T* __restrict__ bh) {
   pdl_wait();
   constexpr int HP = gru_hp(NV);
   extern __shared__ __align__(16) float gru_sm[];
   float* xs = gru_sm;                              // [GRU_CHUNK][HP]
   float* pre = xs + GRU_CHUNK * HP;                // [GRU_CHUNK][3H]: input products with their bias
-  __shared__ __align__(16) float hbuf[2][HP];
-  __shared__ int nonzero[GRU_CHUNK];               // step has a non-zero among its first H input products
+  __shared__ __align__(16) float hbuf[HP];
+  __shared__ float gates[2 * HP];
+  __shared__ int first_s;                          // first step of the chunk with a non-zero among its first H input products
   const int tid = threadIdx.x, G = 3 * H;
-  const int u = tid >> 2, l = tid & 3;             // recurrence: unit and quarter
-  const bool unit = u < H;
+  const bool col = tid < G;                        // gate column tid: r, z, candidate
+  const int u = tid - 2 * H;                       // candidate threads: their unit
   const int64_t b = blockIdx.x;
-  float wi[HP];                                    // column tid of i2h
-  float wh[3][4 * NV];                             // rows 4 * (4 i + l) .. + 3 of the unit's columns
+  float wi[HP], wh[HP];                            // column tid of i2h and of h2h
 #pragma unroll
-  for (int k = 0; k < HP; ++k) wi[k] = (k < H && tid < G) ? to_f32<T>(i2h[k * G + tid]) : 0.f;
-#pragma unroll
-  for (int g = 0; g < 3; ++g)
-#pragma unroll
-    for (int i = 0; i < 4 * NV; ++i) {
-      const int k = 4 * (4 * (i >> 2) + l) + (i & 3);
-      wh[g][i] = (unit && k < H) ? to_f32<T>(h2h[k * G + g * H + u]) : 0.f;
-    }
-  const float bij = tid < G ? to_f32<T>(bi[tid]) : 0.f;
-  const float bh_l = (unit && l < 3) ? to_f32<T>(bh[l * H + u]) : 0.f;
-  for (int i = tid; i < 2 * HP; i += blockDim.x) (&hbuf[0][0])[i] = 0.f;
-  bool started = false;
+  for (int k = 0; k < HP; ++k) {
+    wi[k] = (k < H && col) ? to_f32<T>(i2h[k * G + tid]) : 0.f;
+    wh[k] = (k < H && col) ? to_f32<T>(h2h[k * G + tid]) : 0.f;
+  }
+  const float bij = col ? to_f32<T>(bi[tid]) : 0.f, bhj = col ? to_f32<T>(bh[tid]) : 0.f;
+  for (int i = tid; i < HP; i += blockDim.x) hbuf[i] = 0.f;
+  bool started = false;                            // the same for every thread
   float h = 0.f;
   for (int t0 = 0; t0 < steps; t0 += GRU_CHUNK) {
     const int n = min(GRU_CHUNK, steps - t0);
@@ -90,9 +111,10 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
         if (i < n * HP) xs[i] = v[e];
       }
     }
-    for (int i = tid; i < n; i += blockDim.x) nonzero[i] = 0;
+    if (tid == 0) first_s = n;
     __syncthreads();
-    if (tid < G) {
+    if (col) {
+      int first = n;
       for (int t = 0; t < n; t += 4) {                            // four independent chains (rows past n are not kept)
         float q[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -105,55 +127,44 @@ __global__ void __launch_bounds__(64 * NV) gru_kernel(const T* x, T* y, int step
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          if (t + e < n) {
-            if (tid < H && q[e] != 0.f) nonzero[t + e] = 1;
-            pre[(t + e) * G + tid] = q[e] + bij;
-          }
+          first = q[e] != 0.f ? min(first, t + e) : first;
+          if (t + e < n) pre[(t + e) * G + tid] = q[e] + bij;
         }
       }
+      if (!started && tid < H) atomicMin(&first_s, first);        // (steps past n are no less than n)
     }
     __syncthreads();
     if (t0 + n >= steps) pdl_release();            // (not in the steps: they are the chain)
-    for (int t = 0; t < n; ++t) {
-      const int64_t at = (b * steps + t0 + t) * H + u;
-      if (!started) started = nonzero[t] != 0;     // the same for every thread
-      if (!started) {
-        if (unit && l == 0) y[at] = from_f32<T>(0.f);
-        continue;
-      }
-      const float pre_l = (unit && l < 3) ? pre[t * G + l * H + u] : 0.f;      // lane 0: r, lane 1: z, lane 2: candidate
-      const float4* hv = reinterpret_cast<const float4*>(hbuf[t & 1]);
-      float a[3][2] = {};
+    int t = 0;
+    T* yt = y + (b * steps + t0) * H + u;
+    if (!started) {                                // steps before the list begins: zeros, and a state of zero
+      const int begin = first_s;
+      for (; t < begin; ++t, yt += H)
+        if (col && u >= 0) *yt = from_f32<T>(0.f);
+      started = begin < n;
+    }
+    float pre_next = col && t < n ? pre[t * G + tid] : 0.f;
+    for (; t < n; ++t, yt += H) {
+      const float pre_j = pre_next;
+      if (col && t + 1 < n) pre_next = pre[(t + 1) * G + tid];
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const float4 v = hv[4 * i + l];
-#pragma unroll
-        for (int g = 0; g < 3; ++g) {
-          a[g][0] = fmaf(v.x, wh[g][4 * i], a[g][0]);
-          a[g][1] = fmaf(v.y, wh[g][4 * i + 1], a[g][1]);
-          a[g][0] = fmaf(v.z, wh[g][4 * i + 2], a[g][0]);
-          a[g][1] = fmaf(v.w, wh[g][4 * i + 3], a[g][1]);
-        }
+      for (int k = 0; k < HP; k += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(hbuf + k);
+        a[0] = fmaf(v.x, wh[k], a[0]); a[1] = fmaf(v.y, wh[k + 1], a[1]); a[2] = fmaf(v.z, wh[k + 2], a[2]); a[3] = fmaf(v.w, wh[k + 3], a[3]);
       }
-      const float sr = a[0][0] + a[0][1], sz = a[1][0] + a[1][1], sc = a[2][0] + a[2][1];
-      // even lanes collect r and the candidate, odd lanes z; then lane 0 r, lane 2 the candidate
-      float keep = (l & 1) ? sz : sr;
-      keep += __shfl_xor_sync(0xffffffffu, (l & 1) ? sr : sz, 1);
-      float cand = sc + __shfl_xor_sync(0xffffffffu, sc, 1);
-      const float other = __shfl_xor_sync(0xffffffffu, l == 0 ? cand : keep, 2);
-      const float sum = (l == 2 ? cand : keep) + other + bh_l;
-      const float gate = sigm(pre_l + sum);                                    // lanes 0 and 1
-      const float r = __shfl_sync(0xffffffffu, gate, (threadIdx.x & 28)), z = __shfl_sync(0xffffffffu, gate, (threadIdx.x & 28) + 1);
-      const float c = tanhf(pre_l + r * sum);                                  // lane 2
-      h = c + z * (h - c);
-      if (unit && l == 2) {
-        hbuf[(t + 1) & 1][u] = h;
-        y[at] = from_f32<T>(h);
+      const float sum = (a[0] + a[1]) + (a[2] + a[3]) + bhj;
+      if (tid < 2 * H) gates[tid] = gate_sigmoid<T>(pre_j + sum);
+      __syncthreads();                             // the gates are there, and everyone has read h
+      if (col && u >= 0) {
+        const float r = gates[u], z = gates[H + u];
+        const float c = gate_tanh<T>(pre_j + r * sum);
+        h = c + z * (h - c);
+        hbuf[u] = h;
+        *yt = from_f32<T>(h);
       }
       __syncthreads();
     }
-    // an odd number of steps leaves h in the second buffer: the next chunk counts its steps from zero again, and every
-    // chunk but the last has GRU_CHUNK (even) steps, so it starts in the first
   }
 }
 
@@ -209,7 +220,7 @@ __global__ void augru_kernel(const void* x, const void* att, void* y, int T, int
 // [requests, T, H], att [requests * n_cand, T], only the final states y [requests * n_cand, H] are written.
 // A CTA owns AS_CAND candidates of one request. The terms of x_t are the same for all of them: each chunk of steps they
 // are made once, a gate column per thread. A candidate is four lanes per unit with their quarter of the unit's three
-// recurrent columns in registers (as gru_kernel), and two barriers of its own threads a step: r*h, then h.
+// recurrent columns in registers, and two barriers of its own threads a step: r*h, then h.
 // 4 requests of 1000 candidates, 100 steps, H = 32: 418 us,
 // 973 with a block per candidate and the weights in shared memory
 constexpr int AS_CAND = 4, AS_CHUNK = 32;
@@ -313,7 +324,7 @@ int launch_gru_nv(const T* x, T* y, int64_t batch, int steps, int H, const T* i2
   const size_t smem = sizeof(float) * GRU_CHUNK * (size_t)(gru_hp(NV) + 3 * H);
   static PerDeviceOnce attr;                       // per instantiation
   XB_SET_MAX_SMEM_ONCE(attr, sizeof(float) * GRU_CHUNK * 4 * gru_hp(NV), (const void*)gru_kernel<T, NV>);
-  launch_dependent(gru_kernel<T, NV>, (unsigned)batch, (4 * H + 31) / 32 * 32, smem, s, x, y, steps, H, i2h, h2h, bi, bh);
+  launch_dependent(gru_kernel<T, NV>, (unsigned)batch, (3 * H + 31) / 32 * 32, smem, s, x, y, steps, H, i2h, h2h, bi, bh);
   return check_launch("gru_kernel");
 }
 template <typename T>
