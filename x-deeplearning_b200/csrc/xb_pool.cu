@@ -3,7 +3,7 @@
 // Three kernels share one geometry: a table row is fetched by LPR lanes with 128-bit loads (lane c
 // reads bytes [16c,16c+16) of the row) and accumulated in fp32.
 //   pool_queue_kernel  sum / average, one output per feature group, large batches: one sub-team of LPR
-//                      lanes per segment, 32 segments per warp handed out as sub-teams finish.
+//                      lanes per segment, a warp's run of segments handed out as sub-teams finish.
 //   pool_fast_kernel   one output per feature group (kAssign included), any batch: teams of TL lanes
 //                      per segment, TL/LPR sub-teams that walk the ids s, s+NS, s+2NS..., combined
 //                      with a fixed xor butterfly.
@@ -83,6 +83,7 @@ struct ScanParams {
   int32_t chunk_begin[XB_MAX_POOL_GROUPS + 1];
 };
 
+constexpr int POOL_QUEUE_BLOCKS = 4;           // blocks of pool_queue_kernel resident on an SM
 constexpr int POOL_INLINE_COUNTS = 1024;      // longest count array that pool_fast_kernel adds up itself
 
 __device__ __forceinline__ uint64_t mix64(uint64_t x) {
@@ -790,12 +791,14 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
 }
 
 // Sum / average pooling with one sub-team (LPR lanes) per segment and a per-warp segment queue: a warp
-// owns up to 32 consecutive segments, its 32/LPR sub-teams each take the next unclaimed one as soon as they
-// finish theirs, so lanes stay busy whatever the spread of segment lengths. A sub-team adds the ids of its
+// owns a run of consecutive segments, its 32/LPR sub-teams each take the next unclaimed one as soon as they
+// finish theirs, so lanes stay busy whatever the spread of segment lengths. The run is as long as it takes for the
+// launch to be one wave of warps; the spans of 64 of its segments lie in the lanes' registers, a window of 32 behind the
+// claims and the one after it. A sub-team adds the ids of its
 // segment strictly in order (no cross-lane combine). The ids of the batch after the current one are
 // requested before the rows of the current one, so both latencies overlap.
 template <int TD, int LPR, int KIND>
-__global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constant__ PoolParams p) {
+__global__ void __launch_bounds__(256, POOL_QUEUE_BLOCKS) pool_queue_kernel(const __grid_constant__ PoolParams p) {
   pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;
   constexpr unsigned FULL = 0xffffffffu;
@@ -820,9 +823,10 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
   const int64_t s0 = (warp_id - p.warp_begin[gi]) * g.segs;
   const int nseg = (int)min((int64_t)g.segs, g.batch - s0);
 
-  // lane l keeps the span of segment s0 + l
-  int my_start = 0, my_num = 0;
+  // lane l keeps the spans of segments s0 + win + l and, on their way while those are claimed, s0 + win + 32 + l
+  int win = 0, my_start = 0, my_num = 0, ahead_start = 0, ahead_num = 0;
   if (lane < nseg) pool_span<KIND>(g, s0 + lane, my_start, my_num);
+  if (32 + lane < nseg) pool_span<KIND>(g, s0 + 32 + lane, ahead_start, ahead_num);
   auto load_ids = [&](int st, int nm, int pos, int& row, float& v) {
     const int idx = pos + tlane;
     row = -1; v = 1.f;
@@ -854,13 +858,22 @@ __global__ void __launch_bounds__(256, 4) pool_queue_kernel(const __grid_constan
     const unsigned fmask = __ballot_sync(FULL, finishing && tlane == 0);
     int m2 = m, pos2 = pos + LPR, start2 = start, num2 = num;
     if (fmask) {
-      const int cand = next + __popc(fmask & ((1u << team0) - 1u));
-      const int cs = __shfl_sync(FULL, my_start, cand & 31), cn = __shfl_sync(FULL, my_num, cand & 31);
+      const int cand = next + __popc(fmask & ((1u << team0) - 1u));          // below win + 32 + NT
+      int cs = __shfl_sync(FULL, my_start, cand & 31), cn = __shfl_sync(FULL, my_num, cand & 31);
+      if (next + NT > win + 32) {                    // uniform: some claim may be in the second window
+        const int as = __shfl_sync(FULL, ahead_start, cand & 31), an = __shfl_sync(FULL, ahead_num, cand & 31);
+        if (cand >= win + 32) { cs = as; cn = an; }
+      }
       if (finishing) {
         m2 = cand; pos2 = 0; start2 = cs;
         num2 = cand < nseg ? cn : 0;
       }
       next += __popc(fmask);
+      if (next >= win + 32) {
+        win += 32;
+        my_start = ahead_start; my_num = ahead_num;
+        if (win + 32 + lane < nseg) pool_span<KIND>(g, s0 + win + 32 + lane, ahead_start, ahead_num);
+      }
     }
     int row2;
     float v2;
@@ -1129,13 +1142,53 @@ static int embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* s
         (groups[i].n_items != 1 || groups[i].items[0].udf == XB_UDF_ASSIGN || (double)groups[i].n_ids >= 3.0 * (double)groups[i].batch))
       all_short = false;
   }
-  // Segments a warp of the queue kernel owns: 32 keep its sub-teams busy whatever the spread of lengths, fewer where the
-  // launch would otherwise not fill the chip with resident warps.
-  // 8 groups of 8192 segments of 15.5 ids (25 M x 32 fp16 table): 43 us at 32 a warp (0.43 of a wave), 33 at 8. 32 such
-  // groups: 89 us at 32 (1.7 waves), 100 at 16, so a launch that fills the chip keeps 32.
-  int queue_segs = 32;
-  while (queue_segs > 8 && call_segments / queue_segs < (int64_t)sm_count() * 32) queue_segs >>= 1;
   all_short = all_short && (call_segments + 31) / 32 >= (int64_t)sm_count() * 8;
+  // lanes per row, lanes per segment and kernel of a group
+  struct Lanes { int lpr, tl, bucket; bool fast, queue; };
+  auto lanes_of = [&](const xb_pool_group& h) {
+    Lanes l;
+    const bool f32 = h.table && h.table->dtype == XB_F32;       // (no table: the geometry of fp16, nothing is fetched)
+    const int epc = f32 ? 4 : 8;
+    l.lpr = next_pow2((h.dim + epc - 1) / epc);
+    l.fast = h.n_items == 1 && l.lpr <= 16;
+    if (l.fast && l.lpr < 2) l.lpr = 2;
+    const double avg = (double)h.n_ids / (double)h.batch;
+    int ns = 1;
+    if (l.fast) {
+      // one sub-team per segment gives the fewest instructions per id (no cross-lane combine, whole rows
+      // per lane group); teams grow while the launch would otherwise leave SMs without warps, or while a
+      // segment is so long that one sub-team would walk it in more than a dozen dependent batches of ids
+      // (a 100-step behaviour list on 4 lanes is 25 id-load -> row-load round trips in a row; on a whole warp, 4)
+      const int64_t want_warps = (int64_t)sm_count() * 32;
+      while (ns < 32 / l.lpr && ns < avg &&
+             (call_segments * (int64_t)(l.lpr * ns) / 32 < want_warps || (avg >= 48.0 && avg > 12.0 * ns)))
+        ns <<= 1;
+    } else {
+      while (ns < 32 / l.lpr && ns < avg) ns <<= 1;
+    }
+    l.tl = l.lpr * ns;
+    int lg = 0;
+    while ((2 << lg) < l.lpr) ++lg;                 // lanes per row 2, 4, 8, 16 -> 0..3
+    l.bucket = (f32 ? 0 : 4) + lg;
+    // sum / average groups with plenty of segments go to the segment-queue kernel
+    l.queue = l.fast && l.tl == l.lpr && h.items[0].udf != XB_UDF_ASSIGN && avg >= 3.0 && (call_segments + 31) / 32 >= (int64_t)sm_count() * 8;
+    return l;
+  };
+  // Segments a warp of the queue kernel owns: an equal share of its launch's for each warp that can be resident, so that the
+  // launch is one wave (the groups' last warps have less). Pieces of 32 segments a warp, as many waves as they take: 40 groups
+  // of 8192 lists of 15.5 ids (25 M x 32 fp16) 119 us, 111 in one wave; 20 such groups 79 and 57 (1.1 waves); the sharded step
+  // of one rank 121 and 100; 20 groups of 16 000 lists of 25 over an fp32 table in L2 169 and 135.
+  int64_t queue_total[kBuckets] = {}, queue_groups[kBuckets] = {};
+  for (int i = 0; i < n_groups; ++i) {
+    const xb_pool_group& h = groups[i];
+    if (h.batch <= 0 || h.n_items < 1 || h.dim < 1 || h.dim > 256) continue;
+    const Lanes l = lanes_of(h);
+    if (l.queue) { queue_total[l.bucket] += h.batch; ++queue_groups[l.bucket]; }
+  }
+  auto queue_segs_of = [&](int bucket) {
+    const int64_t warps = std::max<int64_t>((int64_t)sm_count() * POOL_QUEUE_BLOCKS * 8 - queue_groups[bucket], 1);
+    return (int)std::max<int64_t>(8, (queue_total[bucket] + warps - 1) / warps);
+  };
   for (int i = 0; i < n_groups; ++i) {
     const xb_pool_group& h = groups[i];
     XB_REQUIRE(h.batch >= 0 && h.n_ids >= 0, XB_ERR_ARG, "xb_embedding_pool: group %d negative size", i);
@@ -1172,26 +1225,12 @@ static int embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* s
       d.tdtype = XB_F16;   // only fixes the lane geometry: nothing is fetched for a missing table
     }
     d.dim = dim;
-    const int epc = d.tdtype == XB_F32 ? 4 : 8;
-    d.lpr = next_pow2((dim + epc - 1) / epc);
+    const Lanes lanes = lanes_of(h);
+    d.lpr = lanes.lpr;
     if (d.lpr > 32) return fail(XB_ERR_LIMIT, "xb_embedding_pool: row too wide");
-    const bool fast = h.n_items == 1 && d.lpr <= 16;
-    if (fast && d.lpr < 2) d.lpr = 2;
+    const bool fast = lanes.fast;
     const double avg = (double)h.n_ids / (double)h.batch;
-    int ns = 1;
-    if (fast) {
-      // one sub-team per segment gives the fewest instructions per id (no cross-lane combine, whole rows
-      // per lane group); teams grow while the launch would otherwise leave SMs without warps, or while a
-      // segment is so long that one sub-team would walk it in more than a dozen dependent batches of ids
-      // (a 100-step behaviour list on 4 lanes is 25 id-load -> row-load round trips in a row; on a whole warp, 4)
-      const int64_t want_warps = (int64_t)sm_count() * 32;
-      while (ns < 32 / d.lpr && ns < avg &&
-             (call_segments * (int64_t)(d.lpr * ns) / 32 < want_warps || (avg >= 48.0 && avg > 12.0 * ns)))
-        ns <<= 1;
-    } else {
-      while (ns < 32 / d.lpr && ns < avg) ns <<= 1;
-    }
-    d.tl = d.lpr * ns;
+    d.tl = lanes.tl;
     XB_REQUIRE(h.values_dtype == 0 || h.values_dtype == XB_F32 || h.values_dtype == XB_F16, XB_ERR_UNSUPPORTED,
                "xb_embedding_pool: group %d values dtype %d", i, h.values_dtype);
     if (grid) d.grid = grid[i];
@@ -1208,14 +1247,9 @@ static int embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* s
       d.items[k].assign_stride = it.udf == XB_UDF_ASSIGN ? it.assign_stride : 0;
       d.items[k].out = it.out; d.items[k].stride = it.stride;
     }
-    int lg = 0;
-    while ((2 << lg) < d.lpr) ++lg;                 // lanes per row 2, 4, 8, 16 -> 0..3
-    const int bucket = (d.tdtype == XB_F32 ? 0 : 4) + lg;
-    // sum / average groups with plenty of segments go to the segment-queue kernel: 32 segments per warp
-    const bool queue = fast && d.tl == d.lpr && h.items[0].udf != XB_UDF_ASSIGN && avg >= 3.0 &&
-                       (call_segments + 31) / 32 >= (int64_t)sm_count() * 8;
+    const int bucket = lanes.bucket;
     // the queue kernel is instantiated per kind of id list: a bucket takes records only or none
-    const bool queue_ok = queue && (qp[bucket].n_groups == 0 ||
+    const bool queue_ok = lanes.queue && (qp[bucket].n_groups == 0 ||
                                     (qp[bucket].g[0].id_dtype == XB_REC64) == (h.id_dtype == XB_REC64));
     // likewise one instantiation per kind of id list for the short-segment kernel
     const bool short_ok = all_short && fast && d.tl == d.lpr &&
@@ -1238,7 +1272,7 @@ static int embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* s
       d.offsets = off;
     }
     const PoolPath path = short_ok ? PoolPath::SHORT : queue_ok ? PoolPath::QUEUE : fast ? PoolPath::FAST : PoolPath::GENERAL;
-    const PoolSplit split = pool_split(path, h.batch, d.tl, avg, counts_ok, queue_segs, sm_count());
+    const PoolSplit split = pool_split(path, h.batch, d.tl, avg, counts_ok, lanes.queue ? queue_segs_of(bucket) : 32, sm_count());
     d.segs = split.segs;
     dst.total_warps += split.warps;
     dst.g[dst.n_groups++] = d;
