@@ -377,6 +377,142 @@ static int launch_simt_tm(const SimtGemmParams& p, int tn, dim3 grid, cudaStream
   return check_launch("gemm_simt_kernel");
 }
 
+// ---- batches of single rows (fp32): the weighted sum of an attention unit run operator by operator -------------------------
+// A tile has 32 rows at the least and a batch of such products one row each: here a CTA takes a batch, its threads four
+// columns of every few k, and the partial sums are added in order. Bound by the read of B. 500 x ([1, 100] x [100, 36]):
+// 4.5 us, 20 in tiles.
+__global__ void __launch_bounds__(256) gemm_f32_row_kernel(const __grid_constant__ SimtGemmParams p) {
+  extern __shared__ __align__(16) float part[];                 // [groups][N]
+  pdl_wait();
+  const int b = blockIdx.x, N4 = p.N / 4, groups = 256 / N4, g = threadIdx.x / N4, c = threadIdx.x - g * N4;
+  const float* A = reinterpret_cast<const float*>(p.A) + (int64_t)b * p.stride_a;
+  const float* B = reinterpret_cast<const float*>(p.B) + (int64_t)b * p.stride_b;
+  if (g < groups) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = g; k0 < p.K; k0 += 4 * groups) {
+      float a[4];
+      float4 w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int k = k0 + u * groups;
+        const bool in = k < p.K;
+        a[u] = in ? __ldg(A + k) : 0.f;
+        w[u] = in ? __ldg(reinterpret_cast<const float4*>(B + (int64_t)k * p.ldb) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        acc.x = fmaf(a[u], w[u].x, acc.x); acc.y = fmaf(a[u], w[u].y, acc.y);
+        acc.z = fmaf(a[u], w[u].z, acc.z); acc.w = fmaf(a[u], w[u].w, acc.w);
+      }
+    }
+    *reinterpret_cast<float4*>(part + g * p.N + 4 * c) = acc;
+  }
+  __syncthreads();
+  pdl_release();
+  for (int n = threadIdx.x; n < p.N; n += 256) {
+    float v = part[n];
+    for (int i = 1; i < groups; ++i) v += part[i * p.N + n];
+    store_from_f32(p.Y, (int64_t)b * p.stride_y + n, p.y_dtype, finish(p, column_of(p, b, n), b, 0, n, v));
+  }
+}
+
+// ---- one to four output columns: the last layer of a tower or of an attention unit, a stream over A ----------------------
+// A tile of either GEMM engine computes 16 columns at the least and reads A through a ring made for tiles that are used many
+// times. Here `lanes` lanes share a row, each with every lanes-th 16-byte piece of it (up to four, requested together, those
+// of the next row before this one's are used), the weights lie in shared memory as fp32, and the lanes' sums meet by shuffles.
+//
+// Bound by the read of A. [1000, 512] x [512, 4] fp16: 39 us on the tensor cores (one tile walks all of K eight times over), 11 here with
+// the call; [50000, 40] x [40, 1] fp32: 7.4 us after the kernel before, 5.3; [65536, 256] x [256, 1] the same either way.
+constexpr int NARROW_N = 4, NARROW_PIECES = 4;
+template <typename T, int N>
+__global__ void __launch_bounds__(256) gemm_narrow_kernel(const __grid_constant__ SimtGemmParams p, int lanes) {
+  constexpr int E = 16 / (int)sizeof(T);                        // elements of a piece
+  extern __shared__ __align__(16) float ws[];                   // [N][K]
+  __shared__ Column cols[N];
+  pdl_wait();
+  const int b = blockIdx.y, K = p.K, pieces = K / E;
+  const T* A = reinterpret_cast<const T*>(p.A) + (int64_t)b * p.stride_a;
+  const T* B = reinterpret_cast<const T*>(p.B) + (int64_t)b * p.stride_b;
+  const int l = threadIdx.x & (lanes - 1), team = threadIdx.x / lanes, teams = 256 / lanes;
+  const int64_t step = (int64_t)gridDim.x * teams;
+  auto request = [&](int64_t r, uint4 (&raw)[NARROW_PIECES]) {
+    const uint4* row = reinterpret_cast<const uint4*>(A + r * p.lda);
+#pragma unroll
+    for (int i = 0; i < NARROW_PIECES; ++i) {
+      const int c = l + i * lanes;
+      raw[i] = r < p.M && c < pieces ? __ldg(row + c) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  uint4 raw[NARROW_PIECES], next[NARROW_PIECES];                // (the first rows are on their way before the weights)
+  request((int64_t)blockIdx.x * teams + team, raw);
+  for (int i = threadIdx.x; i < N * K; i += 256) {
+    const int n = i / K, k = i - n * K;
+    ws[i] = n < p.N ? to_f32<T>(p.trans_b ? B[(int64_t)n * p.ldb + k] : B[(int64_t)k * p.ldb + n]) : 0.f;
+  }
+  if ((int)threadIdx.x < p.N) cols[threadIdx.x] = column_of(p, b, threadIdx.x);
+  __syncthreads();
+  pdl_release();
+  // (every lane of a warp walks as many rows, so that the shuffles are whole)
+  for (int64_t r0 = (int64_t)blockIdx.x * teams; r0 < p.M; r0 += step) {
+    const int64_t r = r0 + team;
+    request(r + step, next);
+    float acc[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) acc[n] = 0.f;
+#pragma unroll
+    for (int i = 0; i < NARROW_PIECES; ++i) {
+      const int c = l + i * lanes;
+      if (c >= pieces) break;
+      const T* a = reinterpret_cast<const T*>(&raw[i]);
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+#pragma unroll
+        for (int e = 0; e < E; e += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(ws + n * K + c * E + e);
+          acc[n] = fmaf(to_f32<T>(a[e]), w.x, acc[n]);
+          acc[n] = fmaf(to_f32<T>(a[e + 1]), w.y, acc[n]);
+          acc[n] = fmaf(to_f32<T>(a[e + 2]), w.z, acc[n]);
+          acc[n] = fmaf(to_f32<T>(a[e + 3]), w.w, acc[n]);
+        }
+      }
+    }
+    for (int off = lanes >> 1; off > 0; off >>= 1) {
+#pragma unroll
+      for (int n = 0; n < N; ++n) acc[n] += __shfl_xor_sync(0xffffffffu, acc[n], off);
+    }
+#pragma unroll
+    for (int i = 0; i < NARROW_PIECES; ++i) raw[i] = next[i];
+    if (r >= p.M) continue;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      if (n < p.N && n % lanes == l)
+        store_from_f32(p.Y, (int64_t)b * p.stride_y + r * p.ldy + n, p.y_dtype, finish(p, cols[n], b, (int)r, n, acc[n]));
+  }
+}
+
+// What gemm_narrow_kernel takes: whole 16-byte pieces, aligned, and as many rows as the tiles take. (Fewer rows than fill a few
+// blocks gain nothing.)
+bool gemm_narrow_takes(const xb_gemm_args& a) {
+  const int E = a.ab_dtype == XB_F32 ? 4 : 8;
+  return a.N <= NARROW_N && !a.trans_a && a.M >= 128 && a.M <= 65535 * 64 && a.K > 0 && a.K % E == 0 && a.K / E <= 32 * NARROW_PIECES &&
+         a.lda % E == 0 && a.stride_a % E == 0 && (reinterpret_cast<uintptr_t>(a.A) & 15) == 0 && a.batch <= 65535;
+}
+
+template <typename T>
+static int launch_narrow(const SimtGemmParams& p, int batch, cudaStream_t s) {
+  const int pieces = p.K * (int)sizeof(T) / 16;
+  int lanes = 1;
+  while (lanes * NARROW_PIECES < pieces) lanes <<= 1;
+  const int64_t blocks = std::min<int64_t>(((int64_t)p.M * lanes + 255) / 256, (int64_t)sm_count() * 4);
+  const dim3 grid((unsigned)blocks, (unsigned)batch);
+  const int n = p.N == 3 ? 4 : p.N;
+  const size_t smem = (size_t)n * p.K * 4;
+  if (n == 1) launch_dependent(gemm_narrow_kernel<T, 1>, grid, 256, smem, s, p, lanes);
+  else if (n == 2) launch_dependent(gemm_narrow_kernel<T, 2>, grid, 256, smem, s, p, lanes);
+  else launch_dependent(gemm_narrow_kernel<T, 4>, grid, 256, smem, s, p, lanes);
+  return check_launch("gemm_narrow_kernel");
+}
+
 // Tile of a product: a wave of CTAs costs what its busiest SM computes, TM*TN a k slice and output pair, plus what
 // the operand reads (1.5 TN + 0.75 TM) and the slice's barrier and index work (4) cost beside it; the tile with the cheapest sum
 // of waves is taken. The three weights are estimates in units of FMAs, not fitted to measurements of each tile. The general
@@ -419,6 +555,16 @@ int gemm_simt(const xb_gemm_args& a, cudaStream_t stream) {
   pick_simt_tile(a.M, a.N, a.batch, f32, &tm, &tn);
   // (the entry point's limits, whatever the tile; a grid of any of them would take more rows)
   XB_REQUIRE((a.M + 63) / 64 <= 65535 && a.batch <= 65535, XB_ERR_LIMIT, "xb_gemm: M or batch too large for the SIMT engine");
+  // single rows: many of them, each of a size that one CTA reads in a few steps
+  if (f32 && a.M == 1 && a.batch >= 32 && a.N % 4 == 0 && a.N <= 256 && (int64_t)a.N * a.K <= 65536 && p.b_vec) {
+    launch_dependent(gemm_f32_row_kernel, (unsigned)a.batch, 256, (size_t)(256 / (a.N / 4)) * a.N * 4, stream, p);
+    return check_launch("gemm_f32_row_kernel");
+  }
+  if (gemm_narrow_takes(a)) {
+    if (a.ab_dtype == XB_F32) return launch_narrow<float>(p, a.batch, stream);
+    if (a.ab_dtype == XB_F16) return launch_narrow<__half>(p, a.batch, stream);
+    return launch_narrow<__nv_bfloat16>(p, a.batch, stream);
+  }
   p.tiles_n = (a.N + 16 * tn - 1) / (16 * tn);
   const int64_t tiles = (((int64_t)a.M + 16 * tm - 1) / (16 * tm)) * p.tiles_n;
   XB_REQUIRE(tiles < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)tiles);

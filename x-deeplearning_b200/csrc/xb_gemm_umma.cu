@@ -28,6 +28,7 @@
 namespace xb {
 
 int gemm_simt(const xb_gemm_args& a, cudaStream_t stream);
+bool gemm_narrow_takes(const xb_gemm_args& a);           // (gemm_simt hands those to their own kernel)
 
 namespace {
 
@@ -845,7 +846,7 @@ extern "C" int xb_gemm(const xb_gemm_args* a, xb_stream_t stream) {
     return gemm_umma(*a, (cudaStream_t)stream);
   }
   // small problems are launch-bound either way; the CUDA-core engine has no TMA descriptor cost
-  if (a->engine == XB_GEMM_AUTO && umma_eligible(*a) && a->K > 0 &&
+  if (a->engine == XB_GEMM_AUTO && umma_eligible(*a) && a->K > 0 && !gemm_narrow_takes(*a) &&
       (int64_t)a->M * a->N * a->batch >= 128 * 64)
     return gemm_umma(*a, (cudaStream_t)stream);
   return gemm_simt(*a, (cudaStream_t)stream);
