@@ -6,6 +6,8 @@ import os
 
 import numpy as np
 
+from . import capi
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libblaze_b200.so")
 
@@ -52,6 +54,20 @@ def lib():
         L.Blaze_B200_AddDeviceShard.argtypes = [vp, cp, C.c_int64, C.c_int, C.c_int, vp, C.c_int64]
         _lib = L
     return _lib
+
+
+_feed = None
+
+
+def feed_call():
+    """ReshapeInput and Feed in one call of the extension module."""
+    global _feed
+    if _feed is None:
+        m, L = capi.binding(), lib()
+        for name in ("Blaze_PredictorReshapeInput", "Blaze_PredictorFeed"):
+            m.bind(name, C.cast(getattr(L, name), vp).value)
+        _feed = m.feed
+    return _feed
 
 
 class BlazeError(RuntimeError):
@@ -151,12 +167,11 @@ class PredictorManager:
 class Predictor:
     def __init__(self, h):
         self.h = h
+        self._feed = feed_call()
 
     def feed(self, name, array):
         a = np.ascontiguousarray(array)
-        shape = (C.c_int * a.ndim)(*a.shape)
-        _ck(lib().Blaze_PredictorReshapeInput(self.h, name.encode(), shape, a.ndim))
-        _ck(lib().Blaze_PredictorFeed(self.h, name.encode(), a.ctypes.data, a.nbytes))
+        _ck(self._feed(self.h.value, name, a))
         return a            # keep alive until Forward: the copy is asynchronous
 
     def reshape(self, name, shape):

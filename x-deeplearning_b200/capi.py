@@ -1,5 +1,7 @@
 """ctypes bindings of include/xdlb200.h (libxdlb200.so)."""
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 import subprocess
 
@@ -174,6 +176,27 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = L
     return _lib
+
+
+_binding = None
+
+
+def binding():
+    """The extension module with the hot calls (host/binding/xb_binding.cc), bound to this process's kernel library."""
+    global _binding
+    if _binding is None:
+        L = lib()
+        path = os.path.join(HERE, "lib", "xb_binding.so")
+        if not os.path.exists(path):
+            raise RuntimeError("%s is missing: build it first (there is no fallback)" % path)
+        loader = importlib.machinery.ExtensionFileLoader("xb_binding", path)
+        spec = importlib.util.spec_from_file_location("xb_binding", path, loader=loader)
+        m = importlib.util.module_from_spec(spec)
+        loader.exec_module(m)
+        for name in ("xb_gemm", "xb_embedding_pool"):
+            m.bind(name, C.cast(getattr(L, name), C.c_void_p).value)
+        _binding = m
+    return _binding
 
 
 class XbError(RuntimeError):

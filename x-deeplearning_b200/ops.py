@@ -8,7 +8,7 @@ import ctypes as C
 import torch
 
 from . import capi
-from .capi import (XB_F16, XB_F32, XB_BF16, XB_I32, XB_I64, GemmArgs, PoolGroup, TableDesc, DinAttArgs, check, lib)
+from .capi import (XB_F16, XB_F32, XB_BF16, XB_I32, XB_I64, PoolGroup, TableDesc, DinAttArgs, binding, check, lib)
 
 _DT = {torch.float32: XB_F32, torch.float16: XB_F16, torch.bfloat16: XB_BF16, torch.int32: XB_I32,
        torch.int64: XB_I64}
@@ -18,8 +18,18 @@ def dt(t):
     return _DT[t.dtype]
 
 
+_raw_stream, _raw_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+
+
+def raw_stream():
+    """The current stream of the current device as a number (torch.cuda.current_stream() makes an object of it: 3.4 us)."""
+    if _raw_stream is None or _raw_device is None or not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_raw_device())
+
+
 def stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(raw_stream())
 
 
 def ptr(t):
@@ -94,11 +104,14 @@ class PoolPlan:
             need = int(lib().xb_embedding_pool_scratch_bytes(arr, len(part)))
             scratch = torch.empty(max(need, 16), dtype=torch.uint8, device=device)
             self.chunks.append((arr, len(part), scratch, need))
+        # (addresses of what the plan itself owns)
+        self._calls = [(C.addressof(arr), n, scratch.data_ptr(), need) for arr, n, scratch, need in self.chunks]
+        self._pool = binding().pool
 
     def run(self):
-        s = stream()
-        for arr, n, scratch, need in self.chunks:
-            check(lib().xb_embedding_pool(arr, n, ptr(scratch), need, s))
+        s = raw_stream()
+        for arr, n, scratch, need in self._calls:
+            check(self._pool(arr, n, scratch, need, s))
 
 
 def embedding_pool(groups):
@@ -109,29 +122,22 @@ def gemm(A, B, Y=None, bias=None, trans_a=False, trans_b=False, alpha=1.0, beta=
          ep_count=0, nosqrt=False, engine=0, out_dtype=None, batch=1, strides=(0, 0, 0, 0), M=None, N=None, K=None,
          lda=None, ldb=None, ldy=None, bias_kind=None, stride_ep=0, ldbias=None, bias_row_group=0):
     """2-D (or explicitly strided batched) GEMM through xb_gemm. Returns Y."""
-    a = GemmArgs()
     if M is None:
         M, K = (A.shape[-1], A.shape[-2]) if trans_a else (A.shape[-2], A.shape[-1])
         N = B.shape[-2] if trans_b else B.shape[-1]
-    out_dtype = out_dtype or A.dtype
     if Y is None:
-        Y = torch.empty((batch, M, N) if batch > 1 else (M, N), dtype=out_dtype, device=A.device)
-    a.M, a.N, a.K, a.trans_a, a.trans_b, a.alpha, a.beta = M, N, K, int(trans_a), int(trans_b), alpha, beta
-    a.A, a.lda, a.stride_a = A.data_ptr(), lda if lda is not None else A.stride(-2), strides[0]
-    a.B, a.ldb, a.stride_b = B.data_ptr(), ldb if ldb is not None else B.stride(-2), strides[1]
-    if bias is not None:
-        a.bias, a.bias_dtype = bias.data_ptr(), dt(bias)
-        a.bias_kind = bias_kind if bias_kind is not None else (capi.XB_BIAS_ROW if bias.dim() == 1 else capi.XB_BIAS_FULL)
-        a.ldbias = ldbias if ldbias is not None else (bias.stride(-2) if bias.dim() > 1 else 0)
-        a.stride_bias = strides[2]
-        a.bias_row_group = bias_row_group
-    a.Y, a.ldy, a.stride_y = Y.data_ptr(), ldy if ldy is not None else Y.stride(-2), strides[3]
-    a.batch, a.ab_dtype, a.y_dtype = batch, dt(A), dt(Y)
-    a.epilogue = epilogue
-    a.ep_a, a.ep_b, a.ep_c = ptr(ep[0]), ptr(ep[1]), ptr(ep[2])
-    a.ep_count, a.dice_nosqrt, a.stride_ep, a.engine = ep_count, int(nosqrt), stride_ep, engine
-    check(lib().xb_gemm(C.byref(a), stream()))
+        Y = torch.empty((batch, M, N) if batch > 1 else (M, N), dtype=out_dtype or A.dtype, device=A.device)
+    global _gemm
+    if _gemm is None:
+        m = binding()
+        m.dtypes(_DT)
+        _gemm = m.gemm
+    check(_gemm(A, B, Y, bias, trans_a, trans_b, alpha, beta, epilogue, ep, ep_count, nosqrt, engine, batch, strides, M, N, K,
+                lda, ldb, ldy, bias_kind, stride_ep, ldbias, bias_row_group, raw_stream()))
     return Y
+
+
+_gemm = None
 
 
 def pack_weight_kmajor(W, out_dtype=torch.float16, ldk=None, batch=1):
