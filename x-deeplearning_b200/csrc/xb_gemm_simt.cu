@@ -1,8 +1,9 @@
 // CUDA-core GEMM engine with the fused bias/activation epilogue.
 //
 // Serves what the tcgen05 engine does not take: fp32 operands (the reference's
-// 1e-6 operator fixtures need true fp32 products, not tf32), transposed A,
-// leading dimensions that break TMA's 16-byte rule, and tiny shapes.
+// 1e-6 operator fixtures need true fp32 products, not tf32) and fp32 results of
+// 16-bit operands in the layouts and sizes that it leaves. (16-bit results of
+// those go through warp-level matrix instructions, xb_gemm_half.cuh.)
 //
 // 256 threads, tile 16*TM x 16*TN, 16-deep k slices; fp32 accumulation with k
 // ascending, whatever the tile, so every form gives the same bits.
@@ -377,6 +378,10 @@ static int launch_simt_tm(const SimtGemmParams& p, int tn, dim3 grid, cudaStream
   return check_launch("gemm_simt_kernel");
 }
 
+}  // namespace xb
+#include "xb_gemm_half.cuh"
+namespace xb {
+
 // ---- batches of single rows (fp32): the weighted sum of an attention unit run operator by operator -------------------------
 // A tile has 32 rows at the least and a batch of such products one row each: here a CTA takes a batch, its threads four
 // columns of every few k, and the partial sums are added in order. Bound by the read of B. 500 x ([1, 100] x [100, 36]):
@@ -565,6 +570,9 @@ int gemm_simt(const xb_gemm_args& a, cudaStream_t stream) {
     if (a.ab_dtype == XB_F16) return launch_narrow<__half>(p, a.batch, stream);
     return launch_narrow<__nv_bfloat16>(p, a.batch, stream);
   }
+  // 16-bit results of 16-bit operands: the matrix instructions' sums, which are not rounded one by one, end in the same 16 bits.
+  // (An fp32 result would show it, and who asks for this engine by name gets its order of sums.)
+  if (a.engine == XB_GEMM_AUTO && a.ab_dtype != XB_F32 && a.y_dtype != XB_F32) return gemm_half(p, a, stream);
   p.tiles_n = (a.N + 16 * tn - 1) / (16 * tn);
   const int64_t tiles = (((int64_t)a.M + 16 * tm - 1) / (16 * tm)) * p.tiles_n;
   XB_REQUIRE(tiles < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)tiles);

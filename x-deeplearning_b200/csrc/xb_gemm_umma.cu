@@ -845,9 +845,11 @@ extern "C" int xb_gemm(const xb_gemm_args* a, xb_stream_t stream) {
     XB_REQUIRE(a->K > 0, XB_ERR_ARG, "xb_gemm: K = 0");
     return gemm_umma(*a, (cudaStream_t)stream);
   }
-  // small problems are launch-bound either way; the CUDA-core engine has no TMA descriptor cost
+  // Whatever the size where the result has 16 bits: a few outputs of a long sum are a chain of slices in any other kernel
+  // (16 x ([22, 320] x [320, 16]): 4.5 us, 8.3 with warp-level matrix instructions, 24.8 on the CUDA cores; 2 x ([59, 24] x [24, 32]):
+  // 3.3, 4.3, 5.7). An fp32 result of less than 128 x 64 outputs keeps the CUDA cores' order of sums.
   if (a->engine == XB_GEMM_AUTO && umma_eligible(*a) && a->K > 0 && !gemm_narrow_takes(*a) &&
-      (int64_t)a->M * a->N * a->batch >= 128 * 64)
+      (a->y_dtype != XB_F32 || (int64_t)a->M * a->N * a->batch >= 128 * 64))
     return gemm_umma(*a, (cudaStream_t)stream);
   return gemm_simt(*a, (cudaStream_t)stream);
 }
