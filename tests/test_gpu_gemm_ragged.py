@@ -1,0 +1,66 @@
+"""Outputs that end inside a tile, with one tile a block (stored by the threads) and with several (stored by TMA), batches stacked or
+side by side, against plain torch in 64 bits; what lies around the output stays as it was."""
+import pytest
+import torch
+
+import pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def _ops():
+    pkg.load()
+    from x_deeplearning_b200 import ops, capi
+    return ops, capi
+
+
+EPI = ["none", "prelu", "dice", "sigmoid"]
+
+
+@pytest.mark.parametrize("N", [8, 16, 24, 40, 64, 72, 104, 128, 136, 144, 152, 168, 200, 256, 264, 272, 328, 392, 600])
+@pytest.mark.parametrize("M", [6401, 130])
+@pytest.mark.parametrize("beside", [False, True])
+@pytest.mark.parametrize("dtype,out", [(torch.float16, torch.float16), (torch.bfloat16, torch.bfloat16), (torch.float16, torch.float32)])
+def test_ragged_outputs(N, M, beside, dtype, out):
+    ops, capi = _ops()
+    P, K = 3, 72
+    kn = N % 16 == 0 and out != torch.float32
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    A, B = r(P, M, K).to(dtype), (r(P, N, K) / K ** 0.5).to(dtype)
+    bias = r(P, N)
+    act = EPI[(N // 8 + beside) % 4]
+    kw, x = {}, A.double() @ B.double().transpose(1, 2) + bias.double()[:, None]
+    mag = A.double().abs() @ B.double().abs().transpose(1, 2) + bias.double().abs()[:, None]
+    slope = torch.rand((P, N), generator=g, device="cuda")
+    if act == "prelu":
+        kw = dict(epilogue=capi.XB_EPI_PRELU, ep=(slope, None, None), ep_count=N, stride_ep=N)
+        want = torch.where(x < 0, x * slope.double()[:, None], x)
+    elif act == "dice":
+        mean, var = r(P, N), torch.rand((P, N), generator=g, device="cuda") + 0.5
+        kw = dict(epilogue=capi.XB_EPI_DICE, ep=(slope, mean, var), stride_ep=N)
+        p = ((x - mean.double()[:, None]) / var.double().sqrt()[:, None]).sigmoid()
+        want = (1 - p) * slope.double()[:, None] * x + p * x
+    elif act == "sigmoid":
+        kw, want = dict(epilogue=capi.XB_EPI_SIGMOID), x.sigmoid()
+    else:
+        want = x
+    ld = N * P + 16 if beside else N + 8
+    Y = torch.full((M + 1, ld) if beside else (P * M + 1, ld), 9.0, dtype=out, device="cuda")
+    W = B.transpose(1, 2).contiguous() if kn else B
+    ops.gemm(A, W, Y=Y, bias=bias, bias_kind=capi.XB_BIAS_ROW, trans_b=not kn, batch=P, M=M, N=N, K=K, lda=K, ldb=W.shape[-1], ldy=ld,
+             strides=(M * K, N * K, N, N if beside else M * ld), **kw)
+    got = Y[:M, :P * N].view(M, P, N).transpose(0, 1) if beside else Y[:P * M].view(P, M, ld)[:, :, :N]
+    # fp32 sums of K products, not every one rounded; the activations' slopes (Dice: at most 1 + |x| / (2 std)) and their fast
+    # exponential and quotient; the result's rounding
+    eps = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 2.0 ** -24}[out]
+    tol = 2 * (K + 2) * 2.0 ** -24 * mag
+    if act == "dice":
+        tol = tol * (1 + x.abs()) + 2.0 ** -20 * (1 + x.abs())
+    elif act == "sigmoid":
+        tol = tol + 2.0 ** -20
+    assert ((got.double() - want).abs() <= tol + eps * want.abs() + (2.0 ** -25 if out == torch.float16 else 0)).all()
+    if beside:
+        assert (Y[M:] == 9.0).all() and (Y[:, P * N:] == 9.0).all()
+    else:
+        assert (Y[P * M:] == 9.0).all() and (Y[:, N:] == 9.0).all()

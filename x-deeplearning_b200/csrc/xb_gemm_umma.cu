@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <mutex>
 #include <cstring>
+#include <type_traits>
 
 #include "xb_common.cuh"
 #include "xb_umma.cuh"
@@ -51,6 +52,8 @@ struct UmmaGemmParams {
   void* Y; int64_t ldy, stride_y; int y_dtype;
   EpiParams epi; int64_t stride_ep;
   uint32_t idesc;
+  int y_unit, y_bufs;    // results stored by TMA: columns of a copy (32 or 16), staging areas of a warp
+  int y_beside;          // the batches lie beside one another in a row of Y: its map has the batch before the row
 };
 
 template <typename TOut>
@@ -81,74 +84,6 @@ __device__ __forceinline__ void store_row16(TOut* dst, const float (&v)[16], int
 constexpr int EPI_WARPS = 16;
 constexpr int GEMM_THREADS = 64 + EPI_WARPS * 32;
 
-// 16 results of one output row as one (fp32: four) 16-byte store(s)
-template <typename TOut>
-__device__ __forceinline__ void store16_vec(TOut* dst, const float (&v)[16]);
-template <>
-__device__ __forceinline__ void store16_vec<float>(float* dst, const float (&v)[16]) {
-  float4* d = reinterpret_cast<float4*>(dst);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-}
-template <>
-__device__ __forceinline__ void store16_vec<__half>(__half* dst, const float (&v)[16]) {
-  uint32_t w[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-    w[i] = *reinterpret_cast<const uint32_t*>(&h);
-  }
-  uint4* d = reinterpret_cast<uint4*>(dst);
-  d[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  d[1] = make_uint4(w[4], w[5], w[6], w[7]);
-}
-template <>
-__device__ __forceinline__ void store16_vec<__nv_bfloat16>(__nv_bfloat16* dst, const float (&v)[16]) {
-  uint32_t w[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-    w[i] = *reinterpret_cast<const uint32_t*>(&h);
-  }
-  uint4* d = reinterpret_cast<uint4*>(dst);
-  d[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  d[1] = make_uint4(w[4], w[5], w[6], w[7]);
-}
-
-// Activation of 16 adjacent columns of one row; the per-column parameters sit in shared memory and are
-// read as 16-byte vectors (all lanes read the same address: a broadcast).
-template <int KIND>
-__device__ __forceinline__ void epi_apply16(float (&v)[16], const float* s_a, const float* s_b, const float* s_c) {
-  if constexpr (KIND != XB_EPI_NONE) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (KIND == XB_EPI_PRELU) {
-      const float4 a = reinterpret_cast<const float4*>(s_a)[j];
-      // x * (x < 0 ? w : 1): the same value as act_prelu for every x, signed zeros and NaN included
-      v[4 * j] *= v[4 * j] < 0.f ? a.x : 1.f;
-      v[4 * j + 1] *= v[4 * j + 1] < 0.f ? a.y : 1.f;
-      v[4 * j + 2] *= v[4 * j + 2] < 0.f ? a.z : 1.f;
-      v[4 * j + 3] *= v[4 * j + 3] < 0.f ? a.w : 1.f;
-    } else if (KIND == XB_EPI_DICE) {
-      const float4 g = reinterpret_cast<const float4*>(s_a)[j];
-      const float4 b = reinterpret_cast<const float4*>(s_b)[j];
-      const float4 c = reinterpret_cast<const float4*>(s_c)[j];
-      const float gg[4] = {g.x, g.y, g.z, g.w}, bb[4] = {b.x, b.y, b.z, b.w}, cc[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float x = v[4 * j + i];
-        const float pr = __fdividef(1.f, 1.f + __expf(-fmaf(x, cc[i], bb[i])));
-        v[4 * j + i] = x * fmaf(pr, 1.f - gg[i], gg[i]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[4 * j + i] = act_sigmoid(v[4 * j + i]);
-    }
-  }
-  }
-}
-
-// 8 results as one 16-byte piece of 2-byte elements
 template <typename TOut>
 __device__ __forceinline__ uint4 pack8(const float* v);
 template <>
@@ -174,10 +109,71 @@ __device__ __forceinline__ uint4 pack8<__nv_bfloat16>(const float* v) {
 template <>
 __device__ __forceinline__ uint4 pack8<float>(const float*) { return make_uint4(0, 0, 0, 0); }   // not used
 
+// 16 results of one output row as 16-byte stores, those that lie wholly in the `valid` columns left of it
+template <typename TOut>
+__device__ __forceinline__ void store16_vec(TOut* dst, const float (&v)[16], int valid) {
+  if constexpr (sizeof(TOut) == 4) {
+    float4* d = reinterpret_cast<float4*>(dst);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (4 * i + 4 <= valid) d[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+  } else {
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    if (8 <= valid) d[0] = pack8<TOut>(v);
+    if (16 <= valid) d[1] = pack8<TOut>(v + 8);
+  }
+}
+
+// For a 16-bit result the quotient as one multiplication with the hardware's reciprocal (2 ulp of fp32, 2^-11 of what the result's
+// rounding may be off). 4 x ([9854, 24] x [24, 336]) fp16: the division took 6 of 29 us; the error against 64 bits is the same.
+template <typename TOut>
+__device__ __forceinline__ float epi_sigmoid(float x) {
+  if constexpr (sizeof(TOut) == 4) return act_sigmoid(x);
+  else return __fdividef(1.f, 1.f + __expf(-x));
+}
+
+// Activation of 16 adjacent columns of one row; the per-column parameters sit in shared memory and are
+// read as 16-byte vectors (all lanes read the same address: a broadcast).
+template <typename TOut, int KIND>
+__device__ __forceinline__ void epi_apply16(float (&v)[16], const float* s_a, const float* s_b, const float* s_c) {
+  if constexpr (KIND != XB_EPI_NONE) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (KIND == XB_EPI_PRELU) {
+      const float4 a = reinterpret_cast<const float4*>(s_a)[j];
+      // x * (x < 0 ? w : 1): the same value as act_prelu for every x, signed zeros and NaN included
+      v[4 * j] *= v[4 * j] < 0.f ? a.x : 1.f;
+      v[4 * j + 1] *= v[4 * j + 1] < 0.f ? a.y : 1.f;
+      v[4 * j + 2] *= v[4 * j + 2] < 0.f ? a.z : 1.f;
+      v[4 * j + 3] *= v[4 * j + 3] < 0.f ? a.w : 1.f;
+    } else if (KIND == XB_EPI_DICE) {
+      const float4 g = reinterpret_cast<const float4*>(s_a)[j];
+      const float4 b = reinterpret_cast<const float4*>(s_b)[j];
+      const float4 c = reinterpret_cast<const float4*>(s_c)[j];
+      const float gg[4] = {g.x, g.y, g.z, g.w}, bb[4] = {b.x, b.y, b.z, b.w}, cc[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float x = v[4 * j + i];
+        const float pr = __fdividef(1.f, 1.f + __expf(-fmaf(x, cc[i], bb[i])));
+        v[4 * j + i] = x * fmaf(pr, 1.f - gg[i], gg[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[4 * j + i] = epi_sigmoid<TOut>(v[4 * j + i]);
+    }
+  }
+  }
+}
+
 constexpr int EPI_STAGE_BYTES = 32 * 64;      // per epilogue warp: 32 rows x 32 two-byte results
 
-// Epilogue of a tile that lies fully inside the output, with a per-column bias (or none) and 16-byte
-// aligned rows: this thread's row, columns [16 * c_begin, 16 * c_end) of the tile.
+// Epilogue of a tile with a per-column bias (or none) and output rows of whole, aligned 16-byte pieces: this thread's row,
+// columns [16 * c_begin, 16 * c_end) of the tile, as far as `rows` of the warp's 32 and `cols` of the tile's columns lie in the
+// output (a piece is stored or it is not).
+// Bound by shared memory's and L1's data path, which carries a result four times here (staging, both ways, beside the accumulator and
+// the store). Ragged tiles went through epi_tile_edge before: [65536, 88] x [88, 168] fp16 19.6 us, 13.6 here, where whole tiles take
+// 3 % longer for the two comparisons a store ([65536, 88] x [88, 176]: 12.7, 13.0; two forms of this function, one for each, took
+// 14.5, by spills).
 // Two-byte outputs go through a 2 KB staging area of the warp: a thread holds 64 contiguous bytes of its
 // own row, and a store instruction of one piece per lane would touch 32 different lines; after the
 // exchange the 32 lanes of an instruction write 8 rows x 64 contiguous bytes. Piece j of row l is kept at
@@ -186,12 +182,13 @@ constexpr int EPI_STAGE_BYTES = 32 * 64;      // per epilogue warp: 32 rows x 32
 template <typename TOut, int KIND>
 __device__ __forceinline__ void epi_tile_fast(uint32_t tmem_row, int c_begin, int c_end, float alpha,
                                               const float* s_bias, const float* s_a, const float* s_b,
-                                              const float* s_c, TOut* yrow, int64_t ldy, uint4* stage, int lane) {
+                                              const float* s_c, TOut* yrow, int64_t ldy, int rows, int cols,
+                                              uint4* stage, int lane) {
   using namespace umma;
   for (int cg = c_begin; cg < c_end; cg += 2) {
     // two chunks per TMEM round trip when the thread owns two more
     uint32_t raw[32];
-    const bool two = cg + 1 < c_end;                                    // uniform across the CTA
+    const bool two = cg + 1 < c_end;                                    // uniform across the warp
     if (two) {
       tmem_ld32_nowait(tmem_row + (uint32_t)(cg * 16), raw);
     } else {
@@ -213,26 +210,81 @@ __device__ __forceinline__ void epi_tile_fast(uint32_t tmem_row, int c_begin, in
         v[4 * j + 2] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 2]), b.z);
         v[4 * j + 3] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 3]), b.w);
       }
-      epi_apply16<KIND>(v, s_a + c, s_b + c, s_c + c);
+      epi_apply16<TOut, KIND>(v, s_a + c, s_b + c, s_c + c);
       if (sizeof(TOut) == 2 && two) {
         const int sw = (lane >> 1) & 3;
         stage[lane * 4 + ((2 * u) ^ sw)] = pack8<TOut>(v);
         stage[lane * 4 + ((2 * u + 1) ^ sw)] = pack8<TOut>(v + 8);
-      } else {
-        store16_vec<TOut>(yrow + c, v);
+      } else if (lane < rows) {
+        store16_vec<TOut>(yrow + c, v, cols - c);
       }
     }
     if (sizeof(TOut) == 2 && two) {
       __syncwarp();
-      TOut* base = yrow + cg * 16 + (lane & 3) * 8;          // this lane's 16-byte column slot, in its own row
+      const int slot = cg * 16 + (lane & 3) * 8;             // this lane's 16-byte column slot
+      const int in = slot + 8 <= cols ? rows : 0;
+      TOut* base = yrow + slot;                              // (in its own row)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = 8 * i + (lane >> 2);
         const uint4 x = stage[r * 4 + ((lane & 3) ^ ((r >> 1) & 3))];
-        *reinterpret_cast<uint4*>(base + (int64_t)(r - lane) * ldy) = x;
+        if (r < in) *reinterpret_cast<uint4*>(base + (int64_t)(r - lane) * ldy) = x;
       }
       __syncwarp();                                          // the next round overwrites the staging area
     }
+  }
+}
+
+// A unit of W columns of this thread's row into the warp's staging area, as a W-column copy reads it (pieces swizzled as in
+// epi_tile_fast; rows of 32 bytes where W = 16).
+template <typename TOut, int KIND, int W>
+__device__ __forceinline__ void epi_unit(uint32_t tmem_at, float alpha, const float* s_bias, const float* s_a, const float* s_b, const float* s_c,
+                                         uint4* area, int lane) {
+  using namespace umma;
+  uint32_t raw[W];
+  if constexpr (W == 32) tmem_ld32_nowait(tmem_at, raw);
+  else tmem_ld16_nowait(tmem_at, raw);
+  tmem_wait_ld(raw);
+  const int sw = W == 32 ? (lane >> 1) & 3 : (lane >> 2) & 1;
+#pragma unroll
+  for (int u = 0; u < W / 16; ++u) {
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 b = reinterpret_cast<const float4*>(s_bias + 16 * u)[j];
+      v[4 * j] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j]), b.x);
+      v[4 * j + 1] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 1]), b.y);
+      v[4 * j + 2] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 2]), b.z);
+      v[4 * j + 3] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 3]), b.w);
+    }
+    epi_apply16<TOut, KIND>(v, s_a + 16 * u, s_b + 16 * u, s_c + 16 * u);
+    area[lane * (W / 8) + ((2 * u) ^ sw)] = pack8<TOut>(v);
+    area[lane * (W / 8) + ((2 * u + 1) ^ sw)] = pack8<TOut>(v + 8);
+  }
+}
+
+// Epilogue of a tile whose results leave by TMA, a warp's 32 rows x W columns at a time: units `part`, `part` + 4, ... of the tile.
+// A warp with two units a tile has two areas, so that it fills one while the other is read. What the threads' own stores and their
+// reads of the staging area took of the data path (4900 wavefronts a tile of 128 x 256, 5000 cycles) is the copy engine's work here.
+// [65536, 88] x [88, 256] fp16: 16.1 -> 11.8 us, N = 192 14.4 -> 10.5, 8 x ([4096, 256] x [256, 128]) side by side 8.3 -> 7.9,
+// 8 x ([33434, 88] x [88, 32]) with a sigmoid 24.2 -> 22.5.
+template <typename TOut, int KIND, int W>
+__device__ __forceinline__ void epi_tile_tma(const CUtensorMap& map_y, uint32_t tmem_row, int part, int cols, float alpha, const float* s_bias,
+                                             const float* s_a, const float* s_b, const float* s_c, uint8_t* stage, int bufs, uint32_t& turn,
+                                             int x, int y, int z, bool rows, int lane) {
+  using namespace umma;
+  for (int c = part * W; c < cols; c += 4 * W) {
+    uint8_t* area = stage + (bufs == 2 ? (turn & 1u) * (32 * W * 2) : 0u);
+    ++turn;
+    if (lane == 0) {                                         // the copy that read this area last has done so
+      if (bufs == 2) tma_store_wait_read<1>();
+      else tma_store_wait_read<0>();
+    }
+    __syncwarp();
+    epi_unit<TOut, KIND, W>(tmem_row + (uint32_t)c, alpha, s_bias + c, s_a + c, s_b + c, s_c + c, reinterpret_cast<uint4*>(area), lane);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0 && rows) tma_store_3d(&map_y, smem_u32(area), x + c, y, z);
   }
 }
 
@@ -252,9 +304,9 @@ __device__ __forceinline__ void stage_columns(const UmmaGemmParams& p, int b, in
   s_bias[e] = bv; s_a[e] = pa; s_b[e] = pb; s_c[e] = pc;
 }
 
-// Epilogue of any tile: checks rows and columns against the output, adds a full bias matrix where there is one.
+// Epilogue of any output: rows that start or end anywhere, a full bias matrix where there is one.
 template <typename TOut>
-__device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t tmem_row, int c_begin, int c_end, const float* s_bias,
+__device__ __noinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t tmem_row, int c_begin, int c_end, const float* s_bias,
                                               const float* s_a, const float* s_b, const float* s_c, TOut* yrow, int b, int gm,
                                               int brow, int n0, bool vec_base) {
   using namespace umma;
@@ -297,7 +349,7 @@ __device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t 
       }
     } else if (p.epi.kind == XB_EPI_SIGMOID) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = act_sigmoid(v[i]);
+      for (int i = 0; i < 16; ++i) v[i] = epi_sigmoid<TOut>(v[i]);
     }
     if (gm < p.M) store_row16<TOut>(yrow + gn0, v, valid, vec_base && ((gn0 * sizeof(TOut)) % 16 == 0));
   }
@@ -305,10 +357,11 @@ __device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t 
 
 // B_MN is a template parameter because the K-major kernel must not pay for the other layout: with a run-time test of it in the
 // MMA and load loops 8 products of [65536, 256] x [256, 128] took 78 us, 74 without.
-template <typename TOut, bool B_MN>
+// Y_TMA: results leave by TMA (map_y; otherwise it is not read).
+template <typename TOut, bool B_MN, bool Y_TMA>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                 const __grid_constant__ UmmaGemmParams p) {
+                 const __grid_constant__ CUtensorMap map_y, const __grid_constant__ UmmaGemmParams p) {
   using namespace umma;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -354,6 +407,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     fence_barrier_init();
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
+    if (Y_TMA) prefetch_tensormap(&map_y);
   }
   if (warp == 1) tmem_alloc(smem_u32(&tmem_base_s), (uint32_t)p.tmem_cols);
   tc_fence_before_sync();
@@ -463,6 +517,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     float* s_c = s_b + 256;
     int it = 0, cur_n0 = -1, cur_b = -1;
     bool ok = true;
+    uint8_t* area = Y_TMA ? reinterpret_cast<uint8_t*>(s_bias + 4 * 256) + ew * p.y_bufs * p.y_unit * 64 : nullptr;
+    uint32_t turn = 0;                                        // units that this warp has stored
     // A warp whose accumulator wait ran out keeps walking the tile sequence without touching tensor memory,
     // global memory or the acc_empty barrier: the other epilogue warps may have passed the same wait (each
     // lane keeps its own clock), and they still need this warp at the two named barriers below.
@@ -483,19 +539,39 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (!ok) continue;
       tc_fence_after_sync();
       const uint32_t tmem_acc = tmem_base + as * acc_stride + ((uint32_t)(q * 32) << 16);
+      if constexpr (Y_TMA) {
+        const int y = m0 + q * 32, cols = min(p.block_n, p.N - n0), y1 = p.y_beside ? b : y, y2 = p.y_beside ? y : b;
+        auto tile_out = [&](auto kind) {
+          constexpr int KIND = decltype(kind)::value;
+          if (p.y_unit == 32)
+            epi_tile_tma<TOut, KIND, 32>(map_y, tmem_acc, part, cols, p.alpha, s_bias, s_a, s_b, s_c, area, p.y_bufs, turn, n0, y1, y2, y < p.M, lane);
+          else
+            epi_tile_tma<TOut, KIND, 16>(map_y, tmem_acc, part, cols, p.alpha, s_bias, s_a, s_b, s_c, area, p.y_bufs, turn, n0, y1, y2, y < p.M, lane);
+        };
+        switch (p.epi.kind) {
+          case XB_EPI_PRELU: tile_out(std::integral_constant<int, XB_EPI_PRELU>()); break;
+          case XB_EPI_DICE: tile_out(std::integral_constant<int, XB_EPI_DICE>()); break;
+          case XB_EPI_SIGMOID: tile_out(std::integral_constant<int, XB_EPI_SIGMOID>()); break;
+          default: tile_out(std::integral_constant<int, XB_EPI_NONE>()); break;
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[as]));
+        continue;
+      } else {
       TOut* yrow = reinterpret_cast<TOut*>(p.Y) + (int64_t)b * p.stride_y + (int64_t)gm * p.ldy;
-      if (vec_base && p.bias_kind != XB_BIAS_FULL && m0 + BLOCK_M <= p.M && n0 + p.block_n <= p.N &&
-          (n0 * sizeof(TOut)) % 16 == 0) {
-        // the common case, without the per-chunk edge and bias-matrix handling of the loop below
+      if (vec_base && p.bias_kind != XB_BIAS_FULL && (p.N * sizeof(TOut)) % 16 == 0) {       // (n0 is a multiple of 16)
+        // the common case, without the per-element edge and bias-matrix handling of the loop below
+        const int rows = p.M - (m0 + q * 32), cols = p.N - n0;
         switch (p.epi.kind) {
           case XB_EPI_PRELU:
-            epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, stage, lane); break;
+            epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
           case XB_EPI_DICE:
-            epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, stage, lane); break;
+            epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
           case XB_EPI_SIGMOID:
-            epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, stage, lane); break;
+            epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
           default:
-            epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, stage, lane); break;
+            epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
         }
         tc_fence_before_sync();
         __syncwarp();
@@ -506,7 +582,9 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&acc_empty[as]));              // one arrival per epilogue warp
+      }
     }
+    if (Y_TMA && lane == 0) tma_store_wait_read<0>();
   }
 
   pdl_release();
@@ -536,30 +614,31 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// [batch, rows, K] tensor of 2-byte elements, box {64, box_rows, 1}, 128-byte swizzle (an N-major B is the same with
-// its k rows as rows and its columns as the inner extent)
+// [batch, rows, K] tensor of 2-byte elements, box {box_cols, box_rows, box_batch}, swizzled over the box's row (an N-major B is the same with
+// its k rows as rows and its columns as the inner extent; so is Y)
 int make_map(CUtensorMap* map, const void* base, int is_bf16, int64_t K, int64_t rows, int64_t ld, int64_t batch,
-             int64_t batch_stride, int box_rows) {
+             int64_t batch_stride, int box_rows, int box_cols = BLOCK_K, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B, int box_batch = 1) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(XB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)batch};
   cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)(batch > 1 ? batch_stride : ld * rows) * 2};
   if (strides[1] == 0) strides[1] = strides[0];
-  cuuint32_t box[3] = {(cuuint32_t)BLOCK_K, (cuuint32_t)box_rows, 1};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, (cuuint32_t)box_batch};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(XB_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
   return 0;
 }
 
-// Columns of a tile: all of a narrow product, 256 or 128 of a wide one; narrower (down to 32, or to the 64 of a box of an
+// Columns of a tile: all of a product of up to 256, equal shares of a wider one (128 columns each until it
+// was so: [65536, 24] x [24, 272] fp16, three tiles of which the last held 16 columns, 18.9 us, 15.5 as two of 144); narrower (down to 32, or to the 64 of a box of an
 // N-major B) where the tiles would leave SMs idle: a CTA's time is the latency of its operand stream, which shrinks with the
 // tile, and A comes from L2 for every column of tiles. 8 products of
 // [1000, 256] x [256, 128] fp16 (64 tiles of 128 columns, 128 of 64): 6.8 -> 5.8 us.
 int pick_block_n(const xb_gemm_args& a) {
-  const int bn = a.N <= 256 ? (a.N + 15) / 16 * 16 : (a.N % 256 == 0) ? 256 : 128;
+  const int wide = (a.N + 255) / 256, bn = ((a.N + wide - 1) / wide + 15) / 16 * 16;
   const int64_t rows = ((int64_t)a.M + BLOCK_M - 1) / BLOCK_M * a.batch;
   const int least = a.trans_b ? 32 : 64;
   const int64_t split = std::min<int64_t>(sm_count() / std::max<int64_t>(rows, 1), (a.N + least - 1) / least);
@@ -581,13 +660,19 @@ bool umma_eligible(const xb_gemm_args& a) {
   return true;
 }
 
-template <typename TOut, bool B_MN>
-int launch_umma(const CUtensorMap& ma, const CUtensorMap& mb, const UmmaGemmParams& p, dim3 grid, size_t smem,
+template <typename TOut, bool B_MN, bool Y_TMA>
+int launch_umma(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const UmmaGemmParams& p, dim3 grid, size_t smem,
                 cudaStream_t s) {
   static PerDeviceOnce attr_set;   // per instantiation
-  XB_SET_MAX_SMEM_ONCE(attr_set, SMEM_BUDGET + 6 * 1024, (const void*)gemm_umma_kernel<TOut, B_MN>);
-  launch_dependent(gemm_umma_kernel<TOut, B_MN>, grid, GEMM_THREADS, smem, s, ma, mb, p);
+  XB_SET_MAX_SMEM_ONCE(attr_set, SMEM_BUDGET + 6 * 1024, (const void*)gemm_umma_kernel<TOut, B_MN, Y_TMA>);
+  launch_dependent(gemm_umma_kernel<TOut, B_MN, Y_TMA>, grid, GEMM_THREADS, smem, s, ma, mb, my, p);
   return check_launch("gemm_umma_kernel");
+}
+template <typename TOut>
+int launch_umma_half(bool y_tma, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const UmmaGemmParams& p, dim3 grid,
+                     size_t smem, cudaStream_t s) {
+  if (p.b_mn) return y_tma ? launch_umma<TOut, true, true>(ma, mb, my, p, grid, smem, s) : launch_umma<TOut, true, false>(ma, mb, mb, p, grid, smem, s);
+  return y_tma ? launch_umma<TOut, false, true>(ma, mb, my, p, grid, smem, s) : launch_umma<TOut, false, false>(ma, mb, mb, p, grid, smem, s);
 }
 
 void fill_umma_params(UmmaGemmParams& p, const xb_gemm_args& a) {
@@ -642,7 +727,7 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   CUtensorMap ma, mb;
   if (int rc = make_map(&ma, a.A, is_bf16, a.K, a.M, a.lda, p.a_batched ? a.batch : 1, a.stride_a, BLOCK_M)) return rc;
   // after the ring: per-column epilogue parameters [4][256] fp32, then the epilogue warps' staging areas
-  const int tail = 4 * 256 * (int)sizeof(float) + (a.y_dtype == XB_F32 ? 0 : EPI_WARPS * EPI_STAGE_BYTES);
+  int tail = 4 * 256 * (int)sizeof(float) + (a.y_dtype == XB_F32 ? 0 : EPI_WARPS * EPI_STAGE_BYTES);
   if (pair_wanted(a)) {
     if (int rc = make_map(&mb, a.B, is_bf16, a.K, a.N, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, PAIR_N / 2)) return rc;
     p.tiles_m = (a.M + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
@@ -666,6 +751,23 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   p.tiles_n = (a.N + p.block_n - 1) / p.block_n;
   const int64_t total = (int64_t)p.tiles_m * p.tiles_n * p.batch;
   XB_REQUIRE(total < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)total);
+  // Results by TMA where a CTA has several tiles and rows of whole 16-byte pieces. (One tile is a chain of latencies that the copy
+  // lengthens: 2 x ([1862, 88] x [88, 24]) bf16 3.5 us, 3.9 by TMA; [1000, 88] x [88, 168] fp16 3.8 and 4.0.)
+  const bool stacked = a.batch == 1 || a.stride_y >= (int64_t)a.M * a.ldy, beside = !stacked && a.stride_y >= a.N && a.stride_y * a.batch <= a.ldy;
+  bool y_tma = a.y_dtype != XB_F32 && total > sm_count() && p.bias_kind != XB_BIAS_FULL && (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0 &&
+                     a.ldy % 8 == 0 && a.N % 8 == 0 && (a.batch == 1 || a.stride_y % 8 == 0) && (stacked || beside);
+  CUtensorMap my;
+  if (y_tma) {
+    // copies of 32 columns, 16 where the tile has few or where 32 would reach into the next tile
+    p.y_unit = p.block_n >= 128 && (p.block_n % 32 == 0 || p.tiles_n == 1) ? 32 : 16;
+    p.y_bufs = p.block_n > 4 * p.y_unit ? 2 : 1;
+    p.y_beside = beside;
+    const CUtensorMapSwizzle sw = p.y_unit == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+    const int bf = a.y_dtype == XB_BF16;
+    y_tma = 0 == (beside ? make_map(&my, a.Y, bf, a.N, a.batch, a.stride_y, a.M, a.ldy, 1, p.y_unit, sw, 32)
+                         : make_map(&my, a.Y, bf, a.N, a.M, a.ldy, a.batch, a.stride_y, 32, p.y_unit, sw));
+    if (y_tma) tail = 4 * 256 * (int)sizeof(float) + EPI_WARPS * p.y_bufs * p.y_unit * 64;
+  }
   // persistent: one CTA per SM walks the tiles; the accumulator is double-buffered in TMEM so the
   // epilogue of one tile overlaps the loads and MMAs of the next
   dim3 grid((unsigned)std::min<int64_t>(total, sm_count()));
@@ -694,10 +796,9 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
     smem = (size_t)p.stages * stage_bytes + tail + 1024;
   }
   switch (a.y_dtype) {
-    case XB_F16: return p.b_mn ? launch_umma<__half, true>(ma, mb, p, grid, smem, stream) : launch_umma<__half, false>(ma, mb, p, grid, smem, stream);
-    case XB_BF16:
-      return p.b_mn ? launch_umma<__nv_bfloat16, true>(ma, mb, p, grid, smem, stream) : launch_umma<__nv_bfloat16, false>(ma, mb, p, grid, smem, stream);
-    default: return launch_umma<float, false>(ma, mb, p, grid, smem, stream);      // (never b_mn: umma_eligible)
+    case XB_F16: return launch_umma_half<__half>(y_tma, ma, mb, my, p, grid, smem, stream);
+    case XB_BF16: return launch_umma_half<__nv_bfloat16>(y_tma, ma, mb, my, p, grid, smem, stream);
+    default: return launch_umma<float, false, false>(ma, mb, mb, p, grid, smem, stream);      // (never b_mn: umma_eligible)
   }
 }
 

@@ -161,16 +161,13 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       tc_fence_after_sync();
       const uint32_t tmem_acc = tmem_base + as * PAIR_N + ((uint32_t)(q * 32) << 16);
       TOut* yrow = reinterpret_cast<TOut*>(p.Y) + (int64_t)b * p.stride_y + (int64_t)gm * p.ldy;
-      if (m0 + BLOCK_M > p.M) {                                    // the last rows, or none
-        epi_tile_edge<TOut>(p, tmem_acc, c_begin, c_end, s_bias, s_a, s_b, s_c, yrow, b, gm, gm, n0, true);
-      } else {
-        yrow += n0;
-        switch (p.epi.kind) {
-          case XB_EPI_PRELU: epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, stage, lane); break;
-          case XB_EPI_DICE: epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, stage, lane); break;
-          case XB_EPI_SIGMOID: epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, stage, lane); break;
-          default: epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, stage, lane); break;
-        }
+      const int rows = p.M - (m0 + q * 32);                        // of the warp's 32; the columns are all there
+      yrow += n0;
+      switch (p.epi.kind) {
+        case XB_EPI_PRELU: epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
+        case XB_EPI_DICE: epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
+        case XB_EPI_SIGMOID: epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
+        default: epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
       }
       tc_fence_before_sync();
       __syncwarp();
