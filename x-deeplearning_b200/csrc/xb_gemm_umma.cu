@@ -171,9 +171,8 @@ constexpr int EPI_STAGE_BYTES = 32 * 64;      // per epilogue warp: 32 rows x 32
 // columns [16 * c_begin, 16 * c_end) of the tile, as far as `rows` of the warp's 32 and `cols` of the tile's columns lie in the
 // output (a piece is stored or it is not).
 // Bound by shared memory's and L1's data path, which carries a result four times here (staging, both ways, beside the accumulator and
-// the store). Ragged tiles went through epi_tile_edge before: [65536, 88] x [88, 168] fp16 19.6 us, 13.6 here, where whole tiles take
-// 3 % longer for the two comparisons a store ([65536, 88] x [88, 176]: 12.7, 13.0; two forms of this function, one for each, took
-// 14.5, by spills).
+// the store). Ragged tiles went through epi_tile_edge before: [1000, 88] x [88, 168] fp16 4.8 us, 3.8 here; 8 x ([300, 256] x [256, 200])
+// 5.1, 4.3.
 // Two-byte outputs go through a 2 KB staging area of the warp: a thread holds 64 contiguous bytes of its
 // own row, and a store instruction of one piece per lane would touch 32 different lines; after the
 // exchange the 32 lanes of an instruction write 8 rows x 64 contiguous bytes. Piece j of row l is kept at
@@ -306,9 +305,9 @@ __device__ __forceinline__ void stage_columns(const UmmaGemmParams& p, int b, in
 
 // Epilogue of any output: rows that start or end anywhere, a full bias matrix where there is one.
 template <typename TOut>
-__device__ __noinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t tmem_row, int c_begin, int c_end, const float* s_bias,
+__device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t tmem_row, int c_begin, int c_end, const float* s_bias,
                                               const float* s_a, const float* s_b, const float* s_c, TOut* yrow, int b, int gm,
-                                              int brow, int n0, bool vec_base) {
+                                              int brow, int n0, bool vec_base, uint16_t* stage, int lane) {
   using namespace umma;
   for (int cg = c_begin; cg < c_end; ++cg) {
     uint32_t raw[16];
@@ -351,14 +350,36 @@ __device__ __noinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t tme
 #pragma unroll
       for (int i = 0; i < 16; ++i) v[i] = epi_sigmoid<TOut>(v[i]);
     }
-    if (gm < p.M) store_row16<TOut>(yrow + gn0, v, valid, vec_base && ((gn0 * sizeof(TOut)) % 16 == 0));
+    const bool vec = vec_base && ((gn0 * sizeof(TOut)) % 16 == 0);
+    if (sizeof(TOut) == 2 && !(vec && valid == 16)) {
+      // Rows that start anywhere: a store of one element per lane and row touches 32 lines, so the warp turns its 32 x 16 results
+      // and writes two rows at a time. [65536, 256] x [256, 255] fp16: 173 -> 29 us; [40594, 104] x [104, 41] 24 -> 8.3;
+      // 8 x ([4198, 48] x [48, 398]) with a sigmoid 178 -> 24.
+      const int piece = (lane >> 2) & 1;                              // (swapped in every other four rows: no bank conflicts)
+      reinterpret_cast<uint4*>(stage)[lane * 2 + piece] = pack8<TOut>(v);
+      reinterpret_cast<uint4*>(stage)[lane * 2 + (piece ^ 1)] = pack8<TOut>(v + 8);
+      __syncwarp();
+      const int col = lane & 15, rows = p.M - (gm - lane);            // (gm - lane: the warp's first row)
+      uint16_t* at = reinterpret_cast<uint16_t*>(yrow + gn0) + (int64_t)((lane >> 4) - lane) * p.ldy + col;
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i, at += 2 * p.ldy) {
+        const int r = 2 * i + (lane >> 4);
+        const uint16_t x = stage[r * 16 + ((col >> 3) ^ ((r >> 2) & 1)) * 8 + (col & 7)];
+        if (r < rows && col < valid) *at = x;
+      }
+      __syncwarp();
+    } else if (gm < p.M) {
+      store_row16<TOut>(yrow + gn0, v, valid, vec);
+    }
   }
 }
 
 // B_MN is a template parameter because the K-major kernel must not pay for the other layout: with a run-time test of it in the
 // MMA and load loops 8 products of [65536, 256] x [256, 128] took 78 us, 74 without.
-// Y_TMA: results leave by TMA (map_y; otherwise it is not read).
-template <typename TOut, bool B_MN, bool Y_TMA>
+// Y: how results leave, one kernel each: with two of them in one, whole tiles took 3 % longer ([65536, 88] x [88, 176] fp16 12.7 us,
+// 13.0), with three 14 %, by spills. map_y is read where that is by TMA.
+enum { Y_PIECES, Y_TMA, Y_ANY };
+template <typename TOut, bool B_MN, int Y>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_y, const __grid_constant__ UmmaGemmParams p) {
@@ -407,7 +428,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     fence_barrier_init();
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
-    if (Y_TMA) prefetch_tensormap(&map_y);
+    if (Y == Y_TMA) prefetch_tensormap(&map_y);
   }
   if (warp == 1) tmem_alloc(smem_u32(&tmem_base_s), (uint32_t)p.tmem_cols);
   tc_fence_before_sync();
@@ -517,7 +538,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     float* s_c = s_b + 256;
     int it = 0, cur_n0 = -1, cur_b = -1;
     bool ok = true;
-    uint8_t* area = Y_TMA ? reinterpret_cast<uint8_t*>(s_bias + 4 * 256) + ew * p.y_bufs * p.y_unit * 64 : nullptr;
+    uint8_t* area = Y == Y_TMA ? reinterpret_cast<uint8_t*>(s_bias + 4 * 256) + ew * p.y_bufs * p.y_unit * 64 : nullptr;
     uint32_t turn = 0;                                        // units that this warp has stored
     // A warp whose accumulator wait ran out keeps walking the tile sequence without touching tensor memory,
     // global memory or the acc_empty barrier: the other epilogue warps may have passed the same wait (each
@@ -527,7 +548,6 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       place(tile, b, m0, n0);
       const int as = it & 1;
       const int gm = m0 + row;
-      const int brow = p.bias_group > 1 ? (int)((uint32_t)gm / (uint32_t)p.bias_group) : gm;   // bias row of this output row
       if (n0 != cur_n0 || b != cur_b) {
         cur_n0 = n0; cur_b = b;
         asm volatile("bar.sync 2, 512;" ::: "memory");                  // everyone is done with the old columns
@@ -539,7 +559,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (!ok) continue;
       tc_fence_after_sync();
       const uint32_t tmem_acc = tmem_base + as * acc_stride + ((uint32_t)(q * 32) << 16);
-      if constexpr (Y_TMA) {
+      if constexpr (Y == Y_TMA) {
         const int y = m0 + q * 32, cols = min(p.block_n, p.N - n0), y1 = p.y_beside ? b : y, y2 = p.y_beside ? y : b;
         auto tile_out = [&](auto kind) {
           constexpr int KIND = decltype(kind)::value;
@@ -554,37 +574,31 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           case XB_EPI_SIGMOID: tile_out(std::integral_constant<int, XB_EPI_SIGMOID>()); break;
           default: tile_out(std::integral_constant<int, XB_EPI_NONE>()); break;
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[as]));
-        continue;
       } else {
-      TOut* yrow = reinterpret_cast<TOut*>(p.Y) + (int64_t)b * p.stride_y + (int64_t)gm * p.ldy;
-      if (vec_base && p.bias_kind != XB_BIAS_FULL && (p.N * sizeof(TOut)) % 16 == 0) {       // (n0 is a multiple of 16)
-        // the common case, without the per-element edge and bias-matrix handling of the loop below
-        const int rows = p.M - (m0 + q * 32), cols = p.N - n0;
-        switch (p.epi.kind) {
-          case XB_EPI_PRELU:
-            epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
-          case XB_EPI_DICE:
-            epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
-          case XB_EPI_SIGMOID:
-            epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
-          default:
-            epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
+        TOut* yrow = reinterpret_cast<TOut*>(p.Y) + (int64_t)b * p.stride_y + (int64_t)gm * p.ldy;
+        if constexpr (Y == Y_ANY) {
+          const int brow = p.bias_group > 1 ? (int)((uint32_t)gm / (uint32_t)p.bias_group) : gm;   // bias row of this output row
+          epi_tile_edge<TOut>(p, tmem_acc, c_begin, c_end, s_bias, s_a, s_b, s_c, yrow, b, gm, brow, n0, vec_base,
+                              reinterpret_cast<uint16_t*>(stage), lane);
+        } else {
+          const int rows = p.M - (m0 + q * 32), cols = p.N - n0;
+          switch (p.epi.kind) {
+            case XB_EPI_PRELU:
+              epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
+            case XB_EPI_DICE:
+              epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
+            case XB_EPI_SIGMOID:
+              epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
+            default:
+              epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
+          }
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&acc_empty[as]));
-        continue;
       }
-      epi_tile_edge<TOut>(p, tmem_acc, c_begin, c_end, s_bias, s_a, s_b, s_c, yrow, b, gm, brow, n0, vec_base);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&acc_empty[as]));              // one arrival per epilogue warp
-      }
     }
-    if (Y_TMA && lane == 0) tma_store_wait_read<0>();
+    if (Y == Y_TMA && lane == 0) tma_store_wait_read<0>();
   }
 
   pdl_release();
@@ -660,19 +674,20 @@ bool umma_eligible(const xb_gemm_args& a) {
   return true;
 }
 
-template <typename TOut, bool B_MN, bool Y_TMA>
+template <typename TOut, bool B_MN, int Y>
 int launch_umma(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const UmmaGemmParams& p, dim3 grid, size_t smem,
                 cudaStream_t s) {
   static PerDeviceOnce attr_set;   // per instantiation
-  XB_SET_MAX_SMEM_ONCE(attr_set, SMEM_BUDGET + 6 * 1024, (const void*)gemm_umma_kernel<TOut, B_MN, Y_TMA>);
-  launch_dependent(gemm_umma_kernel<TOut, B_MN, Y_TMA>, grid, GEMM_THREADS, smem, s, ma, mb, my, p);
+  XB_SET_MAX_SMEM_ONCE(attr_set, SMEM_BUDGET + 6 * 1024, (const void*)gemm_umma_kernel<TOut, B_MN, Y>);
+  launch_dependent(gemm_umma_kernel<TOut, B_MN, Y>, grid, GEMM_THREADS, smem, s, ma, mb, my, p);
   return check_launch("gemm_umma_kernel");
 }
-template <typename TOut>
-int launch_umma_half(bool y_tma, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const UmmaGemmParams& p, dim3 grid,
-                     size_t smem, cudaStream_t s) {
-  if (p.b_mn) return y_tma ? launch_umma<TOut, true, true>(ma, mb, my, p, grid, smem, s) : launch_umma<TOut, true, false>(ma, mb, mb, p, grid, smem, s);
-  return y_tma ? launch_umma<TOut, false, true>(ma, mb, my, p, grid, smem, s) : launch_umma<TOut, false, false>(ma, mb, mb, p, grid, smem, s);
+template <typename TOut, bool B_MN>
+int launch_umma_half(int y, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const UmmaGemmParams& p, dim3 grid, size_t smem,
+                     cudaStream_t s) {
+  if (y == Y_TMA) return launch_umma<TOut, B_MN, Y_TMA>(ma, mb, my, p, grid, smem, s);
+  if (y == Y_PIECES) return launch_umma<TOut, B_MN, Y_PIECES>(ma, mb, mb, p, grid, smem, s);
+  return launch_umma<TOut, B_MN, Y_ANY>(ma, mb, mb, p, grid, smem, s);
 }
 
 void fill_umma_params(UmmaGemmParams& p, const xb_gemm_args& a) {
@@ -751,22 +766,26 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   p.tiles_n = (a.N + p.block_n - 1) / p.block_n;
   const int64_t total = (int64_t)p.tiles_m * p.tiles_n * p.batch;
   XB_REQUIRE(total < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)total);
-  // Results by TMA where a CTA has several tiles and rows of whole 16-byte pieces. (One tile is a chain of latencies that the copy
-  // lengthens: 2 x ([1862, 88] x [88, 24]) bf16 3.5 us, 3.9 by TMA; [1000, 88] x [88, 168] fp16 3.8 and 4.0.)
+  // Rows of whole, aligned 16-byte pieces, and no bias matrix; those by TMA where a CTA has several tiles. (One tile is a chain of
+  // latencies that the copy lengthens: 2 x ([1862, 88] x [88, 24]) bf16 3.5 us, 3.9 by TMA; [1000, 88] x [88, 168] fp16 3.8 and 4.0.)
+  const int64_t es = a.y_dtype == XB_F32 ? 4 : 2;
+  const bool pieces = p.bias_kind != XB_BIAS_FULL && (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0 && a.ldy * es % 16 == 0 &&
+                      (a.batch == 1 || a.stride_y * es % 16 == 0) && a.N * es % 16 == 0;
   const bool stacked = a.batch == 1 || a.stride_y >= (int64_t)a.M * a.ldy, beside = !stacked && a.stride_y >= a.N && a.stride_y * a.batch <= a.ldy;
-  bool y_tma = a.y_dtype != XB_F32 && total > sm_count() && p.bias_kind != XB_BIAS_FULL && (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0 &&
-                     a.ldy % 8 == 0 && a.N % 8 == 0 && (a.batch == 1 || a.stride_y % 8 == 0) && (stacked || beside);
+  int y = pieces ? Y_PIECES : Y_ANY;
   CUtensorMap my;
-  if (y_tma) {
+  if (pieces && es == 2 && total > sm_count() && (stacked || beside)) {
     // copies of 32 columns, 16 where the tile has few or where 32 would reach into the next tile
     p.y_unit = p.block_n >= 128 && (p.block_n % 32 == 0 || p.tiles_n == 1) ? 32 : 16;
     p.y_bufs = p.block_n > 4 * p.y_unit ? 2 : 1;
     p.y_beside = beside;
     const CUtensorMapSwizzle sw = p.y_unit == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
     const int bf = a.y_dtype == XB_BF16;
-    y_tma = 0 == (beside ? make_map(&my, a.Y, bf, a.N, a.batch, a.stride_y, a.M, a.ldy, 1, p.y_unit, sw, 32)
-                         : make_map(&my, a.Y, bf, a.N, a.M, a.ldy, a.batch, a.stride_y, 32, p.y_unit, sw));
-    if (y_tma) tail = 4 * 256 * (int)sizeof(float) + EPI_WARPS * p.y_bufs * p.y_unit * 64;
+    if (0 == (beside ? make_map(&my, a.Y, bf, a.N, a.batch, a.stride_y, a.M, a.ldy, 1, p.y_unit, sw, 32)
+                     : make_map(&my, a.Y, bf, a.N, a.M, a.ldy, a.batch, a.stride_y, 32, p.y_unit, sw))) {
+      y = Y_TMA;
+      tail = 4 * 256 * (int)sizeof(float) + EPI_WARPS * p.y_bufs * p.y_unit * 64;
+    }
   }
   // persistent: one CTA per SM walks the tiles; the accumulator is double-buffered in TMEM so the
   // epilogue of one tile overlaps the loads and MMAs of the next
@@ -796,9 +815,14 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
     smem = (size_t)p.stages * stage_bytes + tail + 1024;
   }
   switch (a.y_dtype) {
-    case XB_F16: return launch_umma_half<__half>(y_tma, ma, mb, my, p, grid, smem, stream);
-    case XB_BF16: return launch_umma_half<__nv_bfloat16>(y_tma, ma, mb, my, p, grid, smem, stream);
-    default: return launch_umma<float, false, false>(ma, mb, mb, p, grid, smem, stream);      // (never b_mn: umma_eligible)
+    case XB_F16:
+      return p.b_mn ? launch_umma_half<__half, true>(y, ma, mb, my, p, grid, smem, stream) : launch_umma_half<__half, false>(y, ma, mb, my, p, grid, smem, stream);
+    case XB_BF16:
+      return p.b_mn ? launch_umma_half<__nv_bfloat16, true>(y, ma, mb, my, p, grid, smem, stream)
+                    : launch_umma_half<__nv_bfloat16, false>(y, ma, mb, my, p, grid, smem, stream);
+    default:                                             // (never b_mn: umma_eligible)
+      return y == Y_PIECES ? launch_umma<float, false, Y_PIECES>(ma, mb, mb, p, grid, smem, stream)
+                           : launch_umma<float, false, Y_ANY>(ma, mb, mb, p, grid, smem, stream);
   }
 }
 
