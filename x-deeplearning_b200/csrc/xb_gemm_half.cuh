@@ -6,10 +6,9 @@
 // while this one is multiplied. fp32 accumulation; the outputs leave through shared memory, whole rows of 64.
 //
 // Bound by the issue of these narrow loads where the product is large, by the latency of the slices where it is small (up to K / 64
-// trips to memory one after the other). fp16, on the CUDA cores before and here: [30000, 500] x [500, 511] 1314 -> 140 us (rows of
-// A at 4-byte addresses, N = 512: 1312 -> 106), [30000, 313] x [313, 31] 91 -> 19, 16 x ([1617, 143] x [143, 66]) with Dice 81 -> 25,
-// 4 x ([9310, 29] x [29, 325]) with a sigmoid 132 -> 62, 4 x ([38, 374] x [374, 128]) 37 -> 8. One predicate an element on every
-// slice, where most need none, took 165 us of the first.
+// trips to memory one after the other). fp16, on the CUDA cores before and here: [30000, 500] x [500, 511] 1313 -> 145 us (rows of
+// A at 4-byte addresses, N = 512: 1313 -> 110), [30000, 313] x [313, 31] 91 -> 15, 8 x ([2254, 117] x [117, 144]) 70 -> 19,
+// 2 x ([47350, 28] x [28, 27]) bf16 with a sigmoid 31 -> 19 (31 before narrow rows shared a warp), 2 x ([2585, 67] x [67, 45]) 24 -> 7.
 #pragma once
 
 namespace xb {
@@ -34,17 +33,18 @@ __device__ __forceinline__ void mma_half(float (&c)[4], const uint32_t (&a)[4], 
 }
 
 // Blocks of `R` rows x 64 adjacent elements on their way to shared memory: warp w takes rows w, w + 8, ..., a lane elements 2 lane
-// and the next. Zero past `rows` and `ext`.
+// and the next. Zero past `rows` and `ext`. Where no more than 32 elements of a row are left, half a warp takes one (`narrow`; the
+// upper 32 columns in shared memory are then not written).
 template <int R>
 struct HalfSlice {
   uint32_t v[R / 8];
   // ALL: every element is there (what most slices of a large product are, and half the instructions)
-  template <bool ALL, bool EVEN>
-  __device__ __forceinline__ void fetch(const uint16_t* at, int64_t step, int rows, bool one, bool two) {
-    uint16_t lo[R / 8], hi[R / 8];
+  template <int PASS, bool ALL, bool EVEN>
+  __device__ __forceinline__ void fetch(const uint16_t* at, int64_t ld, int rows, bool one, bool two) {
+    uint16_t lo[R / PASS], hi[R / PASS];
 #pragma unroll
-    for (int i = 0; i < R / 8; ++i, at += step) {
-      const bool in = ALL || 8 * i < rows;
+    for (int i = 0; i < R / PASS; ++i, at += PASS * ld) {
+      const bool in = ALL || PASS * i < rows;
       if (EVEN) {
         v[i] = 0;
         if (ALL || (in && two)) v[i] = __ldg(reinterpret_cast<const uint32_t*>(at));
@@ -57,26 +57,36 @@ struct HalfSlice {
     }
     if (!EVEN) {
 #pragma unroll
-      for (int i = 0; i < R / 8; ++i) v[i] = (uint32_t)lo[i] | (uint32_t)hi[i] << 16;
+      for (int i = 0; i < R / PASS; ++i) v[i] = (uint32_t)lo[i] | (uint32_t)hi[i] << 16;
     }
   }
+  static __device__ __forceinline__ bool narrow(int c0, int ext) { return ext - c0 <= 32; }
   __device__ __forceinline__ void load(const uint16_t* base, int64_t ld, int row0, int rows, int c0, int ext, bool even) {
-    const int w = threadIdx.x >> 5, c = c0 + 2 * (threadIdx.x & 31);
+    const bool nar = narrow(c0, ext);
+    const int lane = threadIdx.x & 31, w = nar ? threadIdx.x >> 4 : threadIdx.x >> 5, c = c0 + 2 * (nar ? lane & 15 : lane);
     const bool one = c < ext, two = c + 1 < ext, all = row0 + R <= rows && c0 + 64 <= ext;
     const uint16_t* at = base + (int64_t)(row0 + w) * ld + c;
     const int left = rows - row0 - w;
     if (even) {
-      if (all) fetch<true, true>(at, 8 * ld, left, one, two);
-      else fetch<false, true>(at, 8 * ld, left, one, two);
+      if (all) fetch<8, true, true>(at, ld, left, one, two);
+      else if (nar) fetch<16, false, true>(at, ld, left, one, two);
+      else fetch<8, false, true>(at, ld, left, one, two);
     } else {
-      if (all) fetch<true, false>(at, 8 * ld, left, one, two);
-      else fetch<false, false>(at, 8 * ld, left, one, two);
+      if (all) fetch<8, true, false>(at, ld, left, one, two);
+      else if (nar) fetch<16, false, false>(at, ld, left, one, two);
+      else fetch<8, false, false>(at, ld, left, one, two);
     }
   }
-  __device__ __forceinline__ void store(uint16_t* s, int pitch) const {
+  __device__ __forceinline__ void store(uint16_t* s, int pitch, bool nar) const {
+    if (nar) {
 #pragma unroll
-    for (int i = 0; i < R / 8; ++i)
-      *reinterpret_cast<uint32_t*>(s + ((threadIdx.x >> 5) + 8 * i) * pitch + 2 * (threadIdx.x & 31)) = v[i];
+      for (int i = 0; i < R / 16; ++i)
+        *reinterpret_cast<uint32_t*>(s + ((threadIdx.x >> 4) + 16 * i) * pitch + 2 * (threadIdx.x & 15)) = v[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < R / 8; ++i)
+        *reinterpret_cast<uint32_t*>(s + ((threadIdx.x >> 5) + 8 * i) * pitch + 2 * (threadIdx.x & 31)) = v[i];
+    }
   }
 };
 
@@ -133,7 +143,8 @@ __global__ void __launch_bounds__(256, 2) gemm_half_kernel(const __grid_constant
     if constexpr (TB) sb.load(B, p.ldb, n0, p.N, k0, p.K, b_even);
     else sb.load(B, p.ldb, k0, p.K, n0, p.N, b_even);
   };
-  auto store = [&](const Slices& s) {
+  auto store = [&](const Slices& s, int kb) {
+    const int k0 = kb * HALF_BK;
     const HalfSlice<BM>& sa = s.a;
     const HalfSlice<64>& sb = s.b;
     if constexpr (TA) {
@@ -142,12 +153,12 @@ __global__ void __launch_bounds__(256, 2) gemm_half_kernel(const __grid_constant
         HalfSlice<64> t;
 #pragma unroll
         for (int i = 0; i < 8; ++i) t.v[i] = sa.v[8 * h + i];
-        t.store(As + 64 * h, APITCH);
+        t.store(As + 64 * h, APITCH, HalfSlice<64>::narrow(m0 + 64 * h, p.M));
       }
     } else {
-      sa.store(As, APITCH);
+      sa.store(As, APITCH, HalfSlice<BM>::narrow(k0, p.K));
     }
-    sb.store(Bs, HALF_PITCH);
+    sb.store(Bs, HALF_PITCH, HalfSlice<64>::narrow(TB ? k0 : n0, TB ? p.K : p.N));
   };
 
   const int wm = BM == 128 ? (warp >> 1) * 32 : (warp >> 2) * 32, wn = BM == 128 ? (warp & 1) * WN : (warp & 3) * WN;
@@ -174,11 +185,13 @@ __global__ void __launch_bounds__(256, 2) gemm_half_kernel(const __grid_constant
     for (int u = 0; u < AHEAD; ++u) {
       const int kb = kb0 + u;
       if (kb >= nk) break;                                      // (the same for every thread)
-      store(on_way[u]);
+      store(on_way[u], kb);
       __syncthreads();
       if (kb + AHEAD < nk) load(on_way[u], kb + AHEAD);
+      const int depth = min(HALF_BK, p.K - kb * HALF_BK);       // (zeros up to a multiple of 16)
 #pragma unroll
       for (int k = 0; k < HALF_BK; k += 16) {
+        if (k >= depth) break;
         uint32_t af[2][4], bf[NF / 2][4];
 #pragma unroll
         for (int i = 0; i < 2; ++i) ldmatrix4<TA>(af[i], a_at + 2 * (TA ? k * APITCH + 16 * i : 16 * i * APITCH + k));
@@ -204,14 +217,15 @@ __global__ void __launch_bounds__(256, 2) gemm_half_kernel(const __grid_constant
         *reinterpret_cast<float2*>(out + (wm + 16 * i + 8 * h + (lane >> 2)) * HALF_OPITCH + wn + 8 * j + 2 * (lane & 3)) =
             make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
   __syncthreads();
-  // a thread keeps its two columns and takes every eighth row
-  const int gn = n0 + 2 * lane;
+  // a thread keeps its two columns and takes every eighth row (every sixteenth of up to 32 columns)
+  const bool nar = p.N - n0 <= 32;
+  const int cl = 2 * (nar ? lane & 15 : lane), gn = n0 + cl, step = nar ? 16 : 8;
   if (gn >= p.N) return;
   const bool two = gn + 1 < p.N;
   const Column c0 = column_of(p, b, gn), c1 = column_of(p, b, two ? gn + 1 : gn);
 #pragma unroll 4
-  for (int r = warp; r < BM && m0 + r < p.M; r += 8) {
-    const float2 x = *reinterpret_cast<const float2*>(out + r * HALF_OPITCH + 2 * lane);
+  for (int r = nar ? threadIdx.x >> 4 : warp; r < BM && m0 + r < p.M; r += step) {
+    const float2 x = *reinterpret_cast<const float2*>(out + r * HALF_OPITCH + cl);
     const float v0 = half_finish(p, c0, b, m0 + r, gn, x.x), v1 = two ? half_finish(p, c1, b, m0 + r, gn + 1, x.y) : 0.f;
     const int64_t at = (int64_t)b * p.stride_y + (int64_t)(m0 + r) * p.ldy + gn;
     if (p.y_pairs && two) {
