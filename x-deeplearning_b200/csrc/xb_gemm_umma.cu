@@ -262,6 +262,16 @@ __device__ __forceinline__ void epi_unit(uint32_t tmem_at, float alpha, const fl
   }
 }
 
+template <typename F>
+__device__ __forceinline__ void with_kind(int kind, F f) {
+  switch (kind) {
+    case XB_EPI_PRELU: f(std::integral_constant<int, XB_EPI_PRELU>()); break;
+    case XB_EPI_DICE: f(std::integral_constant<int, XB_EPI_DICE>()); break;
+    case XB_EPI_SIGMOID: f(std::integral_constant<int, XB_EPI_SIGMOID>()); break;
+    default: f(std::integral_constant<int, XB_EPI_NONE>()); break;
+  }
+}
+
 // Epilogue of a tile whose results leave by TMA, a warp's 32 rows x W columns at a time: units `part`, `part` + 4, ... of the tile.
 // A warp with two units a tile has two areas, so that it fills one while the other is read. What the threads' own stores and their
 // reads of the staging area took of the data path (4900 wavefronts a tile of 128 x 256, 5000 cycles) is the copy engine's work here.
@@ -561,19 +571,13 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const uint32_t tmem_acc = tmem_base + as * acc_stride + ((uint32_t)(q * 32) << 16);
       if constexpr (Y == Y_TMA) {
         const int y = m0 + q * 32, cols = min(p.block_n, p.N - n0), y1 = p.y_beside ? b : y, y2 = p.y_beside ? y : b;
-        auto tile_out = [&](auto kind) {
+        with_kind(p.epi.kind, [&](auto kind) {
           constexpr int KIND = decltype(kind)::value;
           if (p.y_unit == 32)
             epi_tile_tma<TOut, KIND, 32>(map_y, tmem_acc, part, cols, p.alpha, s_bias, s_a, s_b, s_c, area, p.y_bufs, turn, n0, y1, y2, y < p.M, lane);
           else
             epi_tile_tma<TOut, KIND, 16>(map_y, tmem_acc, part, cols, p.alpha, s_bias, s_a, s_b, s_c, area, p.y_bufs, turn, n0, y1, y2, y < p.M, lane);
-        };
-        switch (p.epi.kind) {
-          case XB_EPI_PRELU: tile_out(std::integral_constant<int, XB_EPI_PRELU>()); break;
-          case XB_EPI_DICE: tile_out(std::integral_constant<int, XB_EPI_DICE>()); break;
-          case XB_EPI_SIGMOID: tile_out(std::integral_constant<int, XB_EPI_SIGMOID>()); break;
-          default: tile_out(std::integral_constant<int, XB_EPI_NONE>()); break;
-        }
+        });
       } else {
         TOut* yrow = reinterpret_cast<TOut*>(p.Y) + (int64_t)b * p.stride_y + (int64_t)gm * p.ldy;
         if constexpr (Y == Y_ANY) {
@@ -582,16 +586,9 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                               reinterpret_cast<uint16_t*>(stage), lane);
         } else {
           const int rows = p.M - (m0 + q * 32), cols = p.N - n0;
-          switch (p.epi.kind) {
-            case XB_EPI_PRELU:
-              epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
-            case XB_EPI_DICE:
-              epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
-            case XB_EPI_SIGMOID:
-              epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
-            default:
-              epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane); break;
-          }
+          with_kind(p.epi.kind, [&](auto kind) {
+            epi_tile_fast<TOut, decltype(kind)::value>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow + n0, p.ldy, rows, cols, stage, lane);
+          });
         }
       }
       tc_fence_before_sync();
@@ -709,6 +706,17 @@ void fill_umma_params(UmmaGemmParams& p, const xb_gemm_args& a) {
   p.idesc = umma::make_idesc(BLOCK_M, p.block_n, a.ab_dtype == XB_BF16) | (p.b_mn ? umma::IDESC_B_MN : 0u);
 }
 
+// Where the batches of Y lie: one after the other, or beside one another in its rows (an axis-1 concat).
+bool y_stacked(const xb_gemm_args& a) { return a.batch == 1 || a.stride_y >= (int64_t)a.M * a.ldy; }
+bool y_beside(const xb_gemm_args& a) { return !y_stacked(a) && a.stride_y >= a.N && a.stride_y * a.batch <= a.ldy; }
+// map of a two-byte Y for copies of 32 rows x `unit` columns
+int make_y_map(CUtensorMap* map, const xb_gemm_args& a, int unit) {
+  const CUtensorMapSwizzle sw = unit == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+  const int bf = a.y_dtype == XB_BF16;
+  return y_beside(a) ? make_map(map, a.Y, bf, a.N, a.batch, a.stride_y, a.M, a.ldy, 1, unit, sw, 32)
+                     : make_map(map, a.Y, bf, a.N, a.M, a.ldy, a.batch, a.stride_y, 32, unit, sw);
+}
+
 // Two-CTA tiles where they fill the chip (a 256 x 256 tile for every pair of SMs) and the epilogue is the plain one: whole
 // 256-column tiles, aligned output rows, no bias matrix. Below that the one-CTA kernel spreads the work over more SMs.
 // [65536, 1280] x [1280, 1024] and the two layers after it (bf16): 207 us as pairs, 290 one CTA at a time.
@@ -716,7 +724,7 @@ bool pair_wanted(const xb_gemm_args& a) {
   const int64_t es = a.y_dtype == XB_F32 ? 4 : 2;
   return a.trans_b && a.N % 256 == 0 && a.K >= 256 && !(a.bias && a.bias_kind == XB_BIAS_FULL) &&
          (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0 && (a.ldy * es) % 16 == 0 && (a.stride_y * es) % 16 == 0 &&
-         ((int64_t)a.M + 255) / 256 * (a.N / 256) * a.batch >= sm_count() / 2;
+         ((int64_t)a.M + 255) / 256 * (a.N / 256) * a.batch >= sm_count() / 2 && (es == 4 || y_stacked(a) || y_beside(a));
 }
 
 }  // namespace
@@ -728,10 +736,11 @@ namespace xb {
 namespace {
 
 template <typename TOut>
-int launch_umma_pair(const CUtensorMap& ma, const CUtensorMap& mb, const UmmaGemmParams& p, dim3 grid, size_t smem, cudaStream_t s) {
+int launch_umma_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& my, const UmmaGemmParams& p, dim3 grid, size_t smem,
+                     cudaStream_t s) {
   static PerDeviceOnce attr_set;   // per instantiation
   XB_SET_MAX_SMEM_ONCE(attr_set, 226 * 1024, (const void*)gemm_umma_pair_kernel<TOut>);
-  launch_dependent(gemm_umma_pair_kernel<TOut>, grid, GEMM_THREADS, smem, s, ma, mb, p);
+  launch_dependent(gemm_umma_pair_kernel<TOut>, grid, GEMM_THREADS, smem, s, ma, mb, my, p);
   return check_launch("gemm_umma_pair_kernel");
 }
 
@@ -739,11 +748,13 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   UmmaGemmParams p;
   fill_umma_params(p, a);
   const int is_bf16 = a.ab_dtype == XB_BF16;
-  CUtensorMap ma, mb;
+  CUtensorMap ma, mb, my;
   if (int rc = make_map(&ma, a.A, is_bf16, a.K, a.M, a.lda, p.a_batched ? a.batch : 1, a.stride_a, BLOCK_M)) return rc;
   // after the ring: per-column epilogue parameters [4][256] fp32, then the epilogue warps' staging areas
   int tail = 4 * 256 * (int)sizeof(float) + (a.y_dtype == XB_F32 ? 0 : EPI_WARPS * EPI_STAGE_BYTES);
-  if (pair_wanted(a)) {
+  if (pair_wanted(a) && (a.y_dtype == XB_F32 || make_y_map(&my, a, 32) == 0)) {
+    p.y_unit = 32; p.y_bufs = PAIR_Y_BUFS; p.y_beside = y_beside(a);
+    tail = 4 * 256 * (int)sizeof(float) + (a.y_dtype == XB_F32 ? 0 : EPI_WARPS * PAIR_Y_BUFS * 32 * 64);
     if (int rc = make_map(&mb, a.B, is_bf16, a.K, a.N, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, PAIR_N / 2)) return rc;
     p.tiles_m = (a.M + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
     p.tiles_n = a.N / PAIR_N;
@@ -754,9 +765,9 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
     XB_REQUIRE(total < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)total);
     const dim3 grid(2 * (unsigned)std::min<int64_t>(total, sm_count() / 2));
     switch (a.y_dtype) {
-      case XB_F16: return launch_umma_pair<__half>(ma, mb, p, grid, smem, stream);
-      case XB_BF16: return launch_umma_pair<__nv_bfloat16>(ma, mb, p, grid, smem, stream);
-      default: return launch_umma_pair<float>(ma, mb, p, grid, smem, stream);
+      case XB_F16: return launch_umma_pair<__half>(ma, mb, my, p, grid, smem, stream);
+      case XB_BF16: return launch_umma_pair<__nv_bfloat16>(ma, mb, my, p, grid, smem, stream);
+      default: return launch_umma_pair<float>(ma, mb, mb, p, grid, smem, stream);
     }
   }
   if (int rc = p.b_mn ? make_map(&mb, a.B, is_bf16, a.N, a.K, a.ldb, p.b_batched ? a.batch : 1, a.stride_b, BLOCK_K)
@@ -771,18 +782,13 @@ int gemm_umma(const xb_gemm_args& a, cudaStream_t stream) {
   const int64_t es = a.y_dtype == XB_F32 ? 4 : 2;
   const bool pieces = p.bias_kind != XB_BIAS_FULL && (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0 && a.ldy * es % 16 == 0 &&
                       (a.batch == 1 || a.stride_y * es % 16 == 0) && a.N * es % 16 == 0;
-  const bool stacked = a.batch == 1 || a.stride_y >= (int64_t)a.M * a.ldy, beside = !stacked && a.stride_y >= a.N && a.stride_y * a.batch <= a.ldy;
   int y = pieces ? Y_PIECES : Y_ANY;
-  CUtensorMap my;
-  if (pieces && es == 2 && total > sm_count() && (stacked || beside)) {
+  if (pieces && es == 2 && total > sm_count() && (y_stacked(a) || y_beside(a))) {
     // copies of 32 columns, 16 where the tile has few or where 32 would reach into the next tile
     p.y_unit = p.block_n >= 128 && (p.block_n % 32 == 0 || p.tiles_n == 1) ? 32 : 16;
     p.y_bufs = p.block_n > 4 * p.y_unit ? 2 : 1;
-    p.y_beside = beside;
-    const CUtensorMapSwizzle sw = p.y_unit == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
-    const int bf = a.y_dtype == XB_BF16;
-    if (0 == (beside ? make_map(&my, a.Y, bf, a.N, a.batch, a.stride_y, a.M, a.ldy, 1, p.y_unit, sw, 32)
-                     : make_map(&my, a.Y, bf, a.N, a.M, a.ldy, a.batch, a.stride_y, 32, p.y_unit, sw))) {
+    p.y_beside = y_beside(a);
+    if (make_y_map(&my, a, p.y_unit) == 0) {
       y = Y_TMA;
       tail = 4 * 256 * (int)sizeof(float) + EPI_WARPS * p.y_bufs * p.y_unit * 64;
     }

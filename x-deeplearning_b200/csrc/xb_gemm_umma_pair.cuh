@@ -8,6 +8,9 @@
 // both halves. Each CTA keeps the accumulator of its own 128 rows in its tensor memory, so the epilogue is that of the
 // one-CTA kernel. Each CTA loads what it needs itself; nothing is multicast but the arrivals of tcgen05.commit.
 // [65536, 1280] x [1280, 1024] bf16 + bias + PReLU and the 1024-512-256 layers after it: 207 us, 290 with one CTA a tile.
+// Results leave by TMA (two-byte ones), which the epilogue of a layer with K <= 640 waited for: those three layers and the last one
+// 226 -> 219 us, 640-512-256-1 on 65536 rows 81 -> 74, [65536, 256] x [256, 256] 22.4 -> 19.3. One staging area a warp: a second costs
+// a stage of the ring (235, 78 and 19.9 us).
 #pragma once
 
 namespace xb {
@@ -17,6 +20,7 @@ constexpr int PAIR_N = 256;                         // columns of a tile; rows: 
 constexpr int PAIR_B_BYTES = (PAIR_N / 2) * BLOCK_K * 2;
 constexpr int PAIR_STAGE_BYTES = A_STAGE_BYTES + PAIR_B_BYTES;
 constexpr int PAIR_MAX_STAGES = 6;
+constexpr int PAIR_Y_BUFS = 1;                      // staging areas of an epilogue warp
 
 // TMA tile load into this CTA that signals a barrier of the pair's leader
 __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int c0, int c1, int c2) {
@@ -45,7 +49,7 @@ __device__ __forceinline__ void mma_commit_pair_elect(uint32_t bar) {
 
 template <typename TOut>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
-gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_y,
                       const __grid_constant__ UmmaGemmParams p) {
   using namespace umma;
   extern __shared__ uint8_t smem_raw[];
@@ -77,6 +81,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     for (int s = 0; s < STAGES; ++s) { mbar_init(smem_u32(&full_bar[s]), 1); mbar_init(smem_u32(&empty_bar[s]), 1); }
     for (int s = 0; s < 2; ++s) { mbar_init(smem_u32(&acc_full[s]), 1); mbar_init(smem_u32(&acc_empty[s]), 2 * EPI_WARPS); }
     fence_barrier_init();
+    if (sizeof(TOut) == 2) prefetch_tensormap(&map_y);
     prefetch_tensormap(&map_a);
     prefetch_tensormap(&map_b);
   }
@@ -138,9 +143,10 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
   } else {
     const int ew = warp - 2, q = warp & 3, part = ew >> 2, row = q * 32 + lane;
-    const int c_begin = PAIR_N / 16 * part / 4, c_end = PAIR_N / 16 * (part + 1) / 4;
+    [[maybe_unused]] const int c_begin = PAIR_N / 16 * part / 4, c_end = PAIR_N / 16 * (part + 1) / 4;
     float* s_bias = reinterpret_cast<float*>(smem + STAGES * PAIR_STAGE_BYTES);                    // [4][256]
-    uint4* stage = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s_bias + 4 * 256) + ew * EPI_STAGE_BYTES);
+    uint8_t* area = reinterpret_cast<uint8_t*>(s_bias + 4 * 256) + ew * PAIR_Y_BUFS * 32 * 64;
+    uint32_t turn = 0;
     float *s_a = s_bias + 256, *s_b = s_a + 256, *s_c = s_b + 256;
     int it = 0, cur_n0 = -1, cur_b = -1;
     bool ok = true;
@@ -160,19 +166,21 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       if (!ok) continue;
       tc_fence_after_sync();
       const uint32_t tmem_acc = tmem_base + as * PAIR_N + ((uint32_t)(q * 32) << 16);
-      TOut* yrow = reinterpret_cast<TOut*>(p.Y) + (int64_t)b * p.stride_y + (int64_t)gm * p.ldy;
-      const int rows = p.M - (m0 + q * 32);                        // of the warp's 32; the columns are all there
-      yrow += n0;
-      switch (p.epi.kind) {
-        case XB_EPI_PRELU: epi_tile_fast<TOut, XB_EPI_PRELU>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
-        case XB_EPI_DICE: epi_tile_fast<TOut, XB_EPI_DICE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
-        case XB_EPI_SIGMOID: epi_tile_fast<TOut, XB_EPI_SIGMOID>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
-        default: epi_tile_fast<TOut, XB_EPI_NONE>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c, yrow, p.ldy, rows, PAIR_N, stage, lane); break;
-      }
+      const int y = m0 + q * 32, rows = p.M - y;                   // of the warp's 32; the columns are all there
+      with_kind(p.epi.kind, [&](auto kind) {
+        constexpr int KIND = decltype(kind)::value;
+        if constexpr (sizeof(TOut) == 2)
+          epi_tile_tma<TOut, KIND, 32>(map_y, tmem_acc, part, PAIR_N, p.alpha, s_bias, s_a, s_b, s_c, area, PAIR_Y_BUFS, turn, n0,
+                                       p.y_beside ? b : y, p.y_beside ? y : b, rows > 0, lane);
+        else
+          epi_tile_fast<TOut, KIND>(tmem_acc, c_begin, c_end, p.alpha, s_bias, s_a, s_b, s_c,
+                                    reinterpret_cast<TOut*>(p.Y) + (int64_t)b * p.stride_y + (int64_t)gm * p.ldy + n0, p.ldy, rows, PAIR_N, nullptr, lane);
+      });
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(smem_u32(&acc_empty[as]), 0);
     }
+    if (sizeof(TOut) == 2 && lane == 0) tma_store_wait_read<0>();
   }
 
   pdl_release();
