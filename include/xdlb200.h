@@ -289,7 +289,8 @@ int xb_sharded_pool(xb_shard_ctx* ctx, const int64_t* ids, const int32_t* seg_of
  * xb_sharded_pool_finish takes the oldest begun step, makes `stream` wait for that exchange and enqueues the rest.
  * At most two steps may be begun and not finished; every rank must issue begin and finish calls in the same order
  * (exchanges of one communicator run in issue order); the id and offset arrays of a begun step stay untouched
- * until its work has run. xb_sharded_pool is begin followed by finish on one stream. */
+ * until its work has run. xb_sharded_pool is begin followed by finish on one stream; where one rank holds the whole tables it
+ * pools the caller's lists in place, with the same results. */
 int xb_sharded_pool_begin(xb_shard_ctx* ctx, const int64_t* ids, const int32_t* seg_offsets, int64_t n_ids, xb_stream_t stream);
 int xb_sharded_pool_finish(xb_shard_ctx* ctx, int64_t groups, int32_t avg, void* out, int64_t out_stride, int32_t out_dtype,
                            xb_stream_t stream);

@@ -64,3 +64,27 @@ def test_ragged_outputs(N, M, beside, dtype, out):
         assert (Y[M:] == 9.0).all() and (Y[:, P * N:] == 9.0).all()
     else:
         assert (Y[P * M:] == 9.0).all() and (Y[:, N:] == 9.0).all()
+
+
+@pytest.mark.parametrize("M,N,K,P,beside", [(9700, 512, 392, 1, False), (9700, 256, 640, 2, True), (4990, 512, 384, 2, False), (18945, 256, 400, 1, False)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_two_cta_tiles_end_anywhere(M, N, K, P, beside, dtype):
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    A, B, bias = r(P, M, K).to(dtype), (r(P, N, K) / K ** 0.5).to(dtype), r(P, N)
+    slope = torch.rand((P, N), generator=g, device="cuda")
+    ld = N * P + 16 if beside else N + 8
+    Y = torch.full((M + 1, ld) if beside else (P * M + 1, ld), 9.0, dtype=dtype, device="cuda")
+    ops.gemm(A, B, Y=Y, bias=bias, bias_kind=capi.XB_BIAS_ROW, trans_b=True, batch=P, M=M, N=N, K=K, lda=K, ldb=K, ldy=ld,
+             strides=(M * K, N * K, N, N if beside else M * ld), epilogue=capi.XB_EPI_PRELU, ep=(slope, None, None), ep_count=N, stride_ep=N)
+    x = A.double() @ B.double().transpose(1, 2) + bias.double()[:, None]
+    mag = A.double().abs() @ B.double().abs().transpose(1, 2) + bias.double().abs()[:, None]
+    want = torch.where(x < 0, x * slope.double()[:, None], x)
+    got = Y[:M, :P * N].view(M, P, N).transpose(0, 1) if beside else Y[:P * M].view(P, M, ld)[:, :, :N]
+    eps = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    assert ((got.double() - want).abs() <= 2 * (K + 2) * 2.0 ** -24 * mag + eps * want.abs() + (2.0 ** -25 if dtype == torch.float16 else 0)).all()
+    if beside:
+        assert (Y[M:] == 9.0).all() and (Y[:, P * N:] == 9.0).all()
+    else:
+        assert (Y[P * M:] == 9.0).all() and (Y[:, N:] == 9.0).all()

@@ -719,10 +719,12 @@ int make_y_map(CUtensorMap* map, const xb_gemm_args& a, int unit) {
 
 // Two-CTA tiles where they fill the chip (a 256 x 256 tile for every pair of SMs) and the epilogue is the plain one: whole
 // 256-column tiles, aligned output rows, no bias matrix. Below that the one-CTA kernel spreads the work over more SMs.
-// [65536, 1280] x [1280, 1024] and the two layers after it (bf16): 207 us as pairs, 290 one CTA at a time.
+// [65536, 1280] x [1280, 1024] and the two layers after it (bf16): 207 us as pairs, 290 one CTA at a time. Less depth than 384 is
+// an epilogue with a few MMAs beside it, and the one-CTA kernel has two staging areas a warp (65536 rows, N = 512: K = 256 26.8 us,
+// 31.3 as pairs; 320 29.9, 33.7; 384 33.4, 35.1; 448 37.3, 36.3; 640 48.9, 44.0. 20000 rows: 13.5, 13.9; 14.9, 14.8; 16.3, 15.4).
 bool pair_wanted(const xb_gemm_args& a) {
   const int64_t es = a.y_dtype == XB_F32 ? 4 : 2;
-  return a.trans_b && a.N % 256 == 0 && a.K >= 256 && !(a.bias && a.bias_kind == XB_BIAS_FULL) &&
+  return a.trans_b && a.N % 256 == 0 && a.K >= (es == 4 ? 256 : 384) && !(a.bias && a.bias_kind == XB_BIAS_FULL) &&
          (reinterpret_cast<uintptr_t>(a.Y) & 15) == 0 && (a.ldy * es) % 16 == 0 && (a.stride_y * es) % 16 == 0 &&
          ((int64_t)a.M + 255) / 256 * (a.N / 256) * a.batch >= sm_count() / 2 && (es == 4 || y_stacked(a) || y_beside(a));
 }
