@@ -525,6 +525,10 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
   pdl_begin();
   constexpr int EPC = TD == XB_F32 ? 4 : 8;          // elements per 16-byte chunk
   constexpr int RB = LPR < 4 ? LPR : 4;              // row loads in flight per lane
+  // A list's next ids are requested with the rows of these: 20 groups of 512 lists of 25.5 ids over 1 M x 16 fp32 10.9 -> 10.1 us,
+  // of 50 ids 14.7 -> 13.9, 33 groups of 66 lists of 33 ids over 64 fp16 columns through an index 16.3 -> 15.2. Eight lanes a row of
+  // fp32 have no registers left for it (64 bytes spilled; 7 groups of 1543 lists of one id 5.25 -> 5.66 us).
+  constexpr bool KEYS_AHEAD = !(TD == XB_F32 && LPR == 8);
   constexpr unsigned FULL = 0xffffffffu;
   const int64_t warp_id = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (warp_id >= p.total_warps) return;              // whole warp leaves together
@@ -580,19 +584,28 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
     }
     st = sum + incl - nm;
   };
-  // one id, value and table row number per lane: position base + tlane of the segment
-  auto load_ids = [&](int st, int nm, int base, int& row, float& v) {
+  // one id and value per lane, position base + tlane of the segment; its table row (-1: past the segment's end, or missing) is
+  // looked up where it is needed, so that a list's next ids are on their way while the rows of these are
+  auto load_keys = [&](int st, int nm, int base, int64_t& key, float& v) {
     const int idx = base + tlane;
-    row = -1; v = 1.f;
+    key = 0; v = 1.f;
     if (idx < nm) {
       const int64_t at = (int64_t)st + idx;
-      int64_t key = id64 ? (int64_t)__ldcs(reinterpret_cast<const long long*>(g.ids) + at)
-                         : (int64_t)__ldcs(reinterpret_cast<const int32_t*>(g.ids) + at);
-      if (rec) key &= 0xffffffffll;
-      if (has_table) row = (int)lookup_row(g, key);
+      key = id64 ? (int64_t)__ldcs(reinterpret_cast<const long long*>(g.ids) + at)
+                 : (int64_t)__ldcs(reinterpret_cast<const int32_t*>(g.ids) + at);
       if (vmode == 1) v = __ldcs(reinterpret_cast<const float*>(g.values) + at);
       else if (vmode == 2) v = __half2float(reinterpret_cast<const __half*>(g.values)[at]);
     }
+  };
+  auto row_of = [&](int nm, int base, int64_t key) {
+    if (base + tlane >= nm || !has_table) return -1;
+    if (rec) key &= 0xffffffffll;
+    return (int)lookup_row(g, key);
+  };
+  auto load_ids = [&](int st, int nm, int base, int& row, float& v) {
+    int64_t key;
+    load_keys(st, nm, base, key, v);
+    row = row_of(nm, base, key);
   };
 
   int st0, nm0, st1, nm1, st2, nm2, row, row_next;
@@ -617,8 +630,13 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
 #pragma unroll
     for (int e = 0; e < EPC; ++e) acc[e] = 0.f;
 
+    int64_t key = 0;
+    float key_v = 1.f;
     for (int base = 0; __any_sync(FULL, base < num); base += tl) {
-      if (base > 0) load_ids(start, num, base, row, v);
+      if (base > 0) {
+        if (KEYS_AHEAD) { row = row_of(num, base, key); v = key_v; }
+        else load_ids(start, num, base, row, v);
+      }
 #pragma unroll
       for (int r0 = 0; r0 < LPR; r0 += RB) {
         if (r0 > 0 && !__any_sync(FULL, base + r0 * ns < num)) break;      // no team has ids left in this batch
@@ -636,6 +654,7 @@ __global__ void __launch_bounds__(256, 4) pool_fast_kernel(const __grid_constant
           raw[u] = make_uint4(0, 0, 0, 0);
           if (rr[u] >= 0 && cvalid) raw[u] = ld_row16(wrow + (int64_t)rr[u] * pitch, keep);
         }
+        if (KEYS_AHEAD && r0 == 0) load_keys(start, num, base + tl, key, key_v);
 #pragma unroll
         for (int u = 0; u < RB; ++u) {
           float w[8];
