@@ -748,7 +748,7 @@ def bench_dien(reps=20, R=74):
     return {"ms_per_step": ms, "requests_per_step": R, "candidates_per_request": N_CAND, "T": T_STEPS,
             "predictions_per_s": R * N_CAND / (ms * 1e-3),
             "path": "pooling, xb_gru, attention scores (sigmoid, softmax over steps), xb_augru_shared (tcgen05), "
-                    "tower GEMMs with PReLU epilogues"}
+                    "fused tower with PReLU"}
 
 
 def run_micro(args):
