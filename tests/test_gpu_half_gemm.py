@@ -71,3 +71,23 @@ def test_zero_depth_is_the_bias():
     Y = ops.gemm(torch.empty((40, 1), dtype=torch.float16, device="cuda"), torch.empty((1, 70), dtype=torch.float16, device="cuda"), bias=bias,
                  bias_kind=capi.XB_BIAS_ROW, M=40, N=70, K=0, lda=1, ldb=70)
     assert torch.equal(Y, bias.half().expand(40, 70))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 8, 8), (3, 2, 17), (1, 5, 64), (2, 16, 65), (16, 1, 200), (127, 3, 8)])
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_smallest_aligned_products(M, N, K, trans_b, dtype):
+    """(rows at 16-byte addresses: the tensor-memory path from one output on)"""
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(K)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    up = lambda n: (n + 7) // 8 * 8
+    A, B = r(2, M, up(K)).to(dtype), r(2, *((N, up(K)) if trans_b else (K, up(N)))).to(dtype)
+    Y = torch.full((2, M, N + 1), 9.0, dtype=dtype, device="cuda")
+    ops.gemm(A, B, Y=Y, trans_b=trans_b, batch=2, M=M, N=N, K=K, lda=up(K), ldb=B.shape[-1], ldy=N + 1,
+             strides=(M * up(K), B[0].numel(), 0, M * (N + 1)))
+    a = A[:, :, :K].double()
+    w = B[:, :, :K].double().transpose(1, 2) if trans_b else B[:, :, :N].double()
+    eps, tiny = (2.0 ** -11, 2.0 ** -25) if dtype == torch.float16 else (2.0 ** -8, 0.0)
+    assert ((Y[:, :, :N].double() - a @ w).abs() <= 2 * (K + 2) * 2.0 ** -24 * (a.abs() @ w.abs()) + eps * (a @ w).abs() + tiny).all()
+    assert (Y[:, :, N] == 9.0).all()
