@@ -88,3 +88,27 @@ def test_two_cta_tiles_end_anywhere(M, N, K, P, beside, dtype):
         assert (Y[M:] == 9.0).all() and (Y[:, P * N:] == 9.0).all()
     else:
         assert (Y[P * M:] == 9.0).all() and (Y[:, N:] == 9.0).all()
+
+
+@pytest.mark.parametrize("N", [80, 104, 160, 200, 256, 272])
+@pytest.mark.parametrize("M,P,K", [(289, 500, 8), (289, 500, 24), (545, 300, 24), (130, 800, 16)])
+def test_ragged_tiles_between_whole_ones(N, M, P, K):
+    """Ten and more tiles a block, every third or fifth of them with warps whose rows all lie past the output, stores that the copies
+    queue behind: each launch has the bits that the batches have one at a time (one tile a block, stored by the threads)."""
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    A, B, bias = r(P, M, K).half(), (r(P, N, K) / K ** 0.5).half(), r(P, N)
+    one = torch.empty((P, M, N), dtype=torch.float16, device="cuda")
+    for b in range(P):
+        ops.gemm(A[b], B[b], Y=one[b], bias=bias[b], trans_b=True)
+    many = [torch.full((P, M, N), 9.0, dtype=torch.float16, device="cuda") for _ in range(4)]
+    for Y in many:
+        ops.gemm(A, B, Y=Y, bias=bias, bias_kind=capi.XB_BIAS_ROW, trans_b=True, batch=P, M=M, N=N, K=K, lda=K, ldb=K, ldy=N,
+                 strides=(M * K, N * K, N, M * N))
+    for Y in many:
+        assert torch.equal(Y, one)
+    x = A.double() @ B.double().transpose(1, 2) + bias.double()[:, None]
+    mag = A.double().abs() @ B.double().abs().transpose(1, 2) + bias.double().abs()[:, None]
+    # fp32 sums of K products, not every one rounded, and the result's rounding
+    assert ((one.double() - x).abs() <= 2 * (K + 2) * 2.0 ** -24 * mag + 2.0 ** -11 * x.abs() + 2.0 ** -25).all()

@@ -277,11 +277,15 @@ __device__ __forceinline__ void with_kind(int kind, F f) {
 // reads of the staging area took of the data path (4900 wavefronts a tile of 128 x 256, 5000 cycles) is the copy engine's work here.
 // [65536, 88] x [88, 256] fp16: 16.1 -> 11.8 us, N = 192 14.4 -> 10.5, 8 x ([4096, 256] x [256, 128]) side by side 8.3 -> 7.9,
 // 8 x ([33434, 88] x [88, 32]) with a sigmoid 24.2 -> 22.5.
+// A turn is a copy: the wait counts committed groups, so a warp whose rows all lie past the output (`rows` false) takes no turn and
+// leaves the areas as they are. (With turns that commit nothing, the wait for all but the latest copy would name the copy of the other
+// area, and a later unit could overwrite what that copy still reads.)
 template <typename TOut, int KIND, int W>
 __device__ __forceinline__ void epi_tile_tma(const CUtensorMap& map_y, uint32_t tmem_row, int part, int cols, float alpha, const float* s_bias,
                                              const float* s_a, const float* s_b, const float* s_c, uint8_t* stage, int bufs, uint32_t& turn,
                                              int x, int y, int z, bool rows, int lane) {
   using namespace umma;
+  if (!rows) return;                                         // (the same for the warp)
   for (int c = part * W; c < cols; c += 4 * W) {
     uint8_t* area = stage + (bufs == 2 ? (turn & 1u) * (32 * W * 2) : 0u);
     ++turn;
@@ -293,7 +297,7 @@ __device__ __forceinline__ void epi_tile_tma(const CUtensorMap& map_y, uint32_t 
     epi_unit<TOut, KIND, W>(tmem_row + (uint32_t)c, alpha, s_bias + c, s_a + c, s_b + c, s_c + c, reinterpret_cast<uint4*>(area), lane);
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0 && rows) tma_store_3d(&map_y, smem_u32(area), x + c, y, z);
+    if (lane == 0) tma_store_3d(&map_y, smem_u32(area), x + c, y, z);
   }
 }
 
