@@ -84,3 +84,19 @@ def test_augru_tcgen05_engine_declines_shapes_without_selector_slots():
     rc = L.xb_augru_shared(ops.ptr(z), ops.ptr(z), ops.ptr(z), 1, 4, 3, 32, ops.ptr(z), ops.ptr(z), ops.ptr(z), ops.ptr(z),
                            capi.XB_GEMM_TCGEN05, ops.stream())
     assert rc == -2 and b"tcgen05 engine" in L.xb_last_error()
+
+
+@pytest.mark.parametrize("B,T,H", [(8, 100, 36), (5, 70, 64), (40, 33, 16), (3, 129, 20)])
+def test_gru_of_fp16_sequences_computes_as_that_of_fp32_ones(B, T, H):
+    """The data type is that of the arrays: the state, the sums and the gates are the same fp32 numbers, so the fp16 result is the
+    rounding of the fp32 one over the same inputs."""
+    ops, capi, L = _ops()
+    g = torch.Generator(device="cuda").manual_seed(B + T + H)
+    h16 = lambda sd, *s: (torch.randn(s, generator=g, device="cuda") * sd).half()
+    a = [h16(1, B, T, H), h16(H ** -0.5, H, 3 * H), h16(H ** -0.5, H, 3 * H), h16(0.1, 3 * H), h16(0.1, 3 * H)]
+    got = []
+    for t in (a, [v.float() for v in a]):
+        y = torch.empty_like(t[0])
+        capi.check(L.xb_gru(ops.ptr(t[0]), ops.ptr(y), B, T, H, *[ops.ptr(v) for v in t[1:]], ops.dt(y), ops.stream()))
+        got.append(y)
+    assert torch.equal(got[0], got[1].half())

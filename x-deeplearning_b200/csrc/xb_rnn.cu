@@ -37,36 +37,12 @@ namespace {
 // gate columns, its recurrent weights in registers, and a step is: read h as broadcast 16-byte vectors, four chains of FMAs,
 // the reset and update threads evaluate their gates and leave them in shared memory, the candidate threads the candidate and the
 // new h. Two barriers a step, but no shuffles, and each scheduler has one warp (H = 36).
-// fp16 sequences evaluate the gates with the hardware's exponential and reciprocal (gate_tanh below; the state stays fp32, and
-// what their few units in the last place of fp32 leave of a result that is rounded to fp16 is nothing: the same error against
-// 64 bits, 2.0e-4); fp32 sequences keep expf, tanhf and the division.
-// 16 sequences of 100 steps, H = 36: 36 us fp16, 39 fp32; 62 and 58 with four lanes a unit, three shuffles and one barrier a step.
-// 1000 sequences 180 and 275, 16 of H = 64 52 and 70. (The register bound lets the compiler have every h vector of a step on its
+// The data type is that of the arrays: state, sums and gates (expf, tanhf, a division) are fp32 for either.
+// 16 sequences of 100 steps, H = 36: 41 us fp16, 38 fp32; 61 and 57 with four lanes a unit, three shuffles and one barrier a step.
+// 1000 sequences 205 and 193, 16 of H = 64 56 and 52. (The register bound lets the compiler have every h vector of a step on its
 // way at once: at 128 registers, which it picks otherwise, 56 us.)
 constexpr int GRU_CHUNK = 64;
 __host__ __device__ constexpr int gru_hp(int nv) { return 16 * nv; }          // h and x rows padded with zeros
-
-__device__ __forceinline__ float ex2_approx(float v) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v)); return y; }
-__device__ __forceinline__ float rcp_approx(float v) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(v)); return y; }
-template <typename T> __device__ __forceinline__ float gate_sigmoid(float v) {
-  if constexpr (sizeof(T) == 4) return sigm(v);
-  else return rcp_approx(1.f + ex2_approx(-1.4426950408889634f * v));
-}
-// tanh from one exponential, 1 - 2 / (1 + e^2x); below 1/2, where that would cancel, x + x^3 P(x^2) with P of degree 3 fitted to
-// (tanh x - x) / x^3 by iteratively reweighted least squares (Lawson's method), 1.5e-8 relative. Both are evaluated: a branch
-// would take longer.
-template <typename T> __device__ __forceinline__ float gate_tanh(float x) {
-  if constexpr (sizeof(T) == 4) {
-    return tanhf(x);
-  } else {
-    const float s = x * x;
-    float p = fmaf(s, 0.01724149f, -0.05304549f);
-    p = fmaf(p, s, 0.13325879f);
-    p = fmaf(p, s, -0.33333144f);
-    const float small = fmaf(x * s, p, x), large = fmaf(-2.f, rcp_approx(1.f + ex2_approx(2.8853900817779268f * x)), 1.f);
-    return fabsf(x) < 0.5f ? small : large;
-  }
-}
 
 template <typename T, int NV>
 __global__ void __launch_bounds__((48 * NV + 31) / 32 * 32, 1) gru_kernel(const T* x, T* y, int steps, int H,
@@ -154,11 +130,11 @@ __global__ void __launch_bounds__((48 * NV + 31) / 32 * 32, 1) gru_kernel(const 
         a[0] = fmaf(v.x, wh[k], a[0]); a[1] = fmaf(v.y, wh[k + 1], a[1]); a[2] = fmaf(v.z, wh[k + 2], a[2]); a[3] = fmaf(v.w, wh[k + 3], a[3]);
       }
       const float sum = (a[0] + a[1]) + (a[2] + a[3]) + bhj;
-      if (tid < 2 * H) gates[tid] = gate_sigmoid<T>(pre_j + sum);
+      if (tid < 2 * H) gates[tid] = sigm(pre_j + sum);
       __syncthreads();                             // the gates are there, and everyone has read h
       if (col && u >= 0) {
         const float r = gates[u], z = gates[H + u];
-        const float c = gate_tanh<T>(pre_j + r * sum);
+        const float c = tanhf(pre_j + r * sum);
         h = c + z * (h - c);
         hbuf[u] = h;
         *yt = from_f32<T>(h);
