@@ -93,3 +93,32 @@ def test_dice_tower_over_several_tiles_a_block(R, n_cand, T, d, du, dims):
     # Dice on fp16 pairs: half-precision tanh (5e-4) and three roundings (2^-11) of a value, twice, and the logits' rounding
     tol = 4e-3 * (1 + float((x.abs() @ W3.double().abs()).max()))
     assert (got - want).abs().max() <= tol, (float((got - want).abs().max()), tol)
+
+
+@pytest.mark.parametrize("R,n_cand,T,d,du,dims", [(16, 500, 100, 36, 144, (200, 80, 2)), (3, 130, 20, 32, 128, (64, 32, 2)), (40, 64, 50, 16, 8, (48, 24, 8))])
+def test_prelu_tower_rounds_where_its_layers_do(R, n_cand, T, d, du, dims):
+    """The fused tower and the chain that it stands for (input kernel, three GEMMs): the same fp16 layer input and activations, so
+    they differ by the order of fp32 sums and by the few activations that this moves to the next fp16 number. A further rounding of
+    a layer's input (his_sum before its products, for one) moves them by 2^-13 of the layer's spread and more."""
+    ops, capi, L = _ops()
+    g = torch.Generator(device="cuda").manual_seed(R + d)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    n1, n2, n3 = dims
+    W1, W2, W3 = r(du + 5 * d, n1) / (du + 5 * d) ** 0.5, r(n1, n2) / n1 ** 0.5, r(n2, n3) / n2 ** 0.5
+    b1, b2, b3 = r(n1) * 0.1, r(n2) * 0.1, r(n3) * 0.1
+    s1, s2 = torch.rand(n1, generator=g, device="cuda") * 0.5, torch.rand(n2, generator=g, device="cuda") * 0.5
+    user, q, k, att = [r(*s).half() for s in ((R, du), (R * n_cand, d), (R * T, d), (R * n_cand, d))]
+    c = lambda t: t.cpu()
+    tower = ops.DinTower(d, du, c(W1), c(b1), [c(s1)], c(W2), c(b2), [c(s2)], c(W3), c(b3), softmax=False, act=capi.XB_ACT_PRELU)
+    got = tower(user, q, k, att, R, n_cand, T)
+    N, ldx = R * n_cand, (du + 5 * d + 7) // 8 * 8
+    X = torch.empty((N, ldx), dtype=torch.float16, device="cuda")
+    capi.check(L.xb_din_tower_input(ops.ptr(user), du, ops.ptr(q), d, ops.ptr(k), d, ops.ptr(att), d, ops.ptr(X), ldx, R, n_cand, T, d, du,
+                                    ops.stream()))
+    prelu = lambda s: dict(epilogue=capi.XB_EPI_PRELU, ep=(s, None, None), ep_count=s.numel())
+    y = ops.gemm(X, ops.pack_weight_kmajor(W1, ldk=ldx), bias=b1, trans_b=True, M=N, N=n1, K=ldx, **prelu(s1))
+    y = ops.gemm(y, ops.pack_weight_kmajor(W2), bias=b2, trans_b=True, M=N, N=n2, K=n1, **prelu(s2))
+    want = ops.gemm(y, ops.pack_weight_kmajor(W3), bias=b3, trans_b=True, M=N, N=n3, K=n2, out_dtype=torch.float32)
+    # one activation in some thirty meets another fp16 neighbour (fp32 sums of a few hundred terms, 2^-21 apart, against steps of
+    # 2^-10): 2^-10 / 30^0.5 of a value at the most, where every rounding moved would be 2^-11 / 3^0.5 = 2.8e-4
+    assert float((got - want).double().norm() / want.double().norm()) < 8e-5

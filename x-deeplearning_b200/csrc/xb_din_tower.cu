@@ -223,10 +223,11 @@ __global__ void __launch_bounds__(PT_THREADS, 2) din_tower_partial_kernel(const 
   for (int e = threadIdx.x; e < d; e += blockDim.x) {
     float s = 0.f;
     for (int gi = 0; gi < G; ++gi) s += part[gi * d + e];
-    // his_sum is an fp16 tensor in the model's graph: every use sees the rounded value
-    s = __half2float(__float2half_rn(s));
-    hs[e] = s;
-    if (blockIdx.y == 0) p.hs[(int64_t)r * d + e] = s;
+    // his_sum is an fp16 tensor in the DIN model's graph: every use sees the rounded value. The PReLU tower's layer input holds
+    // it in fp16 too, and beside it products and differences of the unrounded one (din_tower_input_kernel)
+    const float s16 = __half2float(__float2half_rn(s));
+    hs[e] = s16;
+    if (blockIdx.y == 0) p.hs[(int64_t)r * d + e] = p.act == XB_ACT_PRELU ? s : s16;
   }
   __syncthreads();
   float2 acc = make_float2(0.f, 0.f);
