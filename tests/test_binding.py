@@ -115,3 +115,12 @@ def test_pool_and_feed_arguments(bound):
     with pytest.raises(blaze_api.BlazeError):
         p.feed("x", whole)
     assert len(seen) == 1                              # nothing is fed into an input that could not be reshaped
+
+
+def test_feed_of_a_closed_predictor(bound):
+    _, _, blaze_api, seen, _ = bound
+    p = blaze_api.Predictor(C.c_void_p(99))
+    p.h = None                                         # what close() leaves
+    with pytest.raises(blaze_api.BlazeError):
+        p.feed("user_0.ids", np.zeros(3, np.float32))
+    assert not seen

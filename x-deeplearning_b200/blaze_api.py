@@ -170,6 +170,8 @@ class Predictor:
         self._feed = feed_call()
 
     def feed(self, name, array):
+        if self.h is None:
+            raise BlazeError("feed: the predictor is closed")
         a = np.ascontiguousarray(array)
         _ck(self._feed(self.h.value, name, a))
         return a            # keep alive until Forward: the copy is asynchronous
