@@ -82,6 +82,16 @@ def test_gemm_arguments(bound):
     assert (seen[-1][0]["M"], seen[-1][0]["K"], seen[-1][0]["N"], seen[-1][0]["trans_a"]) == (10, 6, 4, 1)
 
 
+def test_gemm_takes_any_indexable(bound):
+    ops, capi, _, seen, _ = bound
+    A, rows = torch.zeros((4, 4)), torch.zeros((3, 4))
+    for ep, strides in ((rows, [1, 2, 3, 4]), ([rows[0], None, rows[2]], range(1, 5)), (dict(enumerate(rows)), torch.Size((1, 2, 3, 4, 5)))):
+        ops.gemm(A, A, ep=ep, strides=strides)
+        a, _ = seen[-1]
+        assert [a["ep_a"], a["ep_b"], a["ep_c"]] == [ep[i] if ep[i] is None else ep[i].data_ptr() for i in range(3)]
+        assert (a["stride_a"], a["stride_b"], a["stride_y"]) == (1, 2, 4)
+
+
 def test_gemm_refuses_and_raises(bound):
     ops, capi, _, seen, result = bound
     A = torch.zeros((4, 4))

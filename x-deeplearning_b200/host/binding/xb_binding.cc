@@ -80,19 +80,18 @@ PyObject* py_gemm(PyObject*, PyObject* const* v, Py_ssize_t n) {
   memset(&a, 0, sizeof(a));
   void* p = nullptr;
   PyObject *A = v[0], *B = v[1], *Y = v[2], *bias = v[3], *ep = v[9], *strides = v[14];
-  if (!PyTuple_Check(strides) && !PyList_Check(strides)) { PyErr_SetString(PyExc_TypeError, "gemm: strides"); return nullptr; }
-  if (!PyTuple_Check(ep) && !PyList_Check(ep)) { PyErr_SetString(PyExc_TypeError, "gemm: ep"); return nullptr; }
-  if (PySequence_Fast_GET_SIZE(strides) < 4 || PySequence_Fast_GET_SIZE(ep) < 3) {
+  if (!PyTuple_Check(strides) || !PyTuple_Check(ep)) { PyErr_SetString(PyExc_TypeError, "gemm: strides and ep are tuples"); return nullptr; }
+  if (PyTuple_GET_SIZE(strides) < 4 || PyTuple_GET_SIZE(ep) < 3) {
     PyErr_SetString(PyExc_IndexError, "gemm: four strides and three activation parameters");
     return nullptr;
   }
-  PyObject** st = PySequence_Fast_ITEMS(strides);
+  auto st = [&](int i) { return PyTuple_GET_ITEM(strides, i); };
   if (as_i32(v[15], &a.M) || as_i32(v[16], &a.N) || as_i32(v[17], &a.K) || as_flag(v[4], &a.trans_a) || as_flag(v[5], &a.trans_b) ||
       as_f32(v[6], &a.alpha) || as_f32(v[7], &a.beta))
     return nullptr;
-  if (tensor_ptr(A, &p) || leading(v[18], A, &a.lda) || as_i64(st[0], &a.stride_a)) return nullptr;
+  if (tensor_ptr(A, &p) || leading(v[18], A, &a.lda) || as_i64(st(0), &a.stride_a)) return nullptr;
   a.A = p;
-  if (tensor_ptr(B, &p) || leading(v[19], B, &a.ldb) || as_i64(st[1], &a.stride_b)) return nullptr;
+  if (tensor_ptr(B, &p) || leading(v[19], B, &a.ldb) || as_i64(st(1), &a.stride_b)) return nullptr;
   a.B = p;
   if (bias != Py_None) {
     int32_t kind = 0;
@@ -108,17 +107,17 @@ PyObject* py_gemm(PyObject*, PyObject* const* v, Py_ssize_t n) {
     else if (as_i32(v[21], &kind)) return nullptr;
     if (v[23] == Py_None && dim <= 1) a.ldbias = 0;
     else if (leading(v[23], bias, &a.ldbias)) return nullptr;
-    if (tensor_ptr(bias, &p) || tensor_dtype(bias, &a.bias_dtype) || as_i64(st[2], &a.stride_bias) || as_i64(v[24], &a.bias_row_group))
+    if (tensor_ptr(bias, &p) || tensor_dtype(bias, &a.bias_dtype) || as_i64(st(2), &a.stride_bias) || as_i64(v[24], &a.bias_row_group))
       return nullptr;
     a.bias = p;
     a.bias_kind = kind;
   }
-  if (tensor_ptr(Y, &p) || leading(v[20], Y, &a.ldy) || as_i64(st[3], &a.stride_y)) return nullptr;
+  if (tensor_ptr(Y, &p) || leading(v[20], Y, &a.ldy) || as_i64(st(3), &a.stride_y)) return nullptr;
   a.Y = p;
   if (as_i32(v[13], &a.batch) || tensor_dtype(A, &a.ab_dtype) || tensor_dtype(Y, &a.y_dtype) || as_i32(v[8], &a.epilogue)) return nullptr;
   const float** slots[3] = {&a.ep_a, &a.ep_b, &a.ep_c};
   for (int i = 0; i < 3; ++i) {
-    PyObject* e = PySequence_Fast_ITEMS(ep)[i];
+    PyObject* e = PyTuple_GET_ITEM(ep, i);
     if (e == Py_None) continue;
     if (tensor_ptr(e, &p)) return nullptr;
     *slots[i] = static_cast<const float*>(p);

@@ -127,6 +127,11 @@ def gemm(A, B, Y=None, bias=None, trans_a=False, trans_b=False, alpha=1.0, beta=
         N = B.shape[-2] if trans_b else B.shape[-1]
     if Y is None:
         Y = torch.empty((batch, M, N) if batch > 1 else (M, N), dtype=out_dtype or A.dtype, device=A.device)
+    # any indexable will do (a [3, N] tensor of activation parameters, an array of strides); the extension module takes tuples
+    if type(ep) is not tuple:
+        ep = (ep[0], ep[1], ep[2])
+    if type(strides) is not tuple:
+        strides = (strides[0], strides[1], strides[2], strides[3])
     global _gemm
     if _gemm is None:
         m = binding()
