@@ -4,6 +4,7 @@ import importlib.machinery
 import importlib.util
 import os
 import subprocess
+import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libxdlb200.so")
@@ -156,7 +157,7 @@ def build_native(verbose=False):
     subprocess.check_call(cmd, stdout=None if verbose else subprocess.DEVNULL)
     host = os.path.join(HERE, "host", "Makefile")
     if os.path.exists(host):
-        subprocess.check_call(["make", "-s", "-j8", "-C", os.path.join(HERE, "host")],
+        subprocess.check_call(["make", "-s", "-j8", "-C", os.path.join(HERE, "host"), "all", "python", "PYTHON=" + sys.executable],
                               stdout=None if verbose else subprocess.DEVNULL)
 
 
