@@ -521,9 +521,9 @@ int xb_prelu(const void* x, void* y, int64_t size, const void* w, int64_t inner,
 /* SigmoidOp, blaze/blaze/operator/op/sigmoid_op.cu:11-17 */
 int xb_sigmoid(const void* x, void* y, int64_t size, int32_t dtype, xb_stream_t stream);
 /* SoftmaxOp, blaze/blaze/operator/op/softmax_op.cu:25-67: softmax over c with outer n, inner w */
+int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t w, int32_t dtype, xb_stream_t stream);
 /* xb_softmax of n rows of c fp32 scores, written as fp32 and, rounded from it, as fp16 (the gates of xb_augru_shared) */
 int xb_softmax_scores(const float* x, float* y, void* y16, int64_t n, int32_t c, xb_stream_t stream);
-int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t w, int32_t dtype, xb_stream_t stream);
 /* BatchNormalizationOp (inference), blaze/blaze/operator/op/batch_normalization_op.cu:12 */
 int xb_batchnorm(const void* x, void* y, int64_t size, int32_t c, const void* gamma, const void* beta,
                  const void* mean, const void* var, float eps, int32_t nosqrt, int32_t dtype,
