@@ -56,3 +56,21 @@ def test_batches_of_single_rows(P, N, K, epi):
     if epi == "sigmoid":
         want, tol = want.sigmoid(), tol + 2.0 ** -20            # __expf and the division
     assert ((Y[:, :N].double() - want).abs() <= tol).all() and (Y[:, N:] == 9.0).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_the_named_engine_keeps_its_order_of_sums(dtype):
+    """XB_GEMM_SIMT adds k ascending whatever the number of rows or batches: a row has the bits that it has in a smaller call."""
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(2)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda").to(dtype)
+    kw = dict(out_dtype=torch.float32, engine=capi.XB_GEMM_SIMT)
+    for N in (1, 2, 4):
+        A, B = r(1000, 512), r(512, N)
+        few = torch.cat([ops.gemm(A[i:i + 100], B, **kw) for i in range(0, 1000, 100)])
+        for M in (127, 128, 1000):
+            assert torch.equal(ops.gemm(A[:M], B, **kw), few[:M])
+    A, B = r(64, 1, 300), r(64, 300, 36)
+    one = torch.stack([ops.gemm(A[i], B[i], **kw) for i in range(64)])
+    for P in (31, 32, 64):
+        assert torch.equal(ops.gemm(A[:P], B[:P], batch=P, M=1, N=36, K=300, strides=(300, 300 * 36, 0, 36), **kw), one[:P])

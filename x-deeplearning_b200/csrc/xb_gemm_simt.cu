@@ -6,7 +6,9 @@
 // those go through warp-level matrix instructions, xb_gemm_half.cuh.)
 //
 // 256 threads, tile 16*TM x 16*TN, 16-deep k slices; fp32 accumulation with k
-// ascending, whatever the tile, so every form gives the same bits.
+// ascending, whatever the tile, so every form gives the same bits. XB_GEMM_SIMT
+// is these tiles; XB_GEMM_AUTO also takes the kernels for a few columns and for
+// batches of single rows, which add up partial sums.
 // gemm_f32_kernel (fp32, neither operand transposed: Blaze's own layout) keeps
 // a ring of slices in flight with cp.async, which hides the latency that bounds
 // a small launch, and puts two columns' FMAs into one fma.rn.f32x2 (each
@@ -560,19 +562,21 @@ int gemm_simt(const xb_gemm_args& a, cudaStream_t stream) {
   pick_simt_tile(a.M, a.N, a.batch, f32, &tm, &tn);
   // (the entry point's limits, whatever the tile; a grid of any of them would take more rows)
   XB_REQUIRE((a.M + 63) / 64 <= 65535 && a.batch <= 65535, XB_ERR_LIMIT, "xb_gemm: M or batch too large for the SIMT engine");
+  // Who asks for this engine by name gets its order of sums; the kernels from here to the tiles have others.
+  const bool any = a.engine == XB_GEMM_AUTO;
   // single rows: many of them, each of a size that one CTA reads in a few steps
-  if (f32 && a.M == 1 && a.batch >= 32 && a.N % 4 == 0 && a.N <= 256 && (int64_t)a.N * a.K <= 65536 && p.b_vec) {
+  if (any && f32 && a.M == 1 && a.batch >= 32 && a.N % 4 == 0 && a.N <= 256 && (int64_t)a.N * a.K <= 65536 && p.b_vec) {
     launch_dependent(gemm_f32_row_kernel, (unsigned)a.batch, 256, (size_t)(256 / (a.N / 4)) * a.N * 4, stream, p);
     return check_launch("gemm_f32_row_kernel");
   }
-  if (gemm_narrow_takes(a)) {
+  if (any && gemm_narrow_takes(a)) {
     if (a.ab_dtype == XB_F32) return launch_narrow<float>(p, a.batch, stream);
     if (a.ab_dtype == XB_F16) return launch_narrow<__half>(p, a.batch, stream);
     return launch_narrow<__nv_bfloat16>(p, a.batch, stream);
   }
   // 16-bit results of 16-bit operands: the matrix instructions' sums, which are not rounded one by one, end in the same 16 bits.
-  // (An fp32 result would show it, and who asks for this engine by name gets its order of sums.)
-  if (a.engine == XB_GEMM_AUTO && a.ab_dtype != XB_F32 && a.y_dtype != XB_F32) return gemm_half(p, a, stream);
+  // (An fp32 result would show it.)
+  if (any && a.ab_dtype != XB_F32 && a.y_dtype != XB_F32) return gemm_half(p, a, stream);
   p.tiles_n = (a.N + 16 * tn - 1) / (16 * tn);
   const int64_t tiles = (((int64_t)a.M + 16 * tm - 1) / (16 * tm)) * p.tiles_n;
   XB_REQUIRE(tiles < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_gemm: %lld output tiles are too many for one call", (long long)tiles);
