@@ -112,3 +112,17 @@ def test_ragged_tiles_between_whole_ones(N, M, P, K):
     mag = A.double().abs() @ B.double().abs().transpose(1, 2) + bias.double().abs()[:, None]
     # fp32 sums of K products, not every one rounded, and the result's rounding
     assert ((one.double() - x).abs() <= 2 * (K + 2) * 2.0 ** -24 * mag + 2.0 ** -11 * x.abs() + 2.0 ** -25).all()
+
+
+# (by TMA, in pieces, rows that start anywhere)
+@pytest.mark.parametrize("M,N", [(40000, 200), (5000, 200), (20000, 199)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_sigmoid_of_16_bits_is_the_rounding_of_fp32(M, N, dtype):
+    """The activation is fp32 arithmetic whatever the result's type: the same product with an fp32 result, rounded."""
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    A, W, bias = r(M, 88).to(dtype), (r(N, 88) / 6).to(dtype), r(N)
+    kw = dict(bias=bias, trans_b=True, epilogue=capi.XB_EPI_SIGMOID, engine=capi.XB_GEMM_TCGEN05)
+    got, fp32 = ops.gemm(A, W, out_dtype=dtype, **kw), ops.gemm(A, W, out_dtype=torch.float32, **kw)
+    assert torch.equal(got, fp32.to(dtype))

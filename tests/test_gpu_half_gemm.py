@@ -91,3 +91,19 @@ def test_smallest_aligned_products(M, N, K, trans_b, dtype):
     eps, tiny = (2.0 ** -11, 2.0 ** -25) if dtype == torch.float16 else (2.0 ** -8, 0.0)
     assert ((Y[:, :, :N].double() - a @ w).abs() <= 2 * (K + 2) * 2.0 ** -24 * (a.abs() @ w.abs()) + eps * (a @ w).abs() + tiny).all()
     assert (Y[:, :, N] == 9.0).all()
+
+
+@pytest.mark.parametrize("M,N", [(3000, 257), (70, 33)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("epi", ["sigmoid", "dice"])
+def test_activations_as_on_the_cuda_cores(M, N, dtype, epi):
+    """Sums that any order leaves exact (one product each): bias and activation give the bits of XB_GEMM_SIMT."""
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    A, W = torch.zeros((M, 65), dtype=dtype, device="cuda"), r(65, N).to(dtype)
+    A[:, 40] = r(M).to(dtype)
+    u = lambda lo, hi: torch.rand((N,), generator=g, device="cuda") * (hi - lo) + lo
+    kw = dict(epilogue=capi.XB_EPI_SIGMOID) if epi == "sigmoid" else dict(epilogue=capi.XB_EPI_DICE, ep=(u(0, 0.5), u(-0.1, 0.1), u(0.5, 1.5)))
+    got, simt = [ops.gemm(A, W, bias=r(N) * 0 + 0.3, engine=e, **kw) for e in (capi.XB_GEMM_AUTO, capi.XB_GEMM_SIMT)]
+    assert torch.equal(got, simt)

@@ -90,20 +90,6 @@ struct HalfSlice {
   }
 };
 
-// `finish` for a result of 16 bits: the quotient of a sigmoid as a multiplication with the hardware's reciprocal (2 ulp of fp32)
-__device__ __forceinline__ float half_finish(const SimtGemmParams& p, const Column& c, int b, int gm, int gn, float acc) {
-  float v = p.alpha * acc;
-  if (p.bias_kind == XB_BIAS_ROW)
-    v += p.beta * c.bias;
-  else if (p.bias_kind == XB_BIAS_FULL)
-    v += p.beta * load_as_f32(p.bias, (int64_t)b * p.stride_bias + (int64_t)(gm / p.bias_group) * p.ldbias + gn, p.bias_dtype);
-  if (p.epi.kind == XB_EPI_PRELU) return act_prelu(v, c.a);
-  if (p.epi.kind == XB_EPI_NONE) return v;
-  const bool dice = p.epi.kind == XB_EPI_DICE;
-  const float s = __fdividef(1.f, 1.f + __expf(dice ? -(v - c.b) * c.c : -v));
-  return dice ? (1.f - s) * c.a * v + s * v : s;
-}
-
 // BM = 128: 4 x 2 warps of 32 x 32 outputs; BM = 64: 2 x 4 of 32 x 16.
 template <bool BF16, int BM, bool TA, bool TB>
 __global__ void __launch_bounds__(256, 2) gemm_half_kernel(const __grid_constant__ SimtGemmParams p, int a_even, int b_even) {
@@ -226,7 +212,7 @@ __global__ void __launch_bounds__(256, 2) gemm_half_kernel(const __grid_constant
 #pragma unroll 4
   for (int r = nar ? threadIdx.x >> 4 : warp; r < BM && m0 + r < p.M; r += step) {
     const float2 x = *reinterpret_cast<const float2*>(out + r * HALF_OPITCH + cl);
-    const float v0 = half_finish(p, c0, b, m0 + r, gn, x.x), v1 = two ? half_finish(p, c1, b, m0 + r, gn + 1, x.y) : 0.f;
+    const float v0 = finish(p, c0, b, m0 + r, gn, x.x), v1 = two ? finish(p, c1, b, m0 + r, gn + 1, x.y) : 0.f;
     const int64_t at = (int64_t)b * p.stride_y + (int64_t)(m0 + r) * p.ldy + gn;
     if (p.y_pairs && two) {
       uint32_t w;

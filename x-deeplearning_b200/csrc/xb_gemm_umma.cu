@@ -124,17 +124,9 @@ __device__ __forceinline__ void store16_vec(TOut* dst, const float (&v)[16], int
   }
 }
 
-// For a 16-bit result the quotient as one multiplication with the hardware's reciprocal (2 ulp of fp32, 2^-11 of what the result's
-// rounding may be off). 4 x ([9854, 24] x [24, 336]) fp16: the division took 6 of 29 us; the error against 64 bits is the same.
-template <typename TOut>
-__device__ __forceinline__ float epi_sigmoid(float x) {
-  if constexpr (sizeof(TOut) == 4) return act_sigmoid(x);
-  else return __fdividef(1.f, 1.f + __expf(-x));
-}
-
 // Activation of 16 adjacent columns of one row; the per-column parameters sit in shared memory and are
 // read as 16-byte vectors (all lanes read the same address: a broadcast).
-template <typename TOut, int KIND>
+template <int KIND>
 __device__ __forceinline__ void epi_apply16(float (&v)[16], const float* s_a, const float* s_b, const float* s_c) {
   if constexpr (KIND != XB_EPI_NONE) {
 #pragma unroll
@@ -159,7 +151,7 @@ __device__ __forceinline__ void epi_apply16(float (&v)[16], const float* s_a, co
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[4 * j + i] = epi_sigmoid<TOut>(v[4 * j + i]);
+      for (int i = 0; i < 4; ++i) v[4 * j + i] = act_sigmoid(v[4 * j + i]);
     }
   }
   }
@@ -209,7 +201,7 @@ __device__ __forceinline__ void epi_tile_fast(uint32_t tmem_row, int c_begin, in
         v[4 * j + 2] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 2]), b.z);
         v[4 * j + 3] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 3]), b.w);
       }
-      epi_apply16<TOut, KIND>(v, s_a + c, s_b + c, s_c + c);
+      epi_apply16<KIND>(v, s_a + c, s_b + c, s_c + c);
       if (sizeof(TOut) == 2 && two) {
         const int sw = (lane >> 1) & 3;
         stage[lane * 4 + ((2 * u) ^ sw)] = pack8<TOut>(v);
@@ -256,7 +248,7 @@ __device__ __forceinline__ void epi_unit(uint32_t tmem_at, float alpha, const fl
       v[4 * j + 2] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 2]), b.z);
       v[4 * j + 3] = fmaf(alpha, __uint_as_float(raw[16 * u + 4 * j + 3]), b.w);
     }
-    epi_apply16<TOut, KIND>(v, s_a + 16 * u, s_b + 16 * u, s_c + 16 * u);
+    epi_apply16<KIND>(v, s_a + 16 * u, s_b + 16 * u, s_c + 16 * u);
     area[lane * (W / 8) + ((2 * u) ^ sw)] = pack8<TOut>(v);
     area[lane * (W / 8) + ((2 * u + 1) ^ sw)] = pack8<TOut>(v + 8);
   }
@@ -362,7 +354,7 @@ __device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t 
       }
     } else if (p.epi.kind == XB_EPI_SIGMOID) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) v[i] = epi_sigmoid<TOut>(v[i]);
+      for (int i = 0; i < 16; ++i) v[i] = act_sigmoid(v[i]);
     }
     const bool vec = vec_base && ((gn0 * sizeof(TOut)) % 16 == 0);
     if (sizeof(TOut) == 2 && !(vec && valid == 16)) {
