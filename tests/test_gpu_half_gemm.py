@@ -107,3 +107,25 @@ def test_activations_as_on_the_cuda_cores(M, N, dtype, epi):
     kw = dict(epilogue=capi.XB_EPI_SIGMOID) if epi == "sigmoid" else dict(epilogue=capi.XB_EPI_DICE, ep=(u(0, 0.5), u(-0.1, 0.1), u(0.5, 1.5)))
     got, simt = [ops.gemm(A, W, bias=r(N) * 0 + 0.3, engine=e, **kw) for e in (capi.XB_GEMM_AUTO, capi.XB_GEMM_SIMT)]
     assert torch.equal(got, simt)
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(300, 65, 301, 2), (9000, 65, 129, 1), (60, 64, 320, 1), (22, 16, 512, 16)])
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("positive", [False, True])
+def test_sums_are_no_worse_than_fp32_fmas(M, N, K, batch, trans_b, dtype, positive):
+    """A full bias takes the exact sums away and a factor brings what is left, the errors of the sums, into a 16-bit result."""
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(K)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    A, B = r(batch, M, K), r(batch, *((N, K) if trans_b else (K, N))) / K ** 0.5
+    A, B = [(x.abs() if positive else x).to(dtype) for x in (A, B)]
+    exact = A.double() @ (B.transpose(1, 2) if trans_b else B).double()
+    full, scale = exact.float(), 2.0 ** 20
+    rms = []
+    for e in (capi.XB_GEMM_AUTO, capi.XB_GEMM_SIMT):
+        Y = ops.gemm(A, B, bias=-full, bias_kind=capi.XB_BIAS_FULL, trans_b=trans_b, batch=batch, M=M, N=N, K=K, lda=K, ldb=B.shape[-1], ldy=N,
+                     ldbias=N, strides=(M * K, N * K, M * N, M * N), alpha=scale, beta=scale, engine=e,
+                     Y=torch.empty((batch, M, N), dtype=dtype, device="cuda"))
+        rms.append((Y.double() / scale + (full.double() - exact)).pow(2).mean().sqrt().item())
+    assert rms[0] <= rms[1], rms

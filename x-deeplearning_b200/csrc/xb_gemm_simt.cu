@@ -574,8 +574,8 @@ int gemm_simt(const xb_gemm_args& a, cudaStream_t stream) {
     if (a.ab_dtype == XB_F16) return launch_narrow<__half>(p, a.batch, stream);
     return launch_narrow<__nv_bfloat16>(p, a.batch, stream);
   }
-  // 16-bit results of 16-bit operands: the matrix instructions' sums, which are not rounded one by one, end in the same 16 bits.
-  // (An fp32 result would show it.)
+  // 16-bit results of 16-bit operands: sums of 16 products by matrix instructions, which are no further from 64 bits than FMAs.
+  // (Their bits differ from the FMAs', which an fp32 result would show.)
   if (any && a.ab_dtype != XB_F32 && a.y_dtype != XB_F32) return gemm_half(p, a, stream);
   p.tiles_n = (a.N + 16 * tn - 1) / (16 * tn);
   const int64_t tiles = (((int64_t)a.M + 16 * tm - 1) / (16 * tm)) * p.tiles_n;

@@ -974,11 +974,11 @@ extern "C" int xb_gemm(const xb_gemm_args* a, xb_stream_t stream) {
     XB_REQUIRE(a->K > 0, XB_ERR_ARG, "xb_gemm: K = 0");
     return gemm_umma(*a, (cudaStream_t)stream);
   }
-  // Whatever the size where the result has 16 bits: a few outputs of a long sum are a chain of slices in any other kernel
-  // (16 x ([22, 320] x [320, 16]): 4.5 us, 8.3 with warp-level matrix instructions, 24.8 on the CUDA cores; 2 x ([59, 24] x [24, 32]):
-  // 3.3, 4.3, 5.7). An fp32 result of less than 128 x 64 outputs keeps the CUDA cores' order of sums.
-  if (a->engine == XB_GEMM_AUTO && umma_eligible(*a) && a->K > 0 && !gemm_narrow_takes(*a) &&
-      (a->y_dtype != XB_F32 || (int64_t)a->M * a->N * a->batch >= 128 * 64))
+  // Less than 128 x 64 outputs keep sums that are rounded, fp32 FMAs or gemm_half_kernel's, whose error against 64 bits is no larger;
+  // an accumulator in tensor memory is cut off at every MMA instead (rms before the result's rounding, positive fp16 values 5.6e-7,
+  // FMAs 1.3e-7). What that costs: 16 x ([22, 320] x [320, 16]) fp16 8.5 us, 4.3 in tensor memory (24.8 on the CUDA cores);
+  // 2 x ([59, 24] x [24, 32]) 3.7, 3.1 (5.7).
+  if (a->engine == XB_GEMM_AUTO && umma_eligible(*a) && a->K > 0 && !gemm_narrow_takes(*a) && (int64_t)a->M * a->N * a->batch >= 128 * 64)
     return gemm_umma(*a, (cudaStream_t)stream);
   return gemm_simt(*a, (cudaStream_t)stream);
 }
