@@ -505,7 +505,8 @@ int xb_augru(const void* x, const void* att, void* y, int64_t batch, int32_t T, 
  * y_final [requests * n_cand, H] is kept. All tensors fp16. `engine`: XB_GEMM_AUTO / _SIMT / _TCGEN05; the tcgen05
  * engine (one CTA per 128 candidates, both per-candidate products as MMAs with the state in tensor memory, the
  * request-side terms x_t Wg_x + bg and x_t Wc_x + bc computed once per request) takes an even H <= 64 whose padding
- * to a multiple of 8 leaves at least 4 slots (H = 36 does). Same cell as xb_augru. */
+ * to a multiple of 8 leaves at least 4 slots (H = 36 does). XB_GEMM_AUTO takes it where the call has more such tiles than
+ * the GPU has SMs, and warp-level MMAs with the state in registers for fewer. Same cell as xb_augru. */
 int xb_augru_shared(const void* x, const void* att, void* y_final, int32_t requests, int32_t n_cand, int32_t T, int32_t H,
                     const void* Wg, const void* bg, const void* Wc, const void* bc, int32_t engine, xb_stream_t stream);
 

@@ -32,3 +32,47 @@ def test_augru_over_chunks_of_steps(H, T, R, n_cand):
     f = lambda t: t.float().cpu().numpy()
     want = orc.augru(f(dx)[np.array(few) // n_cand], f(da)[few], f(dWg), f(dbg), f(dWc), f(dbc))[:, T - 1, :]
     np.testing.assert_allclose(f(y)[few], want, rtol=0, atol=8e-3)
+
+
+def _augru(R, n_cand, T, H, seed):
+    from x_deeplearning_b200 import ops, capi
+    rng = np.random.default_rng(seed)
+    h16 = lambda a: torch.from_numpy(a.astype(np.float32)).to("cuda", torch.float16)
+    x, att = h16(rng.normal(0, 0.7, (R, T, H))), h16(rng.dirichlet(np.ones(T) * 0.3, R * n_cand))
+    w = [h16(rng.normal(0, 1 / np.sqrt(2 * H), (2 * H, 2 * H))), h16(rng.normal(0.5, 0.2, 2 * H)),
+         h16(rng.normal(0, 1 / np.sqrt(2 * H), (2 * H, H))), h16(rng.normal(0, 0.1, H))]
+
+    def run(requests, engine):
+        y = torch.empty((requests * n_cand, H), dtype=torch.float16, device="cuda")
+        capi.check(capi.lib().xb_augru_shared(ops.ptr(x), ops.ptr(att), ops.ptr(y), requests, n_cand, T, H, *[ops.ptr(t) for t in w],
+                                              engine, ops.stream()))
+        return y
+    return x, att, w, run
+
+
+@pytest.mark.parametrize("H,T", [(36, 100), (4, 257), (60, 130)])
+@pytest.mark.parametrize("n_cand", [17, 200])
+def test_the_named_engine_whatever_the_number_of_tiles(H, T, n_cand):
+    """A candidate's state does not depend on the call's size where the engine is named: few tiles and more than any GPU has SMs."""
+    pkg.load()
+    from x_deeplearning_b200 import capi
+    run = _augru(300, n_cand, T, H, 1)[3]
+    many = run(300, capi.XB_GEMM_TCGEN05)
+    for few in (1, 3):
+        assert torch.equal(run(few, capi.XB_GEMM_TCGEN05), many[:few * n_cand])
+
+
+@pytest.mark.parametrize("H,T", [(36, 127), (36, 128), (36, 129), (36, 200), (4, 257), (60, 130), (18, 5)])
+@pytest.mark.parametrize("R,n_cand", [(1, 17), (2, 65), (16, 1000)])
+def test_few_tiles_by_the_engine_that_the_library_picks(H, T, R, n_cand):
+    pkg.load()
+    from x_deeplearning_b200 import capi
+    x, att, w, run = _augru(R, n_cand, T, H, H + T)
+    bad = n_cand // 2
+    att[bad] = torch.nan
+    y = run(R, capi.XB_GEMM_AUTO)
+    assert y[bad].isnan().all()
+    few = [i for r in {0, R - 1} for i in range(r * n_cand, (r + 1) * n_cand) if i != bad][:200] + [R * n_cand - 1]
+    f = lambda t: t.float().cpu().numpy()
+    want = orc.augru(f(x)[np.array(few) // n_cand], f(att)[few], *[f(t) for t in w])[:, T - 1, :]
+    np.testing.assert_allclose(f(y)[few], want, rtol=0, atol=8e-3)

@@ -373,7 +373,7 @@ extern "C" int xb_augru_shared(const void* x, const void* att, void* y_final, in
   p.x = (const __half*)x; p.att = (const __half*)att; p.y = (__half*)y_final;
   p.Wg = (const __half*)Wg; p.bg = (const __half*)bg; p.Wc = (const __half*)Wc; p.bc = (const __half*)bc;
   p.requests = requests; p.n_cand = n_cand; p.T = T; p.H = H;
-  if (tc) return augru_mma_wanted(p) ? launch_augru_mma(p, (cudaStream_t)s) : launch_augru_tc(p, (cudaStream_t)s);
+  if (tc) return engine == XB_GEMM_AUTO && augru_mma_wanted(p) ? launch_augru_mma(p, (cudaStream_t)s) : launch_augru_tc(p, (cudaStream_t)s);
   XB_REQUIRE((int64_t)requests * n_cand < ((int64_t)1 << 31), XB_ERR_LIMIT, "xb_augru_shared: batch too large");
   switch ((H + 15) / 16) {
     case 1: return launch_augru_shared<1>(p, (cudaStream_t)s);
