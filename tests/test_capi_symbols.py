@@ -48,3 +48,24 @@ def test_host_index_builder_matches_lookup_rule():
     found = {int(k): int(r) for k, r in zip(sk, sr) if r >= 0}
     assert found == {5: 0, 1 << 40: 1, -7: 2, 99: 4}
     assert m.lib().xb_table_build_index_host(keys.ctypes.data, len(keys), 8, sk.ctypes.data, sr.ctypes.data) == -1
+
+
+def test_uses_tcgen05_answers_what_the_dispatch_does():
+    """Host logic alone: products of up to four columns, few outputs, no depth and fp32 results of [K, N] weights go elsewhere."""
+    m = pkg.load()
+    c = m.capi
+
+    def uses(M=1000, N=64, K=64, y=None, trans_b=1, engine=c.XB_GEMM_AUTO, lda=None):
+        a = c.GemmArgs()
+        a.M, a.N, a.K, a.trans_b, a.batch, a.engine = M, N, K, trans_b, 1, engine
+        a.A = a.B = a.Y = 4096                               # 16-byte aligned; nothing is read
+        a.lda, a.ldb, a.ldy = lda or max(K, 8), (K if trans_b else N) or 8, N
+        a.ab_dtype, a.y_dtype = c.XB_F16, y or c.XB_F16
+        return m.lib().xb_gemm_uses_tcgen05(ctypes.byref(a))
+    assert uses() == 1 and uses(trans_b=0) == 1 and uses(y=c.XB_F32) == 1
+    assert uses(N=4) == 0 and uses(N=4, lda=72) == 0 and uses(M=100000, N=5) == 1
+    assert uses(K=0) == 0 and uses(K=0, engine=c.XB_GEMM_TCGEN05) == 0
+    assert uses(M=127) == 0 and uses(M=128) == 1 and uses(M=127, y=c.XB_F32) == 0
+    assert uses(y=c.XB_F32, trans_b=0) == 0 and uses(lda=65) == 0
+    assert uses(M=127, engine=c.XB_GEMM_TCGEN05) == 1 and uses(trans_b=0, engine=c.XB_GEMM_TCGEN05) == 0
+    assert uses(engine=c.XB_GEMM_SIMT) == 0

@@ -959,9 +959,19 @@ static int validate_gemm(const xb_gemm_args* a) {
   return 0;
 }
 
+// Whether XB_GEMM_AUTO runs these arguments on the tcgen05 engine.
+// Less than 128 x 64 outputs keep sums that are rounded, fp32 FMAs or gemm_half_kernel's, whose error against 64 bits is no larger;
+// an accumulator in tensor memory is cut off at every MMA instead (rms before the result's rounding, positive fp16 values 5.6e-7,
+// FMAs 1.3e-7). What that costs: 16 x ([22, 320] x [320, 16]) fp16 8.5 us, 4.3 in tensor memory (24.8 on the CUDA cores);
+// 2 x ([59, 24] x [24, 32]) 3.7, 3.1 (5.7).
+static bool auto_takes_umma(const xb_gemm_args& a) {
+  return umma_eligible(a) && a.K > 0 && !gemm_narrow_takes(a) && (int64_t)a.M * a.N * a.batch >= 128 * 64;
+}
+
 extern "C" int xb_gemm_uses_tcgen05(const xb_gemm_args* a) {
-  if (!a || a->engine == XB_GEMM_SIMT || (a->engine == XB_GEMM_TCGEN05 && !a->trans_b)) return 0;
-  return umma_eligible(*a) ? 1 : 0;
+  if (!a || (a->engine != XB_GEMM_AUTO && a->engine != XB_GEMM_TCGEN05)) return 0;
+  if (a->engine == XB_GEMM_TCGEN05) return a->trans_b && a->K > 0 && umma_eligible(*a) ? 1 : 0;
+  return auto_takes_umma(*a) ? 1 : 0;
 }
 
 extern "C" int xb_gemm(const xb_gemm_args* a, xb_stream_t stream) {
@@ -974,11 +984,6 @@ extern "C" int xb_gemm(const xb_gemm_args* a, xb_stream_t stream) {
     XB_REQUIRE(a->K > 0, XB_ERR_ARG, "xb_gemm: K = 0");
     return gemm_umma(*a, (cudaStream_t)stream);
   }
-  // Less than 128 x 64 outputs keep sums that are rounded, fp32 FMAs or gemm_half_kernel's, whose error against 64 bits is no larger;
-  // an accumulator in tensor memory is cut off at every MMA instead (rms before the result's rounding, positive fp16 values 5.6e-7,
-  // FMAs 1.3e-7). What that costs: 16 x ([22, 320] x [320, 16]) fp16 8.5 us, 4.3 in tensor memory (24.8 on the CUDA cores);
-  // 2 x ([59, 24] x [24, 32]) 3.7, 3.1 (5.7).
-  if (a->engine == XB_GEMM_AUTO && umma_eligible(*a) && a->K > 0 && !gemm_narrow_takes(*a) && (int64_t)a->M * a->N * a->batch >= 128 * 64)
-    return gemm_umma(*a, (cudaStream_t)stream);
+  if (a->engine == XB_GEMM_AUTO && auto_takes_umma(*a)) return gemm_umma(*a, (cudaStream_t)stream);
   return gemm_simt(*a, (cudaStream_t)stream);
 }
