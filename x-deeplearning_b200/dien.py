@@ -7,7 +7,8 @@ xdl-algorithm-solution/DIEN/script/utils.py:139-207, attention MLP and tower as 
     f[n]      = last state of AUGRU(h[r], s[n])                      [H]
     prob[n]   = softmax(PReLU-MLP([user | q_n | his_sum | q_n*his_sum | f_n]))
 Pooling, GRU, the fused attention unit (scores only), softmax, AUGRU and the fused tower with PReLU run as kernels of the
-library; with an engine of the caller's choice the tower is its assembly kernel and GEMMs of that engine.
+library; with an engine of the caller's choice, or sizes that the fused kernel does not take, the tower is its assembly
+kernel and GEMMs.
 """
 import ctypes as C
 
@@ -43,12 +44,15 @@ class DienModel(DinModel):
         self.dW3 = ops.pack_weight_kmajor(t(tw["W3"]).to(device), torch.float16)
         self.db = [f32(tw["b1"]), f32(tw["b2"]), f32(tw["b3"])]
         self.dslope = [f32(tw["slope1"]), f32(tw["slope2"])]
-        # the same tower in one kernel: the layer input's columns up to the fourth candidate-side segment, which is where that
-        # kernel has the attention output, and zero rows for the fifth
-        W1 = np.zeros((self.dtin + D["d"], tw["W1"].shape[1]), np.float32)
-        W1[:self.dtin] = tw["W1"]
-        self.dtower = ops.DinTower(D["d"], D["user_groups"] * D["emb"], t(W1), t(tw["b1"]), [t(tw["slope1"])], t(tw["W2"]),
-                                   t(tw["b2"]), [t(tw["slope2"])], t(tw["W3"]), t(tw["b3"]), device=device, act=capi.XB_ACT_PRELU)
+        # the same tower in one kernel, where that takes its shape: the layer input's columns up to the fourth candidate-side
+        # segment, which is where that kernel has the attention output, and zero rows for the fifth
+        self.dtower = None
+        if lib().xb_din_tower_packed_bytes(D["d"], *tw["W2"].shape, tw["W3"].shape[1]) > 0:
+            W1 = np.zeros((self.dtin + D["d"], tw["W1"].shape[1]), np.float32)
+            W1[:self.dtin] = tw["W1"]
+            self.dtower = ops.DinTower(D["d"], D["user_groups"] * D["emb"], t(W1), t(tw["b1"]), [t(tw["slope1"])], t(tw["W2"]),
+                                       t(tw["b2"]), [t(tw["slope2"])], t(tw["W3"]), t(tw["b3"]), device=device,
+                                       act=capi.XB_ACT_PRELU)
 
     def forward_dien(self, p):
         """Inputs already uploaded by DinModel.upload(). Returns probabilities [R*n_cand, 2] fp32."""
@@ -76,7 +80,7 @@ class DienModel(DinModel):
         a = self.augru
         check(L.xb_augru_shared(ops.ptr(hseq), ops.ptr(score16), ops.ptr(final), R, n_cand, T, H, ops.ptr(a["Wg"]),
                                 ops.ptr(a["bg"]), ops.ptr(a["Wc"]), ops.ptr(a["bc"]), self.augru_engine, s))
-        if self.engine == capi.XB_GEMM_AUTO:
+        if self.engine == capi.XB_GEMM_AUTO and self.dtower is not None:
             ws = self.dtower.workspace(R, dev)
             prob = self.dtower(p["user_emb"], q, k.view(R * T, H), final, R, n_cand, T, ws=ws)
             p["dien_keep"] = (hseq, raw, sm, score16, final, ws)                      # alive until the stream drains
