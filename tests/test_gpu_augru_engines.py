@@ -76,3 +76,23 @@ def test_few_tiles_by_the_engine_that_the_library_picks(H, T, R, n_cand):
     f = lambda t: t.float().cpu().numpy()
     want = orc.augru(f(x)[np.array(few) // n_cand], f(att)[few], *[f(t) for t in w])[:, T - 1, :]
     np.testing.assert_allclose(f(y)[few], want, rtol=0, atol=8e-3)
+
+
+@pytest.mark.parametrize("H", [4, 18, 36, 60])
+@pytest.mark.parametrize("R,n_cand", [(1, 40), (3, 300)])
+def test_both_engines_round_in_the_same_places(H, R, n_cand):
+    """One input column and one state column a gate, that with weight 1: every sum has one product of each, and what is left of it
+    after its roundings to fp16 is exact in fp32 (states are multiples of 2^-24, sums below 1 where a state is small)."""
+    pkg.load()
+    from x_deeplearning_b200 import capi
+    x, att, w, run = _augru(R, n_cand, 30, H, H + R)
+    rng = np.random.default_rng(H)
+    values = lambda *s: torch.from_numpy(rng.uniform(0.5, 0.7, s) * rng.choice([-1, 1], s)).to("cuda", torch.float16)
+    x.zero_()
+    x[:, :, 1] = values(R, 30)
+    for W in w:
+        W.zero_()
+    w[0][1], w[2][1] = values(2 * H), values(H)
+    eye = torch.eye(H, device="cuda", dtype=torch.float16)
+    w[0][H:, :H], w[0][H:, H:], w[2][H:] = eye, eye, eye
+    assert torch.equal(run(R, capi.XB_GEMM_AUTO), run(R, capi.XB_GEMM_TCGEN05))
