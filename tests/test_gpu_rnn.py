@@ -100,3 +100,26 @@ def test_gru_of_fp16_sequences_computes_as_that_of_fp32_ones(B, T, H):
         capi.check(L.xb_gru(ops.ptr(t[0]), ops.ptr(y), B, T, H, *[ops.ptr(v) for v in t[1:]], ops.dt(y), ops.stream()))
         got.append(y)
     assert torch.equal(got[0], got[1].half())
+
+
+def test_gru_adds_its_recurrent_sums_by_quarters_of_the_units():
+    """Units 0 and 16 have the same state and weights 2^30 and -2^30: in the quarter that both belong to they cancel before the term
+    of unit 4, which belongs to another, is added. Added between the two it would be lost."""
+    ops, capi, L = _ops()
+    B, H = 3, 20
+    g = torch.Generator().manual_seed(7)
+    r = lambda *s: torch.randn(s, generator=g)
+    x, Wi, Wh, bi = r(B, 2, H), r(H, 3 * H) / H ** 0.5, torch.zeros((H, 3 * H)), r(3 * H) * 0.1
+    for k in range(3):
+        Wi[:, k * H + 16], bi[k * H + 16] = Wi[:, k * H], bi[k * H]
+    Wh[0, 2 * H:], Wh[4, 2 * H:], Wh[16, 2 * H:] = 2.0 ** 30, 1.0, -2.0 ** 30
+    dx, dWi, dWh, dbi, dbh = x.cuda(), Wi.cuda(), Wh.cuda(), bi.cuda(), torch.zeros(3 * H).cuda()
+    y = torch.empty_like(dx)
+    capi.check(L.xb_gru(ops.ptr(dx), ops.ptr(y), B, 2, H, ops.ptr(dWi), ops.ptr(dWh), ops.ptr(dbi), ops.ptr(dbh), capi.XB_F32, ops.stream()))
+    h = torch.zeros((B, H), dtype=torch.float64)
+    for t in range(2):
+        pre, rec = x[:, t].double() @ Wi.double() + bi.double(), h[:, 4:5]
+        reset, z = pre[:, :H].sigmoid(), pre[:, H:2 * H].sigmoid()
+        c = (pre[:, 2 * H:] + reset * rec).tanh()
+        h = c + z * (h - c)
+        assert (y[:, t].double().cpu() - h).abs().max() <= 2e-5

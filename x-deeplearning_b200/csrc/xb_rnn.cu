@@ -34,12 +34,13 @@ namespace {
 //
 // What bounds it is the chain h(t) -> h(t+1), in which every instruction waits for the one before; everything else is kept off
 // it. The input products of up to GRU_CHUNK steps are made first (they do not depend on h). Then a thread owns one of the 3H
-// gate columns, its recurrent weights in registers, and a step is: read h as broadcast 16-byte vectors, four chains of FMAs,
+// gate columns, its recurrent weights in registers, and a step is: read h as broadcast 16-byte vectors, eight chains of FMAs,
 // the reset and update threads evaluate their gates and leave them in shared memory, the candidate threads the candidate and the
 // new h. Two barriers a step, but no shuffles, and each scheduler has one warp (H = 36).
 // The data type is that of the arrays: state, sums and gates (expf, tanhf, a division) are fp32 for either.
-// 16 sequences of 100 steps, H = 36: 41 us fp16, 38 fp32; 61 and 57 with four lanes a unit, three shuffles and one barrier a step.
-// 1000 sequences 205 and 193, 16 of H = 64 56 and 52. (The register bound lets the compiler have every h vector of a step on its
+// 16 sequences of 100 steps, H = 36: 42 us fp16, 38 fp32; 61 and 57 with four lanes a unit, three shuffles and one barrier a step.
+// The chains add up as those lanes did, so the results are the same (four chains, one a component of the vectors: 41.5 and 38).
+// 1000 sequences 210 and 194, 16 of H = 64 57 and 53. (The register bound lets the compiler have every h vector of a step on its
 // way at once: at 128 registers, which it picks otherwise, 56 us.)
 constexpr int GRU_CHUNK = 64;
 __host__ __device__ constexpr int gru_hp(int nv) { return 16 * nv; }          // h and x rows padded with zeros
@@ -123,13 +124,14 @@ __global__ void __launch_bounds__((48 * NV + 31) / 32 * 32, 1) gru_kernel(const 
     for (; t < n; ++t, yt += H) {
       const float pre_j = pre_next;
       if (col && t + 1 < n) pre_next = pre[(t + 1) * G + tid];
-      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      float a[4][2] = {};                          // quarter l of the units: 4 l .. 4 l + 3 of every 16
 #pragma unroll
       for (int k = 0; k < HP; k += 4) {
         const float4 v = *reinterpret_cast<const float4*>(hbuf + k);
-        a[0] = fmaf(v.x, wh[k], a[0]); a[1] = fmaf(v.y, wh[k + 1], a[1]); a[2] = fmaf(v.z, wh[k + 2], a[2]); a[3] = fmaf(v.w, wh[k + 3], a[3]);
+        float (&q)[2] = a[k / 4 % 4];
+        q[0] = fmaf(v.x, wh[k], q[0]); q[1] = fmaf(v.y, wh[k + 1], q[1]); q[0] = fmaf(v.z, wh[k + 2], q[0]); q[1] = fmaf(v.w, wh[k + 3], q[1]);
       }
-      const float sum = (a[0] + a[1]) + (a[2] + a[3]) + bhj;
+      const float sum = (((a[0][0] + a[0][1]) + (a[1][0] + a[1][1])) + ((a[2][0] + a[2][1]) + (a[3][0] + a[3][1]))) + bhj;
       if (tid < 2 * H) gates[tid] = sigm(pre_j + sum);
       __syncthreads();                             // the gates are there, and everyone has read h
       if (col && u >= 0) {
