@@ -96,3 +96,13 @@ def test_both_engines_round_in_the_same_places(H, R, n_cand):
     eye = torch.eye(H, device="cuda", dtype=torch.float16)
     w[0][H:, :H], w[0][H:, H:], w[2][H:] = eye, eye, eye
     assert torch.equal(run(R, capi.XB_GEMM_AUTO), run(R, capi.XB_GEMM_TCGEN05))
+
+
+@pytest.mark.parametrize("H", [4, 10, 12, 18, 20, 26, 28, 34, 36, 42, 44, 50, 52, 58, 60])
+@pytest.mark.parametrize("R,n_cand,T", [(1, 40, 100), (5, 1000, 100), (2, 65, 131)])
+def test_both_engines_give_the_same_states(H, R, n_cand, T):
+    """The same chunks in k, the terms of x_t among them, and the same roundings: equal bits, whichever the call's size picks."""
+    pkg.load()
+    from x_deeplearning_b200 import capi
+    run = _augru(R, n_cand, T, H, H + R)[3]
+    assert torch.equal(run(R, capi.XB_GEMM_AUTO), run(R, capi.XB_GEMM_TCGEN05))

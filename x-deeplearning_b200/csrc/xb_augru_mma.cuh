@@ -5,14 +5,15 @@
 // accumulators lie in registers as their A operand wants them, so h and r*h go from one product into the next without leaving
 // the thread, and no thread waits for another one anywhere in the walk. The tcgen05 engine pays two tensor-memory round trips
 // with their barriers a step, but its products cost the SM almost nothing, while these take the schedulers' slow path to the
-// tensor cores: with one warp a scheduler a step is its chain (1200 cycles, 2250 there), with two the products bound it (1850).
+// tensor cores: with one warp a scheduler a step is its chain (1180 cycles, 2110 there), with two the products bound it (1680).
 // So this engine takes the calls that give every SM one CTA at the most: tcgen05 tiles share an SM in pairs beyond that.
-// H = 36, 100 steps, us (tcgen05 engine): 200 candidates 66 (114), 4 x 1000 67 (115), 16 x 1000 96 (115); more CTAs than SMs,
-// 19 x 1000: 185 (178), 74 x 1000: 375 (342).
+// H = 36, 100 steps, us (tcgen05 engine): 200 candidates 65 (113), 4 x 1000 65 (114), 16 x 1000 90 (114); more CTAs than SMs,
+// 19 x 1000: 178 (178), 74 x 1000: 356 (341).
 //
-// The terms of x_t are made once per CTA and chunk of steps in fp32 and are what the accumulators of a step start from. They are
-// rounded to fp16 first, as the tcgen05 engine holds them: a state then does not depend on which of the two the call's size
-// picks but for the order of sums (2-norm of the difference 5e-5, 3.7e-4 unrounded; 100 steps, H = 36). The recurrent weights stay in registers (H <= 36) or are read from shared memory as fragments. The state h stays
+// The terms of x_t are made once per CTA and chunk of steps and enter the products as they do in the tcgen05 engine: summed in
+// fp32 in its order, rounded to fp16, and multiplied by a one in the first spare row of the last k chunk. With the same chunks of 16
+// in k a state then has the same bits whichever engine the call's size picks. (As the fp32 start of the accumulators: 67 us instead
+// of 65, 4 x 1000.) The recurrent weights stay in registers (H <= 36) or are read from shared memory as fragments. The state h stays
 // in fp32; it is rounded to fp16 only as an MMA operand.
 //
 // Columns of the gate product in tiles of 8: the whole tiles of r, those of u, then one tile with what is left of both, so that
@@ -31,7 +32,7 @@ struct AmGeom {
   static constexpr int KT = HT + 1;                             // chunks of 8 in k
   static constexpr int NG = 2 * HT + 1, NC = HT + 1, NT = NG + NC;
   static constexpr int NPX = NT * 8;                            // request-side terms of a step, in tile order
-  static constexpr int XP = (KT & 1) ? KT * 8 : KT * 8 + 8;     // pitch of an x row: fragment loads on different banks
+  static constexpr int XP = KT * 8;                             // pitch of an x row
   static constexpr bool WREG = H <= 36;                         // recurrent weights in registers
   static_assert(W == 2 || W == 4, "two or four columns left over");
 };
@@ -44,7 +45,7 @@ __host__ __device__ inline AmSmem am_smem(int T, int warps) {
   s.ap = s.n16 + 2;                                             // an odd number of words: the rows of a warp on different banks
   int off = 0;
   s.wb = off; off += G::NT * G::KT * 128;                       // fragments of the recurrent weights: [tile][k chunk][lane]
-  s.px = off; off += (s.n16 + 1) * G::NPX * 4;                  // (one row more: the last step requests a next one)
+  s.px = off; off += (s.n16 + 1) * G::NPX * 2;                  // (one row more: the last step requests a next one)
   s.xs = off; off += s.n16 * G::XP * 2;
   s.att = off; off += warps * 16 * s.ap * 2;
   s.total = (off + 15) / 16 * 16;
@@ -79,14 +80,14 @@ __device__ __forceinline__ int am_column(int j, int n) {
   const int c = (j - G::NG) * 8 + n;
   return c < H ? c : -1;
 }
-// rows k0 and k0 + 1 of the x part (`row0` 0) or h part (`row0` H) of a weight column, as one fragment word
+// rows k0 and k0 + 1 of the h part of a weight column, as one fragment word
 template <int H>
-__device__ __forceinline__ uint32_t am_weights(const AuParams& p, int j, int col, int row0, int k0) {
+__device__ __forceinline__ uint32_t am_weights(const AuParams& p, int j, int col, int k0) {
   const bool gate = j < AmGeom<H>::NG;
   const __half* W = gate ? p.Wg : p.Wc;
   const int ld = gate ? 2 * H : H;
   const __half zero = __float2half(0.f);
-  const __half lo = col >= 0 && k0 < H ? W[(row0 + k0) * ld + col] : zero, hi = col >= 0 && k0 + 1 < H ? W[(row0 + k0 + 1) * ld + col] : zero;
+  const __half lo = col >= 0 && k0 < H ? W[(H + k0) * ld + col] : zero, hi = col >= 0 && k0 + 1 < H ? W[(H + k0 + 1) * ld + col] : zero;
   return h2_bits(__halves2half2(lo, hi));
 }
 
@@ -100,17 +101,19 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
   const int g = lane >> 2, q = lane & 3;                        // row of the warp's 16 (and g + 8), column pair of a tile
   const AmSmem S = am_smem<H>(p.T, warps);
   uint32_t* wb = reinterpret_cast<uint32_t*>(smem + S.wb);
-  float* px = reinterpret_cast<float*>(smem + S.px);
+  __half* px = reinterpret_cast<__half*>(smem + S.px);
   __half* xs = reinterpret_cast<__half*>(smem + S.xs);
   __half* atts = reinterpret_cast<__half*>(smem + S.att);
   const int r = blockIdx.x / p.tiles_per_req, first = (blockIdx.x - r * p.tiles_per_req) * warps * 16;
   const int rows = min(warps * 16, p.n_cand - first), T = p.T;
   const __half zero = __float2half(0.f);
+  const bool slot = q == G::W / 2;                              // this lane has the first spare row of the last k chunk: a one in A
+  const uint32_t one = slot ? 0x3C00u : 0u;
 
 #pragma unroll 4
   for (int i = tid; i < NT * KT * 32; i += blockDim.x) {
     const int l = i & 31, k = (i >> 5) % KT, j = (i >> 5) / KT;
-    wb[i] = am_weights<H>(p, j, am_column<H>(j, l >> 2), H, 8 * k + 2 * (l & 3));
+    wb[i] = am_weights<H>(p, j, am_column<H>(j, l >> 2), 8 * k + 2 * (l & 3));
   }
 
   float h[NC][4];
@@ -119,7 +122,7 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
   for (int j = 0; j < NC; ++j) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) h[j][e] = 0.f;
-    hp[j][0] = hp[j][1] = 0u;
+    hp[j][0] = hp[j][1] = j == HT ? one : 0u;
   }
   uint32_t wr[G::WREG ? NT : 1][KT];
   const __half* xr = p.x + (int64_t)r * T * H;
@@ -157,25 +160,29 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
       }
     }
     __syncthreads();
-    // ---- request-side terms x_t Wx + b of every tile's columns: a warp takes every warps-th tile, 16 steps a product
-    for (int j = warp; j < NT; j += warps) {
-      uint32_t wx[KT];
+    // ---- request-side terms x_t Wx + b: a column a thread, its weights in registers, four steps at a time
+    for (int i = tid & 127; i < NPX; i += 128) {
+      const int j = i >> 3, c = am_column<H>(j, i & 7);
+      const bool gate = j < NG;
+      const __half* W = gate ? p.Wg : p.Wc;
+      const int ld = gate ? 2 * H : H;
+      float w[H];
 #pragma unroll
-      for (int k = 0; k < KT; ++k) wx[k] = am_weights<H>(p, j, am_column<H>(j, g), 0, 8 * k + 2 * q);
-      const int c0 = am_column<H>(j, 2 * q), c1 = am_column<H>(j, 2 * q + 1);
-      const __half* bias = j < NG ? p.bg : p.bc;
-      const float b0 = c0 >= 0 ? __half2float(bias[c0]) : 0.f, b1 = c1 >= 0 ? __half2float(bias[c1]) : 0.f;
-      for (int t = 0; t < n16; t += 16) {
-        uint32_t xa[KT][2];
+      for (int k = 0; k < H; ++k) w[k] = c >= 0 ? __half2float(W[k * ld + c]) : 0.f;
+      const float bias = c >= 0 ? __half2float((gate ? p.bg : p.bc)[c]) : 0.f;
+      const int share = tid >> 7, shares = blockDim.x >> 7;
+      for (int t = 4 * share; t < n; t += 4 * shares) {
+        float v[4] = {bias, bias, bias, bias};
 #pragma unroll
-        for (int k = 0; k < KT; ++k) {
-          xa[k][0] = *reinterpret_cast<const uint32_t*>(xs + (t + g) * G::XP + 8 * k + 2 * q);
-          xa[k][1] = *reinterpret_cast<const uint32_t*>(xs + (t + g + 8) * G::XP + 8 * k + 2 * q);
+        for (int k = 0; k < H; k += 2) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {                         // (rows up to a multiple of 16 are there, zero past the last step)
+            const float2 xv = __half22float2(*reinterpret_cast<const __half2*>(xs + (t + e) * G::XP + k));
+            v[e] = fmaf(xv.y, w[k + 1], fmaf(xv.x, w[k], v[e]));
+          }
         }
-        float acc[4] = {b0, b1, b0, b1};
-        am_product<KT>(acc, xa, [&](int k) { return wx[k]; });
-        *reinterpret_cast<float2*>(px + (t + g) * NPX + j * 8 + 2 * q) = __half22float2(__floats2half2_rn(acc[0], acc[1]));
-        *reinterpret_cast<float2*>(px + (t + g + 8) * NPX + j * 8 + 2 * q) = __half22float2(__floats2half2_rn(acc[2], acc[3]));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) px[(t + e) * NPX + i] = __float2half_rn(v[e]);
       }
     }
     if constexpr (G::WREG) {
@@ -189,14 +196,15 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
     __syncthreads();
 
     // ---- the steps
-    const float* pxl = px + 2 * q;
+    const uint16_t* pxl = reinterpret_cast<const uint16_t*>(px) + g;
     const __half* al = atts + (warp * 16 + g) * S.ap;
     float acc[NT][4];
+    uint32_t last[NT];                                          // fragments of the last k chunk: weights, in the slot's lanes the step's term
     auto start = [&](int j, int t) {
-      const float2 v = *reinterpret_cast<const float2*>(pxl + t * NPX + j * 8);
-      acc[j][0] = v.x; acc[j][1] = v.y; acc[j][2] = v.x; acc[j][3] = v.y;
+      if (slot) last[j] = pxl[t * NPX + j * 8];
     };
     auto weight = [&](int j, int k) {
+      if (k == KT - 1) return last[j];
       if constexpr (G::WREG) return wr[j][k];
       else return wb[(j * KT + k) * 32 + lane];
     };
@@ -207,12 +215,19 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
       return h2_bits(__hfma2(th, __floats2half2_rn(0.5f, 0.5f), __floats2half2_rn(0.5f, 0.5f)));
     };
 #pragma unroll
-    for (int j = 0; j < NT; ++j) start(j, 0);
+    for (int j = 0; j < NT; ++j) {
+      last[j] = wb[(j * KT + KT - 1) * 32 + lane];
+      start(j, 0);
+    }
 #pragma unroll 1
     for (int t = 0; t < n; ++t) {
       const float om[2] = {1.f - __half2float(al[t]), 1.f - __half2float(al[8 * S.ap + t])};
       // gates: r's tiles first, r*h is what the candidate product waits for
-      auto gate = [&](int j) { am_product<KT>(acc[j], hp, [&](int k) { return weight(j, k); }); };
+      auto product = [&](int j, const uint32_t (&a)[KT][2]) {
+        acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+        am_product<KT>(acc[j], a, [&](int k) { return weight(j, k); });
+      };
+      auto gate = [&](int j) { product(j, hp); };
 #pragma unroll
       for (int j = 0; j < HT; ++j) gate(j);
       gate(2 * HT);
@@ -227,6 +242,7 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
           const uint32_t s = sigm2(acc[tile][2 * e], acc[tile][2 * e + 1]);
           const float2 rf = __half22float2(bits_h2(s));
           rh[j][e] = h2_bits(__floats2half2_rn(rf.x * h[j][2 * e], rf.y * h[j][2 * e + 1]));   // (h is zero past column H)
+          if (j == HT && slot) rh[j][e] = one;
           if (j == HT) {
             const uint32_t moved = __shfl_down_sync(0xffffffffu, s, G::W / 2);
             u[HT][e] = q < G::W / 2 ? moved : 0u;               // (padding columns take nothing from another candidate)
@@ -235,7 +251,7 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
         start(tile, t + 1);
       }
 #pragma unroll
-      for (int j = 0; j < NC; ++j) am_product<KT>(acc[NG + j], rh, [&](int k) { return weight(NG + j, k); });
+      for (int j = 0; j < NC; ++j) product(NG + j, rh);
 #pragma unroll
       for (int j = 0; j < HT; ++j) {
 #pragma unroll
@@ -254,6 +270,7 @@ __global__ void __launch_bounds__(256, 1) augru_mma_kernel(const __grid_constant
           h[j][2 * e] = u0 * h[j][2 * e] + (1.f - u0) * c.x;
           h[j][2 * e + 1] = u1 * h[j][2 * e + 1] + (1.f - u1) * c.y;
           hp[j][e] = h2_bits(__floats2half2_rn(h[j][2 * e], h[j][2 * e + 1]));
+          if (j == HT && slot) hp[j][e] = one;
         }
         start(NG + j, t + 1);
       }
