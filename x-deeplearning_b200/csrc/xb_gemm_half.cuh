@@ -1,14 +1,15 @@
 // 16-bit products that the tcgen05 engine does not take: rows that TMA cannot address (odd leading dimensions, operands that
-// start anywhere) and transposed A. Included by xb_gemm_simt.cu.
+// start anywhere), transposed A and less than 128 x 64 outputs. Included by xb_gemm_simt.cu.
 //
 // Warp-level matrix instructions on operands that the threads fetch themselves: a warp reads 64 adjacent elements of a row, a lane
 // two of them, with one 4-byte load where the rows allow it and two 2-byte loads otherwise, the next slice of 64 k in registers
 // while this one is multiplied. fp32 accumulation; the outputs leave through shared memory, whole rows of 64.
 //
 // Bound by the issue of these narrow loads where the product is large, by the latency of the slices where it is small (up to K / 64
-// trips to memory one after the other). fp16, on the CUDA cores before and here: [30000, 500] x [500, 511] 1313 -> 145 us (rows of
-// A at 4-byte addresses, N = 512: 1313 -> 110), [30000, 313] x [313, 31] 91 -> 15, 8 x ([2254, 117] x [117, 144]) 70 -> 19,
-// 2 x ([47350, 28] x [28, 27]) bf16 with a sigmoid 31 -> 19 (31 before narrow rows shared a warp), 2 x ([2585, 67] x [67, 45]) 24 -> 7.
+// trips to memory one after the other). fp16, on the CUDA cores before and here: [30000, 500] x [500, 511] 1125 -> 146 us (rows of
+// A at 4-byte addresses, N = 512: 1131 -> 120), [30000, 313] x [313, 31] 90 -> 16, 8 x ([2254, 117] x [117, 144]) 69 -> 19,
+// 2 x ([47350, 28] x [28, 27]) bf16 with a sigmoid 30 -> 22 (12 us more where narrow rows do not share a warp),
+// 2 x ([2585, 67] x [67, 45]) 23 -> 8, 16 x ([22, 320] x [320, 16]) 30 -> 8.
 #pragma once
 
 namespace xb {
@@ -96,6 +97,21 @@ struct HalfSlice {
     }
   }
 };
+
+// `finish` with one quotient for both activations that have one: with two, and their special cases, the loop over the outputs is so
+// long that products without an activation pay for it ([30000, 500] x [500, 511] 153 us, 146; 8 x ([2254, 117] x [117, 144]) 22, 19)
+__device__ __forceinline__ float half_finish(const SimtGemmParams& p, const Column& c, int b, int gm, int gn, float acc) {
+  float v = p.alpha * acc;
+  if (p.bias_kind == XB_BIAS_ROW)
+    v += p.beta * c.bias;
+  else if (p.bias_kind == XB_BIAS_FULL)
+    v += p.beta * load_as_f32(p.bias, (int64_t)b * p.stride_bias + (int64_t)(gm / p.bias_group) * p.ldbias + gn, p.bias_dtype);
+  if (p.epi.kind == XB_EPI_PRELU) return act_prelu(v, c.a);
+  if (p.epi.kind == XB_EPI_NONE) return v;
+  const bool dice = p.epi.kind == XB_EPI_DICE;
+  const float s = 1.f / (1.f + __expf(dice ? -(v - c.b) * c.c : -v));
+  return dice ? (1.f - s) * c.a * v + s * v : s;
+}
 
 // BM = 128: 4 x 2 warps of 32 x 32 outputs; BM = 64: 2 x 4 of 32 x 16.
 template <bool BF16, int BM, bool TA, bool TB>
@@ -219,7 +235,7 @@ __global__ void __launch_bounds__(256, 2) gemm_half_kernel(const __grid_constant
 #pragma unroll 4
   for (int r = nar ? threadIdx.x >> 4 : warp; r < BM && m0 + r < p.M; r += step) {
     const float2 x = *reinterpret_cast<const float2*>(out + r * HALF_OPITCH + cl);
-    const float v0 = finish(p, c0, b, m0 + r, gn, x.x), v1 = two ? finish(p, c1, b, m0 + r, gn + 1, x.y) : 0.f;
+    const float v0 = half_finish(p, c0, b, m0 + r, gn, x.x), v1 = two ? half_finish(p, c1, b, m0 + r, gn + 1, x.y) : 0.f;
     const int64_t at = (int64_t)b * p.stride_y + (int64_t)(m0 + r) * p.ldy + gn;
     if (p.y_pairs && two) {
       uint32_t w;

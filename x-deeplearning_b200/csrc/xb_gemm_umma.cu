@@ -267,8 +267,8 @@ __device__ __forceinline__ void with_kind(int kind, F f) {
 // Epilogue of a tile whose results leave by TMA, a warp's 32 rows x W columns at a time: units `part`, `part` + 4, ... of the tile.
 // A warp with two units a tile has two areas, so that it fills one while the other is read. What the threads' own stores and their
 // reads of the staging area took of the data path (4900 wavefronts a tile of 128 x 256, 5000 cycles) is the copy engine's work here.
-// [65536, 88] x [88, 256] fp16: 16.1 -> 11.8 us, N = 192 14.4 -> 10.5, 8 x ([4096, 256] x [256, 128]) side by side 8.3 -> 7.9,
-// 8 x ([33434, 88] x [88, 32]) with a sigmoid 24.2 -> 22.5.
+// [65536, 88] x [88, 256] fp16: 16.1 -> 11.8 us, N = 192 14.4 -> 10.5, 8 x ([4096, 256] x [256, 128]) side by side 8.3 -> 7.9.
+// A sigmoid's division is most of an epilogue that has one (8 x ([33434, 88] x [88, 32]) 32 us, 20 without an activation).
 // A turn is a copy: the wait counts committed groups, so a warp whose rows all lie past the output (`rows` false) takes no turn and
 // leaves the areas as they are. (With turns that commit nothing, the wait for all but the latest copy would name the copy of the other
 // area, and a later unit could overwrite what that copy still reads.)
@@ -360,7 +360,7 @@ __device__ __forceinline__ void epi_tile_edge(const UmmaGemmParams& p, uint32_t 
     if (sizeof(TOut) == 2 && !(vec && valid == 16)) {
       // Rows that start anywhere: a store of one element per lane and row touches 32 lines, so the warp turns its 32 x 16 results
       // and writes two rows at a time. [65536, 256] x [256, 255] fp16: 173 -> 29 us; [40594, 104] x [104, 41] 24 -> 8.3;
-      // 8 x ([4198, 48] x [48, 398]) with a sigmoid 178 -> 24.
+      // 8 x ([4198, 48] x [48, 398]) with a sigmoid 170 -> 36.
       const int piece = (lane >> 2) & 1;                              // (swapped in every other four rows: no bank conflicts)
       reinterpret_cast<uint4*>(stage)[lane * 2 + piece] = pack8<TOut>(v);
       reinterpret_cast<uint4*>(stage)[lane * 2 + (piece ^ 1)] = pack8<TOut>(v + 8);
@@ -962,8 +962,8 @@ static int validate_gemm(const xb_gemm_args* a) {
 // Whether XB_GEMM_AUTO runs these arguments on the tcgen05 engine.
 // Less than 128 x 64 outputs keep sums that are rounded, fp32 FMAs or gemm_half_kernel's, whose error against 64 bits is no larger;
 // an accumulator in tensor memory is cut off at every MMA instead (rms before the result's rounding, positive fp16 values 5.6e-7,
-// FMAs 1.3e-7). What that costs: 16 x ([22, 320] x [320, 16]) fp16 8.5 us, 4.3 in tensor memory (24.8 on the CUDA cores);
-// 2 x ([59, 24] x [24, 32]) 3.7, 3.1 (5.7).
+// FMAs 1.3e-7). What that costs: 16 x ([22, 320] x [320, 16]) fp16 8.0 us, 4.3 in tensor memory (30 on the CUDA cores);
+// 2 x ([59, 24] x [24, 32]) 3.6, 3.2 (5.5); K-major [1, 1280] x [1280, 512] 21, 7.9 (90).
 static bool auto_takes_umma(const xb_gemm_args& a) {
   return umma_eligible(a) && a.K > 0 && !gemm_narrow_takes(a) && (int64_t)a.M * a.N * a.batch >= 128 * 64;
 }
