@@ -3,7 +3,7 @@
 // Three kernels share one geometry: a table row is fetched by LPR lanes with 128-bit loads (lane c
 // reads bytes [16c,16c+16) of the row) and accumulated in fp32.
 //   pool_queue_kernel  sum / average, one output per feature group, large batches: one sub-team of LPR
-//                      lanes per segment, a warp's run of segments handed out as sub-teams finish.
+//                      lanes per segment, a warp's share of them handed out as sub-teams finish.
 //   pool_fast_kernel   one output per feature group (kAssign included), any batch: teams of TL lanes
 //                      per segment, TL/LPR sub-teams that walk the ids s, s+NS, s+2NS..., combined
 //                      with a fixed xor butterfly.
@@ -810,10 +810,10 @@ __global__ void __launch_bounds__(256) pool_short_kernel(const __grid_constant__
 }
 
 // Sum / average pooling with one sub-team (LPR lanes) per segment and a per-warp segment queue: a warp
-// owns a run of consecutive segments, its 32/LPR sub-teams each take the next unclaimed one as soon as they
-// finish theirs, so lanes stay busy whatever the spread of segment lengths. The run is as long as it takes for the
-// launch to be one wave of warps; the spans of 64 of its segments lie in the lanes' registers, a window of 32 behind the
-// claims and the one after it. A sub-team adds the ids of its
+// owns pieces of consecutive segments, its 32/LPR sub-teams each take the next unclaimed one as soon as they
+// finish theirs, so lanes stay busy whatever the spread of segment lengths. The pieces are as many as it takes for the
+// launch to be one wave of warps; the numbers and spans of 64 of its segments lie in the lanes' registers, a window of 32 behind
+// the claims and the one after it. A sub-team adds the ids of its
 // segment strictly in order (no cross-lane combine). The ids of the batch after the current one are
 // requested before the rows of the current one, so both latencies overlap.
 template <int TD, int LPR, int KIND>
@@ -839,13 +839,19 @@ __global__ void __launch_bounds__(256, POOL_QUEUE_BLOCKS) pool_queue_kernel(cons
   const char* wrow = g.weights + tlane * 16;
   const int pitch = (int)g.pitch;
   const uint64_t keep = l2_policy_keep();
-  const int64_t s0 = (warp_id - p.warp_begin[gi]) * g.segs;
-  const int nseg = (int)min((int64_t)g.segs, g.batch - s0);
+  const int64_t w0 = warp_id - p.warp_begin[gi], warps = (gi + 1 < p.n_groups ? p.warp_begin[gi + 1] : p.total_warps) - p.warp_begin[gi];
+  // number and span of the warp's i-th segment, -1 and no ids past its last one
+  auto load_span = [&](int i, int& seg, int& st, int& nm) {
+    const int64_t at = pool_queue_segment(i, w0, warps, g.segs);
+    const bool in = i < g.segs && at < g.batch;
+    seg = -1; nm = 0;
+    if (in) { seg = (int)at; pool_span<KIND>(g, at, st, nm); }
+  };
 
-  // lane l keeps the spans of segments s0 + win + l and, on their way while those are claimed, s0 + win + 32 + l
-  int win = 0, my_start = 0, my_num = 0, ahead_start = 0, ahead_num = 0;
-  if (lane < nseg) pool_span<KIND>(g, s0 + lane, my_start, my_num);
-  if (32 + lane < nseg) pool_span<KIND>(g, s0 + 32 + lane, ahead_start, ahead_num);
+  // lane l keeps the warp's segments win + l and, on their way while those are claimed, win + 32 + l
+  int win = 0, my_seg, my_start = 0, my_num, ahead_seg, ahead_start = 0, ahead_num;
+  load_span(lane, my_seg, my_start, my_num);
+  load_span(32 + lane, ahead_seg, ahead_start, ahead_num);
   auto load_ids = [&](int st, int nm, int pos, int& row, float& v) {
     const int idx = pos + tlane;
     row = -1; v = 1.f;
@@ -860,9 +866,8 @@ __global__ void __launch_bounds__(256, POOL_QUEUE_BLOCKS) pool_queue_kernel(cons
     }
   };
 
-  int m = team, next = NT;                           // my segment (relative), first unclaimed one
-  int start = __shfl_sync(FULL, my_start, m & 31), num = __shfl_sync(FULL, my_num, m & 31);
-  if (m >= nseg) num = 0;
+  int seg = __shfl_sync(FULL, my_seg, team), next = NT;          // my segment (-1: none is left), first unclaimed one of the warp's
+  int start = __shfl_sync(FULL, my_start, team), num = __shfl_sync(FULL, my_num, team);
   int pos = 0, row;
   float v;
   load_ids(start, num, 0, row, v);
@@ -870,33 +875,30 @@ __global__ void __launch_bounds__(256, POOL_QUEUE_BLOCKS) pool_queue_kernel(cons
 #pragma unroll
   for (int e = 0; e < EPC; ++e) acc[e] = 0.f;
 
-  while (__any_sync(FULL, m < nseg)) {
+  while (__any_sync(FULL, seg >= 0)) {
     // where this sub-team goes after the current batch: on in its segment, or to the next unclaimed one
-    const bool live = m < nseg;
-    const bool finishing = live && pos + LPR >= num;
+    const bool finishing = seg >= 0 && pos + LPR >= num;
     const unsigned fmask = __ballot_sync(FULL, finishing && tlane == 0);
-    int m2 = m, pos2 = pos + LPR, start2 = start, num2 = num;
+    int seg2 = seg, pos2 = pos + LPR, start2 = start, num2 = num;
     if (fmask) {
       const int cand = next + __popc(fmask & ((1u << team0) - 1u));          // below win + 32 + NT
-      int cs = __shfl_sync(FULL, my_start, cand & 31), cn = __shfl_sync(FULL, my_num, cand & 31);
+      int ci = __shfl_sync(FULL, my_seg, cand & 31), cs = __shfl_sync(FULL, my_start, cand & 31), cn = __shfl_sync(FULL, my_num, cand & 31);
       if (next + NT > win + 32) {                    // uniform: some claim may be in the second window
-        const int as = __shfl_sync(FULL, ahead_start, cand & 31), an = __shfl_sync(FULL, ahead_num, cand & 31);
-        if (cand >= win + 32) { cs = as; cn = an; }
+        const int ai = __shfl_sync(FULL, ahead_seg, cand & 31), as = __shfl_sync(FULL, ahead_start, cand & 31),
+                  an = __shfl_sync(FULL, ahead_num, cand & 31);
+        if (cand >= win + 32) { ci = ai; cs = as; cn = an; }
       }
-      if (finishing) {
-        m2 = cand; pos2 = 0; start2 = cs;
-        num2 = cand < nseg ? cn : 0;
-      }
+      if (finishing) { seg2 = ci; pos2 = 0; start2 = cs; num2 = cn; }
       next += __popc(fmask);
       if (next >= win + 32) {
         win += 32;
-        my_start = ahead_start; my_num = ahead_num;
-        if (win + 32 + lane < nseg) pool_span<KIND>(g, s0 + win + 32 + lane, ahead_start, ahead_num);
+        my_seg = ahead_seg; my_start = ahead_start; my_num = ahead_num;
+        load_span(win + 32 + lane, ahead_seg, ahead_start, ahead_num);
       }
     }
     int row2;
     float v2;
-    load_ids(start2, m2 < nseg ? num2 : 0, pos2, row2, v2);
+    load_ids(start2, num2, pos2, row2, v2);
 
     // rows of the current batch: id r of the batch sits in lane team0 + r
     int rr[LPR];
@@ -932,12 +934,12 @@ __global__ void __launch_bounds__(256, POOL_QUEUE_BLOCKS) pool_queue_kernel(cons
 #pragma unroll
           for (int e = 0; e < EPC; ++e) acc[e] = acc[e] * scale;
         }
-        store_vec<EPC>(it.out, pool_out_at<KIND>(g, it, s0 + m) + col0, out16, acc, nvalid);
+        store_vec<EPC>(it.out, pool_out_at<KIND>(g, it, seg) + col0, out16, acc, nvalid);
       }
 #pragma unroll
       for (int e = 0; e < EPC; ++e) acc[e] = 0.f;
     }
-    m = m2; pos = pos2; start = start2; num = num2; row = row2; v = v2;
+    seg = seg2; pos = pos2; start = start2; num = num2; row = row2; v = v2;
   }
 }
 
@@ -1190,24 +1192,27 @@ static int embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* s
     while ((2 << lg) < l.lpr) ++lg;                 // lanes per row 2, 4, 8, 16 -> 0..3
     l.bucket = (f32 ? 0 : 4) + lg;
     // sum / average groups with plenty of segments go to the segment-queue kernel
-    l.queue = l.fast && l.tl == l.lpr && h.items[0].udf != XB_UDF_ASSIGN && avg >= 3.0 && (call_segments + 31) / 32 >= (int64_t)sm_count() * 8;
+    l.queue = l.fast && l.tl == l.lpr && h.batch < ((int64_t)1 << 31) && h.items[0].udf != XB_UDF_ASSIGN && avg >= 3.0 && (call_segments + 31) / 32 >= (int64_t)sm_count() * 8;
     return l;
   };
-  // Segments a warp of the queue kernel owns: an equal share of its launch's for each warp that can be resident, so that the
-  // launch is one wave (the groups' last warps have less). Pieces of 32 segments a warp, as many waves as they take: 40 groups
-  // of 8192 lists of 15.5 ids (25 M x 32 fp16) 119 us, 111 in one wave; 20 such groups 79 and 57 (1.1 waves); the sharded step
-  // of one rank 121 and 100; 20 groups of 16 000 lists of 25 over an fp32 table in L2 169 and 135.
-  int64_t queue_total[kBuckets] = {}, queue_groups[kBuckets] = {};
+  // Segments a warp of the queue kernel owns: an equal share of its launch's time for each warp that can be resident, so that the
+  // launch is one wave (xb_pool_plan.h). us as pieces of 32 segments a warp, as many waves as they take; in one wave of equal numbers
+  // of neighbouring segments; as here (tables of 1 M rows, 32 fp16 columns): 20 groups of 8192 lists of 15.5 ids 72, 52, 54; 32 such
+  // groups 80, 78, 78, sorted by length 78, 87, 61; one group of 45 ids and 31 of 4 74, 133, 35; 8 groups of 65 536 lists with means
+  // from 3 to 45 over 16 columns 128, 216, 115; 2 groups of 131 072 lists of 15.5 79, 74, 75, sorted 56, 83, 57.
+  auto queue_cost = [](const xb_pool_group& h, const Lanes& l) { return pool_queue_cost((double)h.n_ids / (double)h.batch, l.lpr); };
+  PoolQueueGroup queue_groups[kBuckets][XB_MAX_POOL_GROUPS];
+  PoolQueueShare queue_share[kBuckets];
+  int queue_count[kBuckets] = {};
   for (int i = 0; i < n_groups; ++i) {
     const xb_pool_group& h = groups[i];
     if (h.batch <= 0 || h.n_items < 1 || h.dim < 1 || h.dim > 256) continue;
     const Lanes l = lanes_of(h);
-    if (l.queue) { queue_total[l.bucket] += h.batch; ++queue_groups[l.bucket]; }
+    if (l.queue) queue_groups[l.bucket][queue_count[l.bucket]++] = {h.batch, queue_cost(h, l)};
   }
-  auto queue_segs_of = [&](int bucket) {
-    const int64_t warps = std::max<int64_t>((int64_t)sm_count() * POOL_QUEUE_BLOCKS * 8 - queue_groups[bucket], 1);
-    return (int)std::max<int64_t>(8, (queue_total[bucket] + warps - 1) / warps);
-  };
+  for (int b = 0; b < kBuckets; ++b)
+    if (queue_count[b]) queue_share[b] = pool_queue_share(queue_groups[b], queue_count[b], 32 >> ((b & 3) + 1), (int64_t)sm_count() * POOL_QUEUE_BLOCKS * 8);
+  auto queue_segs_of = [&](const xb_pool_group& h, const Lanes& l) { return pool_queue_segs(queue_share[l.bucket], queue_cost(h, l), 32 / l.lpr); };
   for (int i = 0; i < n_groups; ++i) {
     const xb_pool_group& h = groups[i];
     XB_REQUIRE(h.batch >= 0 && h.n_ids >= 0, XB_ERR_ARG, "xb_embedding_pool: group %d negative size", i);
@@ -1291,7 +1296,7 @@ static int embedding_pool(const xb_pool_group* groups, int32_t n_groups, void* s
       d.offsets = off;
     }
     const PoolPath path = short_ok ? PoolPath::SHORT : queue_ok ? PoolPath::QUEUE : fast ? PoolPath::FAST : PoolPath::GENERAL;
-    const PoolSplit split = pool_split(path, h.batch, d.tl, avg, counts_ok, lanes.queue ? queue_segs_of(bucket) : 32, sm_count());
+    const PoolSplit split = pool_split(path, h.batch, d.tl, avg, counts_ok, lanes.queue ? queue_segs_of(h, lanes) : 32, sm_count());
     d.segs = split.segs;
     dst.total_warps += split.warps;
     dst.g[dst.n_groups++] = d;
