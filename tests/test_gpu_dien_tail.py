@@ -122,3 +122,14 @@ def test_prelu_tower_rounds_where_its_layers_do(R, n_cand, T, d, du, dims):
     # one activation in some thirty meets another fp16 neighbour (fp32 sums of a few hundred terms, 2^-21 apart, against steps of
     # 2^-10): 2^-10 / 30^0.5 of a value at the most, where every rounding moved would be 2^-11 / 3^0.5 = 2.8e-4
     assert float((got - want).double().norm() / want.double().norm()) < 8e-5
+
+
+@pytest.mark.parametrize("n,c", [(2000, 100), (9000, 37), (5000, 255), (2047, 64), (3000, 132)])
+def test_softmax_of_fp16_rows_computes_as_that_of_fp32_ones(n, c):
+    """A warp a row for either type where the eight lanes a row of many aligned fp32 rows are not faster: the same sums."""
+    ops, capi, L = _ops()
+    x = (torch.randn((n, c), generator=torch.Generator(device="cuda").manual_seed(c), device="cuda") * 3).half()
+    y16, y32 = torch.empty_like(x), torch.empty((n, c), device="cuda")
+    capi.check(L.xb_softmax(ops.ptr(x), ops.ptr(y16), n, c, 1, capi.XB_F16, ops.stream()))
+    capi.check(L.xb_softmax(ops.ptr(x.float()), ops.ptr(y32), n, c, 1, capi.XB_F32, ops.stream()))
+    assert torch.equal(y16, y32.half())

@@ -93,7 +93,7 @@ __global__ void softmax_kernel(const void* x, void* y, int64_t n, int c, int64_t
 // 256 columns stay in registers between the three passes. 16 000 rows of 100 fp32: 7.3 us, 34 before (one thread per row
 // touches 32 rows with every load).
 template <int PER>
-__global__ void __launch_bounds__(256) softmax_rows_kernel(const void* x, void* y, int64_t n, int c, int dt) {
+__global__ void __launch_bounds__(256) softmax_rows_kernel(const void* x, void* y, __half* y16, int64_t n, int c, int dt) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * 8;
@@ -120,17 +120,22 @@ __global__ void __launch_bounds__(256) softmax_rows_kernel(const void* x, void* 
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
       const int j = lane + 32 * i;
-      if (j < c) store_from_f32(y, base + j, dt, v[i] / s);
+      if (j >= c) continue;
+      v[i] /= s;
+      store_from_f32(y, base + j, dt, v[i]);
+      if (y16) y16[base + j] = __float2half_rn(v[i]);
     }
   }
 }
 
-// The same for fp32 rows, eight lanes a row and four columns a lane at a time: a quarter of the shuffles, loads of 16 bytes
-// where the rows allow them. y16, where given, receives the fp16 rounding of y, which saves the pass that would convert it.
-// 16 000 rows of 100 with the fp16 copy: 5.6 us after the kernel before, 9.5 as two launches.
+// The same for fp32 rows of whole, aligned 16-byte pieces, eight lanes a row and four columns a lane at a time: a quarter of the
+// shuffles. Many rows of up to 128 columns alone: with few rows the two are the same, with more columns or single loads a lane's
+// chain is longer than a warp's (33 523 rows of 137 24 us, 19 a warp a row). 16 000 rows of 100 4.5 us, 6.4 a warp a row; 74 000 11.1,
+// 24.6; 2048 2.4 either way.
 template <int PER4>
-__global__ void __launch_bounds__(256) softmax_f32_kernel(const float* x, float* y, __half* y16, int64_t n, int c, int vec) {
+__global__ void __launch_bounds__(256) softmax_f32_kernel(const float* x, float* y, __half* y16, int64_t n, int c) {
   pdl_begin();
+  const bool y16_vec = (reinterpret_cast<uintptr_t>(y16) & 7) == 0;
   const int l = threadIdx.x & 7, sub = threadIdx.x >> 3 & 3;
   const int64_t rows = (int64_t)gridDim.x * 32;
   for (int64_t at = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 5) * 4; at < n; at += rows) {       // the same for a warp: its shuffles stay whole
@@ -141,13 +146,8 @@ __global__ void __launch_bounds__(256) softmax_f32_kernel(const float* x, float*
 #pragma unroll
     for (int i = 0; i < PER4; ++i) {
       const int j = 4 * (l + 8 * i);
-      if (vec) {
-        const float4 q = in && j < c ? *reinterpret_cast<const float4*>(xr + j) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-        v[i][0] = q.x; v[i][1] = q.y; v[i][2] = q.z; v[i][3] = q.w;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[i][e] = in && j + e < c ? xr[j + e] : -INFINITY;
-      }
+      const float4 q = in && j < c ? *reinterpret_cast<const float4*>(xr + j) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      v[i][0] = q.x; v[i][1] = q.y; v[i][2] = q.z; v[i][3] = q.w;
     }
 #pragma unroll
     for (int i = 0; i < PER4; ++i)
@@ -169,34 +169,37 @@ __global__ void __launch_bounds__(256) softmax_f32_kernel(const float* x, float*
 #pragma unroll
     for (int i = 0; i < PER4; ++i) {
       const int j = 4 * (l + 8 * i);
+      if (j >= c) continue;
 #pragma unroll
       for (int e = 0; e < 4; ++e) v[i][e] /= s;
-      if (vec && j < c) {
-        *reinterpret_cast<float4*>(y + r * c + j) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
-        if (y16) {
-          const __half2 lo = __floats2half2_rn(v[i][0], v[i][1]), hi = __floats2half2_rn(v[i][2], v[i][3]);
-          *reinterpret_cast<uint2*>(y16 + r * c + j) =
-              make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-        }
+      *reinterpret_cast<float4*>(y + r * c + j) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+      if (!y16) continue;
+      const __half2 lo = __floats2half2_rn(v[i][0], v[i][1]), hi = __floats2half2_rn(v[i][2], v[i][3]);
+      if (y16_vec) {
+        *reinterpret_cast<uint2*>(y16 + r * c + j) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
       } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (j + e < c) {
-            y[r * c + j + e] = v[i][e];
-            if (y16) y16[r * c + j + e] = __float2half_rn(v[i][e]);
-          }
+        y16[r * c + j] = __low2half(lo); y16[r * c + j + 1] = __high2half(lo);
+        y16[r * c + j + 2] = __low2half(hi); y16[r * c + j + 3] = __high2half(hi);
       }
     }
   }
 }
-static int launch_softmax_f32(const float* x, float* y, __half* y16, int64_t n, int c, cudaStream_t s) {
-  const int vec = c % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
-                  (reinterpret_cast<uintptr_t>(y16) & 7) == 0;
-  const unsigned grid = stream_grid(n, 32);
-  if (c <= 64) launch_dependent(softmax_f32_kernel<2>, grid, 256, 0, s, x, y, y16, n, c, vec);
-  else if (c <= 128) launch_dependent(softmax_f32_kernel<4>, grid, 256, 0, s, x, y, y16, n, c, vec);
-  else launch_dependent(softmax_f32_kernel<8>, grid, 256, 0, s, x, y, y16, n, c, vec);
-  return check_launch("softmax_f32_kernel");
+
+// Rows of 16 to 256 columns. y16, where given, receives the fp16 rounding of an fp32 y, which saves the pass that would convert it
+// (16 000 rows of 100: 4.7 us, 9.5 as two launches).
+static int launch_softmax_rows(const void* x, void* y, __half* y16, int64_t n, int c, int dt, cudaStream_t s) {
+  if (dt == XB_F32 && c % 4 == 0 && c <= 128 && n >= 2048 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
+    const float* xf = static_cast<const float*>(x);
+    float* yf = static_cast<float*>(y);
+    if (c <= 64) launch_dependent(softmax_f32_kernel<2>, stream_grid(n, 32), 256, 0, s, xf, yf, y16, n, c);
+    else launch_dependent(softmax_f32_kernel<4>, stream_grid(n, 32), 256, 0, s, xf, yf, y16, n, c);
+    return check_launch("softmax_f32_kernel");
+  }
+  const unsigned grid = stream_grid(n, 8);
+  if (c <= 64) launch_dependent(softmax_rows_kernel<2>, grid, 256, 0, s, x, y, y16, n, c, dt);
+  else if (c <= 128) launch_dependent(softmax_rows_kernel<4>, grid, 256, 0, s, x, y, y16, n, c, dt);
+  else launch_dependent(softmax_rows_kernel<8>, grid, 256, 0, s, x, y, y16, n, c, dt);
+  return check_launch("softmax_rows_kernel");
 }
 
 struct EwParams {
@@ -602,14 +605,7 @@ extern "C" int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t 
   XB_REQUIRE(x && y && n >= 0 && c > 0 && w > 0, XB_ERR_ARG, "xb_softmax: bad arguments");
   XB_REQUIRE(float_dtype(dtype), XB_ERR_UNSUPPORTED, "xb_softmax: dtype %d", dtype);
   if (n == 0) return 0;
-  if (w == 1 && c >= 16 && c <= 256) {
-    if (dtype == XB_F32) return launch_softmax_f32((const float*)x, (float*)y, nullptr, n, c, (cudaStream_t)s);
-    const unsigned grid = stream_grid(n, 8);
-    if (c <= 64) launch_dependent(softmax_rows_kernel<2>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
-    else if (c <= 128) launch_dependent(softmax_rows_kernel<4>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
-    else launch_dependent(softmax_rows_kernel<8>, grid, 256, 0, (cudaStream_t)s, x, y, n, c, dtype);
-    return check_launch("softmax_rows_kernel");
-  }
+  if (w == 1 && c >= 16 && c <= 256) return launch_softmax_rows(x, y, nullptr, n, c, dtype, (cudaStream_t)s);
   launch_dependent(softmax_kernel, stream_grid(n * w, 128), 128, 0, (cudaStream_t)s, x, y, n, c, w, dtype);
   return check_launch("softmax_kernel");
 }
@@ -617,7 +613,7 @@ extern "C" int xb_softmax(const void* x, void* y, int64_t n, int32_t c, int64_t 
 extern "C" int xb_softmax_scores(const float* x, float* y, void* y16, int64_t n, int32_t c, xb_stream_t s) {
   XB_REQUIRE(x && y && y16 && n >= 0 && c > 0, XB_ERR_ARG, "xb_softmax_scores: bad arguments");
   if (n == 0) return 0;
-  if (c >= 16 && c <= 256) return launch_softmax_f32(x, y, (__half*)y16, n, c, (cudaStream_t)s);
+  if (c >= 16 && c <= 256) return launch_softmax_rows(x, y, (__half*)y16, n, c, XB_F32, (cudaStream_t)s);
   if (int rc = xb_softmax(x, y, n, c, 1, XB_F32, s)) return rc;
   return xb_copy2d(y, c, XB_F32, y16, c, XB_F16, n, c, s);
 }
