@@ -129,3 +129,17 @@ def test_sums_are_no_worse_than_fp32_fmas(M, N, K, batch, trans_b, dtype, positi
                      Y=torch.empty((batch, M, N), dtype=dtype, device="cuda"))
         rms.append((Y.double() / scale + (full.double() - exact)).pow(2).mean().sqrt().item())
     assert rms[0] <= rms[1], rms
+
+
+@pytest.mark.parametrize("M,N,K,batch", [(706, 43, 14, 1), (46002, 15, 16, 1), (42, 119, 7, 1), (38, 11, 8, 2), (5, 3, 1, 1)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_one_shallow_slice_is_the_cuda_cores(M, N, K, batch, dtype):
+    """The low bits of the sums, brought into a 16-bit result as above, are those of XB_GEMM_SIMT."""
+    ops, capi = _ops()
+    g = torch.Generator(device="cuda").manual_seed(K)
+    A, B = [torch.randn(s, generator=g, device="cuda").to(dtype) for s in ((batch, M, K), (batch, K, N))]
+    full = -(A.double() @ B.double()).float()
+    got = [ops.gemm(A, B, bias=full, bias_kind=capi.XB_BIAS_FULL, batch=batch, M=M, N=N, K=K, lda=K, ldb=N, ldy=N, ldbias=N, alpha=2.0 ** 20,
+                    beta=2.0 ** 20, strides=(M * K, K * N, M * N, M * N), engine=e, Y=torch.empty((batch, M, N), dtype=dtype, device="cuda"))
+           for e in (capi.XB_GEMM_AUTO, capi.XB_GEMM_SIMT)]
+    assert torch.equal(*got)
