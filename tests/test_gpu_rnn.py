@@ -123,3 +123,23 @@ def test_gru_adds_its_recurrent_sums_by_quarters_of_the_units():
         c = (pre[:, 2 * H:] + reset * rec).tanh()
         h = c + z * (h - c)
         assert (y[:, t].double().cpu() - h).abs().max() <= 2e-5
+
+
+@pytest.mark.parametrize("H", [22, 32, 36, 42, 43, 48, 64])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_gru_of_many_sequences(H, dtype):
+    """More sequences than are resident at a time, under another register bound: each has the bits that it has in a small call."""
+    ops, capi, L = _ops()
+    B, T = 5 * torch.cuda.get_device_properties(0).multi_processor_count + 3, 70
+    g = torch.Generator(device="cuda").manual_seed(H)
+    r = lambda sd, *s: (torch.randn(s, generator=g, device="cuda") * sd).to(dtype)
+    x, w = r(1, B, T, H), [r(H ** -0.5, H, 3 * H), r(H ** -0.5, H, 3 * H), r(0.1, 3 * H), r(0.1, 3 * H)]
+    x[::7, :T // 2] = 0
+
+    def run(x):
+        y = torch.empty_like(x)
+        capi.check(L.xb_gru(ops.ptr(x), ops.ptr(y), len(x), T, H, *[ops.ptr(v) for v in w], ops.dt(y), ops.stream()))
+        return y
+    many = run(x)
+    for i in range(0, B, 100):
+        assert torch.equal(run(x[i:i + 100]), many[i:i + 100])

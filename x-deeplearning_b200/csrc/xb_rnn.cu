@@ -40,13 +40,13 @@ namespace {
 // The data type is that of the arrays: state, sums and gates (expf, tanhf, a division) are fp32 for either.
 // 16 sequences of 100 steps, H = 36: 42 us fp16, 38 fp32; 61 and 57 with four lanes a unit, three shuffles and one barrier a step.
 // The chains add up as those lanes did, so the results are the same (four chains, one a component of the vectors: 41.5 and 38).
-// 1000 sequences 210 and 194, 16 of H = 64 57 and 53. (The register bound lets the compiler have every h vector of a step on its
-// way at once: at 128 registers, which it picks otherwise, 56 us.)
+// 16 of H = 64 57 and 53. (The register bound lets the compiler have every h vector of a step on its way at once: at 128
+// registers, which it picks otherwise, 56 us; calls of many sequences have other bounds, see launch_gru_nv.)
 constexpr int GRU_CHUNK = 64;
 __host__ __device__ constexpr int gru_hp(int nv) { return 16 * nv; }          // h and x rows padded with zeros
 
-template <typename T, int NV>
-__global__ void __launch_bounds__((48 * NV + 31) / 32 * 32, 1) gru_kernel(const T* x, T* y, int steps, int H,
+template <typename T, int NV, int BLOCKS>
+__global__ void __launch_bounds__((48 * NV + 31) / 32 * 32, BLOCKS) gru_kernel(const T* x, T* y, int steps, int H,
                                                                        const T* __restrict__ i2h, const T* __restrict__ h2h,
                                                                        const T* __restrict__ bi, const T* __restrict__ bh) {
   pdl_wait();
@@ -296,14 +296,26 @@ int launch_augru_shared(const AuParams& p, cudaStream_t s) {
   return check_launch("augru_shared_kernel");
 }
 
+template <typename T, int NV, int BLOCKS>
+int launch_gru_blocks(const T* x, T* y, int64_t batch, int steps, int H, const T* i2h, const T* h2h, const T* bi, const T* bh,
+                      cudaStream_t s) {
+  const size_t smem = sizeof(float) * GRU_CHUNK * (size_t)(gru_hp(NV) + 3 * H);
+  static PerDeviceOnce attr;                       // per instantiation
+  XB_SET_MAX_SMEM_ONCE(attr, sizeof(float) * GRU_CHUNK * 4 * gru_hp(NV), (const void*)gru_kernel<T, NV, BLOCKS>);
+  launch_dependent(gru_kernel<T, NV, BLOCKS>, (unsigned)batch, (3 * H + 31) / 32 * 32, smem, s, x, y, steps, H, i2h, h2h, bi, bh);
+  return check_launch("gru_kernel");
+}
 template <typename T, int NV>
 int launch_gru_nv(const T* x, T* y, int64_t batch, int steps, int H, const T* i2h, const T* h2h, const T* bi, const T* bh,
                   cudaStream_t s) {
-  const size_t smem = sizeof(float) * GRU_CHUNK * (size_t)(gru_hp(NV) + 3 * H);
-  static PerDeviceOnce attr;                       // per instantiation
-  XB_SET_MAX_SMEM_ONCE(attr, sizeof(float) * GRU_CHUNK * 4 * gru_hp(NV), (const void*)gru_kernel<T, NV>);
-  launch_dependent(gru_kernel<T, NV>, (unsigned)batch, (3 * H + 31) / 32 * 32, smem, s, x, y, steps, H, i2h, h2h, bi, bh);
-  return check_launch("gru_kernel");
+  // More sequences than are resident with all the registers that a step would like: a bound that lets more of them in. A quarter of
+  // the register file holds three warps of 146 registers (NV = 2), two of 174 and 206. us of 40 steps in fp32, all registers and
+  // bounded: 600 of H = 32 31, 23 (445: 20, 23); 300 of H = 36 37, 33 (200: 22, 26); 200 of H = 45 39, 28, 2000 269, 151;
+  // 200 of H = 64 45, 31.
+  constexpr int BLOCKS = NV == 2 ? 5 : NV == 3 ? 3 : NV == 4 ? 2 : 1;
+  const int fit = NV == 2 ? 4 : NV == 3 && 3 * H <= 128 ? 2 : 1;
+  if (BLOCKS > 1 && batch > (int64_t)fit * sm_count()) return launch_gru_blocks<T, NV, BLOCKS>(x, y, batch, steps, H, i2h, h2h, bi, bh, s);
+  return launch_gru_blocks<T, NV, 1>(x, y, batch, steps, H, i2h, h2h, bi, bh, s);
 }
 template <typename T>
 int launch_gru(const T* x, T* y, int64_t batch, int steps, int H, const T* i2h, const T* h2h, const T* bi, const T* bh,
