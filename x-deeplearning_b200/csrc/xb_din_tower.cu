@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
       if (h > 0) {
 #pragma unroll
         for (int j = 0; j < NL; ++j)
-          if (j < n3) lg[((h - 1) * 128 + row) * n3 + j] = logit[j];
+          if (j < n3) lg[((h - 1) * n3 + j) * 128 + row] = logit[j];          // (rows side by side: no bank conflicts)
       }
       workers_sync();
       if (h == 0 && ok) {                    // (the others write the next tile's sums after a2_full, where these warps arrive too)
@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) din_tower_tc_kernel(const __gri
           if (j < n3) {
             // layer-3 output rounded to the model's fp16, as the un-fused graph stores it
 #pragma unroll
-            for (int g = 0; g < TW_GROUPS - 1; ++g) logit[j] += lg[(g * 128 + row) * n3 + j];
+            for (int g = 0; g < TW_GROUPS - 1; ++g) logit[j] += lg[(g * n3 + j) * 128 + row];
             logit[j] += b3[j];
             if (ACT == XB_ACT_DICE) logit[j] = __half2float(__float2half_rn(logit[j]));
             mx = fmaxf(mx, logit[j]);
