@@ -131,7 +131,7 @@ def test_sums_are_no_worse_than_fp32_fmas(M, N, K, batch, trans_b, dtype, positi
     assert rms[0] <= rms[1], rms
 
 
-@pytest.mark.parametrize("M,N,K,batch", [(706, 43, 14, 1), (46002, 15, 16, 1), (42, 119, 7, 1), (38, 11, 8, 2), (5, 3, 1, 1)])
+@pytest.mark.parametrize("M,N,K,batch", [(706, 43, 14, 1), (46002, 15, 16, 1), (42, 119, 7, 1), (1087, 121, 3, 1), (38, 11, 8, 2), (5, 3, 1, 1)])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_one_shallow_slice_is_the_cuda_cores(M, N, K, batch, dtype):
     """The low bits of the sums, brought into a 16-bit result as above, are those of XB_GEMM_SIMT."""

@@ -577,9 +577,9 @@ int gemm_simt(const xb_gemm_args& a, cudaStream_t stream) {
   // 16-bit results of 16-bit operands: sums of 16 products by matrix instructions, which are no further from 64 bits than FMAs.
   // (Their bits differ from the FMAs', which an fp32 result would show.) One slice of up to 16 k is quicker on the CUDA cores unless
   // there are more columns than a tile and many outputs: K = 14, us there and here: [706, 14] x [14, 43] 4.5, 6.0,
-  // [46002, 14] x [14, 15] 9.6, 11.6, [42, 14] x [14, 119] 4.6, 5.8; 4 x ([3001, 14] x [14, 65]) 12.6, 9.1, [20000, 14] x [14, 255] 36, 25;
+  // [46002, 14] x [14, 15] 9.6, 11.6, [42, 14] x [14, 119] 4.6, 5.8, [1087, 3] x [3, 121] 4.8, 6.3; 4 x ([3001, 14] x [14, 65]) 12.6, 9.1, [20000, 14] x [14, 255] 36, 25;
   // K = 17: 5.4, 6.2; 12.9, 11.9; 5.6, 6.1; 16, 9.6; 46, 26.
-  const bool shallow = a.K <= 16 && (a.N <= 64 || (int64_t)a.M * a.N * a.batch < 65536);
+  const bool shallow = a.K <= 16 && (a.N <= 64 || (int64_t)a.M * a.N * a.batch < 1 << 18);
   if (any && a.ab_dtype != XB_F32 && a.y_dtype != XB_F32 && !shallow) return gemm_half(p, a, stream);
   p.tiles_n = (a.N + 16 * tn - 1) / (16 * tn);
   const int64_t tiles = (((int64_t)a.M + 16 * tm - 1) / (16 * tm)) * p.tiles_n;
