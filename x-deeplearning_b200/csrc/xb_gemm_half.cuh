@@ -26,7 +26,7 @@ __device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
 // c += a b as sums of 16 products, each added to c by an fp32 addition of its own: what the matrix instruction adds to an accumulator
 // is cut off, not rounded, and a long chain of such sums drifts. The products of [16..512]-deep sums against 64 bits, rms relative to
 // the result, before the result's rounding (fp32 FMAs; matrix instructions that accumulate): fp16 normal values 6.5e-8 (1.5e-7; 1.6e-7),
-// positive ones 5.7e-8 (9.0e-8; 2.9e-7); bf16 4.5e-8 (5.6e-8; 1.0e-7) and 3.5e-8 (4.3e-8; 1.0e-7). Largest error: less than half the FMAs'.
+// positive ones 5.7e-8 (9.0e-8; 2.9e-7); bf16 4.5e-8 (5.6e-8; 1.0e-7) and 3.5e-8 (4.3e-8; 1.0e-7). Largest error: 0.3 to 0.7 of the FMAs'.
 template <bool BF16>
 __device__ __forceinline__ void mma_half(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   float d[4] = {0.f, 0.f, 0.f, 0.f};
