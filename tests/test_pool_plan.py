@@ -89,8 +89,9 @@ def test_the_queue_kernels_shares_take_the_same_time(queue, groups, lanes, warps
     cost = [max(1.0, a / lanes + 0.5) for _, a in groups]
     assert sum(-(-b // s) for (b, _), s in zip(groups, segs)) <= warps
     fair = sum(b * c for (b, _), c in zip(groups, cost)) / warps
+    mean = sum(b * c for (b, _), c in zip(groups, cost)) / sum(b for b, _ in groups)
     for s, c in zip(segs, cost):
-        assert s >= max(8, spw) and (s * c <= 1.34 * fair + c or s == max(8, spw))
+        assert s >= spw and (s >= 8 or c > mean) and (s * c <= 1.34 * fair + c or s <= max(8, spw))
 
 
 @pytest.mark.parametrize("batch,segs", [(1, 8), (9, 8), (100, 17), (101, 33), (8192, 69), (5000, 16), (70001, 55), (300, 299), (37900, 8)])

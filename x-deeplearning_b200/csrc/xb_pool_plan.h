@@ -55,13 +55,14 @@ inline double pool_queue_cost(double avg, int lanes) { return std::max(1.0, avg 
 struct PoolQueueGroup { int64_t batch; double cost; };
 struct PoolQueueShare { double share, mean; };          // cost of a warp's share, mean cost of a list
 
-// Segments a warp owns in a group whose lists cost `cost`. Lists much longer than the launch's other ones go to whole rounds of
-// the `spw` sub-teams: with one list more than those a warp takes twice the time.
+// Segments a warp owns in a group whose lists cost `cost`, no less than 8 mean lists' worth. Lists much longer than the launch's
+// other ones go to whole rounds of the `spw` sub-teams: with one list more than those a warp takes twice the time.
 inline int pool_queue_segs(const PoolQueueShare& q, double cost, int spw) {
   int64_t segs = (int64_t)(q.share / cost);
   if (cost >= 2 * q.mean && segs < 4 * spw) segs = segs / spw * spw;
   else if ((double)segs * cost < q.share) ++segs;
-  return (int)std::max<int64_t>(std::max(8, spw), std::min<int64_t>(segs, 1 << 30));
+  const int least = std::max(spw, (int)std::min(8.0, 8 * q.mean / cost + 0.999));
+  return (int)std::max<int64_t>(least, std::min<int64_t>(segs, 1 << 30));
 }
 
 // The share with which the groups of a launch fit `warps` warps.
